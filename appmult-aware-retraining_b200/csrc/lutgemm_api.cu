@@ -50,7 +50,7 @@ std::atomic<unsigned long long> g_kernel_launches{0};
 
 struct BackwardPlan {
     bool gw_slab, ga_slab;
-    bool gw_tall, ga_tall;  // slab kernel with the 1024 x 32 tile instead of 512 x 64
+    bool gw_tall, ga_tall;  // fp32 slab with the 1024 x 32 tile instead of the packed slab with the 512 x 64 tile
     int gw_splits;        // row-broadcast grad_w kernel: slabs of M
     size_t gw_scratch, ga_scratch;
     // slab grad_w kernels read the activation codes from a transposed copy at[k][m] kept behind the partial
@@ -60,34 +60,61 @@ struct BackwardPlan {
     int gw_at_pitch;      // 0 = no transposed copy
 };
 
-// Kernel choice for the two gradients.  Slab kernels amortise one slab build over 512 rows of the
-// reduction dimension (M for grad_w, N for grad_a), so they need that dimension long and the tiles
-// reasonably full; everything else goes to the row/column-broadcast kernels.
-// lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
-BackwardPlan plan_backward(int bits, int M, int K, int N, int sms) {
-    BackwardPlan pl{};
-    // measured on B200 at 4096^3 (ms, grad_w / grad_a): tall fp32-slab 15.9 / 16.4 (8 bit), 14.1 / 14.4 (7 bit)
-    // against broadcast about 24 / 24 and 17 / 17: the slab kernels win where the broadcast gathers suffer
-    // bank conflicts (7 and 8 bits); at 4 and 6 bits a table row is conflict-free and the broadcast kernels
-    // (11.5 / 11.6) beat the slab kernels.  grad_a needs N >= 768 for a slab: on convolution shapes with
-    // N <= 512 the column-broadcast kernel is faster at both 7 and 8 bits.
-    pl.gw_slab = bits >= 7 && M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6;
-    // (a partly filled slab tile only pays against the column-broadcast kernel, which runs at about 37 % of the
-    // roofline at 7 bits and 29 % at 8 bits whatever N is, when the better of the two tilings is this full)
-    const double ga_fill = slab_fill(N, M) > tall_fill(N, M) ? slab_fill(N, M) : tall_fill(N, M);
-    pl.ga_slab = bits >= 7 && N >= 768 && M >= 32 && ga_fill >= (bits == 7 ? 0.85 : 0.7);
-    const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
-    if (force == LUTGEMM_BACKWARD_BCAST) pl.gw_slab = pl.ga_slab = false;
-    if (force == LUTGEMM_BACKWARD_SLAB) pl.gw_slab = pl.ga_slab = true;
-    // (the tall kernel is the faster one per look-up: at N = 1536, where its tiles are 75 % full and the wide ones
-    // full, grad_a of a 12608 x 384 problem takes 1.82 against 1.89 ms, at N = 2560 (83 %) 2.40 against 2.76 ms)
-    pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
-    pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
-    if (tile == LUTGEMM_TILE_WIDE) pl.gw_tall = pl.ga_tall = false;
-    if (tile == LUTGEMM_TILE_TALL) { pl.gw_tall = pl.gw_slab; pl.ga_tall = pl.ga_slab; }
+// ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
+// Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
+// The clocks are measured on B200, at 4096^3 unless said otherwise:
+//   slab kernels, per k and tile      packed 512 x 64: 1540 (4 and 6 bits), 1560 (7), 2180 (8); tall 1024 x 32: 1540, 1690, 1880;
+//                                     forward 512 x 64: 1000, 1100, 1330 and 40e3 / 55e3 at the start (code transposition)
+//   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
+//                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.7, 1.9, 2.8
+// A slab kernel's time does not depend on the codes and it can cut K into many work items; a broadcast kernel has no slab
+// to build, so it stays the better one for few rows.  Against the fixed limits on M, N and tile fill that came before
+// (base_plan below) the estimates move small and ragged problems to the slab kernels: 256 x 512 x 256 at 7 bits, forward 0.291 ms,
+// grad_w 0.088 ms and grad_a 0.092 ms with the broadcast kernels, both gradients 0.034 ms with the slab kernels.
+struct FamilyClocks {
+    double packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start;
+};
+FamilyClocks family_clocks(int bits) {
+    if (bits == 8) return {2180, 1880, 1330, 3.1, 3.3, 4.2, 2.8, 55e3};
+    if (bits == 7) return {1560, 1690, 1100, 2.33, 2.4, 2.6, 1.9, 40e3};
+    return {1540, 1540, 1000, 1.48, 1.6, 1.6, 1.7, 40e3};
+}
+constexpr double kBcastStart = 12e3, kSlabStart = 5e3;
+constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
+
+long div_up(long a, long b) { return (a + b - 1) / b; }
+
+double slab_grad_clocks(long rows, long cols, int K, int rt, int ct, int overhead, double per_step, double start, int sms) {
+    const long blocks = div_up(rows, rt);
+    const lutgemm::KSplit ks = lutgemm::choose_ksplit(blocks * div_up(cols, ct), K, sms, overhead);
+    const double reduce = blocks > 1 ? 8e3 + 8.0 * blocks * K * cols / kReduceBytesPerClock : 0;
+    return (double)ks.waves * (ks.per + overhead) * per_step + start + reduce;
+}
+double packed_clocks(int bits, long rows, long cols, int K, int sms) {
+    const FamilyClocks f = family_clocks(bits);
+    return slab_grad_clocks(rows, cols, K, 512, 64, lutgemm::kPackedItemOverhead, f.packed, kSlabStart, sms);
+}
+double tall_clocks(int bits, long rows, long cols, int K, int sms) {
+    const FamilyClocks f = family_clocks(bits);
+    return slab_grad_clocks(rows, cols, K, 1024, 32, lutgemm::kTallItemOverhead, f.tall, kSlabStart, sms);
+}
+double gw_bcast_clocks(int bits, int M, int K, int N, int sms) {
+    const long kt = N <= 128 ? 128 : 32, nt = N <= 128 ? 64 : 256, splits = lutgemm::gw_num_splits(bits, M, K, N, sms);
+    const long items = div_up(K, kt) * div_up(N, nt) * splits;
+    return (double)div_up(items, sms) * kt * nt * div_up(M, splits) * family_clocks(bits).gw_bcast / 32 + kBcastStart +
+           (splits > 1 ? 8e3 + 8.0 * splits * K * N / kReduceBytesPerClock : 0);
+}
+double ga_bcast_clocks(int bits, int M, int K, int N, int sms) {
+    const long mt = bits == 8 ? 512 : 256;
+    return (double)div_up(div_up(M, mt) * div_up(K, 32), sms) * mt * N * family_clocks(bits).ga_bcast + kBcastStart;
+}
+
+void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms) {
     pl.gw_splits = pl.gw_slab ? 1 : lutgemm::gw_num_splits(bits, M, K, N, sms);
+    pl.gw_at_offset = 0;
+    pl.gw_at_pitch = 0;
     if (pl.gw_slab) {
-        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::slab_f32_row_blocks(M);
+        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::slab_packed_row_blocks(M);
         pl.gw_scratch = rb > 1 ? (size_t)rb * K * N * sizeof(float) : 0;
         pl.gw_at_offset = (pl.gw_scratch + 15) & ~(size_t)15;
         pl.gw_at_pitch = (M + 15) & ~15;
@@ -95,10 +122,44 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms) {
     } else {
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
-    if (pl.ga_slab) {
-        const int rb = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::slab_f32_row_blocks(N);
-        pl.ga_scratch = rb > 1 ? (size_t)rb * K * M * sizeof(float) : 0;
-    }
+}
+void set_ga_scratch(BackwardPlan &pl, int M, int K, int N) {
+    const int rb = !pl.ga_slab ? 1 : pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::slab_packed_row_blocks(N);
+    pl.ga_scratch = rb > 1 ? (size_t)rb * K * M * sizeof(float) : 0;
+}
+
+// Choice by fixed limits: the plan for callers whose scratch buffer is too small for the faster one (a fixed buffer, or
+// one sized for this choice), so that what fitted such a buffer keeps running.
+BackwardPlan base_plan(int bits, int M, int K, int N, int sms) {
+    BackwardPlan pl{};
+    pl.gw_slab = bits >= 7 && M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6;
+    const double ga_fill = slab_fill(N, M) > tall_fill(N, M) ? slab_fill(N, M) : tall_fill(N, M);
+    pl.ga_slab = bits >= 7 && N >= 768 && M >= 32 && ga_fill >= (bits == 7 ? 0.85 : 0.7);
+    pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
+    pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
+    set_gw_scratch(pl, bits, M, K, N, sms);
+    set_ga_scratch(pl, M, K, N);
+    return pl;
+}
+
+// Choice by estimated time.  A convolution's grad_a (non-overlapping windows) gathers its column codes from the image and
+// writes in place; there the slab kernels pay from N = 768 on (1x1, 128 -> 512 channels, 7 bits: 0.75 against 0.68 ms; 1024 -> 512:
+// 1.24 against 1.22 ms).  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
+BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv) {
+    BackwardPlan pl{};
+    const double gw_p = packed_clocks(bits, M, N, K, sms), gw_t = tall_clocks(bits, M, N, K, sms);
+    const double ga_p = packed_clocks(bits, N, M, K, sms), ga_t = tall_clocks(bits, N, M, K, sms);
+    pl.gw_slab = (gw_p < gw_t ? gw_p : gw_t) < gw_bcast_clocks(bits, M, K, N, sms);
+    pl.ga_slab = (!conv || N >= 768) && (ga_p < ga_t ? ga_p : ga_t) < ga_bcast_clocks(bits, M, K, N, sms);
+    const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
+    if (force == LUTGEMM_BACKWARD_BCAST) pl.gw_slab = pl.ga_slab = false;
+    if (force == LUTGEMM_BACKWARD_SLAB) pl.gw_slab = pl.ga_slab = true;
+    pl.gw_tall = pl.gw_slab && gw_t < gw_p;
+    pl.ga_tall = pl.ga_slab && ga_t < ga_p;
+    if (tile == LUTGEMM_TILE_WIDE) pl.gw_tall = pl.ga_tall = false;
+    if (tile == LUTGEMM_TILE_TALL) { pl.gw_tall = pl.gw_slab; pl.ga_tall = pl.ga_slab; }
+    set_gw_scratch(pl, bits, M, K, N, sms);
+    set_ga_scratch(pl, M, K, N);
     return pl;
 }
 
@@ -107,6 +168,11 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms) {
 namespace lutgemm {
 
 void record_cuda_error(cudaError_t e) { g_last_cuda_error = e; }
+
+size_t base_gw_scratch_bytes(int bits, int M, int K, int N) {
+    const int sms = current_num_sms();
+    return sms > 0 ? base_plan(bits, M, K, N, sms).gw_scratch : 0;
+}
 
 int launch_status() {
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
@@ -171,14 +237,20 @@ int lutgemm_bits_from_elem_num(long elem_num) {
 }
 
 // ---- shared bodies of the GEMM and the implicit-im2col entry points ------------------------------------
-// Large-M problems with reasonably filled 512x64 tiles go to the slab kernel; small or skinny ones to the
-// row-broadcast kernel.  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
-static bool forward_uses_slab(int M, int N) {
-    bool slab = M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6;
+// The forward kernel by estimated time (see family_clocks); base_forward_uses_slab is the choice by fixed limits, for
+// callers whose workspace is too small for it.  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
+static bool base_forward_uses_slab(int M, int N) { return M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6; }
+
+static bool forward_uses_slab(int bits, int M, int K, int N, int sms) {
     const int force = g_force_forward.load(std::memory_order_relaxed);
-    if (force == LUTGEMM_FORWARD_ROWBCAST) slab = false;
-    if (force == LUTGEMM_FORWARD_SLAB) slab = true;
-    return slab;
+    if (force == LUTGEMM_FORWARD_ROWBCAST) return false;
+    if (force == LUTGEMM_FORWARD_SLAB) return true;
+    const FamilyClocks f = family_clocks(bits);
+    const long tiles = div_up(M, 512) * div_up(N, 64), chunks = div_up(K, 16);
+    const double slab = (double)div_up(tiles * chunks, sms) * 16 * f.fwd_slab + f.fwd_start;
+    const long mt = N <= 128 ? 128 : 64, nt = N <= 128 ? 64 : 256;
+    const double bcast = (double)div_up(div_up(M, mt) * div_up(N, nt), sms) * mt * nt * K * f.fwd_bcast / 32 + kBcastStart;
+    return base_forward_uses_slab(M, N) || slab < bcast;
 }
 
 static int codes_pitch(int M) { return (M + 15) & ~15; }
@@ -196,11 +268,15 @@ static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const u
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (forward_uses_slab(M, N)) {
+    const int pitch = codes_pitch(M);
+    bool slab = forward_uses_slab(bits, M, K, N, sms);
+    if (slab && scratch && scratch_bytes < (size_t)pitch * K) {
+        if (base_forward_uses_slab(M, N) || g_force_forward.load(std::memory_order_relaxed)) return LUTGEMM_E_SCRATCH;
+        slab = false;
+    }
+    if (slab) {
         const uint8_t *at = nullptr;
-        const int pitch = codes_pitch(M);
         if (scratch) {
-            if (scratch_bytes < (size_t)pitch * K) return LUTGEMM_E_SCRATCH;
             const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, s);
             if (trc != LUTGEMM_OK) return trc;
             at = static_cast<const uint8_t *>(scratch);
@@ -218,7 +294,8 @@ int lutgemm_forward(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint1
 
 size_t lutgemm_forward_scratch_bytes(int bits, int M, int K, int N) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
-    if (!forward_uses_slab(M, N)) return 0;
+    const int sms = current_num_sms();
+    if (sms <= 0 || !forward_uses_slab(bits, M, K, N, sms)) return 0;
     return (size_t)codes_pitch(M) * K;
 }
 
@@ -241,7 +318,7 @@ size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    const BackwardPlan pl = plan_backward(bits, M, K, N, sms);
+    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false);
     return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch;
 }
 
@@ -259,11 +336,13 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const BackwardPlan pl = plan_backward(bits, M, K, N, sms);
+    const size_t given = scratch ? scratch_bytes : 0;
+    BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0);
+    if ((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) pl = base_plan(bits, M, K, N, sms);
     float *sc = static_cast<float *>(scratch);
     if (gw) {
         // the weight gradient goes first: under data parallelism its all-reduce can then overlap gA
-        if (pl.gw_scratch && (!scratch || scratch_bytes < pl.gw_scratch)) return LUTGEMM_E_SCRATCH;
+        if (pl.gw_scratch > given) return LUTGEMM_E_SCRATCH;
         const uint8_t *at = codes_t;  // left by the forward pass (same layout), or made here
         if (pl.gw_slab && pl.gw_at_pitch && !at) {
             uint8_t *dst = static_cast<uint8_t *>(scratch) + pl.gw_at_offset;
@@ -273,14 +352,14 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
         }
         int rc = !pl.gw_slab ? lutgemm::backward_gw(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, pl.gw_splits, sms, s)
                  : pl.gw_tall ? lutgemm::backward_gw_slab_tall(gc, a, w, gw, lut_gw, nullptr, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s)
-                             : lutgemm::backward_gw_slab_f32(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s);
+                             : lutgemm::backward_gw_slab_packed(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s);
         if (rc != LUTGEMM_OK) return rc;
     }
     if (ga) {
-        if (pl.ga_scratch && (!scratch || scratch_bytes < pl.ga_scratch)) return LUTGEMM_E_SCRATCH;
+        if (pl.ga_scratch > given) return LUTGEMM_E_SCRATCH;
         int rc = !pl.ga_slab ? lutgemm::backward_ga(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sms, s)
                  : pl.ga_tall ? lutgemm::backward_ga_slab_tall(gc, a, w, ga, lut_ga, nullptr, bits, M, K, N, conv, sc, sms, s)
-                             : lutgemm::backward_ga_slab_f32(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sc, sms, s);
+                             : lutgemm::backward_ga_slab_packed(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sc, sms, s);
         if (rc != LUTGEMM_OK) return rc;
     }
     return LUTGEMM_OK;
@@ -413,38 +492,73 @@ static bool pixel_mode_supported(const lutgemm::ConvGeom &g) {
     return g.kh * g.kw <= lutgemm::kMaxTaps && g.kh * g.kw <= 256 && max_d <= 127 && g.pad <= 127;
 }
 
-// Per stride class: the slab kernel in pixel mode pays where its row dimension taps * Cout is long enough to
-// amortise the slab build; otherwise, and always at 4 and 6 bits where a table row is free of bank conflicts, the
-// column-broadcast gather kernel in pixel mode.  The slab kernel's time does not depend on the codes; the broadcast
-// kernel's bank conflicts do (weight codes clustered around the zero point conflict less than uniform ones).
-// Measured on B200, ResNet-18 layers at batch 256, broadcast with uniform / clustered codes against slab, ms:
-//   7 bits  3x3 512->512 (4608 rows) 2.92 / 2.13 : 2.42    3x3 256->256 (2304 rows) 2.91 / 2.12 : 3.13
-//   8 bits  3x3 512->512             3.94 / 2.73 : 2.68    3x3 256->256             3.92 / 2.69 : 3.63
-//           3x3 256->512 stride 2 (classes of 2048, 1024, 1024, 512 rows) 2.63 / 1.82 : 1.53
-// Trained layers have clustered codes, so the choice leans that way: from 8192 rows at 7 bits (a wash between the two
-// distributions at 4608), from 4096 rows or Cout >= 512 at 8 bits, where the gather is up to four-way conflicted.
-static bool gx_class_uses_slab(int bits, const lutgemm::PixelClass &px, int Cout) {
+// f(class) for every stride class of the convolution that has pixels and taps
+extern "C++" {
+template <typename F>
+static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
+    lutgemm::PixelClass px;
+    for (int ph = 0; ph < g.stride; ++ph)
+        for (int pw = 0; pw < g.stride; ++pw)
+            if (make_pixel_class(g, ph, pw, &px)) f(px);
+}
+}
+
+// Slab kernel in pixel mode (rows = taps * Cout) or column-broadcast gather kernel in pixel mode, by estimated time (see
+// family_clocks).  The slab kernel's time does not depend on the codes, the broadcast kernel's bank conflicts do; the
+// estimate takes the clustered codes of a trained layer.  Measured on B200, 3x3 layers at batch 256, clustered codes,
+// broadcast against slab, ms:
+//   7 bits  64 channels (576 rows) 1.79 : 2.17   128 (1152) 1.99 : 1.96   256 (2304) 2.00 : 1.81   512 (4608) 2.02 : 1.79
+//   8 bits  64 channels            2.32 : 2.81   128        2.66 : 2.57   256        2.66 : 2.39   512        2.74 : 2.36
+static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
     const int force = g_force_backward.load(std::memory_order_relaxed);
     if (force == LUTGEMM_BACKWARD_BCAST) return false;
     if (force == LUTGEMM_BACKWARD_SLAB) return true;
-    const long rows = (long)px.ntaps * Cout;
-    return bits == 7 ? rows >= 8192 : bits == 8 && (rows >= 4096 || Cout >= 512);
+    const FamilyClocks f = family_clocks(bits);
+    const long mt = bits == 8 ? 512 : 256;
+    double slab = 0, rows_tiles = 0;
+    long tiles = 0, most_rows = 0;
+    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
+        const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
+        const int rt = lutgemm::gx_tile_rows(bits, rows);
+        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, 20, f.packed * (rt > 512 ? 1.15 : 1.0), kSlabStart, sms);
+        tiles += t;
+        rows_tiles += (double)t * rows;
+        if (rows > most_rows) most_rows = rows;
+    });
+    const double mean = (double)div_up(tiles, sms) * rows_tiles / tiles;  // (a class with pixels exists: kernel extent > stride)
+    const double per_sm = mean > most_rows ? mean : (double)most_rows;
+    return slab < per_sm * mt * f.gx_bcast + kBcastStart;
+}
+
+// Scratch that the choice by fixed limits (see base_plan) asked for: a buffer of at least that size is not refused, the
+// broadcast kernel, which needs none, runs where the slab kernel's partial sums do not fit.
+static size_t gx_base_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout) {
+    size_t need = 0;
+    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
+        const long rows = (long)px.ntaps * Cout;
+        if (!(bits == 7 ? rows >= 8192 : bits == 8 && (rows >= 4096 || Cout >= 512))) return;
+        auto cost = [&](long rt) { return div_up(rows, rt) * (rt + (bits == 8 ? 384 : 256)); };
+        long rt = 1024;
+        for (long cand : {576L, 512L})
+            if (cost(cand) < cost(rt)) rt = cand;
+        const long blocks = div_up(rows, rt);
+        const size_t n = blocks > 1 ? (size_t)blocks * px.C * px.P * sizeof(float) : 0;
+        need = n > need ? n : need;
+    });
+    return need;
 }
 
 static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout) {
     const int M = g.B * g.Ho * g.Wo, K = g.C * g.kh * g.kw;
-    if (!conv_windows_overlap(g)) {
-        const int sms = current_num_sms();
-        return sms > 0 ? plan_backward(bits, M, K, Cout, sms).ga_scratch : 0;
-    }
+    const int sms = current_num_sms();
+    if (sms <= 0) return 0;
+    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true).ga_scratch;
     size_t need = 0;
-    lutgemm::PixelClass px;
-    for (int ph = 0; ph < g.stride; ++ph)
-        for (int pw = 0; pw < g.stride; ++pw)
-            if (make_pixel_class(g, ph, pw, &px) && gx_class_uses_slab(bits, px, Cout)) {
-                const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B);
-                need = n > need ? n : need;
-            }
+    if (gx_uses_slab(bits, g, Cout, sms))
+        for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
+            const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B);
+            need = n > need ? n : need;
+        });
     return need;
 }
 
@@ -457,7 +571,7 @@ size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int 
     if (sms <= 0) return 0;
     const int M = B * g.Ho * g.Wo, K = C * kh * kw;
     // the weight-gradient and the activation-gradient kernels run one after the other on the same buffer
-    const size_t gw_need = plan_backward(bits, M, K, Cout, sms).gw_scratch;
+    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true).gw_scratch;
     const size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
     return gw_need > gx_need ? gw_need : gx_need;
 }
@@ -492,16 +606,22 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
         return backward_impl(gy, x, wmat, gx, nullptr, lut_ga, nullptr, bits, M, K, Cout, g, nullptr, scratch, scratch_bytes,
                              stream);
     if (!pixel_mode_supported(g)) return LUTGEMM_E_TOOLARGE;
-    if (conv_gx_scratch_bytes(bits, g, Cout) > (scratch ? scratch_bytes : 0)) return LUTGEMM_E_SCRATCH;
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
+    bool slab = gx_uses_slab(bits, g, Cout, sms);
+    const size_t given = scratch ? scratch_bytes : 0;
+    if (slab && conv_gx_scratch_bytes(bits, g, Cout) > given) {
+        if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
+            return LUTGEMM_E_SCRATCH;
+        slab = false;
+    }
     lutgemm::PixelClass px;
     lutgemm::PixelClass bcast[lutgemm::kMaxClassesPerLaunch];  // classes for the broadcast kernel, launched in groups
     int nb = 0;
     for (int ph = 0; ph < stride; ++ph)
         for (int pw = 0; pw < stride; ++pw) {
             if (!make_pixel_class(g, ph, pw, &px)) continue;
-            if (gx_class_uses_slab(bits, px, Cout)) {
+            if (slab) {
                 rc = lutgemm::backward_gx_class(gy, x, wmat, gx, lut_ga, bits, Cout, px, B, static_cast<float *>(scratch), sms, s);
                 if (rc != LUTGEMM_OK) return rc;
                 continue;
@@ -541,8 +661,8 @@ static int make_epilogue(const float *box, const float *sumw_t, const float *tap
 // `scratch` and the one-pass epilogue kernel finishes them.
 static size_t align16(size_t n) { return (n + 15) & ~(size_t)15; }
 
-static bool layer_forward_needs_sums(int M, int K, int N, int sms) {
-    return forward_uses_slab(M, N) && lutgemm::slab_fwd_ksplits(M, K, N, sms) > 1;
+static bool layer_forward_needs_sums(int bits, int M, int K, int N, int sms) {
+    return forward_uses_slab(bits, M, K, N, sms) && lutgemm::slab_fwd_ksplits(M, K, N, sms) > 1;
 }
 
 static size_t layer_forward_scratch_bytes(int bits, int M, int K, int N) {
@@ -550,7 +670,7 @@ static size_t layer_forward_scratch_bytes(int bits, int M, int K, int N) {
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
     const size_t codes = align16(lutgemm_forward_scratch_bytes(bits, M, K, N));
-    return codes + (layer_forward_needs_sums(M, K, N, sms) ? (size_t)M * N * sizeof(uint32_t) : 0);
+    return codes + (layer_forward_needs_sums(bits, M, K, N, sms) ? (size_t)M * N * sizeof(uint32_t) : 0);
 }
 
 static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t *lut, int bits, int M, int K, int N,
@@ -561,9 +681,12 @@ static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
     const size_t codes = lutgemm_forward_scratch_bytes(bits, M, K, N);
-    if (!layer_forward_needs_sums(M, K, N, sms))
-        return forward_impl(a, w, nullptr, lut, bits, M, K, N, conv, scratch, scratch ? codes : 0, stream, &e);
-    if (!scratch || scratch_bytes < layer_forward_scratch_bytes(bits, M, K, N)) return LUTGEMM_E_SCRATCH;
+    if (!layer_forward_needs_sums(bits, M, K, N, sms))
+        return forward_impl(a, w, nullptr, lut, bits, M, K, N, conv, scratch, scratch_bytes, stream, &e);
+    if (!scratch || scratch_bytes < layer_forward_scratch_bytes(bits, M, K, N)) {
+        if (base_forward_uses_slab(M, N) || g_force_forward.load(std::memory_order_relaxed)) return LUTGEMM_E_SCRATCH;
+        return lutgemm::forward_rowbcast(a, w, nullptr, lut, bits, M, K, N, conv, &e, sms, static_cast<cudaStream_t>(stream));
+    }
     uint32_t *sums = reinterpret_cast<uint32_t *>(static_cast<char *>(scratch) + align16(codes));
     const int rc = forward_impl(a, w, sums, lut, bits, M, K, N, conv, scratch, codes, stream);
     if (rc != LUTGEMM_OK) return rc;

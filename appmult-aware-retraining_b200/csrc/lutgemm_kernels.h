@@ -18,6 +18,9 @@ inline bool cuda_ok(cudaError_t e) {
 // status of the launch just made on this thread
 int launch_status();
 
+// scratch of the weight gradient under the choice by fixed limits (lutgemm_api.cu)
+size_t base_gw_scratch_bytes(int bits, int M, int K, int N);
+
 struct ConvGeom;    // lutgemm_common.cuh; geometry.enabled == 0 means `a` is a plain [M,K] matrix
 struct PixelClass;  // lutgemm_common.cuh; the input pixels of one stride class of a convolution and their taps
 struct LayerEpilogue;  // lutgemm_common.cuh; optional de-quantisation applied where the forward kernels store
@@ -36,18 +39,39 @@ void slab_fwd_set_tma(bool on);
 // number of K ranges forward_slab cuts a problem into when it is free to (1 = none; a fused epilogue needs 1)
 int slab_fwd_ksplits(int M, int K, int N, int num_sms);
 
-// rows of the reduction dimension per CTA tile of the fp32-slab gradient kernels, and the block count
-constexpr int kSlabF32Rows = 512;
-int slab_f32_row_blocks(int rdim);
-// gradient slab kernels with an fp32 slab (conversion done once per slab entry, in the build)
-// `at` (optional): the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
-int backward_gw_slab_f32(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
-                         int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                         int at_pitch, int num_sms, cudaStream_t stream);
-int backward_ga_slab_f32(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
-                         int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
-                         cudaStream_t stream);
-// the same with a tall tile (1024 rows x 32 columns): half the slab-build work per look-up
+// How a slab kernel cuts K (outputs are per k, so the parts are independent work items): the number of parts and the k
+// per part (a multiple of 16) for which a persistent grid of num_sms CTAs finishes first, when an item of `per` k costs
+// per + item_overhead steps.  Up to 64 parts, so that few tiles still fill the GPU.
+struct KSplit {
+    int parts, per;
+    long waves;
+};
+inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
+    const int chunks = (K + 15) / 16;
+    KSplit best{1, chunks * 16, (tiles + num_sms - 1) / num_sms};
+    long cost = best.waves * (best.per + item_overhead);
+    for (int s = 2; s <= 64 && s <= chunks; ++s) {
+        const int per = ((chunks + s - 1) / s) * 16;
+        if ((K + per - 1) / per != s) continue;
+        const long waves = (tiles * s + num_sms - 1) / num_sms, c = waves * (per + item_overhead);
+        if (c < cost) { cost = c; best = KSplit{s, per, waves}; }
+    }
+    return best;
+}
+constexpr int kPackedItemOverhead = 12, kTallItemOverhead = 8;  // in k steps: operand fetch, grad_out block, first slabs
+
+// rows of the reduction dimension per CTA tile of the packed-slab gradient kernels, and the block count
+constexpr int kSlabPackedRows = 512;
+int slab_packed_row_blocks(int rdim);
+// gradient slab kernels with 16-bit slab entries (converted where they are used)
+// `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
+int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
+                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
+                            int at_pitch, int num_sms, cudaStream_t stream);
+int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
+                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
+                            cudaStream_t stream);
+// fp32 slab entries and a tall tile (1024 rows x 32 columns)
 constexpr int kSlabTallRows = 1024;
 int slab_tall_row_blocks(int rdim);
 // lut_f32 (optional, bits <= 7): the gradient table as fp32 in the same padded layout; it replaces the int16
@@ -68,7 +92,8 @@ int bounded_wait_selftest(cudaStream_t stream);
 int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks, bool transpose, const ConvGeom *scatter,
                        const PixelClass *px, float scale, int num_sms, cudaStream_t stream);
 // activation gradient of a convolution for the input pixels of one stride class, written into gx[B,C,H,W]
-// (tall slab kernel in pixel mode: no unfolded gradient, no col2im); scratch: gx_class_scratch_bytes()
+// (packed slab kernel in pixel mode: no unfolded gradient, no col2im); scratch: gx_class_scratch_bytes()
+int gx_tile_rows(int bits, long rdim);  // rows of its tile for a class of rdim = taps * Cout rows
 size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B);
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
                       int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream);

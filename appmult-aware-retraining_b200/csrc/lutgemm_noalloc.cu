@@ -48,6 +48,10 @@ int lutgemm_backward_gw_noalloc(const float *gc, const uint8_t *a, const uint8_t
     if (!gc || !a || !w || !gw || !lut_gw || M <= 0 || K <= 0 || N <= 0) return LUTGEMM_E_BADARG;
     void *scratch = scratch_on_current_device();
     if (!scratch) return LUTGEMM_E_CUDA;
+    // What fits is decided by the dispatch with fixed limits: lutgemm_backward falls back to it where the partial sums of
+    // the faster choice exceed the array.
+    if (lutgemm_lut_elem_num(bits) > 0 && lutgemm::base_gw_scratch_bytes(bits, M, K, N) > kNoAllocScratchBytes)
+        return LUTGEMM_E_TOOLARGE;
     // Same kernels and dispatch as lutgemm_backward with ga == NULL; only the home of the partial sums
     // differs.  Every partial sum the reduction reads is written earlier in the same call, so nothing in
     // the array has to start at zero and nothing is cleared here.

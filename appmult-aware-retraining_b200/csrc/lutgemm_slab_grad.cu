@@ -1,54 +1,105 @@
-// Gradient LUT-GEMM kernels for sm_100a with an fp32 "column-gathered slab" (grad_w and grad_a).
+// Gradient LUT-GEMM kernels for sm_100a with a packed 16-bit "column-gathered slab" (512 x 64 tile).
 //
 //   grad_w:  gw[k,n] = 1/16 * sum_m T(a[m,k], w[k,n]) * gc[m,n]     rows r = m, columns c = n
 //   grad_a:  ga[m,k] = 1/16 * sum_n gc[m,n] * T(a[m,k], w[k,n])     rows r = n, columns c = m
+//   grad_x:  gx[b,c,h,w] = 1/16 * sum_{taps (i,j)} sum_n gy[m(b,h,w,i,j), n] * T(x[b,c,h,w], wmat[(c,i,j), n])
+//            rows r = (tap, n), columns = input pixels, the k loop runs over the input channels c
 //
-// As in the forward slab kernel, for every k the CTA first gathers a slab U_k[x][c] = T(x, cc[k,c]) for
-// all 2^b row codes x and its 64 columns c, and each of its 512 rows then reads slab row rc[r,k]
-// contiguously.  Here the slab holds fp32 values, converted ONCE per slab entry while it is built:
-// the use phase is then  "extract code, form address, one 64-bit shared load, two FMAs"  per row and
-// lane pair of columns - 5 instructions per 64 table look-ups, with no int16->fp32 conversion (the XU
-// pipe converts only 16 lanes/clk) and no unpacking in the hot loop.  The grad_out block of the tile
-// (32 rows x 2 columns per thread) stays in registers for the whole k loop.
+// Per k a slab U_k[x][c] = T(x, cc[k,c]) is gathered once for all 2^b row codes x and the 64 columns of the tile, then
+// every row reads slab row rc[r,k] contiguously (half a warp per row, four columns per lane in one 64-bit load,
+// conflict-free by construction) and multiplies it with its grad_out entries, which stay in registers for the whole
+// k loop.
 //
-// Shared memory: the gradient table (fp32 [cc][x] for b <= 7, 66 KB at 7 bits; int16 pairs at 8 bits,
-// 129 KB, converted with the magic-number trick during the build), the slab(s) (2^b rows x 264 B; two
-// buffers for b <= 7, one at 8 bits where two do not fit), operand code stages and the per-warp partial
-// sums.  Every k yields one partial sum per column and warp; the 16 warps are combined in a fixed
-// tree, 512-row blocks by slab_reduce_blocks in ascending order: results are deterministic.
-// Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492.
-#include <stdlib.h>
+// grad_x is the activation gradient of a convolution WITHOUT the unfolded intermediate: every tap that touches an input
+// pixel sees the same activation code, so the sum over taps joins the sum over n in one long row dimension (kh*kw*Cout
+// rows; the kernel exists with 576-row tiles for it as well), the column codes are the code image itself, the row codes are
+// kh*kw rows of the weight matrix, and the result is written straight into the image gradient - no col2im, no atomics.  A
+// strided convolution is cut into stride^2 classes of input pixels that each see a fixed subset of the taps.
+//
+// What bounds it: the shared-memory pipe (one 128-byte wavefront per clock) and instruction issue (four per clock).
+// The slab keeps the table's own 16 bits per entry, so a look-up costs half the wavefronts of an fp32 slab; the price
+// is the conversion at each use.  It is done for two entries at a time: each 16-bit half goes, in offset-binary, behind
+// the exponent of 2^23 (one byte permutation), one packed subtraction of 2^23 + 2^15 leaves the two signed entries
+// exactly, and one packed multiply-add (fma.rn.f32x2) consumes them - 10 instructions per 128 look-ups of a warp
+// against 8 with an fp32 slab, but 512 + build instead of 1024 + build wavefronts per 32768 look-ups.  Products and
+// sums are the same fp32 operations as with an fp32 slab.
+//
+// Hand-over between the warps of a CTA: per slab buffer a "full" and an "empty" mbarrier with one arrival per warp
+// (see lutgemm_slab_grad_tall.cu); at 7 bits and below a buffer holds the slabs of two k, so that waits, arrivals and
+// loop overhead are paid once per two k.  Every wait is bounded (lutgemm_waits.cuh).
+// Partial sums: one per lane group, warp and k; one warp (rotating with k) adds the 32 of a column in ascending order,
+// row blocks are added by slab_reduce_blocks in ascending order: results are deterministic.
+// Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492, and for
+// grad_x the unfold backward of self_ops/ops_py/approx_ops.py:556-571.
+#include <type_traits>
 
 #include "lutgemm_common.cuh"
 #include "lutgemm_kernels.h"
+#include "lutgemm_waits.cuh"
 
 namespace lutgemm {
-namespace sg {
+namespace sp {
 
-enum { kGw = 1, kGa = 2 };
+enum { kGw = 1, kGa = 2, kGx = 3 };
 
-template <int BITS, int WARPS, int RW_>
+// two fp32 values in one 64-bit register (the operand form of the packed fp32 instructions)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 t;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t.x), "=f"(t.y) : "l"(v));
+    return t;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// the two signed table entries of a slab word: 0x4B000000 | u is the float 2^23 + u, u = entry + 2^15
+__device__ __forceinline__ f32x2 entries2(uint32_t word, f32x2 bias) {
+    const float lo = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7610));
+    const float hi = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7632));
+    return add2(pack2(lo, hi), bias);
+}
+
+template <int BITS, int RW_>
 struct Cfg {
     static constexpr int Q = 1 << BITS;
-    static constexpr bool F32_TABLE = BITS <= 7;
-    static constexpr int HALF = Q / 2;
-    static constexpr int TT_STRIDE = F32_TABLE ? Q + 1 : HALF + 1;  // words per table row
-    static constexpr int THREADS = 32 * WARPS, RT = WARPS * RW_, CT = 64, KC = 16;
-    static constexpr int RW = RW_;               // rows per warp (a multiple of 8)
-    static constexpr int PPW = 32 / WARPS;       // slab column pairs built per warp
-    static constexpr int CPW = CT / WARPS;       // columns whose partial sums a warp combines
-    static constexpr int U_STRIDE = 66;  // words per slab row: 64 floats + 2 (conflict-free 64-bit stores)
-    static constexpr int P_STRIDE = 66;
-    static constexpr int NBUF = BITS == 8 ? 1 : 2;   // slab buffers (and partial-sum buffers)
-    static constexpr int TT_BYTES = Q * TT_STRIDE * 4;
-    static constexpr int U_BYTES = Q * U_STRIDE * 4;
-    static constexpr int RC_STAGE = KC * RT, CC_STAGE = KC * CT;
-    static constexpr int P_BYTES = WARPS * P_STRIDE * 4;
+    static constexpr int WARPS = 16, THREADS = 512, RW = RW_, RT = WARPS * RW, CT = 64;
+    static constexpr int E = Q >= 32 ? Q / 32 : 1;      // codes per lane in the build: x = lane + 32 j, j < E
+    // table row of a column code: the E entries of a lane side by side (one 2E-byte load per column and lane); the
+    // 2E bytes of padding spread the transposing stage over the banks
+    static constexpr int TT_ROW = 2 * Q + (E == 1 ? 4 : 2 * E);
+    static constexpr int U_ROW = 2 * CT + 8;            // bytes per slab row: conflict-free 64-bit build stores
+    static constexpr int KC = 16;                       // k per global fetch
+    static constexpr int SC = BITS == 8 ? 8 : 16;       // k per shared-memory stage
+    static constexpr int KP = BITS == 8 ? 1 : 2;        // slabs per buffer
+    static constexpr int NB = BITS == 8 ? 2 : 3;        // buffers (shared memory has no room for a third at 8 bits)
+    static constexpr int NSEG = RT / 16;                // 16-row code segments per k
+    static constexpr int RC_LOADS = (KC * NSEG + THREADS - 1) / THREADS;
+    static constexpr int TT_BYTES = (Q * TT_ROW + 15) & ~15;
+    static constexpr int U_BYTES = Q * U_ROW;
+    static constexpr int RC_STAGE = SC * RT, CC_STAGE = SC * CT;
+    static constexpr int P_FLOATS = 2 * WARPS * CT;     // partial sums of one k: one row per half-warp
     static constexpr int OFF_U = TT_BYTES;
-    static constexpr int OFF_RC = OFF_U + NBUF * U_BYTES;
+    static constexpr int OFF_RC = OFF_U + NB * KP * U_BYTES;
     static constexpr int OFF_CC = OFF_RC + 2 * RC_STAGE;
     static constexpr int OFF_PART = OFF_CC + 2 * CC_STAGE;
-    static constexpr int SMEM = OFF_PART + NBUF * P_BYTES;
+    static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // grad_x: image offset of each column
+    static constexpr int OFF_BAR = OFF_PIX + CT * 8;
+    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // a full and an empty mbarrier per buffer, and the abort word
+    static_assert(RW % 4 == 0 && RT % 16 == 0, "rows per warp");
+    static_assert(U_BYTES % 16 == 0 && RC_STAGE % 16 == 0 && CC_STAGE % 16 == 0, "16-byte vectors");
+    static_assert(SMEM <= 232448, "shared memory budget");
 };
 
 struct Args {
@@ -57,63 +108,61 @@ struct Args {
     const int16_t *lut;
     const float *gc;
     float *out;
-    int M, K, N;
+    int M, K, N;               // kGx: M = pixels of the class (all images), K = channels, N = Cout
+    int RDIM, CDIM;
     int tiles_r, tiles_c;
     int ksplits, k_per_split;  // a tile's k range is cut into independent work items (outputs are per k)
     int direct;
     int vec_a, vec_w, vec_g;
     ConvGeom conv;
-    int ga_scatter;  // grad_a of a convolution: results go straight to the image gradient
-    const uint8_t *at;  // grad_w only, optional: transposed row codes at[k][m], rows at_pitch bytes apart
+    int ga_scatter;     // grad_a of a convolution whose windows do not overlap: results go straight to the image
+    const uint8_t *at;  // grad_w: transposed row codes at[k][m], rows at_pitch bytes apart
     int at_pitch;       // a multiple of 16; columns m >= M hold 0
+    int *error_word;    // device error word of the bounded waits
+    PixelClass px;      // kGx only
 };
 
-// PF = how many slab-row loads are kept in flight ahead of the FMAs that consume them.  Without explicit
-// prefetch the compiler, short of registers, emits load -> use -> load -> use, and a warp's k iteration
-// costs RW shared-memory latencies back to back.
-template <int BITS, int MODE, int WARPS, int RW_, int PF>
-__global__ void __launch_bounds__(32 * WARPS, 1) slab_grad_kernel(const Args p) {
-    using C = Cfg<BITS, WARPS, RW_>;
-    constexpr int RW = C::RW, PPW = C::PPW, CPW = C::CPW;
-    constexpr int Q = C::Q, HALF = C::HALF, TTS = C::TT_STRIDE, RT = C::RT, CT = C::CT, KC = C::KC;
-    constexpr int US = C::U_STRIDE, PS = C::P_STRIDE, THREADS = C::THREADS, NBUF = C::NBUF;
+template <int BITS, int MODE, int RW>
+__global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_constant__ Args p) {
+    using C = Cfg<BITS, RW>;
+    constexpr int Q = C::Q, E = C::E, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC, KP = C::KP, NB = C::NB;
+    constexpr int WARPS = C::WARPS, THREADS = C::THREADS, NSEG = C::NSEG, RCL = C::RC_LOADS;
+    constexpr int HALVES = KC / SC;  // shared-memory stages per fetched group of 16 k
+    constexpr int NW = RW / 4;       // code words per warp; half h of the warp owns rows 4q + 2h and 4q + 2h + 1
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
     constexpr int COL = lut_col_num(BITS);
 
     const int M = p.M, K = p.K, N = p.N;
-    const int CDIM = MODE == kGa ? M : N;
+    const int RDIM = p.RDIM, CDIM = p.CDIM;
 
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t *rc_s = smem + C::OFF_RC;
     uint8_t *cc_s = smem + C::OFF_CC;
     float *part_s = reinterpret_cast<float *>(smem + C::OFF_PART);
+    long long *pix_s = reinterpret_cast<long long *>(smem + C::OFF_PIX);
     const uint32_t tt_addr = smem_u32(smem);
     const uint32_t u_addr = smem_u32(smem + C::OFF_U);
+    const uint32_t bar_full = smem_u32(smem + C::OFF_BAR), bar_empty = bar_full + 8 * NB;
+    volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 16 * NB);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int half = lane >> 4, cq = lane & 15;  // half-warp and column quad (columns 4 cq .. 4 cq + 3)
 
-    // ---- stage the gradient table; x = row code, y = column code, T(x,y) = lut[a*COL + w] ----------------
+    // ---- stage the gradient table in offset-binary; x = row code, y = column code, T(x,y) = lut[a*COL + w] -------
+    // (grad_w: rows are activation codes; grad_a / grad_x: rows are weight codes)
 #pragma unroll 8
     for (int idx = tid; idx < Q * Q; idx += THREADS) {
         const int hi_idx = idx >> BITS, lo_idx = idx & (Q - 1);  // global read contiguous in lo_idx
-        const int16_t v = p.lut[hi_idx * COL + lo_idx];
-        const int x = MODE == kGa ? lo_idx : hi_idx, y = MODE == kGa ? hi_idx : lo_idx;
-        if (C::F32_TABLE) {
-            reinterpret_cast<float *>(smem)[y * TTS + x] = (float)v;
-        } else {
-            // int16 pairs {T(i,y), T(i+HALF,y)} in offset-binary (v + 32768) for the magic-number conversion
-            reinterpret_cast<uint16_t *>(smem)[(y * TTS + (x & (HALF - 1))) * 2 + (x >> (BITS - 1))] =
-                (uint16_t)v ^ (uint16_t)0x8000u;
-        }
+        const int x = MODE == kGw ? hi_idx : lo_idx, y = MODE == kGw ? lo_idx : hi_idx;
+        const int pos = Q >= 32 ? (x & 31) * E + (x >> 5) : x;
+        *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + pos * 2) = (uint16_t)p.lut[hi_idx * COL + lo_idx] ^ (uint16_t)0x8000u;
     }
+    if (tid == 0) *abort_word = 0;
 
-    // grad_a of a convolution (non-overlapping windows) goes straight to its place in the image gradient
-    auto ga_index = [&](int m, int k) -> long {
-        if (!p.ga_scatter) return (long)m * K + k;
-        return conv_scatter_index(p.conv, m, k);
-    };
-
-    // ---- operand chunk staging: rc_s[stage][kk][r] (512 row codes per k), cc_s[stage][kk][c] (64) ------
-    uint4 prc = make_uint4(0, 0, 0, 0), pcc = make_uint4(0, 0, 0, 0);
+    // ---- operand staging: a group of 16 k is fetched into registers and written to shared memory SC k at a time:
+    //      rc_s[stage][kk][r] (RT row codes per k), cc_s[stage][kk][c] (64 column codes per k) ---------------------
+    uint4 prc[RCL], pcc = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < RCL; ++j) prc[j] = make_uint4(0, 0, 0, 0);
     auto load16 = [&](const uint8_t *src, int valid) -> uint4 {  // up to 16 bytes, the rest 0
         uint32_t t[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -135,227 +184,510 @@ __global__ void __launch_bounds__(32 * WARPS, 1) slab_grad_kernel(const Args p) 
         if (p.vec_w) return *reinterpret_cast<const uint4 *>(src);
         return load16(src, min(16, N - n));
     };
-    auto fetch_chunk = [&](int r0, int c0, int chunk) {
-        const int kbase = chunk * KC;
-        if (tid >= RT) return;
-        if (MODE == kGw && p.at) {
-            // row codes from the transposed copy at[k][m]: 16 rows per load, coalesced like the w operand
-            const int gk = kbase + tid / (RT / 16), gm = r0 + (tid % (RT / 16)) * 16;
-            prc = (gk < K && gm < p.at_pitch) ? *reinterpret_cast<const uint4 *>(p.at + (size_t)gk * p.at_pitch + gm)
-                                              : make_uint4(0, 0, 0, 0);
-            if (tid < KC * CT / 16) pcc = w_codes16(kbase + tid / (CT / 16), c0 + (tid % (CT / 16)) * 16);
-        } else if (MODE == kGw) {
-            prc = a_codes16(r0 + tid, kbase);
-            if (tid < KC * CT / 16) pcc = w_codes16(kbase + tid / (CT / 16), c0 + (tid % (CT / 16)) * 16);
-        } else {
-            prc = w_codes16(kbase + tid / (RT / 16), r0 + (tid % (RT / 16)) * 16);
-            if (tid < CT) pcc = a_codes16(c0 + tid, kbase);
+    // grad_x: row codes of channel k, rows r..r+15 with r = tap*N + n -> weight rows (k*T + t[tap])
+    auto gx_row_codes16 = [&](int k, int r) -> uint4 {
+        if (k >= K || r >= RDIM) return make_uint4(0, 0, 0, 0);
+        int q = r / N, n = r - q * N;
+        if (p.vec_w)  // N % 16 == 0: the 16 rows lie inside one tap
+            return *reinterpret_cast<const uint4 *>(p.w + ((size_t)k * p.px.T + p.px.t[q]) * N + n);
+        uint32_t t[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (r + i < RDIM) t[i >> 2] |= (uint32_t)p.w[((size_t)k * p.px.T + p.px.t[q]) * N + n] << (8 * (i & 3));
+            if (++n == N) { n = 0; ++q; }
+        }
+        return make_uint4(t[0], t[1], t[2], t[3]);
+    };
+    // grad_x: the code of pixel column `col` in channels kbase..kbase+15
+    auto gx_col_codes16 = [&](int col, int kbase) -> uint4 {
+        if (col >= CDIM || kbase >= K) return make_uint4(0, 0, 0, 0);
+        const size_t plane = (size_t)p.px.H * p.px.W;
+        const uint8_t *src = p.a + pixel_class_offset(p.px, col) + (size_t)kbase * plane;
+        uint32_t t[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            if (kbase + q < K) t[q >> 2] |= (uint32_t)src[q * plane] << (8 * (q & 3));
+        return make_uint4(t[0], t[1], t[2], t[3]);
+    };
+    auto fetch_group = [&](int r0, int c0, int group) {
+        const int kbase = group * KC;
+#pragma unroll
+        for (int j = 0; j < RCL; ++j) {
+            const int idx = tid + THREADS * j;  // (k, 16-row segment)
+            const int gk = kbase + idx / NSEG, gr = r0 + (idx % NSEG) * 16;
+            if ((KC * NSEG) % THREADS != 0 && idx >= KC * NSEG) prc[j] = make_uint4(0, 0, 0, 0);
+            else if (MODE == kGw)
+                prc[j] = (gk < K && gr < p.at_pitch) ? *reinterpret_cast<const uint4 *>(p.at + (size_t)gk * p.at_pitch + gr)
+                                                     : make_uint4(0, 0, 0, 0);
+            else prc[j] = MODE == kGx ? gx_row_codes16(gk, gr) : w_codes16(gk, gr);
+        }
+        if (tid < CT) {
+            if (MODE == kGw) pcc = w_codes16(kbase + tid / (CT / 16), c0 + (tid % (CT / 16)) * 16);
+            else pcc = MODE == kGx ? gx_col_codes16(c0 + tid, kbase) : a_codes16(c0 + tid, kbase);
         }
     };
-    auto store_chunk = [&](int stage) {
-        if (tid >= RT) return;
+    static_assert(KC * CT / 16 == CT, "column codes: one 16-byte vector for each of the first 64 threads");
+    // writes the k range [hf*SC, hf*SC + SC) of the fetched group to `stage`, cut to BITS bits
+    auto store_stage = [&](int stage, int hf) {
         uint8_t *rs = rc_s + stage * C::RC_STAGE;
         uint8_t *cs = cc_s + stage * C::CC_STAGE;
-        const uint32_t tr[4] = {prc.x & MASK4, prc.y & MASK4, prc.z & MASK4, prc.w & MASK4};
-        const uint32_t tc[4] = {pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4};
-        if (MODE == kGw && p.at) {
-            *reinterpret_cast<uint4 *>(rs + (tid / (RT / 16)) * RT + (tid % (RT / 16)) * 16) =
-                make_uint4(tr[0], tr[1], tr[2], tr[3]);
-            if (tid < KC * CT / 16)
-                *reinterpret_cast<uint4 *>(cs + (tid / (CT / 16)) * CT + (tid % (CT / 16)) * 16) =
-                    make_uint4(tc[0], tc[1], tc[2], tc[3]);
-        } else if (MODE == kGw) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) rs[q * RT + tid] = (uint8_t)(tr[q >> 2] >> (8 * (q & 3)));
-            if (tid < KC * CT / 16)
-                *reinterpret_cast<uint4 *>(cs + (tid / (CT / 16)) * CT + (tid % (CT / 16)) * 16) =
-                    make_uint4(tc[0], tc[1], tc[2], tc[3]);
+        for (int j = 0; j < RCL; ++j) {
+            const int idx = tid + THREADS * j, kq = idx / NSEG;
+            if (idx < KC * NSEG && (kq / SC == hf || HALVES == 1))
+                *reinterpret_cast<uint4 *>(rs + (kq % SC) * RT + (idx % NSEG) * 16) =
+                    make_uint4(prc[j].x & MASK4, prc[j].y & MASK4, prc[j].z & MASK4, prc[j].w & MASK4);
+        }
+        if (tid < CT) {
+            const uint32_t tc[4] = {pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4};
+            if (MODE == kGw) {
+                const int kq = tid / (CT / 16);
+                if (kq / SC == hf || HALVES == 1)
+                    *reinterpret_cast<uint4 *>(cs + (kq % SC) * CT + (tid % (CT / 16)) * 16) = make_uint4(tc[0], tc[1], tc[2], tc[3]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    if (q / SC == hf || HALVES == 1) cs[(q % SC) * CT + tid] = (uint8_t)(tc[q >> 2] >> (8 * (q & 3)));
+            }
+        }
+    };
+    // build the slab at shared address `ub` for the k at (stage, kk): warp wp fills columns 4 wp .. 4 wp + 3.  Lane l
+    // reads the entries of codes l + 32 j of each column in one load and stores four columns of one code at a time;
+    // all table reads of the share are issued before the first store (the stores order later reads behind them).
+    const uint32_t tt_lane = tt_addr + lane * (2 * E);
+    const uint32_t us = u_addr + wp * 8 + lane * C::U_ROW;
+    auto build = [&](uint32_t off, const uint8_t *codes) {  // off: byte offset of the slab
+        const uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + wp * 4);
+        constexpr int EW = (E + 1) / 2;  // table words per lane and column
+        uint32_t r[4][EW];
+        if (Q >= 32 || lane < Q) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t addr = tt_lane + byte_of(cw, c) * C::TT_ROW;
+                if constexpr (E == 8)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(r[c][0]), "=r"(r[c][1]), "=r"(r[c][2]), "=r"(r[c][3]) : "r"(addr));
+                else if constexpr (E == 4)
+                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r[c][0]), "=r"(r[c][1]) : "r"(addr));
+                else if constexpr (E == 2) r[c][0] = lds_u32(addr);
+                else r[c][0] = lds_u16(addr);
+            }
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(us + off + j * 32 * C::U_ROW),
+                             "r"(__byte_perm(r[0][j / 2], r[1][j / 2], sel)), "r"(__byte_perm(r[2][j / 2], r[3][j / 2], sel))
+                             : "memory");
+            }
+        }
+    };
+    // add the 32 partial sums of one k in ascending order and store the tile's 64 columns (two per lane)
+    auto reduce_store = [&](int k, const float *ps, float *obase, int c0) {
+        const f32x2 *p2 = reinterpret_cast<const f32x2 *>(ps) + lane;
+        f32x2 v = p2[0];
+#pragma unroll 8
+        for (int i = 1; i < 2 * WARPS; ++i) v = add2(v, p2[i * (CT / 2)]);
+        float2 o = unpack2(v);
+        if (p.direct) {
+            o.x *= kGradFactor;
+            o.y *= kGradFactor;
+        }
+        const int col = c0 + 2 * lane;
+        if (MODE != kGw && p.direct) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (col + e >= CDIM) break;
+                const float ov = e ? o.y : o.x;
+                if (MODE == kGx) {
+                    obase[pix_s[2 * lane + e] + (long long)k * p.px.H * p.px.W] = ov;
+                } else if (p.ga_scatter) {
+                    const long ix = conv_scatter_index(p.conv, col + e, k);
+                    if (ix >= 0) obase[ix] = ov;
+                } else {
+                    obase[(size_t)(col + e) * K + k] = ov;
+                }
+            }
+            return;
+        }
+        float *dst = obase + (size_t)k * CDIM + col;
+        if (col + 1 < CDIM && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+            *reinterpret_cast<float2 *>(dst) = o;
         } else {
-            *reinterpret_cast<uint4 *>(rs + (tid / (RT / 16)) * RT + (tid % (RT / 16)) * 16) =
-                make_uint4(tr[0], tr[1], tr[2], tr[3]);
-            if (tid < CT) {
-#pragma unroll
-                for (int q = 0; q < 16; ++q) cs[q * CT + tid] = (uint8_t)(tc[q >> 2] >> (8 * (q & 3)));
-            }
-        }
-    };
-    // build slab `buf` for the k at (stage, kk): warp wp fills PPW 64-bit column pairs (columns 2*PPW*wp ...).
-    // Lanes run over x, so the table reads are contiguous and the 64-bit slab stores (row stride 66 words)
-    // fall on distinct bank pairs within each half-warp.
-    auto build = [&](int buf, int stage, int kk) {
-        const uint8_t *cp = cc_s + stage * C::CC_STAGE + kk * CT + wp * (2 * PPW);
-        const uint32_t cw = PPW == 2 ? *reinterpret_cast<const uint32_t *>(cp) : *reinterpret_cast<const uint16_t *>(cp);
-        const uint32_t ub = u_addr + buf * C::U_BYTES;
-#pragma unroll
-        for (int pp = 0; pp < PPW; ++pp) {
-            const uint32_t y0 = byte_of(cw, 2 * pp), y1 = byte_of(cw, 2 * pp + 1);
-            const uint32_t col_off = (2 * PPW * wp + 2 * pp) * 4;
-            if constexpr (C::F32_TABLE) {
-#pragma unroll
-                for (int j = 0; j < (Q + 31) / 32; ++j) {
-                    const int x = lane + 32 * j;
-                    if (Q >= 32 || x < Q) {
-                        const uint32_t r0 = lds_u32(tt_addr + (y0 * TTS + x) * 4);
-                        const uint32_t r1 = lds_u32(tt_addr + (y1 * TTS + x) * 4);
-                        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + x * (US * 4) + col_off), "r"(r0), "r"(r1)
-                                     : "memory");
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < HALF / 32; ++j) {
-                    const int i = lane + 32 * j;
-                    const uint32_t r0 = lds_u32(tt_addr + (y0 * TTS + i) * 4);
-                    const uint32_t r1 = lds_u32(tt_addr + (y1 * TTS + i) * 4);
-                    // 0x4B000000 | u is the float 2^23 + u; minus (2^23 + 32768) leaves the signed entry exactly
-                    const float f00 = __uint_as_float((r0 & 0xffffu) | 0x4B000000u) - 8421376.0f;
-                    const float f01 = __uint_as_float((r1 & 0xffffu) | 0x4B000000u) - 8421376.0f;
-                    const float f10 = __uint_as_float(__byte_perm(r0, 0x4B000000u, 0x7632)) - 8421376.0f;
-                    const float f11 = __uint_as_float(__byte_perm(r1, 0x4B000000u, 0x7632)) - 8421376.0f;
-                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ub + i * (US * 4) + col_off), "f"(f00), "f"(f01)
-                                 : "memory");
-                    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ub + (i + HALF) * (US * 4) + col_off), "f"(f10),
-                                 "f"(f11)
-                                 : "memory");
-                }
-            }
-        }
-    };
-    // combine the warps' partial sums of one k (fixed tree): warp wp owns CPW columns, lane = CPW*grp + col;
-    // grp adds warps 2grp and 2grp+1, the groups meet by shuffles; then store the columns
-    auto reduce_store = [&](int k, float *obase, int c0) {
-        const float *ps = part_s + (NBUF == 2 ? (k & 1) : 0) * (WARPS * PS);
-        const int col = CPW * wp + (lane & (CPW - 1)), grp = lane / CPW;
-        float v = ps[(2 * grp) * PS + col] + ps[(2 * grp + 1) * PS + col];
-#pragma unroll
-        for (int d = CPW; d < 32; d *= 2) v += __shfl_xor_sync(0xffffffffu, v, d);
-        if (lane < CPW && c0 + col < CDIM) {
-            if (p.direct && MODE == kGa) {
-                const long o = ga_index(c0 + col, k);
-                if (o >= 0) obase[o] = v * kGradFactor;
-            } else {
-                obase[(size_t)k * CDIM + c0 + col] = p.direct ? v * kGradFactor : v;
-            }
+            if (col < CDIM) dst[0] = o.x;
+            if (col + 1 < CDIM) dst[1] = o.y;
         }
     };
 
+    const f32x2 bias = pack2(-8421376.0f, -8421376.0f);  // -(2^23 + 2^15)
+    const uint32_t wsel0 = (uint32_t)C::U_ROW << (16 * half), wsel1 = wsel0 << 8;  // dot-product weights of the lane's two rows
+    static_assert(C::U_ROW < 256, "slab row stride must fit one byte of the dot-product operand");
+
     const int items = p.tiles_r * p.tiles_c * p.ksplits;
+    bool first_item = true;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int tile = item / p.ksplits;
         const int kbeg = (item % p.ksplits) * p.k_per_split, kend = min(K, kbeg + p.k_per_split);
         const int tr = tile / p.tiles_c, tc = tile % p.tiles_c;
         const int r0 = tr * RT, c0 = tc * CT;
 
-        // the grad_out block of this tile: g[r][j] for the warp's RW rows and the lane's 2 columns
-        float g[RW][2];
+        // kbeg is a multiple of 16, so the first stage is half 0 of its group
+        fetch_group(r0, c0, kbeg / KC);
+
+        // the grad_out block of this tile: g[2 (2q + j) + i] = entries of row 4q + 2h + j of the warp for the lane's
+        // column pair i (columns 4 cq + 2 i, + 1)
+        // (adding -0 changes no value; it makes the pair the result of one 64-bit instruction, so that it stays in an
+        // aligned register pair - without it two moves per pair and k were spent on re-pairing the registers in grad_a)
+        f32x2 g[RW];
+        const f32x2 minus_zero = pack2(-0.0f, -0.0f);
+        auto pair = [&](float lo, float hi) { return add2(pack2(lo, hi), minus_zero); };
+        const int rb = r0 + wp * RW + 2 * half;  // row (q, j) of the lane is rb + 4 q + j
+        const int cb = c0 + 4 * cq;
         if (MODE == kGw) {
-            const int n = c0 + 2 * lane;
 #pragma unroll
-            for (int r = 0; r < RW; ++r) {
-                const int m = r0 + wp * RW + r;
-                g[r][0] = g[r][1] = 0.f;
-                if (m < M) {
-                    const float *src = p.gc + (size_t)m * N + n;
-                    if (p.vec_g) {
-                        if (n < N) { const float2 t = *reinterpret_cast<const float2 *>(src); g[r][0] = t.x; g[r][1] = t.y; }
+            for (int q = 0; q < NW; ++q)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int m = rb + 4 * q + j;
+                    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (m < M) {
+                        const float *src = p.gc + (size_t)m * N + cb;
+                        if (p.vec_g && cb < N) t = *reinterpret_cast<const float4 *>(src);  // N % 4 == 0
+                        else {
+                            if (cb < N) t.x = src[0];
+                            if (cb + 1 < N) t.y = src[1];
+                            if (cb + 2 < N) t.z = src[2];
+                            if (cb + 3 < N) t.w = src[3];
+                        }
+                    }
+                    g[2 * (2 * q + j)] = pair(t.x, t.y);
+                    g[2 * (2 * q + j) + 1] = pair(t.z, t.w);
+                }
+        } else {
+            // two rows (n, n + 1 of one output position) of four columns at a time
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float *base[2];
+                int h[2] = {0, 0}, w[2] = {0, 0};
+                bool valid[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int col = cb + 2 * i + e;
+                    valid[e] = col < CDIM;
+                    if (MODE == kGa) {
+                        base[e] = p.gc + (size_t)min(col, CDIM - 1) * N;
                     } else {
-                        if (n < N) g[r][0] = src[0];
-                        if (n + 1 < N) g[r][1] = src[1];
+                        const int per = p.px.Hc * p.px.Wc, cc = min(col, CDIM - 1);
+                        const int b = cc / per, rr = cc - b * per, hh = rr / p.px.Wc;
+                        h[e] = p.px.ph + p.px.s * hh;
+                        w[e] = p.px.pw + p.px.s * (rr - hh * p.px.Wc);
+                        base[e] = p.gc + (size_t)b * p.px.Ho * p.px.Wo * N;
                     }
                 }
-            }
-        } else {
-            // g[r][j] = gc[m = c0 + 2*lane + j][n = r0 + RW*wp + r]
+                // &grad_out of (column e, row r), or nullptr where there is none
+                auto src_of = [&](int e, int r) -> const float * {
+                    if (!valid[e] || r >= RDIM) return nullptr;
+                    if (MODE == kGa) return base[e] + r;
+                    const int q = r / N, n = r - q * N;
+                    const int th = h[e] - p.px.dh[q], tw = w[e] - p.px.dw[q];
+                    if (th < 0 || tw < 0) return nullptr;
+                    const int oh = th / p.px.s, ow = tw / p.px.s;
+                    if (oh * p.px.s != th || ow * p.px.s != tw || oh >= p.px.Ho || ow >= p.px.Wo) return nullptr;
+                    return base[e] + ((size_t)oh * p.px.Wo + ow) * N + n;
+                };
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int m = c0 + 2 * lane + j;
-                const int nb = r0 + wp * RW;
-                const float *src = p.gc + (size_t)min(m, M - 1) * N + nb;
-                if (m < M && p.vec_g && nb + RW <= N) {
+                for (int q = 0; q < NW; ++q) {
+                    const int r = rb + 4 * q;
+                    float2 t[2];
 #pragma unroll
-                    for (int r = 0; r < RW; r += 4) {
-                        const float4 t = *reinterpret_cast<const float4 *>(src + r);
-                        g[r][j] = t.x; g[r + 1][j] = t.y; g[r + 2][j] = t.z; g[r + 3][j] = t.w;
+                    for (int e = 0; e < 2; ++e) {
+                        t[e] = make_float2(0.f, 0.f);
+                        const float *src = src_of(e, r);
+                        if (p.vec_g) {  // N % 4 == 0: both rows share their tap and lie inside one 8-byte vector
+                            if (src) t[e] = *reinterpret_cast<const float2 *>(src);
+                        } else {
+                            if (src) t[e].x = *src;
+                            src = src_of(e, r + 1);
+                            if (src) t[e].y = *src;
+                        }
                     }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < RW; ++r) g[r][j] = (m < M && nb + r < N) ? src[r] : 0.f;
+                    g[2 * (2 * q) + i] = pair(t[0].x, t[1].x);
+                    g[2 * (2 * q + 1) + i] = pair(t[0].y, t[1].y);
                 }
             }
         }
 
-        fetch_chunk(r0, c0, kbeg / KC);
         __syncthreads();  // previous item (or the table staging) is done with every buffer
-        store_chunk((kbeg / KC) & 1);
+        store_stage((kbeg / SC) & 1, 0);
+        if (MODE == kGx && tid < CT) pix_s[tid] = (long long)pixel_class_offset(p.px, min(c0 + tid, CDIM - 1));
+        if (tid == 0) {
+            // fresh barriers for this item: phases restart at 0 (nobody is waiting or arriving here)
+#pragma unroll
+            for (int b = 0; b < 2 * NB; ++b) {
+                if (!first_item) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar_full + 8 * b) : "memory");
+                mbar_init(bar_full + 8 * b, WARPS);
+            }
+        }
+        first_item = false;
         __syncthreads();
-        build(NBUF == 2 ? (kbeg & 1) : 0, (kbeg / KC) & 1, 0);
-        __syncthreads();
+        // unit u = KP consecutive k of one stage, in buffer u % NB; with NB buffers the slabs of unit u + NB - 1 are built
+        // during unit u
+        constexpr int UB = KP * C::U_BYTES;
+        auto build_unit = [&](uint32_t buf, const uint8_t *codes, bool second) {
+            build(buf * UB, codes);
+            if constexpr (KP == 2)
+                if (second) build(buf * UB + C::U_BYTES, codes + CT);
+        };
+#pragma unroll
+        for (int u = 0; u < NB - 1; ++u)
+            if (kbeg + u * KP < kend)
+                build_unit(u, cc_s + ((kbeg / SC) & 1) * C::CC_STAGE + u * KP * CT, kbeg + u * KP + 1 < kend);
+        __syncwarp();
+        // the first units are complete once every warp has arrived; the last buffer starts out released
+        if (lane == 0) {
+#pragma unroll
+            for (int u = 0; u < NB - 1; ++u) mbar_arrive(bar_full + 8 * u);
+            mbar_arrive(bar_empty + 8 * (NB - 1));
+        }
 
         float *obase = p.out + (p.direct ? (size_t)0 : (size_t)tr * K * CDIM);
 
-        for (int k = kbeg; k < kend; ++k) {
-            const int chunk = k / KC, kk = k % KC, stage = chunk & 1;
-            const bool have_next_chunk = (chunk + 1) * KC < kend;
-            if (kk == 0 && have_next_chunk) fetch_chunk(r0, c0, chunk + 1);
-            // Half of the warps (alternating groups of four, so that every scheduler has both kinds) run
-            // the side work - building slab k+1 and combining the partial sums of k-1 - before their gathers,
-            // the other half after them: the dependent shared-memory chains of the side work then overlap
-            // the other group's gather stream instead of all lining up behind the barrier.
-            const bool side_first = (wp >> 2) & 1;
-            auto side_work = [&]() {
-                if (NBUF == 2 && k + 1 < kend) build((k + 1) & 1, ((k + 1) / KC) & 1, (k + 1) % KC);
-                if (NBUF == 2 && k > kbeg) reduce_store(k - 1, obase, c0);
+        const uint32_t uc = u_addr + cq * 8;
+        f32x2 acc[2][2];  // [row parity j][column pair i]
+        // rows of code words [QB, QE) of the warp: the lane's columns of the slab at `ua`, row codes of this k at `rbase`
+        auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag) {
+            constexpr int QB = decltype(qb_tag)::value, QE = decltype(qe_tag)::value, NR = 2 * (QE - QB);
+            constexpr int PF = 4;  // slab reads in flight ahead of their use
+            uint32_t rv[QE - QB];
+            if constexpr (RW % 16 == 0 && QB % 4 == 0 && QE % 4 == 0) {
+#pragma unroll
+                for (int q = 0; q < (QE - QB) / 4; ++q) {
+                    const uint4 t = reinterpret_cast<const uint4 *>(rbase + QB * 4)[q];
+                    rv[4 * q] = t.x; rv[4 * q + 1] = t.y; rv[4 * q + 2] = t.z; rv[4 * q + 3] = t.w;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < QE - QB; ++q) rv[q] = reinterpret_cast<const uint32_t *>(rbase + QB * 4)[q];
+            }
+            uint32_t w0[PF], w1[PF];
+            auto fetch = [&](int i) {  // slab row address = base + 136 * code in one integer dot-product instruction
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w0[i % PF]), "=r"(w1[i % PF])
+                             : "r"(__dp4a(rv[i >> 1], i & 1 ? wsel1 : wsel0, ua)));
             };
-            auto use_phase = [&]() {
-            // use slab k: slab row rc[r,k], two fp32 columns per lane, for this warp's RW rows
-                const uint2 *rp = reinterpret_cast<const uint2 *>(rc_s + stage * C::RC_STAGE + kk * RT + wp * RW);
-                uint32_t rv[RW / 4];
 #pragma unroll
-                for (int q = 0; q < RW / 8; ++q) {
-                    const uint2 t = rp[q];
-                    rv[2 * q] = t.x; rv[2 * q + 1] = t.y;
-                }
-                const uint32_t ub = u_addr + (NBUF == 2 ? (k & 1) : 0) * C::U_BYTES + lane * 8;
-                float s0a = 0.f, s0b = 0.f, s1a = 0.f, s1b = 0.f;
-                float pf0[PF], pf1[PF];
-                auto row_addr = [&](uint32_t v, int i) { return ub + byte_of(v, i) * (US * 4); };
+            for (int i = 0; i < PF && i < NR; ++i) fetch(i);
 #pragma unroll
-                for (int r = 0; r < PF; ++r) {
-                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                                 : "=f"(pf0[r]), "=f"(pf1[r]) : "r"(row_addr(rv[r >> 2], r & 3)));
-                }
-#pragma unroll
-                for (int r = 0; r < RW; ++r) {
-                    const float f0 = pf0[r % PF], f1 = pf1[r % PF];
-                    if (r + PF < RW) {
-                        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                                     : "=f"(pf0[r % PF]), "=f"(pf1[r % PF])
-                                     : "r"(row_addr(rv[(r + PF) >> 2], (r + PF) & 3)));
+            for (int i = 0; i < NR; ++i) {
+                const uint32_t a0 = w0[i % PF], a1 = w1[i % PF];
+                if (i + PF < NR) fetch(i + PF);
+                const int gi = 2 * (2 * QB + i);
+                acc[i & 1][0] = fma2(entries2(a0, bias), g[gi], acc[i & 1][0]);
+                acc[i & 1][1] = fma2(entries2(a1, bias), g[gi + 1], acc[i & 1][1]);
+            }
+        };
+        using Q0 = std::integral_constant<int, 0>;
+        using QH = std::integral_constant<int, NW / 2>;
+        using QN = std::integral_constant<int, NW>;
+        auto clear_acc = [&]() { acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = pack2(0.f, 0.f); };
+        // partial sums of one k: row 2 wp + h, the lane's four columns
+        float *part_lane = part_s + (2 * wp + half) * CT + 4 * cq;
+        auto store_part = [&](int slot) {
+            const float2 lo = unpack2(add2(acc[0][0], acc[1][0])), hi = unpack2(add2(acc[0][1], acc[1][1]));
+            *reinterpret_cast<float4 *>(part_lane + slot * C::P_FLOATS) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        };
+
+        // Unit by unit: read the slabs, release them, then - once every warp has released the unit before, whose buffer
+        // it is - add up that unit's partial sums if it is this warp's turn and build the unit NB - 1 ahead.  With three
+        // buffers each wait has a whole unit of slack, with two (8 bits) the build sits in the middle of the reads.
+        constexpr int AHEAD = NB - 1;
+        constexpr int UNITS = SC / KP;  // per stage
+        static_assert(UNITS > 2 * AHEAD, "the next stage is written while no warp can still be reading it");
+        uint32_t buf = 0, prev = NB - 1, par = 0;  // buffers of this unit and of the one before, parity of this round
+        int stage = (kbeg / SC) & 1, hf = 0;
+        for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
+            const bool more = ks + SC < kend;
+            // the registers are free for the next group once the last stage of the current one is written
+            if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC);
+            const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
+            const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + AHEAD * KP * CT;  // column codes of the unit AHEAD
+#pragma unroll 1
+            for (int it = 0; it < UNITS; ++it) {
+                const int k = ks + KP * it;
+                if (k >= kend) break;
+                const uint32_t ua = uc + buf * UB;
+                clear_acc();
+                mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);  // the slabs of this unit are complete
+                if constexpr (KP == 2) {
+                    use_rows(ua, rb_, Q0{}, QN{});
+                    store_part(buf * KP);
+                    if (k + 1 < kend) {
+                        clear_acc();
+                        use_rows(ua + C::U_BYTES, rb_ + RT, Q0{}, QN{});
+                        store_part(buf * KP + 1);
                     }
-                    if (r & 1) { s0b = fmaf(f0, g[r][0], s0b); s1b = fmaf(f1, g[r][1], s1b); }
-                    else       { s0a = fmaf(f0, g[r][0], s0a); s1a = fmaf(f1, g[r][1], s1a); }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
+                } else {
+                    use_rows(ua, rb_, Q0{}, QH{});
                 }
-                *reinterpret_cast<float2 *>(part_s + (NBUF == 2 ? (k & 1) : 0) * (WARPS * PS) + wp * PS + 2 * lane) =
-                    make_float2(s0a + s0b, s1a + s1b);
-            };
-            if (side_first) { side_work(); use_phase(); } else { use_phase(); side_work(); }
-            if (kk == KC - 2 && have_next_chunk) store_chunk(stage ^ 1);
-            __syncthreads();
-            if (NBUF == 1) {
-                // one slab and one partial-sum buffer: everybody has left slab k, so rebuild it for k+1 and
-                // combine the partial sums of k, then meet again before slab k+1 is read
-                if (k + 1 < kend) build(0, ((k + 1) / KC) & 1, (k + 1) % KC);
-                reduce_store(k, obase, c0);
-                __syncthreads();
+                // (same parity: the last buffer, which unit 0 waits for, starts out released)
+                mbar_wait(bar_empty + 8 * prev, par, 1 + NB + prev, abort_word, p.error_word);
+                if (k > kbeg && ((wp ^ (k - KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
+                    const int i = wp & (KP - 1);
+                    reduce_store(k - KP + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0);
+                }
+                if (k + AHEAD * KP < kend) {
+                    build_unit(prev, cb_, k + AHEAD * KP + 1 < kend);
+                    // the next stage is written before the full arrival of the unit during which its first slab is built
+                    if (it == UNITS - 2 * AHEAD && more) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + 8 * prev);
+                }
+                if constexpr (KP == 1) {
+                    use_rows(ua, rb_, QH{}, QN{});
+                    store_part(buf);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
+                }
+                rb_ += KP * RT;
+                cb_ = it == UNITS - 1 - AHEAD ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
+                prev = buf;
+                if (++buf == NB) { buf = 0; par ^= 1; }
             }
         }
-        if (NBUF == 2) reduce_store(kend - 1, obase, c0);
+        __syncthreads();  // every warp has stored its partial sums of the last unit
+        {
+            const int kl = kend - 1 - (kend - 1 - kbeg) % KP;  // first k of the last unit, in buffer prev
+            const int i = wp & (KP - 1);
+            if (kl + i < kend && ((wp ^ kl) & (WARPS - KP)) == 0)
+                reduce_store(kl + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0);
+        }
     }
 }
 
-}  // namespace sg
+}  // namespace sp
 
-int slab_f32_row_blocks(int rdim) { return (rdim + kSlabF32Rows - 1) / kSlabF32Rows; }
+namespace {
+
+template <int BITS, int MODE, int RW>
+int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStream_t stream) {
+    using C = sp::Cfg<BITS, RW>;
+    auto kern = sp::slab_grad_packed_kernel<BITS, MODE, RW>;
+    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM))) return LUTGEMM_E_CUDA;
+    p.error_word = device_error_word();
+    if (!p.error_word) return LUTGEMM_E_CUDA;
+    p.tiles_r = (p.RDIM + C::RT - 1) / C::RT;
+    p.tiles_c = (p.CDIM + C::CT - 1) / C::CT;
+    p.direct = p.tiles_r == 1;
+    p.out = p.direct ? out : scratch;
+    const long tiles = (long)p.tiles_r * p.tiles_c;
+    const KSplit ks = choose_ksplit(tiles, p.K, num_sms, kPackedItemOverhead);
+    p.ksplits = ks.parts;
+    p.k_per_split = ks.per;
+    const long items = tiles * ks.parts;
+    const int grid = (int)(items < num_sms ? items : num_sms);
+    kern<<<grid, C::THREADS, C::SMEM, stream>>>(p);
+    return launch_status();
+}
+
+template <int BITS, int MODE>
+int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, float *out, const int16_t *lut, int M, int K,
+                       int N, const ConvGeom &conv, float *scratch, const uint8_t *at, int at_pitch, int num_sms,
+                       cudaStream_t stream) {
+    static_assert(sp::Cfg<BITS, 32>::RT == kSlabPackedRows, "tile height");
+    sp::Args p{};
+    p.a = a; p.w = w; p.lut = lut; p.gc = gc; p.M = M; p.K = K; p.N = N;
+    p.RDIM = MODE == sp::kGa ? N : M;
+    p.CDIM = MODE == sp::kGa ? M : N;
+    p.conv = conv;
+    p.at = at;
+    p.at_pitch = at_pitch;
+    p.ga_scatter = (MODE == sp::kGa && conv.enabled) ? 1 : 0;
+    p.vec_a = !conv.enabled && (K % 16 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
+    p.vec_w = (N % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+    p.vec_g = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(gc) & 15) == 0);
+    const int rc = launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+    if (rc != LUTGEMM_OK) return rc;
+    const int tiles_r = slab_packed_row_blocks(p.RDIM);
+    if (tiles_r > 1)
+        return slab_reduce_blocks(scratch, out, K, p.CDIM, tiles_r, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
+                                  kGradFactor, num_sms, stream);
+    return LUTGEMM_OK;
+}
+
+// rows per warp of the grad_x tile (16 warps): 32, or 36 where 576-row tiles leave less padding (576 = 3 x 3 taps of 64
+// channels); a tile costs its rows plus the slab build
+int gx_rows_per_warp(int bits, long rdim) {
+    auto cost = [&](long rt) { return ((rdim + rt - 1) / rt) * (rt + (1L << bits)); };
+    return cost(576) < cost(512) ? 36 : 32;
+}
+
+template <int BITS>
+int launch_packed_gx(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut, int Cout,
+                     const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream) {
+    sp::Args p{};
+    p.a = x; p.w = wmat; p.lut = lut; p.gc = gy;
+    p.M = B * px.Hc * px.Wc; p.K = px.C; p.N = Cout;
+    p.RDIM = px.ntaps * Cout;
+    p.CDIM = p.M;
+    p.px = px;
+    p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
+    p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
+    const int rw = gx_rows_per_warp(BITS, p.RDIM);
+    const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, gx, scratch, num_sms, stream)
+                            : launch_packed<BITS, sp::kGx, 32>(p, gx, scratch, num_sms, stream);
+    if (rc != LUTGEMM_OK) return rc;
+    const int tiles_r = (p.RDIM + 16 * rw - 1) / (16 * rw);
+    if (tiles_r > 1)
+        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, tiles_r, false, nullptr, &px, kGradFactor, num_sms, stream);
+    return LUTGEMM_OK;
+}
+
+}  // namespace
+
+int slab_packed_row_blocks(int rdim) { return (rdim + kSlabPackedRows - 1) / kSlabPackedRows; }
+
+int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
+                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
+                            int at_pitch, int num_sms, cudaStream_t stream) {
+    switch (bits) {
+        case 4: return launch_packed_gemm<4, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
+        case 6: return launch_packed_gemm<6, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
+        case 7: return launch_packed_gemm<7, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
+        case 8: return launch_packed_gemm<8, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
+    }
+    return LUTGEMM_E_BITS;
+}
+
+int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
+                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
+                            cudaStream_t stream) {
+    switch (bits) {
+        case 4: return launch_packed_gemm<4, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
+        case 6: return launch_packed_gemm<6, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
+        case 7: return launch_packed_gemm<7, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
+        case 8: return launch_packed_gemm<8, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
+    }
+    return LUTGEMM_E_BITS;
+}
+
+int gx_tile_rows(int bits, long rdim) { return 16 * gx_rows_per_warp(bits, rdim); }
+
+size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B) {
+    const long rdim = (long)px.ntaps * Cout, rt = 16L * gx_rows_per_warp(bits, rdim);
+    const long tiles_r = (rdim + rt - 1) / rt;
+    return tiles_r > 1 ? (size_t)tiles_r * px.C * ((size_t)B * px.Hc * px.Wc) * sizeof(float) : 0;
+}
+
+int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
+                      int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream) {
+    switch (bits) {
+        case 4: return launch_packed_gx<4>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
+        case 6: return launch_packed_gx<6>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
+        case 7: return launch_packed_gx<7>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
+        case 8: return launch_packed_gx<8>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
+    }
+    return LUTGEMM_E_BITS;
+}
 
 // out[k][c] (TRANSPOSE=false) or out[c][k] (TRANSPOSE=true) = scale * sum_b part[b][k][c], b ascending.
 // PLACE = 1: column c is an unfolded row m of a convolution with non-overlapping windows and (m,k) goes to its
@@ -444,8 +776,48 @@ __global__ void __launch_bounds__(256) slab_reduce_blocks_vec_kernel(const float
     }
 }
 
+// Many blocks of few sums (a convolution's grad_w: M / 512 blocks of K x Cout): the blocks of 32 vectors are shared out
+// over the 16 warps of a CTA in contiguous ranges, and the warps' sums added in ascending order.  One thread per sum
+// and all blocks in a row left most of the GPU idle: 392 blocks of 64 x 256 sums took as long as a tenth of the kernel
+// that made them.
+__global__ void __launch_bounds__(512) slab_reduce_many_kernel(const float *__restrict__ part, float *__restrict__ out,
+                                                               long vecs, int nblocks, float scale) {
+    __shared__ float4 sums[16][32];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int b0 = (int)((long)nblocks * ty / 16), b1 = (int)((long)nblocks * (ty + 1) / 16);
+    const float4 *src = reinterpret_cast<const float4 *>(part);
+    for (long v0 = (long)blockIdx.x * 32; v0 < vecs; v0 += (long)gridDim.x * 32) {
+        const long v = v0 + tx;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v < vecs) {
+#pragma unroll 4
+            for (int b = b0; b < b1; ++b) {
+                const float4 t = src[(size_t)b * vecs + v];
+                s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+            }
+        }
+        sums[ty][tx] = s;
+        __syncthreads();
+        if (ty == 0 && v < vecs) {
+#pragma unroll
+            for (int i = 1; i < 16; ++i) {
+                const float4 t = sums[i][tx];
+                s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+            }
+            reinterpret_cast<float4 *>(out)[v] = make_float4(s.x * scale, s.y * scale, s.z * scale, s.w * scale);
+        }
+        __syncthreads();
+    }
+}
+
 int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks, bool transpose, const ConvGeom *scatter,
                        const PixelClass *px, float scale, int num_sms, cudaStream_t stream) {
+    if (!scatter && !px && !transpose && nblocks >= 16 && (long)K * C % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0 &&
+        (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        const long vecs = (long)K * C / 4, ctas = (vecs + 31) / 32;
+        slab_reduce_many_kernel<<<(int)(ctas < 4L * num_sms ? ctas : 4L * num_sms), 512, 0, stream>>>(part, out, vecs, nblocks, scale);
+        return launch_status();
+    }
     if (!scatter && !px && C % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
         const long vtiles = (long)((K + 31) / 32) * ((C + 127) / 128);
@@ -469,85 +841,6 @@ int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks,
         slab_reduce_blocks_kernel<false, 0><<<rgrid, 256, 0, stream>>>(part, out, K, C, nblocks, scale, pl);
     }
     return launch_status();
-}
-
-template <int BITS, int MODE, int WARPS, int RW, int PF>
-static int launch_slab_grad_w(const float *gc, const uint8_t *a, const uint8_t *w, float *out, const int16_t *lut,
-                            int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                            int at_pitch, int num_sms, cudaStream_t stream) {
-    using C = sg::Cfg<BITS, WARPS, RW>;
-    auto kern = sg::slab_grad_kernel<BITS, MODE, WARPS, RW, PF>;
-    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)))
-        return LUTGEMM_E_CUDA;
-    const int RDIM = MODE == sg::kGa ? N : M, CDIM = MODE == sg::kGa ? M : N;
-    sg::Args p{};
-    p.a = a; p.w = w; p.lut = lut; p.gc = gc; p.M = M; p.K = K; p.N = N;
-    p.conv = conv;
-    p.at = MODE == sg::kGw ? at : nullptr;
-    p.at_pitch = at_pitch;
-    p.ga_scatter = (MODE == sg::kGa && conv.enabled) ? 1 : 0;
-    p.tiles_r = (RDIM + C::RT - 1) / C::RT;
-    p.tiles_c = (CDIM + C::CT - 1) / C::CT;
-    p.direct = p.tiles_r == 1;
-    p.out = p.direct ? out : scratch;
-    p.vec_a = !conv.enabled && (K % 16 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
-    p.vec_w = (N % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
-    p.vec_g = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(gc) & 15) == 0);
-    // cut K so that the persistent grid's last wave is as full as possible (k ranges are multiples of KC)
-    const long tiles = (long)p.tiles_r * p.tiles_c;
-    const int kchunks = (K + C::KC - 1) / C::KC;
-    int ksplits = 1;
-    double best = -1.0;
-    for (int sp = 1; sp <= 16 && sp <= kchunks; ++sp) {
-        const int per = ((kchunks + sp - 1) / sp) * C::KC;
-        if ((K + per - 1) / per != sp) continue;
-        const long it = tiles * sp;
-        const long waves = (it + num_sms - 1) / num_sms;
-        const double eff = (double)it / (double)(waves * num_sms) * (double)per / (double)(per + 8);
-        if (eff > best + 1e-9) { best = eff; ksplits = sp; }
-    }
-    p.ksplits = ksplits;
-    p.k_per_split = ((kchunks + ksplits - 1) / ksplits) * C::KC;
-    const long items = tiles * ksplits;
-    const int grid = (int)(items < num_sms ? items : num_sms);
-    kern<<<grid, C::THREADS, C::SMEM, stream>>>(p);
-    if (launch_status() != LUTGEMM_OK) return LUTGEMM_E_CUDA;
-    if (!p.direct)
-        return slab_reduce_blocks(scratch, out, K, CDIM, p.tiles_r, MODE == sg::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
-                                  kGradFactor, num_sms, stream);
-    return LUTGEMM_OK;
-}
-
-template <int BITS, int MODE>
-static int launch_slab_grad(const float *gc, const uint8_t *a, const uint8_t *w, float *out, const int16_t *lut,
-                            int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                            int at_pitch, int num_sms, cudaStream_t stream) {
-    return launch_slab_grad_w<BITS, MODE, 16, 32, 4>(gc, a, w, out, lut, M, K, N, conv, scratch, at, at_pitch, num_sms,
-                                                     stream);
-}
-
-int backward_gw_slab_f32(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
-                         int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                         int at_pitch, int num_sms, cudaStream_t stream) {
-    switch (bits) {
-        case 4: return launch_slab_grad<4, sg::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 6: return launch_slab_grad<6, sg::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 7: return launch_slab_grad<7, sg::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 8: return launch_slab_grad<8, sg::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-    }
-    return LUTGEMM_E_BITS;
-}
-
-int backward_ga_slab_f32(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
-                         int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
-                         cudaStream_t stream) {
-    switch (bits) {
-        case 4: return launch_slab_grad<4, sg::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 6: return launch_slab_grad<6, sg::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 7: return launch_slab_grad<7, sg::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 8: return launch_slab_grad<8, sg::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-    }
-    return LUTGEMM_E_BITS;
 }
 
 }  // namespace lutgemm

@@ -2,22 +2,12 @@
 //
 //   grad_w:  gw[k,n] = 1/16 * sum_m T(a[m,k], w[k,n]) * gc[m,n]     rows r = m, columns c = n
 //   grad_a:  ga[m,k] = 1/16 * sum_n gc[m,n] * T(a[m,k], w[k,n])     rows r = n, columns c = m
-//   grad_x:  gx[b,c,h,w] = 1/16 * sum_{taps (i,j)} sum_n gy[m(b,h,w,i,j), n] * T(x[b,c,h,w], wmat[(c,i,j), n])
-//            rows r = (tap, n), columns = input pixels, the k loop runs over the input channels c
 //
 // Per k a slab U_k[x][c] = T(x, cc[k,c]) is gathered once, then every row reads slab row rc[r,k] contiguously
 // (conflict-free: with RW = 64 half a warp per row and two fp32 columns per lane in one 64-bit load, otherwise a
 // warp per row and one column per lane) and multiplies it with its grad_out entries held in registers (RW per
 // thread).  The 2^b-row build is paid once per 16*RW rows; two slab buffers, so slab k+1 is built
 // while slab k is read.
-//
-// grad_x is the activation gradient of a convolution WITHOUT the unfolded intermediate: every tap that
-// touches an input pixel sees the same activation code, so the sum over taps joins the sum over n in one
-// long row dimension (kh*kw*Cout rows: 576 for a 3x3 convolution with 64 output channels, which is why the
-// kernel exists with RW = 36 as well), the column codes are the code image itself, the row codes are kh*kw
-// rows of the weight matrix, and the result is written straight into the image gradient - no col2im, no
-// atomics.  A strided convolution is cut into stride^2 classes of input pixels (h mod stride, w mod stride)
-// that each see a fixed subset of the taps; one launch per class.
 //
 // Hand-over between the warps of a CTA: per slab buffer a "full" barrier (all 16 warps have built their part)
 // and an "empty" barrier (all 16 warps have finished reading it), both mbarriers with one arrival per warp.
@@ -28,8 +18,9 @@
 // Partial sums: one per lane, warp and k; the 16 warps are added in ascending order by one warp (rotating
 // with k), row blocks by slab_reduce_blocks in ascending order: results are deterministic.
 // grad_w takes its row codes from a transposed copy at[k][m] of the activation codes when the caller has one.
-// Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492, and for
-// grad_x the unfold backward of self_ops/ops_py/approx_ops.py:556-571.
+// Used at 8 bits, where the slab build weighs most and its 1024 rows halve it (4096^3: 13.53 ms each for grad_w and
+// grad_a, against 15.2 and 15.6 ms with the packed slab of lutgemm_slab_grad.cu), for short K, and for fp32 tables.
+// Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492.
 #include <type_traits>
 
 #include "lutgemm_common.cuh"
@@ -43,7 +34,7 @@
 namespace lutgemm {
 namespace sgt {
 
-enum { kGw = 1, kGa = 2, kGx = 3 };
+enum { kGw = 1, kGa = 2 };
 
 template <int BITS, int RW_>
 struct Cfg {
@@ -79,7 +70,7 @@ struct Args {
     float factor;              // result scale: 1/16 for the 16x fixed-point int16 tables, 1 for fp32 tables
     const float *gc;
     float *out;
-    int M, K, N;               // kGx: M = pixels of the class (all images), K = channels, N = Cout
+    int M, K, N;
     int RDIM, CDIM;
     int tiles_r, tiles_c;
     int ksplits, k_per_split;  // a tile's k range is cut into independent work items (outputs are per k)
@@ -90,7 +81,6 @@ struct Args {
     const uint8_t *at;  // grad_w only, optional: transposed row codes at[k][m], rows at_pitch bytes apart
     int at_pitch;       // a multiple of 16; columns m >= M hold 0
     int *error_word;    // device error word of the bounded waits
-    PixelClass px;      // kGx only
 };
 
 // USE_AT (grad_w only): the row codes come from the transposed copy p.at; the other instantiation keeps the
@@ -108,7 +98,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
     constexpr int PF = BITS == 8 ? 4 : 2;
     // HW: half a warp per slab row and two columns per lane (64-bit slab reads) instead of a warp per row and one
     // column per lane: lanes 0-15 take the first RW/2 rows of the warp, lanes 16-31 the others
-    constexpr bool HW = LUTGEMM_TALL_HALFWARP_ROWS && MODE != kGx && RW == 64 && HANDOVER;
+    constexpr bool HW = LUTGEMM_TALL_HALFWARP_ROWS && RW == 64 && HANDOVER;
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
     constexpr int COL = lut_col_num(BITS);
     static_assert(MODE != kGw || USE_AT || RT % THREADS == 0, "grad_w without a transposed copy: whole rows per thread");
@@ -127,7 +117,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
 
     // ---- stage the gradient table; x = row code, y = column code, T(x,y) = lut[a*COL + w] ----------------
-    // (grad_w: rows are activation codes; grad_a / grad_x: rows are weight codes)
+    // (grad_w: rows are activation codes; grad_a: rows are weight codes)
 #pragma unroll 8
     for (int idx = tid; idx < Q * Q; idx += THREADS) {
         const int hi_idx = idx >> BITS, lo_idx = idx & (Q - 1);  // global read contiguous in lo_idx
@@ -171,31 +161,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
         if (p.vec_w) return *reinterpret_cast<const uint4 *>(src);
         return load16(src, min(16, N - n));
     };
-    // grad_x: row codes of channel k, rows r..r+15 with r = tap*N + n -> weight rows (k*T + t[tap])
-    auto gx_row_codes16 = [&](int k, int r) -> uint4 {
-        if (k >= K || r >= RDIM) return make_uint4(0, 0, 0, 0);
-        int q = r / N, n = r - q * N;
-        if (p.vec_w)  // N % 16 == 0: the 16 rows lie inside one tap
-            return *reinterpret_cast<const uint4 *>(p.w + ((size_t)k * p.px.T + p.px.t[q]) * N + n);
-        uint32_t t[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            if (r + i < RDIM) t[i >> 2] |= (uint32_t)p.w[((size_t)k * p.px.T + p.px.t[q]) * N + n] << (8 * (i & 3));
-            if (++n == N) { n = 0; ++q; }
-        }
-        return make_uint4(t[0], t[1], t[2], t[3]);
-    };
-    // grad_x: the code of pixel column `col` in channels kbase..kbase+15
-    auto gx_col_codes16 = [&](int col, int kbase) -> uint4 {
-        if (col >= CDIM || kbase >= K) return make_uint4(0, 0, 0, 0);
-        const size_t plane = (size_t)p.px.H * p.px.W;
-        const uint8_t *src = p.a + pixel_class_offset(p.px, col) + (size_t)kbase * plane;
-        uint32_t t[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-            if (kbase + q < K) t[q >> 2] |= (uint32_t)src[q * plane] << (8 * (q & 3));
-        return make_uint4(t[0], t[1], t[2], t[3]);
-    };
     auto fetch_group = [&](int r0, int c0, int group) {
         const int kbase = group * KC;
         if (MODE == kGw && USE_AT) {
@@ -219,9 +184,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
                 const int idx = tid + THREADS * j;  // (k, 16-row segment)
                 const int gk = kbase + idx / NSEG, gr = r0 + (idx % NSEG) * 16;
                 if (idx >= KC * NSEG) prc[j] = make_uint4(0, 0, 0, 0);
-                else prc[j] = MODE == kGx ? gx_row_codes16(gk, gr) : w_codes16(gk, gr);
+                else prc[j] = w_codes16(gk, gr);
             }
-            if (tid < CT) pcc = MODE == kGx ? gx_col_codes16(c0 + tid, kbase) : a_codes16(c0 + tid, kbase);
+            if (tid < CT) pcc = a_codes16(c0 + tid, kbase);
         }
     };
     // writes the k range [half*SC, half*SC + SC) of the fetched group to `stage`
@@ -317,9 +282,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
         for (int wv = 1; wv < WARPS; ++wv) v += ps[wv * PS];
         const int col = c0 + lane;
         if (col < CDIM) {
-            if (p.direct && MODE == kGx) {
-                obase[pixel_class_offset(p.px, col) + (size_t)k * p.px.H * p.px.W] = v * p.factor;
-            } else if (p.direct && MODE == kGa) {
+            if (p.direct && MODE == kGa) {
                 if (p.ga_scatter) {
                     const long o = conv_scatter_index(p.conv, col, k);
                     if (o >= 0) obase[o] = v * p.factor;
@@ -384,7 +347,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
                 const int m = r0 + wp * RW + r;
                 g[r] = (m < M && n < N) ? p.gc[(size_t)m * N + n] : 0.f;
             }
-        } else if (MODE == kGa) {
+        } else {
             // g[r] = gc[m = c0 + lane][n = r0 + RW*wp + r]
             const int m = c0 + lane;
             const int nb = r0 + wp * RW;
@@ -398,41 +361,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
             } else {
 #pragma unroll
                 for (int r = 0; r < RW; ++r) g[r] = (m < M && nb + r < N) ? src[r] : 0.f;
-            }
-        } else {
-            // g[r] = gy[m(pixel, tap), n] for row (tap, n) = r0 + RW*wp + r; 0 where the tap leaves the output
-            const int col = c0 + lane;
-            int h = 0, w = 0, b = 0;
-            if (col < CDIM) {
-                const int per = p.px.Hc * p.px.Wc;
-                b = col / per;
-                const int rr = col - b * per, hh = rr / p.px.Wc;
-                h = p.px.ph + p.px.s * hh;
-                w = p.px.pw + p.px.s * (rr - hh * p.px.Wc);
-            }
-            const int rb = r0 + wp * RW;
-            auto row_src = [&](int r) -> const float * {  // &gy[m][n] of row r, or nullptr
-                if (col >= CDIM || r >= RDIM) return nullptr;
-                const int q = r / N, n = r - q * N;
-                const int th = h - p.px.dh[q], tw = w - p.px.dw[q];
-                if (th < 0 || tw < 0) return nullptr;
-                const int oh = th / p.px.s, ow = tw / p.px.s;
-                if (oh * p.px.s != th || ow * p.px.s != tw || oh >= p.px.Ho || ow >= p.px.Wo) return nullptr;
-                return p.gc + ((size_t)(b * p.px.Ho + oh) * p.px.Wo + ow) * N + n;
-            };
-            if (p.vec_g) {  // N % 4 == 0: four consecutive rows share their tap
-#pragma unroll
-                for (int r = 0; r < RW; r += 4) {
-                    const float *src = row_src(rb + r);
-                    const float4 t = src ? *reinterpret_cast<const float4 *>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    g[r] = t.x; g[r + 1] = t.y; g[r + 2] = t.z; g[r + 3] = t.w;
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < RW; ++r) {
-                    const float *src = row_src(rb + r);
-                    g[r] = src ? *src : 0.f;
-                }
             }
         }
 
@@ -618,22 +546,11 @@ int launch_slab_grad_tall(sgt::Args p, float *out, float *scratch, int num_sms, 
     p.tiles_c = (p.CDIM + C::CT - 1) / C::CT;
     p.direct = p.tiles_r == 1;
     p.out = p.direct ? out : scratch;
-    // cut K so that the persistent grid's last wave is as full as possible (k ranges are multiples of 16)
     const long tiles = (long)p.tiles_r * p.tiles_c;
-    const int kchunks = (p.K + C::KC - 1) / C::KC;
-    int ksplits = 1;
-    double best = -1.0;
-    for (int sp = 1; sp <= 16 && sp <= kchunks; ++sp) {
-        const int per = ((kchunks + sp - 1) / sp) * C::KC;
-        if ((p.K + per - 1) / per != sp) continue;
-        const long it = tiles * sp;
-        const long waves = (it + num_sms - 1) / num_sms;
-        const double eff = (double)it / (double)(waves * num_sms) * (double)per / (double)(per + 8);
-        if (eff > best + 1e-9) { best = eff; ksplits = sp; }
-    }
-    p.ksplits = ksplits;
-    p.k_per_split = ((kchunks + ksplits - 1) / ksplits) * C::KC;
-    const long items = tiles * ksplits;
+    const KSplit ks = choose_ksplit(tiles, p.K, num_sms, kTallItemOverhead);
+    p.ksplits = ks.parts;
+    p.k_per_split = ks.per;
+    const long items = tiles * ks.parts;
     const int grid = (int)(items < num_sms ? items : num_sms);
     kern<<<grid, C::THREADS, C::SMEM, stream>>>(p);
     return launch_status();
@@ -667,38 +584,6 @@ int launch_gemm_grad_tall(const float *gc, const uint8_t *a, const uint8_t *w, f
     return LUTGEMM_OK;
 }
 
-// cost of one (k, column tile) step in shared-memory wavefronts: rows read plus the slab build
-long gx_step_cost(int bits, long rdim, int rw) {
-    const long rt = 16L * rw, q = 1L << bits;
-    return ((rdim + rt - 1) / rt) * (rt + (bits == 8 ? 3 * q / 2 : 2 * q));
-}
-
-template <int BITS>
-int launch_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut, int Cout,
-                    const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream) {
-    sgt::Args p{};
-    p.a = x; p.w = wmat; p.lut = lut; p.gc = gy;
-    p.factor = kGradFactor;
-    p.M = B * px.Hc * px.Wc; p.K = px.C; p.N = Cout;
-    p.RDIM = px.ntaps * Cout;
-    p.CDIM = p.M;
-    p.px = px;
-    p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
-    p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
-    int rw = 64;
-    for (int cand : {36, 32})
-        if (gx_step_cost(BITS, p.RDIM, cand) < gx_step_cost(BITS, p.RDIM, rw)) rw = cand;
-    int rc;
-    if (rw == 36) rc = launch_slab_grad_tall<BITS, sgt::kGx, 36>(p, gx, scratch, num_sms, stream);
-    else if (rw == 32) rc = launch_slab_grad_tall<BITS, sgt::kGx, 32>(p, gx, scratch, num_sms, stream);
-    else rc = launch_slab_grad_tall<BITS, sgt::kGx, 64>(p, gx, scratch, num_sms, stream);
-    if (rc != LUTGEMM_OK) return rc;
-    const int tiles_r = (p.RDIM + 16 * rw - 1) / (16 * rw);
-    if (tiles_r > 1)
-        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, tiles_r, false, nullptr, &px, kGradFactor, num_sms, stream);
-    return LUTGEMM_OK;
-}
-
 }  // namespace
 
 void slab_tall_set_handover(bool on) { g_tall_handover = on; }
@@ -723,26 +608,6 @@ int backward_ga_slab_tall(const float *gc, const uint8_t *a, const uint8_t *w, f
         case 6: return launch_gemm_grad_tall<6, sgt::kGa>(gc, a, w, ga, lut_ga, lut_f32, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
         case 7: return launch_gemm_grad_tall<7, sgt::kGa>(gc, a, w, ga, lut_ga, lut_f32, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
         case 8: return launch_gemm_grad_tall<8, sgt::kGa>(gc, a, w, ga, lut_ga, lut_f32, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-    }
-    return LUTGEMM_E_BITS;
-}
-
-size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B) {
-    const long rdim = (long)px.ntaps * Cout;
-    int rw = 64;
-    for (int cand : {36, 32})
-        if (gx_step_cost(bits, rdim, cand) < gx_step_cost(bits, rdim, rw)) rw = cand;
-    const long tiles_r = (rdim + 16L * rw - 1) / (16L * rw);
-    return tiles_r > 1 ? (size_t)tiles_r * px.C * ((size_t)B * px.Hc * px.Wc) * sizeof(float) : 0;
-}
-
-int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
-                      int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream) {
-    switch (bits) {
-        case 4: return launch_gx_class<4>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
-        case 6: return launch_gx_class<6>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
-        case 7: return launch_gx_class<7>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
-        case 8: return launch_gx_class<8>(gy, x, wmat, gx, lut_ga, Cout, px, B, scratch, num_sms, stream);
     }
     return LUTGEMM_E_BITS;
 }

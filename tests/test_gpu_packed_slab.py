@@ -1,0 +1,154 @@
+"""GPU tests of the packed-slab gradient kernels (512 x 64 tiles, 576 x 64 for grad_x) at the sizes where they can go
+wrong - remainders of tiles, of the two-k slab buffers and of the 16-k operand stages - with tables over the whole int16
+range, and of what the dispatcher does when a caller's scratch buffer is too small for the faster kernel.
+
+Tolerance: an fp32 sum of n terms in any order is off by at most about n * 2^-24 times the sum of the absolute terms, and
+the kernels add at most 16 terms per accumulator, 32 accumulators and the row blocks in turn (fewer than 100 additions in
+a chain, 6e-6); 1e-5 of the sum of the absolute terms is what every gradient test here allows."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle_np as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.fail("gpu-marked test started without a CUDA device")
+    import approx_ops
+    approx_ops.library()
+    return torch.device("cuda:0")
+
+
+@pytest.fixture
+def packed():
+    import approx_ops
+    approx_ops.set_kernel_choice(backward="slab", grad_tile="wide")
+    yield
+    approx_ops.set_kernel_choice()
+
+
+def full_range_tables(bits, seed):
+    rng = np.random.default_rng(seed)
+    q = 1 << bits
+    out = []
+    for _ in range(2):
+        t = rng.integers(-2 ** 15, 2 ** 15, (q, q))
+        t[0, 0], t[q - 1, q - 1], t[0, q - 1], t[q - 1, 0] = -2 ** 15, 2 ** 15 - 1, 0, -1
+        out.append(O.pack_padded(t, bits, np.int16))
+    return out
+
+
+def problem(bits, M, K, N, seed):
+    rng = np.random.default_rng(seed)
+    q = 1 << bits
+    a, w = rng.integers(0, q, (M, K)).astype(np.uint8), rng.integers(0, q, (K, N)).astype(np.uint8)
+    return a, w, rng.standard_normal((M, N)).astype(np.float32)
+
+
+def backward(dev, gc, a, w, la, lw):
+    import approx_ops
+    ga = torch.full(a.shape, float("nan"), dtype=torch.float32, device=dev)
+    gw = torch.full(w.shape, float("nan"), dtype=torch.float32, device=dev)
+    t = [torch.from_numpy(x).to(dev) for x in (gc, a, w, la, lw)]
+    approx_ops.approx_gemm_backward(t[0], t[1], t[2], ga, gw, t[3], t[4])
+    torch.cuda.synchronize()
+    assert approx_ops.device_error() == 0
+    return ga.cpu().numpy(), gw.cpu().numpy()
+
+
+def check(got, ref, refabs):
+    assert np.isfinite(got).all()
+    assert (np.abs(got - ref) <= TOL * refabs + 1e-30).all()
+
+
+@pytest.mark.parametrize("bits", [4, 6, 7, 8])
+@pytest.mark.parametrize("M,K,N", [(511, 1, 65), (512, 2, 64), (513, 3, 63), (70, 15, 513), (530, 16, 130), (1030, 17, 40),
+                                   (33, 33, 1100), (600, 47, 66), (20000, 9, 12), (20000, 7, 5)])
+def test_gradients_at_the_edges_of_tiles_and_stages(dev, oracle_c, packed, bits, M, K, N):
+    """(The last two have 40 row blocks: the many-block reduction with and without 16-byte vectors.)"""
+    la, lw = full_range_tables(bits, 3 * bits)
+    a, w, gc = problem(bits, M, K, N, bits + M + K + N)
+    ga, gw = backward(dev, gc, a, w, la, lw)
+    r_ga, r_gw, r_gaa, r_gwa = oracle_c.backward_f64(gc, a, w, la, lw, bits)
+    check(ga, r_ga, r_gaa)
+    check(gw, r_gw, r_gwa)
+
+
+@pytest.mark.parametrize("bits", [4, 6, 7, 8])
+@pytest.mark.parametrize("B,Cin,H,Cout,k,st,p", [(1, 5, 9, 64, 3, 1, 1), (2, 33, 6, 128, 3, 1, 1), (1, 18, 7, 63, 3, 1, 1),
+                                                 (1, 16, 9, 256, 3, 2, 1)])
+def test_image_gradient_of_convolutions(dev, oracle_c, packed, bits, B, Cin, H, Cout, k, st, p):
+    """576-row tiles (one and two of them, and a partly filled one) and the stride classes of a stride-2 convolution."""
+    import approx_ops
+    la, lw = full_range_tables(bits, 5 * bits)
+    rng = np.random.default_rng(bits + Cin + Cout)
+    q = 1 << bits
+    x = rng.integers(0, q, (B, Cin, H, H)).astype(np.uint8)
+    wmat = rng.integers(0, q, (Cin * k * k, Cout)).astype(np.uint8)
+    Ho = (H + 2 * p - k) // st + 1
+    gy = rng.standard_normal((B * Ho * Ho, Cout)).astype(np.float32)
+    col = oracle_c.im2col(x, k, k, st, p, 1)
+    gx = torch.full(x.shape, float("nan"), dtype=torch.float32, device=dev)
+    gw = torch.full(wmat.shape, float("nan"), dtype=torch.float32, device=dev)
+    t = [torch.from_numpy(v).to(dev) for v in (gy, x, wmat, la, lw)]
+    approx_ops.approx_conv2d_backward(t[0], t[1], t[2], gx, gw, t[3], t[4], k, k, st, p, 1)
+    r_ga, r_gw, r_gaa, r_gwa = oracle_c.backward_f64(gy, col, wmat, la, lw, bits)
+    check(gw.cpu().numpy(), r_gw, r_gwa)
+    check(gx.cpu().numpy(), O.col2im_f64(r_ga, x.shape, k, k, st, p, 1), O.col2im_f64(r_gaa, x.shape, k, k, st, p, 1))
+
+
+@pytest.mark.parametrize("bits", [6, 7, 8])
+def test_a_small_scratch_buffer_selects_a_kernel_that_fits(dev, oracle_c, bits):
+    """A buffer that the choice by fixed limits can work with is not refused: the gradients are then computed by its
+    kernels.  Without a buffer the broadcast kernels, which need none here, run."""
+    import approx_ops
+    lib = approx_ops.library()
+    la, lw = full_range_tables(bits, 7 * bits)
+    M, K, N = 300, 200, 600  # slab kernels by estimated time; M < 512 and N < 768: broadcast kernels by fixed limits
+    a, w, gc = problem(bits, M, K, N, bits)
+    assert lib.lutgemm_backward_scratch_bytes(bits, M, K, N) > 0
+    ga, gw = (torch.full(s, float("nan"), dtype=torch.float32, device=dev) for s in (a.shape, w.shape))
+    t = [torch.from_numpy(v).to(dev) for v in (gc, a, w, la, lw)]
+    rc = lib.lutgemm_backward(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), ga.data_ptr(), gw.data_ptr(), t[3].data_ptr(),
+                              t[4].data_ptr(), bits, M, K, N, None, 0, None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    r_ga, r_gw, r_gaa, r_gwa = oracle_c.backward_f64(gc, a, w, la, lw, bits)
+    check(ga.cpu().numpy(), r_ga, r_gaa)
+    check(gw.cpu().numpy(), r_gw, r_gwa)
+    # 4096 rows, the weight gradient by a slab kernel under either choice: a buffer below both needs is refused
+    M = 4096
+    if bits >= 7:
+        rc = lib.lutgemm_backward(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), ga.data_ptr(), gw.data_ptr(), t[3].data_ptr(),
+                                  t[4].data_ptr(), bits, M, K, N, ga.data_ptr(), 16, None)
+        assert rc == -4  # LUTGEMM_E_SCRATCH, before anything is launched
+
+
+@pytest.mark.parametrize("bits", [6, 7, 8])
+def test_image_gradient_without_scratch(dev, oracle_c, bits):
+    import approx_ops
+    lib = approx_ops.library()
+    la, lw = full_range_tables(bits, 9 * bits)
+    B, Cin, H, Cout, k = 1, 64, 8, 256, 3
+    assert lib.lutgemm_conv2d_backward_scratch_bytes(bits, B, Cin, H, H, Cout, k, k, 1, 1, 1) > 0
+    rng = np.random.default_rng(bits)
+    x = rng.integers(0, 1 << bits, (B, Cin, H, H)).astype(np.uint8)
+    wmat = rng.integers(0, 1 << bits, (Cin * k * k, Cout)).astype(np.uint8)
+    gy = rng.standard_normal((B * H * H, Cout)).astype(np.float32)
+    gx = torch.full(x.shape, float("nan"), dtype=torch.float32, device=dev)
+    t = [torch.from_numpy(v).to(dev) for v in (gy, x, wmat, la)]
+    rc = lib.lutgemm_conv2d_backward(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), gx.data_ptr(), None, t[3].data_ptr(), None,
+                                     bits, B, Cin, H, H, Cout, k, k, 1, 1, 1, ctypes.c_void_p(None), 0, None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    col = oracle_c.im2col(x, k, k, 1, 1, 1)
+    r_ga, _, r_gaa, _ = oracle_c.backward_f64(gy, col, wmat, la, lw, bits)
+    check(gx.cpu().numpy(), O.col2im_f64(r_ga, x.shape, k, k, 1, 1, 1), O.col2im_f64(r_gaa, x.shape, k, k, 1, 1, 1))
