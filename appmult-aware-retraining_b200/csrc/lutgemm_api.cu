@@ -64,7 +64,8 @@ struct BackwardPlan {
 // Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
 // The clocks are measured on B200, at 4096^3 unless said otherwise:
 //   slab kernels, per k and tile      packed 512 x 64: 1540 (4 and 6 bits), 1560 (7), 2180 (8); tall 1024 x 32: 1540, 1690, 1880;
-//                                     forward 512 x 64: 1000, 1100, 1330 and 40e3 / 55e3 at the start (code transposition)
+//                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
+//                                     more launches: code transposition, zeroing, and a layer's epilogue)
 //   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
 //                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.7, 1.9, 2.8
 // A slab kernel's time does not depend on the codes and it can cut K into many work items; a broadcast kernel has no slab
@@ -75,11 +76,11 @@ struct FamilyClocks {
     double packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {2180, 1880, 1330, 3.1, 3.3, 4.2, 2.8, 55e3};
-    if (bits == 7) return {1560, 1690, 1100, 2.33, 2.4, 2.6, 1.9, 40e3};
-    return {1540, 1540, 1000, 1.48, 1.6, 1.6, 1.7, 40e3};
+    if (bits == 8) return {2180, 1880, 1330, 3.1, 3.3, 4.2, 2.8, 75e3};
+    if (bits == 7) return {1560, 1690, 940, 2.33, 2.4, 2.6, 1.9, 60e3};
+    return {1540, 1540, 905, 1.48, 1.6, 1.6, 1.7, 60e3};
 }
-constexpr double kBcastStart = 12e3, kSlabStart = 5e3;
+constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
 
 long div_up(long a, long b) { return (a + b - 1) / b; }
@@ -145,21 +146,24 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms) {
 // Choice by estimated time.  A convolution's grad_a (non-overlapping windows) gathers its column codes from the image and
 // writes in place; there the slab kernels pay from N = 768 on (1x1, 128 -> 512 channels, 7 bits: 0.75 against 0.68 ms; 1024 -> 512:
 // 1.24 against 1.22 ms).  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
-BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv) {
+// (want_gw, want_ga: the gradients that are asked for; the plan of the other one is left empty)
+BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bool want_gw, bool want_ga) {
     BackwardPlan pl{};
-    const double gw_p = packed_clocks(bits, M, N, K, sms), gw_t = tall_clocks(bits, M, N, K, sms);
-    const double ga_p = packed_clocks(bits, N, M, K, sms), ga_t = tall_clocks(bits, N, M, K, sms);
-    pl.gw_slab = (gw_p < gw_t ? gw_p : gw_t) < gw_bcast_clocks(bits, M, K, N, sms);
-    pl.ga_slab = (!conv || N >= 768) && (ga_p < ga_t ? ga_p : ga_t) < ga_bcast_clocks(bits, M, K, N, sms);
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
-    if (force == LUTGEMM_BACKWARD_BCAST) pl.gw_slab = pl.ga_slab = false;
-    if (force == LUTGEMM_BACKWARD_SLAB) pl.gw_slab = pl.ga_slab = true;
-    pl.gw_tall = pl.gw_slab && gw_t < gw_p;
-    pl.ga_tall = pl.ga_slab && ga_t < ga_p;
-    if (tile == LUTGEMM_TILE_WIDE) pl.gw_tall = pl.ga_tall = false;
-    if (tile == LUTGEMM_TILE_TALL) { pl.gw_tall = pl.gw_slab; pl.ga_tall = pl.ga_slab; }
-    set_gw_scratch(pl, bits, M, K, N, sms);
-    set_ga_scratch(pl, M, K, N);
+    if (want_gw) {
+        const double packed = packed_clocks(bits, M, N, K, sms), tall = tall_clocks(bits, M, N, K, sms);
+        pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
+        if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
+        pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
+        set_gw_scratch(pl, bits, M, K, N, sms);
+    }
+    if (want_ga) {
+        const double packed = packed_clocks(bits, N, M, K, sms), tall = tall_clocks(bits, N, M, K, sms);
+        pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
+        if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
+        pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
+        set_ga_scratch(pl, M, K, N);
+    }
     return pl;
 }
 
@@ -318,7 +322,7 @@ size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false);
+    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false, true, true);
     return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch;
 }
 
@@ -337,7 +341,7 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t given = scratch ? scratch_bytes : 0;
-    BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0);
+    BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0, gw != nullptr, ga != nullptr);
     if ((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) pl = base_plan(bits, M, K, N, sms);
     float *sc = static_cast<float *>(scratch);
     if (gw) {
@@ -552,7 +556,7 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     const int M = g.B * g.Ho * g.Wo, K = g.C * g.kh * g.kw;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true).ga_scratch;
+    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true).ga_scratch;
     size_t need = 0;
     if (gx_uses_slab(bits, g, Cout, sms))
         for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
@@ -571,7 +575,7 @@ size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int 
     if (sms <= 0) return 0;
     const int M = B * g.Ho * g.Wo, K = C * kh * kw;
     // the weight-gradient and the activation-gradient kernels run one after the other on the same buffer
-    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true).gw_scratch;
+    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false).gw_scratch;
     const size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
     return gw_need > gx_need ? gw_need : gx_need;
 }

@@ -41,24 +41,28 @@ int slab_fwd_ksplits(int M, int K, int N, int num_sms);
 
 // How a slab kernel cuts K (outputs are per k, so the parts are independent work items): the number of parts and the k
 // per part (a multiple of 16) for which a persistent grid of num_sms CTAs finishes first, when an item of `per` k costs
-// per + item_overhead steps.  Up to 64 parts, so that few tiles still fill the GPU.
+// per + item_overhead steps.  Up to 64 parts, so that few tiles still fill the GPU; beyond 12 items per CTA another part
+// gains less than 1 / 12, and the search (a microsecond of host time per call) ends.
 struct KSplit {
     int parts, per;
     long waves;
 };
 inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
-    const int chunks = (K + 15) / 16;
-    KSplit best{1, chunks * 16, (tiles + num_sms - 1) / num_sms};
+    const unsigned chunks = (unsigned)(K + 15) / 16, sms = (unsigned)num_sms;
+    KSplit best{1, (int)chunks * 16, (tiles + num_sms - 1) / num_sms};
     long cost = best.waves * (best.per + item_overhead);
-    for (int s = 2; s <= 64 && s <= chunks; ++s) {
-        const int per = ((chunks + s - 1) / s) * 16;
-        if ((K + per - 1) / per != s) continue;
-        const long waves = (tiles * s + num_sms - 1) / num_sms, c = waves * (per + item_overhead);
-        if (c < cost) { cost = c; best = KSplit{s, per, waves}; }
+    unsigned last = chunks;
+    for (unsigned s = 2; s <= 64 && s <= chunks && tiles * s <= 12L * num_sms; ++s) {
+        const unsigned per = (chunks + s - 1) / s;  // in chunks
+        if (per == last) continue;                  // more parts of the same length: some would get no work
+        last = per;
+        const unsigned parts = (chunks + per - 1) / per, waves = ((unsigned)tiles * parts + sms - 1) / sms;
+        const long c = (long)waves * (16 * per + item_overhead);
+        if (c < cost) { cost = c; best = KSplit{(int)parts, (int)per * 16, (long)waves}; }
     }
     return best;
 }
-constexpr int kPackedItemOverhead = 12, kTallItemOverhead = 8;  // in k steps: operand fetch, grad_out block, first slabs
+constexpr int kPackedItemOverhead = 16, kTallItemOverhead = 8;  // in k steps: operand fetch, grad_out block, first slabs
 
 // rows of the reduction dimension per CTA tile of the packed-slab gradient kernels, and the block count
 constexpr int kSlabPackedRows = 512;

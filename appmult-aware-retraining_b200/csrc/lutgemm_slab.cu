@@ -11,14 +11,12 @@
 //
 // The use-phase read is uniform in x and contiguous in n: half a warp reads one slab row, one 64-bit shared load
 // per lane returns four adjacent uint16 entries (four columns), conflict-free by construction - 64 table
-// look-ups per shared-memory wavefront instead of ~11, and two rows per load instruction.  The build reads the table transposed and paired ([w][x],
-// codes x and x + 2^b/2 in one word) with conflict-free 32-bit loads and writes slab rows (stride 34
+// look-ups per shared-memory wavefront instead of ~11, and two rows per load instruction.  The build reads the table
+// transposed ([w][x], conflict-free, all of a lane's codes of one column in one load) and writes slab rows (stride 34
 // words) with conflict-free 64-bit stores: 2^b * 2 wavefronts per k against 512 for the use phase.
-// Two slab buffers: slab k+1 is built while slab k is read, one CTA barrier per k.  (Handing the buffers over
-// through per-buffer mbarriers, as the gradient kernels do, does not pay here: with polling waits it was slower -
-// 11.5 against 10.7 ms at 8 bits for 4096^3 - and with suspending waits 10.38 against 10.42 ms at 8 bits, 8.63
-// against 8.68 ms at 7 bits, 8.35 against 7.69 ms at 6 bits: the forward's read phase per k is half as long as
-// the gradients'.)
+// At 7 bits and below three buffers of two slabs each are handed over through mbarriers; at 8 bits shared memory has room
+// for two slabs only: slab k+1 is built while slab k is read, one CTA barrier per k (mbarriers do not pay there: 10.38
+// against 10.42 ms for 4096^3).
 // The two halves of a slab word go to the accumulators as  S += word,  H += word >> 16 ; at the end
 // sum(lo) = S - (H << 16) (mod 2^32) and sum(hi) = H.
 // Work items are (tile, k range): whole tiles where they fill the persistent grid's waves, otherwise every CTA
@@ -41,31 +39,31 @@
 #include "lutgemm_tma.cuh"
 #include "lutgemm_waits.cuh"
 
-#ifndef LUTGEMM_FWD_HALFWARP_ROWS
-#define LUTGEMM_FWD_HALFWARP_ROWS 1
-#endif
-
 namespace lutgemm {
 namespace sf {
 
 template <int BITS>
 struct Cfg {
     static constexpr int Q = 1 << BITS;
-    static constexpr int HALF = Q / 2;          // words per transposed-table row (two codes per word)
-    static constexpr int TT_STRIDE = HALF + 1;  // words; +1 keeps the transposing stage conflict-free
+    static constexpr int E = Q >= 32 ? Q / 32 : 1;  // codes per lane in the build: x = lane + 32 j, j < E
+    static constexpr int TT_ROW = table_row_bytes<BITS>();  // table row of a column code
+    static constexpr int KP = BITS == 8 ? 1 : 2;    // slabs per buffer
+    static constexpr int NB = BITS == 8 ? 2 : 3;    // buffers (shared memory has no room for more at 8 bits)
     static constexpr int THREADS = 512;
     static constexpr int RT = 512;              // rows per CTA tile: 32 per warp
     static constexpr int CT = 64;               // columns per CTA tile: 2 per lane
     static constexpr int KC = 16;               // k per operand stage
     static constexpr int U_STRIDE = 34;         // words per slab row (32 + 2 pad: 8-byte aligned rows)
-    static constexpr int TT_BYTES = (Q * TT_STRIDE * 4 + 127) & ~127;  // the stages behind it are TMA destinations
+    static constexpr int TT_BYTES = (Q * TT_ROW + 127) & ~127;  // the stages behind it are TMA destinations
     static constexpr int U_BYTES = Q * U_STRIDE * 4;
     static constexpr int RC_STAGE = KC * RT;   // [half][kk][256]: two boxes of 16 k x 256 rows
     static constexpr int CC_STAGE = KC * CT;   // [kk][64]
-    static constexpr int OFF_BAR = TT_BYTES + 2 * U_BYTES + 2 * RC_STAGE + 2 * CC_STAGE;
-    static constexpr int SMEM = OFF_BAR + 2 * 8 + 16;  // one mbarrier per stage and the abort word
+    static constexpr int OFF_RC = TT_BYTES + NB * KP * U_BYTES;
+    static constexpr int OFF_BAR = OFF_RC + 2 * RC_STAGE + 2 * CC_STAGE;
+    // one mbarrier per stage, a full and an empty one per slab buffer, and the abort word
+    static constexpr int SMEM = OFF_BAR + 2 * 8 + 2 * NB * 8 + 16;
     static_assert(U_BYTES % 128 == 0 && RC_STAGE % 128 == 0 && CC_STAGE % 128 == 0, "TMA destinations are 128-byte aligned");
-    static constexpr int NSETS = HALF > 32 ? HALF / 32 : 1;
+    static_assert(SMEM <= 232448, "shared memory budget");
 };
 
 struct Args {
@@ -95,37 +93,34 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
                                                           const __grid_constant__ CUtensorMap map_w) {
     static_assert(!TMA || USE_AT, "bulk-tensor operand loads read the transposed copy");
     using C = Cfg<BITS>;
-    constexpr int Q = C::Q, HALF = C::HALF, TTS = C::TT_STRIDE, RT = C::RT, CT = C::CT, KC = C::KC;
-    constexpr int US = C::U_STRIDE, THREADS = C::THREADS, NSETS = C::NSETS;
+    constexpr int Q = C::Q, E = C::E, RT = C::RT, CT = C::CT, KC = C::KC, KP = C::KP, NB = C::NB;
+    constexpr int US = C::U_STRIDE, THREADS = C::THREADS;
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
     constexpr int COL = lut_col_num(BITS);
-    constexpr bool HW = LUTGEMM_FWD_HALFWARP_ROWS != 0;  // half a warp per slab row in the use phase (64-bit reads)
     const int M = p.M, K = p.K, N = p.N;
 
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t *rc_s = smem + C::TT_BYTES + 2 * C::U_BYTES;
+    uint8_t *rc_s = smem + C::OFF_RC;
     uint8_t *cc_s = rc_s + 2 * C::RC_STAGE;
     const uint32_t tt_addr = smem_u32(smem);
     const uint32_t u_addr = smem_u32(smem + C::TT_BYTES);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const uint32_t bar_stage = smem_u32(smem + C::OFF_BAR);  // TMA: one barrier per operand stage
-    volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 16);
+    volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 16 + 16 * NB);
+    const uint32_t bar_full = bar_stage + 16, bar_empty = bar_full + 8 * NB;  // KP == 2: slab buffers
     uint32_t stage_phase = 0;                                 // TMA: bit s = parity of the next completion of stage s
+    if (tid == 0) *abort_word = 0;
     if (TMA && tid == 0) {
-        *abort_word = 0;
         mbar_init(bar_stage, 1);
         mbar_init(bar_stage + 8, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");  // visible to the copy engine
     }
 
-    // ---- stage the table transposed and paired: tt[w][i] = { LUT[i][w], LUT[i + HALF][w] } ---------------
-    {
-        uint16_t *tt16 = reinterpret_cast<uint16_t *>(smem);
+    // ---- stage the table transposed: row w holds LUT[x][w], a lane's codes side by side ------------------
 #pragma unroll 8
-        for (int idx = tid; idx < Q * Q; idx += THREADS) {
-            const int x = idx >> BITS, y = idx & (Q - 1);  // global read contiguous in y
-            tt16[(y * TTS + (x & (HALF - 1))) * 2 + (x >> (BITS - 1))] = p.lut[x * COL + y];
-        }
+    for (int idx = tid; idx < Q * Q; idx += THREADS) {
+        const int x = idx >> BITS, y = idx & (Q - 1);  // global read contiguous in y
+        *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + table_pos<BITS>(x) * 2) = p.lut[x * COL + y];
     }
 
     // ---- operand chunk staging: rc_s[stage][kk][m] (512 activation codes per k), cc_s[stage][kk][n] -----
@@ -136,6 +131,15 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
         for (int q = 0; q < 16; ++q)
             if (q < valid) t[q >> 2] |= (uint32_t)src[q] << (8 * (q & 3));
         return make_uint4(t[0], t[1], t[2], t[3]);
+    };
+    auto fetch_cols = [&](int n0, int chunk) {
+        const int kbase = chunk * KC;
+        if (tid < KC * CT / 16) {
+            const int gk = kbase + tid / (CT / 16), gn = n0 + (tid % (CT / 16)) * 16;
+            if (gk >= K || gn >= N) pcc = make_uint4(0, 0, 0, 0);
+            else if (p.vec_w) pcc = *reinterpret_cast<const uint4 *>(p.w + (size_t)gk * N + gn);
+            else pcc = load16(p.w + (size_t)gk * N + gn, min(16, N - gn));
+        }
     };
     auto fetch_chunk = [&](int m0, int n0, int chunk) {
         const int kbase = chunk * KC;
@@ -149,12 +153,12 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
         else if (p.conv.enabled) prc = conv_code16(p.a, p.conv, m, kbase, K);
         else if (p.vec_a) prc = *reinterpret_cast<const uint4 *>(p.a + (size_t)m * K + kbase);
         else prc = load16(p.a + (size_t)m * K + kbase, min(16, K - kbase));
-        if (tid < KC * CT / 16) {
-            const int gk = kbase + tid / (CT / 16), gn = n0 + (tid % (CT / 16)) * 16;
-            if (gk >= K || gn >= N) pcc = make_uint4(0, 0, 0, 0);
-            else if (p.vec_w) pcc = *reinterpret_cast<const uint4 *>(p.w + (size_t)gk * N + gn);
-            else pcc = load16(p.w + (size_t)gk * N + gn, min(16, N - gn));
-        }
+        fetch_cols(n0, chunk);
+    };
+    auto store_cols = [&](int stage) {
+        if (tid < KC * CT / 16)
+            *reinterpret_cast<uint4 *>(cc_s + stage * C::CC_STAGE + (tid / (CT / 16)) * CT + (tid % (CT / 16)) * 16) =
+                make_uint4(pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4);
     };
     auto store_chunk = [&](int stage) {
         // codes are masked to BITS bits here, once, so no stray code can index outside a slab or the table
@@ -167,39 +171,28 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
 #pragma unroll
             for (int q = 0; q < 16; ++q) rs[rc_off(q, tid)] = (uint8_t)(tr[q >> 2] >> (8 * (q & 3)));
         }
-        if (tid < KC * CT / 16)
-            *reinterpret_cast<uint4 *>(cc_s + stage * C::CC_STAGE + (tid / (CT / 16)) * CT + (tid % (CT / 16)) * 16) =
-                make_uint4(pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4);
+        store_cols(stage);
     };
-    // build slab `buf` for the k that sits at (stage, kk): warp wp fills column pairs 2wp and 2wp+1
-    auto build = [&](int buf, int stage, int kk) {
-        const uint32_t cw = *reinterpret_cast<const uint32_t *>(cc_s + stage * C::CC_STAGE + kk * CT + wp * 4);
-        const uint32_t ub = u_addr + buf * C::U_BYTES + wp * 8;  // this warp's four columns: words 2wp and 2wp+1
+    // build the slab at byte offset `off` from the column codes of one k: warp wp fills column pairs 2wp and 2wp+1.  Lane l
+    // reads the entries of codes l + 32 j of each column and stores four columns of one code at a time; all
+    // table reads of the warp's share are issued before its first store (the stores order later reads behind them).
+    const uint32_t tt_lane = tt_addr + lane * table_lane_bytes<BITS>();
+    const uint32_t us = u_addr + wp * 8 + lane * (US * 4);
+    auto build = [&](uint32_t off, const uint8_t *codes) {
+        const uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + wp * 4);
         // (chunks that arrive by bulk copy have not been through the masking store: cut the codes to BITS bits here)
         const uint32_t cwm = TMA ? (cw & MASK4) : cw;
-        const uint32_t y0 = byte_of(cwm, 0), y1 = byte_of(cwm, 1), y2 = byte_of(cwm, 2), y3 = byte_of(cwm, 3);
-        // all table reads of the warp's share are issued before its first store (the stores order later reads behind
-        // them)
-        uint32_t r0[NSETS], r1[NSETS], r2[NSETS], r3[NSETS];
+        constexpr int EW = (E + 1) / 2;  // table words per lane and column
+        uint32_t r[4][EW];
+        if (Q >= 32 || lane < Q) {
 #pragma unroll
-        for (int j = 0; j < NSETS; ++j) {
-            const int i = lane + 32 * j;
-            if (HALF >= 32 || i < HALF) {
-                r0[j] = lds_u32(tt_addr + (y0 * TTS + i) * 4);
-                r1[j] = lds_u32(tt_addr + (y1 * TTS + i) * 4);
-                r2[j] = lds_u32(tt_addr + (y2 * TTS + i) * 4);
-                r3[j] = lds_u32(tt_addr + (y3 * TTS + i) * 4);
-            }
-        }
+            for (int c = 0; c < 4; ++c) load_table_entries<BITS>(tt_lane + byte_of(cwm, c) * C::TT_ROW, r[c]);
 #pragma unroll
-        for (int j = 0; j < NSETS; ++j) {
-            const int i = lane + 32 * j;
-            if (HALF >= 32 || i < HALF) {
-                // { LUT[i][y0], LUT[i][y1] }, { LUT[i][y2], LUT[i][y3] } and the same for code i + HALF
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + i * (US * 4)), "r"(__byte_perm(r0[j], r1[j], 0x5410)),
-                             "r"(__byte_perm(r2[j], r3[j], 0x5410)) : "memory");
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + (i + HALF) * (US * 4)),
-                             "r"(__byte_perm(r0[j], r1[j], 0x7632)), "r"(__byte_perm(r2[j], r3[j], 0x7632)) : "memory");
+            for (int j = 0; j < E; ++j) {
+                const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(us + off + j * 32 * (US * 4)),
+                             "r"(__byte_perm(r[0][j / 2], r[1][j / 2], sel)), "r"(__byte_perm(r[2][j / 2], r[3][j / 2], sel))
+                             : "memory");
             }
         }
     };
@@ -229,6 +222,7 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
     const long total_chunks = (long)p.tiles_r * p.tiles_c * kchunks;
     long cur = p.share ? total_chunks * blockIdx.x / gridDim.x : (long)blockIdx.x;
     const long cur_end = p.share ? total_chunks * (blockIdx.x + 1) / gridDim.x : (long)p.tiles_r * p.tiles_c;
+    bool first_item = true;
     while (cur < cur_end) {
         int tile, kbeg, kend;
         if (p.share) {
@@ -247,8 +241,8 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
         const bool partial = kbeg != 0 || kend != K;
         const int m0 = (tile / p.tiles_c) * RT, n0 = (tile % p.tiles_c) * CT;
 
-        // HW: half a warp per slab row, two words (four columns) per lane: acc[2 * i + w] belongs to row i of the lane's
-        // half and word w.  Otherwise a warp per row, one word (two columns) per lane: acc[r] belongs to row r.
+        // half a warp per slab row, two words (four columns) per lane: acc[2 * i + w] belongs to row i of the lane's
+        // half and word w
         uint32_t acc[32][2];  // [..][0] = sum of whole words, [..][1] = sum of high halves
 #pragma unroll
         for (int r = 0; r < 32; ++r) acc[r][0] = acc[r][1] = 0u;
@@ -263,25 +257,145 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
             store_chunk((kbeg / KC) & 1);
             __syncthreads();
         }
-        build(kbeg & 1, (kbeg / KC) & 1, 0);
-        __syncthreads();
+        if constexpr (KP == 2) {
+            // Two k at a time: the whole words of both are added in one three-operand addition (three additions per
+            // two look-up words instead of four), and waits, arrivals and loop overhead are paid once per two k.
+            // Unit u = two k in slab buffer u % 3; the slabs of unit u + 2 are built after the reads of unit u, once
+            // every warp has released unit u - 1, so each wait has a whole unit of slack and warps drift instead of
+            // lining up behind a CTA barrier per k.  4096^3: 7 bits 7.93 -> 6.78 ms, 6 bits 7.21 -> 6.52 ms, 4 bits 7.20 ->
+            // 6.54 ms; 262144 x 576 x 64 at 7 bits 1.268 -> 1.083 ms.
+            constexpr int AHEAD = NB - 1, UB = KP * C::U_BYTES, UNITS = KC / KP;
+            static_assert(UNITS > 2 * AHEAD, "the next stage is written while no warp can still be reading it");
+            auto build_unit = [&](uint32_t buf, const uint8_t *codes, bool second) {
+                build(buf * UB, codes);
+                if (second) build(buf * UB + C::U_BYTES, codes + CT);
+            };
+            int stage = (kbeg / KC) & 1;
+            if (tid == 0) {
+                // fresh barriers for this item: phases restart at 0 (nobody is waiting or arriving here)
+#pragma unroll
+                for (int b = 0; b < 2 * NB; ++b) {
+                    if (!first_item) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar_full + 8 * b) : "memory");
+                    mbar_init(bar_full + 8 * b, THREADS / 32);
+                }
+            }
+            first_item = false;
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+                if (kbeg + u * KP < kend)
+                    build_unit(u, cc_s + stage * C::CC_STAGE + u * KP * CT, kbeg + u * KP + 1 < kend);
+            __syncwarp();
+            // the first units are complete once every warp has arrived; the last buffer starts out released
+            if (lane == 0) {
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) mbar_arrive(bar_full + 8 * u);
+                mbar_arrive(bar_empty + 8 * AHEAD);
+            }
+            const uint32_t uc = u_addr + (lane & 15) * 8;
+            const int row16 = wp * 32 + (lane >> 4) * 16;  // first of the 16 rows of the lane's half-warp
+            uint32_t buf = 0, prev = NB - 1, par = 0;  // buffers of this unit and of the one before, parity of this round
+            for (int ks = kbeg; ks < kend; ks += KC, stage ^= 1) {
+                const bool more = ks + KC < kend;
+                if (!USE_AT && more) fetch_chunk(m0, n0, ks / KC + 1);
+                const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + rc_off(0, row16);
+                const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + AHEAD * KP * CT;  // column codes of the unit AHEAD
+#pragma unroll 1
+                for (int it = 0; it < UNITS; ++it) {
+                    const int k = ks + KP * it;
+                    if (k >= kend) break;
+                    mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);
+                    // lanes 0-15 read the slab rows of the warp's rows 0-15, lanes 16-31 those of rows 16-31, 64 bits (four
+                    // columns) per lane; slab row address = base + 136 * code in one integer dot-product instruction
+                    const uint32_t ua = uc + buf * UB;
+                    const uint4 q0 = *reinterpret_cast<const uint4 *>(rb_);
+                    const uint32_t rv[4] = {q0.x, q0.y, q0.z, q0.w};
+                    if (k + 1 < kend) {
+                        const uint4 q1 = *reinterpret_cast<const uint4 *>(rb_ + 256);
+                        const uint32_t rw[4] = {q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            uint32_t w0, w1, v0, v1;
+                            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1)
+                                         : "r"(byte_scaled_add<US * 4>(rv[i >> 2], i & 3, ua)));
+                            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v0), "=r"(v1)
+                                         : "r"(byte_scaled_add<US * 4>(rw[i >> 2], i & 3, ua) + C::U_BYTES));
+                            acc[2 * i][0] += w0 + v0;
+                            acc[2 * i][1] += w0 >> 16;
+                            acc[2 * i][1] += v0 >> 16;
+                            acc[2 * i + 1][0] += w1 + v1;
+                            acc[2 * i + 1][1] += w1 >> 16;
+                            acc[2 * i + 1][1] += v1 >> 16;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            uint32_t w0, w1;
+                            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1)
+                                         : "r"(byte_scaled_add<US * 4>(rv[i >> 2], i & 3, ua)));
+                            acc[2 * i][0] += w0;
+                            acc[2 * i][1] += w0 >> 16;
+                            acc[2 * i + 1][0] += w1;
+                            acc[2 * i + 1][1] += w1 >> 16;
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
+                    // (same parity: the last buffer, which unit 0 waits for, starts out released)
+                    mbar_wait(bar_empty + 8 * prev, par, 1 + NB + prev, abort_word, p.error_word);
+                    // every warp has left the unit before, and with it the stage of the chunk before: refill it
+                    if (TMA && it == 0 && more) tma_issue(m0, n0, ks / KC + 1, stage ^ 1);
+                    if (USE_AT && !TMA && it == 0 && more) {
+                        // row codes by asynchronous copies: in registers across the reads they would spill (the transposed
+                        // copy is cut to BITS bits already)
+                        const int gk = ks + KC + tid / (RT / 16), gm = m0 + (tid % (RT / 16)) * 16;
+                        uint8_t *dst = rc_s + (stage ^ 1) * C::RC_STAGE + rc_off(tid / (RT / 16), (tid % (RT / 16)) * 16);
+                        if (gk < K && gm < p.at_pitch) cp_async16(dst, p.at + (size_t)gk * p.at_pitch + gm);
+                        else *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+                        cp_async_commit();
+                    }
+                    if (k + AHEAD * KP < kend) {
+                        if (TMA && it == UNITS - AHEAD) tma_wait(stage ^ 1);  // the first slab of the next chunk
+                        build_unit(prev, cb_, k + AHEAD * KP + 1 < kend);
+                        // without bulk copies the next stage is written before the full arrival of the unit during which
+                        // its first slab is built
+                        if (!TMA && it == UNITS - 2 * AHEAD && more) {
+                            if (USE_AT) {
+                                fetch_cols(n0, ks / KC + 1);
+                                store_cols(stage ^ 1);
+                                cp_async_wait<0>();
+                            } else {
+                                store_chunk(stage ^ 1);
+                            }
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_full + 8 * prev);
+                    }
+                    rb_ += KP * 256;
+                    cb_ = it == UNITS - 1 - AHEAD ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
+                    prev = buf;
+                    if (++buf == NB) { buf = 0; par ^= 1; }
+                }
+            }
+        } else {
+            build((kbeg & 1) * C::U_BYTES, cc_s + ((kbeg / KC) & 1) * C::CC_STAGE);
+            __syncthreads();
 
-        for (int k = kbeg; k < kend; ++k) {
-            const int chunk = k / KC, kk = k % KC, stage = chunk & 1;
-            const bool have_next_chunk = (chunk + 1) * KC < kend;
-            if (TMA) {
-                // the other stage was last read before the barrier that ended the previous k: refill it now, and
-                // make sure it has landed before the last k of this chunk builds the next chunk's first slab
-                if (kk == 0 && have_next_chunk) tma_issue(m0, n0, chunk + 1, stage ^ 1);
-                if (kk == KC - 1 && have_next_chunk) tma_wait(stage ^ 1);
-            } else if (kk == 0 && have_next_chunk) fetch_chunk(m0, n0, chunk + 1);
-            // half of the warps (alternating groups of four, so that every scheduler has both kinds) build their share
-            // of slab k+1 before their reads of slab k, the other half after them: the build's dependent
-            // shared-memory chains then overlap read streams
-            const bool build_first = (wp >> 2) & 1;
-            if (build_first && k + 1 < kend) build((k + 1) & 1, ((k + 1) / KC) & 1, (k + 1) % KC);
+            for (int k = kbeg; k < kend; ++k) {
+                const int chunk = k / KC, kk = k % KC, stage = chunk & 1;
+                const bool have_next_chunk = (chunk + 1) * KC < kend;
+                if (TMA) {
+                    // the other stage was last read before the barrier that ended the previous k: refill it now, and
+                    // make sure it has landed before the last k of this chunk builds the next chunk's first slab
+                    if (kk == 0 && have_next_chunk) tma_issue(m0, n0, chunk + 1, stage ^ 1);
+                    if (kk == KC - 1 && have_next_chunk) tma_wait(stage ^ 1);
+                } else if (kk == 0 && have_next_chunk) fetch_chunk(m0, n0, chunk + 1);
+                // half of the warps (alternating groups of four, so that every scheduler has both kinds) build their share
+                // of slab k+1 before their reads of slab k, the other half after them: the build's dependent
+                // shared-memory chains then overlap read streams
+                const bool build_first = (wp >> 2) & 1;
+                if (build_first && k + 1 < kend) build(((k + 1) & 1) * C::U_BYTES, cc_s + (((k + 1) / KC) & 1) * C::CC_STAGE + ((k + 1) % KC) * CT);
 
-            if constexpr (HW) {
                 // use slab k: lanes 0-15 read the slab rows of the warp's rows 0-15, lanes 16-31 those of rows 16-31,
                 // 64 bits (four columns) per lane
                 const uint4 q0 = *reinterpret_cast<const uint4 *>(rc_s + stage * C::RC_STAGE +
@@ -299,25 +413,10 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
                     acc[2 * i + 1][0] += w1;
                     acc[2 * i + 1][1] += w1 >> 16;
                 }
-            } else {
-                // use slab k: slab row a[m,k], two columns per lane, for this warp's 32 rows
-                const uint4 *rp = reinterpret_cast<const uint4 *>(rc_s + stage * C::RC_STAGE + rc_off(kk, wp * 32));
-                const uint4 q0 = rp[0], q1 = rp[1];
-                const uint32_t rv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                const uint32_t ub = u_addr + (k & 1) * C::U_BYTES + lane * 4;
-#pragma unroll
-                for (int r = 0; r < 32; ++r) {
-                    // slab row address = base + 136 * code in one integer dot-product instruction
-                    const uint32_t addr = byte_scaled_add<US * 4>(rv[r >> 2], r & 3, ub);
-                    uint32_t word;
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(word) : "r"(addr));
-                    acc[r][0] += word;
-                    acc[r][1] += word >> 16;
-                }
+                if (!build_first && k + 1 < kend) build(((k + 1) & 1) * C::U_BYTES, cc_s + (((k + 1) / KC) & 1) * C::CC_STAGE + ((k + 1) % KC) * CT);
+                if (!TMA && kk == KC - 2 && have_next_chunk) store_chunk(stage ^ 1);
+                __syncthreads();
             }
-            if (!build_first && k + 1 < kend) build((k + 1) & 1, ((k + 1) / KC) & 1, (k + 1) % KC);
-            if (!TMA && kk == KC - 2 && have_next_chunk) store_chunk(stage ^ 1);
-            __syncthreads();
         }
 
         LayerEpilogueScalars ev{};
@@ -326,8 +425,8 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
         for (int r = 0; r < 32; ++r) {
             acc[r][0] -= acc[r][1] << 16;  // low-half sum = whole-word sum - 65536 * high-half sum
             // the row and the first of the two columns that acc[r] holds
-            const int m = HW ? m0 + wp * 32 + (lane >> 4) * 16 + (r >> 1) : m0 + wp * 32 + r;
-            const int n = HW ? n0 + 4 * (lane & 15) + 2 * (r & 1) : n0 + 2 * lane;
+            const int m = m0 + wp * 32 + (lane >> 4) * 16 + (r >> 1);
+            const int n = n0 + 4 * (lane & 15) + 2 * (r & 1);
             if (m < M) {
                 if (p.epi.out) {
                     // the layer's de-quantisation applied to the sums in registers (one split per tile here)
@@ -339,7 +438,7 @@ __global__ void __launch_bounds__(512, 1) slab_fwd_kernel(const Args p, const __
                     continue;
                 }
                 uint32_t *crow = p.c + (size_t)m * N;
-                if (HW && !partial && p.vec_c4) {
+                if (!partial && p.vec_c4) {
                     // the lane's four columns of this row in one 16-byte store (acc[r] and acc[r + 1] are one row)
                     if ((r & 1) == 0 && n < N) {
                         const uint32_t lo1 = acc[r + 1][0] - (acc[r + 1][1] << 16);

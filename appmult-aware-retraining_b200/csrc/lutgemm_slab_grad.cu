@@ -76,9 +76,7 @@ struct Cfg {
     static constexpr int Q = 1 << BITS;
     static constexpr int WARPS = 16, THREADS = 512, RW = RW_, RT = WARPS * RW, CT = 64;
     static constexpr int E = Q >= 32 ? Q / 32 : 1;      // codes per lane in the build: x = lane + 32 j, j < E
-    // table row of a column code: the E entries of a lane side by side (one 2E-byte load per column and lane); the
-    // 2E bytes of padding spread the transposing stage over the banks
-    static constexpr int TT_ROW = 2 * Q + (E == 1 ? 4 : 2 * E);
+    static constexpr int TT_ROW = table_row_bytes<BITS>();  // table row of a column code
     static constexpr int U_ROW = 2 * CT + 8;            // bytes per slab row: conflict-free 64-bit build stores
     static constexpr int KC = 16;                       // k per global fetch
     static constexpr int SC = BITS == 8 ? 8 : 16;       // k per shared-memory stage
@@ -153,8 +151,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     for (int idx = tid; idx < Q * Q; idx += THREADS) {
         const int hi_idx = idx >> BITS, lo_idx = idx & (Q - 1);  // global read contiguous in lo_idx
         const int x = MODE == kGw ? hi_idx : lo_idx, y = MODE == kGw ? lo_idx : hi_idx;
-        const int pos = Q >= 32 ? (x & 31) * E + (x >> 5) : x;
-        *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + pos * 2) = (uint16_t)p.lut[hi_idx * COL + lo_idx] ^ (uint16_t)0x8000u;
+        *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + table_pos<BITS>(x) * 2) = (uint16_t)p.lut[hi_idx * COL + lo_idx] ^ (uint16_t)0x8000u;
     }
     if (tid == 0) *abort_word = 0;
 
@@ -252,9 +249,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
     };
     // build the slab at shared address `ub` for the k at (stage, kk): warp wp fills columns 4 wp .. 4 wp + 3.  Lane l
-    // reads the entries of codes l + 32 j of each column in one load and stores four columns of one code at a time;
+    // reads the entries of codes l + 32 j of each column and stores four columns of one code at a time;
     // all table reads of the share are issued before the first store (the stores order later reads behind them).
-    const uint32_t tt_lane = tt_addr + lane * (2 * E);
+    const uint32_t tt_lane = tt_addr + lane * table_lane_bytes<BITS>();
     const uint32_t us = u_addr + wp * 8 + lane * C::U_ROW;
     auto build = [&](uint32_t off, const uint8_t *codes) {  // off: byte offset of the slab
         const uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + wp * 4);
@@ -262,16 +259,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         uint32_t r[4][EW];
         if (Q >= 32 || lane < Q) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t addr = tt_lane + byte_of(cw, c) * C::TT_ROW;
-                if constexpr (E == 8)
-                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(r[c][0]), "=r"(r[c][1]), "=r"(r[c][2]), "=r"(r[c][3]) : "r"(addr));
-                else if constexpr (E == 4)
-                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r[c][0]), "=r"(r[c][1]) : "r"(addr));
-                else if constexpr (E == 2) r[c][0] = lds_u32(addr);
-                else r[c][0] = lds_u16(addr);
-            }
+            for (int c = 0; c < 4; ++c) load_table_entries<BITS>(tt_lane + byte_of(cw, c) * C::TT_ROW, r[c]);
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;

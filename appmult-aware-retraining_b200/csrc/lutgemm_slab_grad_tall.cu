@@ -18,8 +18,8 @@
 // Partial sums: one per lane, warp and k; the 16 warps are added in ascending order by one warp (rotating
 // with k), row blocks by slab_reduce_blocks in ascending order: results are deterministic.
 // grad_w takes its row codes from a transposed copy at[k][m] of the activation codes when the caller has one.
-// Used at 8 bits, where the slab build weighs most and its 1024 rows halve it (4096^3: 13.53 ms each for grad_w and
-// grad_a, against 15.2 and 15.6 ms with the packed slab of lutgemm_slab_grad.cu), for short K, and for fp32 tables.
+// Used at 8 bits, where the slab build weighs most and its 1024 rows halve it (4096^3: 13.33 and 13.47 ms for grad_w and
+// grad_a, against 15.0 and 15.5 ms with the packed slab of lutgemm_slab_grad.cu), for short K, and for fp32 tables.
 // Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492.
 #include <type_traits>
 
@@ -40,8 +40,7 @@ template <int BITS, int RW_>
 struct Cfg {
     static constexpr int Q = 1 << BITS;
     static constexpr bool F32_TABLE = BITS <= 7;
-    static constexpr int HALF = Q / 2;
-    static constexpr int TT_STRIDE = F32_TABLE ? Q + 1 : HALF + 1;  // words per table row
+    static constexpr int TT_STRIDE = F32_TABLE ? Q + 1 : table_row_bytes<BITS>() / 4;  // words per table row
     static constexpr int WARPS = 16, THREADS = 512, RW = RW_, RT = WARPS * RW, CT = 32;
     static constexpr int KC = 16;                       // k per global fetch (16 codes per row in registers)
     static constexpr int SC = BITS == 8 ? 8 : 16;       // k per shared-memory stage
@@ -90,7 +89,7 @@ template <int BITS, int MODE, int RW, bool USE_AT, bool HANDOVER>
 __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
     using C = Cfg<BITS, RW>;
     constexpr int WARPS = C::WARPS;
-    constexpr int Q = C::Q, HALF = C::HALF, TTS = C::TT_STRIDE, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC;
+    constexpr int Q = C::Q, TTS = C::TT_STRIDE, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC;
     constexpr int US = C::U_STRIDE, PS = C::P_STRIDE, THREADS = C::THREADS, NSEG = C::NSEG, RCL = C::RC_LOADS;
     constexpr int HALVES = KC / SC;  // shared-memory stages per fetched group of 16 k
     // slab reads in flight ahead of their use (per row, or per pair of columns with HW): 4 at 8 bits (2 and 3 are 1 - 2 %
@@ -127,9 +126,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
                 p.lut_f32 ? p.lut_f32[hi_idx * COL + lo_idx] : (float)p.lut[hi_idx * COL + lo_idx];
         } else {
             const int16_t v = p.lut[hi_idx * COL + lo_idx];
-            // int16 pairs {T(i,y), T(i+HALF,y)} in offset-binary (v + 32768) for the magic-number conversion
-            reinterpret_cast<uint16_t *>(smem)[(y * TTS + (x & (HALF - 1))) * 2 + (x >> (BITS - 1))] =
-                (uint16_t)v ^ (uint16_t)0x8000u;
+            // 16-bit entries in offset-binary (v + 32768) for the magic-number conversion
+            reinterpret_cast<uint16_t *>(smem)[y * (TTS * 2) + table_pos<BITS>(x)] = (uint16_t)v ^ (uint16_t)0x8000u;
         }
     }
     if (tid == 0) *abort_word = 0;
@@ -232,45 +230,36 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
         const uint32_t cw = *reinterpret_cast<const uint16_t *>(cc_s + stage * C::CC_STAGE + kk * CT + wp * 2);
         const uint32_t y0 = cw & 0xffu, y1 = cw >> 8;
         const uint32_t ub = u_addr + buf * C::U_BYTES + wp * 8;
-        // The table reads of the warp's share are issued before its first store where that measured faster (the
-        // stores order later reads behind them): always with the fp32 table (7 bits: grad_w 13.70 -> 13.28 ms,
-        // grad_a 13.87 -> 13.48 ms at 4096^3), at 8 bits for grad_w only (14.00 -> 13.77 ms; grad_a 14.06 -> 14.50 ms).
-        constexpr bool READS_FIRST = C::F32_TABLE || MODE == kGw;
-        constexpr int NJ = C::F32_TABLE ? (Q + 31) / 32 : HALF / 32;
-        uint32_t r0[NJ], r1[NJ];
-        auto read = [&](int j) {
-            const int x = lane + 32 * j;  // fp32 table: code x; int16 table: the pair of codes (x, x + HALF)
-            if (Q >= 32 || x < Q) {
-                r0[j] = lds_u32(tt_addr + (y0 * TTS + x) * 4);
-                r1[j] = lds_u32(tt_addr + (y1 * TTS + x) * 4);
-            }
-        };
-        auto store = [&](int j) {
-            const int x = lane + 32 * j;
-            if constexpr (C::F32_TABLE) {
-                if (Q >= 32 || x < Q)
-                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + x * (US * 4)), "r"(r0[j]), "r"(r1[j]) : "memory");
-            } else {
+        // The table reads of the warp's share are issued before its first store (the stores order later reads behind
+        // them): 7 bits, grad_w 13.70 -> 13.28 ms, grad_a 13.87 -> 13.48 ms at 4096^3.
+        if constexpr (C::F32_TABLE) {
+            constexpr int NJ = (Q + 31) / 32;
+            uint32_t r0[NJ], r1[NJ];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+                if (Q >= 32 || lane < Q) {
+                    r0[j] = lds_u32(tt_addr + (y0 * TTS + lane + 32 * j) * 4);
+                    r1[j] = lds_u32(tt_addr + (y1 * TTS + lane + 32 * j) * 4);
+                }
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+                if (Q >= 32 || lane < Q)
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + (lane + 32 * j) * (US * 4)), "r"(r0[j]), "r"(r1[j])
+                                 : "memory");
+        } else {
+            uint32_t r0[Q / 64], r1[Q / 64];  // entries of codes lane + 64 j (low halves) and lane + 64 j + 32
+            load_table_entries<BITS>(tt_addr + y0 * (TTS * 4) + lane * table_lane_bytes<BITS>(), r0);
+            load_table_entries<BITS>(tt_addr + y1 * (TTS * 4) + lane * table_lane_bytes<BITS>(), r1);
+#pragma unroll
+            for (int j = 0; j < Q / 64; ++j) {
                 // 0x4B000000 | u is the float 2^23 + u; minus (2^23 + 32768) leaves the signed entry exactly
                 const float f00 = __uint_as_float((r0[j] & 0xffffu) | 0x4B000000u) - 8421376.0f;
                 const float f01 = __uint_as_float((r1[j] & 0xffffu) | 0x4B000000u) - 8421376.0f;
                 const float f10 = __uint_as_float(__byte_perm(r0[j], 0x4B000000u, 0x7632)) - 8421376.0f;
                 const float f11 = __uint_as_float(__byte_perm(r1[j], 0x4B000000u, 0x7632)) - 8421376.0f;
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ub + x * (US * 4)), "f"(f00), "f"(f01) : "memory");
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ub + (x + HALF) * (US * 4)), "f"(f10), "f"(f11)
-                             : "memory");
-            }
-        };
-        if constexpr (READS_FIRST) {
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) read(j);
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) store(j);
-        } else {
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                read(j);
-                store(j);
+                const uint32_t row = ub + (lane + 64 * j) * (US * 4);
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(row), "f"(f00), "f"(f01) : "memory");
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(row + 32 * (US * 4)), "f"(f10), "f"(f11) : "memory");
             }
         }
     };
