@@ -91,9 +91,9 @@ double slab_grad_clocks(long rows, long cols, int K, int rt, int ct, int overhea
     const double reduce = blocks > 1 ? 8e3 + 8.0 * blocks * K * cols / kReduceBytesPerClock : 0;
     return (double)ks.waves * (ks.per + overhead) * per_step + start + reduce;
 }
-double packed_clocks(int bits, long rows, long cols, int K, int sms) {
-    const FamilyClocks f = family_clocks(bits);
-    return slab_grad_clocks(rows, cols, K, 512, 64, lutgemm::kPackedItemOverhead, f.packed, kSlabStart, sms);
+double packed_clocks(int bits, long rows, long cols, int K, int sms, int rt) {
+    const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
+    return slab_grad_clocks(rows, cols, K, rt, 64, lutgemm::kPackedItemOverhead, step, kSlabStart, sms);
 }
 double tall_clocks(int bits, long rows, long cols, int K, int sms) {
     const FamilyClocks f = family_clocks(bits);
@@ -124,8 +124,9 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms) {
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
 }
-void set_ga_scratch(BackwardPlan &pl, int M, int K, int N) {
-    const int rb = !pl.ga_slab ? 1 : pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::slab_packed_row_blocks(N);
+void set_ga_scratch(BackwardPlan &pl, int bits, int M, int K, int N) {
+    const int rt = lutgemm::packed_ga_tile_rows(bits, N);
+    const int rb = !pl.ga_slab ? 1 : pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : (N + rt - 1) / rt;
     pl.ga_scratch = rb > 1 ? (size_t)rb * K * M * sizeof(float) : 0;
 }
 
@@ -139,7 +140,7 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms) {
     pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
     set_gw_scratch(pl, bits, M, K, N, sms);
-    set_ga_scratch(pl, M, K, N);
+    set_ga_scratch(pl, bits, M, K, N);
     return pl;
 }
 
@@ -151,18 +152,18 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
     BackwardPlan pl{};
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (want_gw) {
-        const double packed = packed_clocks(bits, M, N, K, sms), tall = tall_clocks(bits, M, N, K, sms);
+        const double packed = packed_clocks(bits, M, N, K, sms, 512), tall = tall_clocks(bits, M, N, K, sms);
         pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
         set_gw_scratch(pl, bits, M, K, N, sms);
     }
     if (want_ga) {
-        const double packed = packed_clocks(bits, N, M, K, sms), tall = tall_clocks(bits, N, M, K, sms);
+        const double packed = packed_clocks(bits, N, M, K, sms, lutgemm::packed_ga_tile_rows(bits, N)), tall = tall_clocks(bits, N, M, K, sms);
         pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_ga_scratch(pl, M, K, N);
+        set_ga_scratch(pl, bits, M, K, N);
     }
     return pl;
 }
@@ -524,7 +525,7 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(bits, rows);
-        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, 20, f.packed * (rt > 512 ? 1.15 : 1.0), kSlabStart, sms);
+        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, 20, f.packed * (rt > 512 ? 1.12 : 1.0), kSlabStart, sms);
         tiles += t;
         rows_tiles += (double)t * rows;
         if (rows > most_rows) most_rows = rows;

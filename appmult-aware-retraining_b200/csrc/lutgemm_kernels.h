@@ -41,8 +41,8 @@ int slab_fwd_ksplits(int M, int K, int N, int num_sms);
 
 // How a slab kernel cuts K (outputs are per k, so the parts are independent work items): the number of parts and the k
 // per part (a multiple of 16) for which a persistent grid of num_sms CTAs finishes first, when an item of `per` k costs
-// per + item_overhead steps.  Up to 64 parts, so that few tiles still fill the GPU; beyond 12 items per CTA another part
-// gains less than 1 / 12, and the search (a microsecond of host time per call) ends.
+// per + item_overhead steps.  Up to 64 parts, so that few tiles still fill the GPU; beyond 16 items per CTA another part
+// gains less than 1 / 16, and the search (a microsecond of host time per call) ends.
 struct KSplit {
     int parts, per;
     long waves;
@@ -52,7 +52,7 @@ inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
     KSplit best{1, (int)chunks * 16, (tiles + num_sms - 1) / num_sms};
     long cost = best.waves * (best.per + item_overhead);
     unsigned last = chunks;
-    for (unsigned s = 2; s <= 64 && s <= chunks && tiles * s <= 12L * num_sms; ++s) {
+    for (unsigned s = 2; s <= 64 && s <= chunks && tiles * s <= 16L * num_sms; ++s) {
         const unsigned per = (chunks + s - 1) / s;  // in chunks
         if (per == last) continue;                  // more parts of the same length: some would get no work
         last = per;
@@ -62,11 +62,12 @@ inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
     }
     return best;
 }
-constexpr int kPackedItemOverhead = 16, kTallItemOverhead = 8;  // in k steps: operand fetch, grad_out block, first slabs
+constexpr int kPackedItemOverhead = 10, kTallItemOverhead = 4;  // in k steps: operand fetch, grad_out block, first slabs
 
 // rows of the reduction dimension per CTA tile of the packed-slab gradient kernels, and the block count
 constexpr int kSlabPackedRows = 512;
 int slab_packed_row_blocks(int rdim);
+int packed_ga_tile_rows(int bits, int N);  // grad_a: rows of its tile (384, 512 or 576)
 // gradient slab kernels with 16-bit slab entries (converted where they are used)
 // `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
 int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,

@@ -444,13 +444,22 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         // rows of code words [QB, QE) of the warp: the lane's columns of the slab at `ua`, row codes of this k at `rbase`
         auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag) {
             constexpr int QB = decltype(qb_tag)::value, QE = decltype(qe_tag)::value, NR = 2 * (QE - QB);
-            constexpr int PF = 4;  // slab reads in flight ahead of their use
+            // slab reads in flight ahead of their use (4096^3 at 7 bits: grad_w 10.93 / 10.87 / 10.83 / 10.55 ms with 2 / 3 / 4 / 6
+            // (6 bits 10.31 with 4, 10.69 with 6),
+            // grad_a 11.33 / 11.19 / 11.24 / 11.48; 384-row tiles, 12608 x 1536 x 384: 1.323 / 1.283 / 1.344 / 1.323)
+            constexpr int PF = MODE == kGw ? (BITS == 7 ? 6 : 4) : RW == 24 ? 3 : 4;
             uint32_t rv[QE - QB];
             if constexpr (RW % 16 == 0 && QB % 4 == 0 && QE % 4 == 0) {
 #pragma unroll
                 for (int q = 0; q < (QE - QB) / 4; ++q) {
                     const uint4 t = reinterpret_cast<const uint4 *>(rbase + QB * 4)[q];
                     rv[4 * q] = t.x; rv[4 * q + 1] = t.y; rv[4 * q + 2] = t.z; rv[4 * q + 3] = t.w;
+                }
+            } else if constexpr (RW % 8 == 0 && QB % 2 == 0 && QE % 2 == 0) {
+#pragma unroll
+                for (int q = 0; q < (QE - QB) / 2; ++q) {
+                    const uint2 t = reinterpret_cast<const uint2 *>(rbase + QB * 4)[q];
+                    rv[2 * q] = t.x; rv[2 * q + 1] = t.y;
                 }
             } else {
 #pragma unroll
@@ -473,7 +482,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             }
         };
         using Q0 = std::integral_constant<int, 0>;
-        using QH = std::integral_constant<int, NW / 2>;
+        using QH = std::integral_constant<int, RW == 24 ? 4 : NW / 2>;
         using QN = std::integral_constant<int, NW>;
         auto clear_acc = [&]() { acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = pack2(0.f, 0.f); };
         // partial sums of one k: row 2 wp + h, the lane's four columns
@@ -554,6 +563,21 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
 
 }  // namespace sp
 
+// Rows of a packed tile: the height that costs least over all row blocks, a k step of a tile taking about
+// 78 + 5 rows-per-warp instructions per warp (slab build and loop, reads and arithmetic).  576 = 3 x 3 taps of 64 channels
+// and half of 1152, 384 for row counts that would leave a quarter of 512 empty (7 bits, grad_a, 512-row tiles -> these:
+// 12608 x 384 x 384 0.419 -> 0.359 ms, 12608 x 384 x 1152 1.244 -> 0.984 ms).
+static int best_tile_rows(long rdim, bool with_384) {
+    auto cost = [&](long rt, double step) { return (double)((rdim + rt - 1) / rt) * step; };
+    int rt = 512;
+    double c = cost(512, 1.0);
+    if (cost(576, 1.12) < c) { c = cost(576, 1.12); rt = 576; }
+    if (with_384 && cost(384, 0.83) < c) rt = 384;
+    return rt;
+}
+int packed_ga_tile_rows(int, int N) { return best_tile_rows(N, true); }
+int gx_tile_rows(int, long rdim) { return best_tile_rows(rdim, false); }
+
 namespace {
 
 template <int BITS, int MODE, int RW>
@@ -593,20 +617,21 @@ int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, floa
     p.vec_a = !conv.enabled && (K % 16 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
     p.vec_w = (N % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
     p.vec_g = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(gc) & 15) == 0);
-    const int rc = launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+    int rc, rt = kSlabPackedRows;
+    if constexpr (MODE == sp::kGa) {
+        rt = packed_ga_tile_rows(BITS, N);
+        rc = rt == 384   ? launch_packed<BITS, MODE, 24>(p, out, scratch, num_sms, stream)
+             : rt == 576 ? launch_packed<BITS, MODE, 36>(p, out, scratch, num_sms, stream)
+                         : launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+    } else {
+        rc = launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+    }
     if (rc != LUTGEMM_OK) return rc;
-    const int tiles_r = slab_packed_row_blocks(p.RDIM);
+    const int tiles_r = (p.RDIM + rt - 1) / rt;
     if (tiles_r > 1)
         return slab_reduce_blocks(scratch, out, K, p.CDIM, tiles_r, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
                                   kGradFactor, num_sms, stream);
     return LUTGEMM_OK;
-}
-
-// rows per warp of the grad_x tile (16 warps): 32, or 36 where 576-row tiles leave less padding (576 = 3 x 3 taps of 64
-// channels); a tile costs its rows plus the slab build
-int gx_rows_per_warp(int bits, long rdim) {
-    auto cost = [&](long rt) { return ((rdim + rt - 1) / rt) * (rt + (1L << bits)); };
-    return cost(576) < cost(512) ? 36 : 32;
 }
 
 template <int BITS>
@@ -620,7 +645,7 @@ int launch_packed_gx(const float *gy, const uint8_t *x, const uint8_t *wmat, flo
     p.px = px;
     p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
     p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
-    const int rw = gx_rows_per_warp(BITS, p.RDIM);
+    const int rw = gx_tile_rows(BITS, p.RDIM) / 16;
     const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, gx, scratch, num_sms, stream)
                             : launch_packed<BITS, sp::kGx, 32>(p, gx, scratch, num_sms, stream);
     if (rc != LUTGEMM_OK) return rc;
@@ -658,10 +683,8 @@ int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w,
     return LUTGEMM_E_BITS;
 }
 
-int gx_tile_rows(int bits, long rdim) { return 16 * gx_rows_per_warp(bits, rdim); }
-
 size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B) {
-    const long rdim = (long)px.ntaps * Cout, rt = 16L * gx_rows_per_warp(bits, rdim);
+    const long rdim = (long)px.ntaps * Cout, rt = gx_tile_rows(bits, rdim);
     const long tiles_r = (rdim + rt - 1) / rt;
     return tiles_r > 1 ? (size_t)tiles_r * px.C * ((size_t)B * px.Hc * px.Wc) * sizeof(float) : 0;
 }
