@@ -50,26 +50,64 @@ __global__ void update_ranges_kernel(const float *act_lo, const float *act_hi, c
     quant[3] = rintf(__fdiv_rn(wmin, s_w));
 }
 
-// One block per output channel: codes of weight[co, :, :, :] (any strides) written as column co of wmat[K, Cout],
-// K ordered (cin, kh, kw); wsum[co, t] = sum over cin of the codes of tap t (integers: exact in any order).
-__global__ void __launch_bounds__(256) weight_prep_kernel(const float *__restrict__ weight, long s_co, long s_c, long s_h,
+// One block per CO output channels: codes of weight[co, :, :, :] (any strides) written as columns of wmat[K, Cout], K
+// ordered (cin, kh, kw); wsum[co, t] = sum over cin of the codes of tap t.  A thread handles one k of all CO channels, so
+// its reads are independent of each other and its codes leave in one CO-byte store; the sums are integers (exact in any
+// order; shared-memory atomics are native for integers only), added up inside the warp first where there is one tap.
+// 384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> PREP us.
+template <int CO>
+__global__ void __launch_bounds__(512) weight_prep_kernel(const float *__restrict__ weight, long s_co, long s_c, long s_h,
                                                           long s_w, int Cout, int Cin, int kh, int kw,
                                                           const float *__restrict__ quant, float qmax,
-                                                          uint8_t *__restrict__ wmat, float *__restrict__ wsum) {
-    extern __shared__ float tap_sum[];  // [kh*kw]
-    const int T = kh * kw, K = Cin * T, co = blockIdx.x;
+                                                          uint8_t *__restrict__ wmat, float *__restrict__ wsum, int vec) {
+    extern __shared__ uint32_t tap_sum[];  // [CO][kh*kw]
+    const int T = kh * kw, K = Cin * T, co0 = blockIdx.x * CO, lane = threadIdx.x & 31;
     const Divisor scale = make_divisor(quant[2]);
     const float zp = quant[3];
-    for (int t = threadIdx.x; t < T; t += blockDim.x) tap_sum[t] = 0.f;
+    for (int t = threadIdx.x; t < CO * T; t += blockDim.x) tap_sum[t] = 0u;
     __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int c = k / T, t = k - c * T, i = t / kw, j = t - i * kw;
-        const float q = fminf(fmaxf(code_of(weight[co * s_co + c * s_c + i * s_h + j * s_w], scale, zp), 0.f), qmax);
-        wmat[(size_t)k * Cout + co] = (uint8_t)q;
-        atomicAdd(&tap_sum[t], q);
+    for (int k0 = 0; k0 < K; k0 += blockDim.x) {  // (whole warps: the sum over the warp below needs every lane)
+        const int k = k0 + threadIdx.x;
+        uint32_t q[CO];
+        int t = 0;
+        if (k < K) {
+            const int c = k / T;
+            t = k - c * T;
+            const int i = t / kw, j = t - i * kw;
+            const float *src = weight + co0 * s_co + c * s_c + i * s_h + j * s_w;
+            float x[CO];
+#pragma unroll
+            for (int e = 0; e < CO; ++e) x[e] = co0 + e < Cout ? src[e * s_co] : 0.f;
+#pragma unroll
+            for (int e = 0; e < CO; ++e)
+                q[e] = (uint32_t)(uint8_t)fminf(fmaxf(code_of(x[e], scale, zp), 0.f), qmax);
+            uint8_t *dst = wmat + (size_t)k * Cout + co0;
+            if (CO == 8 && vec) {
+                *reinterpret_cast<uint2 *>(dst) = make_uint2(q[0] | q[1 % CO] << 8 | q[2 % CO] << 16 | q[3 % CO] << 24,
+                                                             q[4 % CO] | q[5 % CO] << 8 | q[6 % CO] << 16 | q[7 % CO] << 24);
+            } else {
+#pragma unroll
+                for (int e = 0; e < CO; ++e)
+                    if (co0 + e < Cout) dst[e] = (uint8_t)q[e];
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < CO; ++e) q[e] = 0u;
+        }
+        if (T == 1) {
+#pragma unroll
+            for (int e = 0; e < CO; ++e) {
+                const uint32_t sum = __reduce_add_sync(0xffffffffu, q[e]);
+                if (lane == 0) atomicAdd(&tap_sum[e], sum);
+            }
+        } else if (k < K) {
+#pragma unroll
+            for (int e = 0; e < CO; ++e) atomicAdd(&tap_sum[e * T + t], q[e]);
+        }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < T; t += blockDim.x) wsum[(size_t)co * T + t] = tap_sum[t];
+    for (int t = threadIdx.x; t < CO * T; t += blockDim.x)
+        if (co0 + t / T < Cout) wsum[(size_t)co0 * T + t] = (float)tap_sum[t];
 }
 
 __device__ __forceinline__ bool tap_inside(const ConvGeom &g, int oh, int ow, int i, int j) {
@@ -175,8 +213,15 @@ int layer_update_ranges(const float *act_lo, const float *act_hi, const float *w
 
 int layer_weight_prep(const float *weight, long s_co, long s_c, long s_h, long s_w, int Cout, int Cin, int kh, int kw,
                       const float *quant, float qmax, uint8_t *wmat, float *wsum, cudaStream_t stream) {
-    weight_prep_kernel<<<Cout, 256, kh * kw * sizeof(float), stream>>>(weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw, quant,
-                                                                      qmax, wmat, wsum);
+    const int T = kh * kw, K = Cin * T, threads = K >= 512 ? 512 : (K + 31) / 32 * 32;
+    if (T <= 512) {  // (the sums of eight channels have to fit shared memory)
+        const int vec = Cout % 8 == 0 && (reinterpret_cast<uintptr_t>(wmat) & 7) == 0;
+        weight_prep_kernel<8><<<(Cout + 7) / 8, threads, 8 * T * sizeof(uint32_t), stream>>>(
+            weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw, quant, qmax, wmat, wsum, vec);
+    } else {
+        weight_prep_kernel<1><<<Cout, threads, T * sizeof(uint32_t), stream>>>(weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw,
+                                                                             quant, qmax, wmat, wsum, 0);
+    }
     return launch_status();
 }
 

@@ -152,3 +152,19 @@ def test_image_gradient_without_scratch(dev, oracle_c, bits):
     col = oracle_c.im2col(x, k, k, 1, 1, 1)
     r_ga, _, r_gaa, _ = oracle_c.backward_f64(gy, col, wmat, la, lw, bits)
     check(gx.cpu().numpy(), O.col2im_f64(r_ga, x.shape, k, k, 1, 1, 1), O.col2im_f64(r_gaa, x.shape, k, k, 1, 1, 1))
+
+
+@pytest.mark.parametrize("Cout,Cin,k", [(8, 5, 1), (13, 700, 1), (64, 33, 3), (9, 3, 23), (1, 1, 1)])
+def test_weight_codes_and_their_sums(dev, Cout, Cin, k):
+    """Eight channels per block with and without whole 8-byte stores, one tap, more taps than eight channels' sums fit
+    shared memory, K below a warp and above a block: codes and sums are whole numbers, so the comparison is exact."""
+    import approx_ops
+    g = torch.Generator().manual_seed(Cout + Cin + k)
+    w = torch.randn(Cout, Cin, k, k, generator=g)
+    s, z, qmax = 0.0371, -31.0, 127.0
+    quant = torch.tensor([1.0, 0.0, s, z], device=dev)
+    for weight in (w.to(dev), w.to(dev).to(memory_format=torch.channels_last)):
+        wmat, wsum = approx_ops.layer_weight_prep(weight, quant, qmax)
+        codes = torch.clamp(torch.round(w / quant[2].cpu() - quant[3].cpu()), 0, qmax)
+        assert torch.equal(wmat.cpu().float(), codes.reshape(Cout, -1).t())
+        assert torch.equal(wsum.cpu(), codes.reshape(Cout, Cin, k * k).sum(dim=1))
