@@ -834,4 +834,37 @@ int lutgemm_layer_weight_grad(const float *gwmat, const float *tapg, const float
                                              sms, static_cast<cudaStream_t>(stream));
 }
 
+// ---- a convolution layer's forward pass in one call --------------------------------------------------------------
+size_t lutgemm_conv2d_layer_work_floats(int B, int C, int H, int W, int Cout, int kh, int kw, int stride, int pad, int dil) {
+    lutgemm::ConvGeom g{};
+    if (Cout <= 0 || make_geom(B, C, H, W, kh, kw, stride, pad, dil, &g) != LUTGEMM_OK) return 0;
+    const size_t L = (size_t)g.Ho * g.Wo;
+    return (size_t)B * H * W + (size_t)Cout * kh * kw + L * Cout + L + B * L;
+}
+
+int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, long x_sw, const float *weight, long w_so,
+                              long w_sc, long w_sh, long w_sw, const float *bias, const float *quant, float a_qmax,
+                              float w_qmax, const uint16_t *lut, int bits, int B, int C, int H, int W, int Cout, int kh,
+                              int kw, int stride, int pad, int dil, uint8_t *codes, uint8_t *wmat, float *out, float *work,
+                              void *scratch, size_t scratch_bytes, void *stream) {
+    lutgemm::ConvGeom g{};
+    int rc = make_geom(B, C, H, W, kh, kw, stride, pad, dil, &g);
+    if (rc != LUTGEMM_OK) return rc;
+    if (!quant || !work || Cout <= 0 || (reinterpret_cast<uintptr_t>(work) & 3)) return LUTGEMM_E_BADARG;
+    const size_t L = (size_t)g.Ho * g.Wo, pixels = (size_t)B * H * W;
+    float *chansum = work, *wsum = chansum + pixels, *sumw_t = wsum + (size_t)Cout * kh * kw, *taps = sumw_t + L * Cout,
+          *box = taps + L;
+    // (the quantisation kernel adds its channel tiles to the channel sums)
+    if (!lutgemm::cuda_ok(cudaMemsetAsync(chansum, 0, pixels * sizeof(float), static_cast<cudaStream_t>(stream))))
+        return LUTGEMM_E_CUDA;
+    rc = lutgemm_quantize_activations(x, x_sb, x_sc, x_sh, x_sw, B, C, H, W, quant, quant + 1, a_qmax, codes, chansum, stream);
+    if (rc == LUTGEMM_OK)
+        rc = lutgemm_layer_weight_prep(weight, w_so, w_sc, w_sh, w_sw, Cout, C, kh, kw, quant, w_qmax, wmat, wsum, stream);
+    if (rc == LUTGEMM_OK) rc = lutgemm_layer_cross_terms(wsum, Cout, C, H, W, kh, kw, stride, pad, dil, sumw_t, taps, stream);
+    if (rc == LUTGEMM_OK) rc = lutgemm_layer_window_sum(chansum, B, H, W, kh, kw, stride, pad, dil, box, stream);
+    if (rc != LUTGEMM_OK) return rc;
+    return lutgemm_conv2d_forward_layer(codes, wmat, lut, bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, box, sumw_t, taps,
+                                        quant, quant + 2, quant + 1, quant + 3, bias, out, scratch, scratch_bytes, stream);
+}
+
 }  // extern "C"

@@ -90,22 +90,16 @@ class _AppConvLayer(torch.autograd.Function):
         # quant = [s_a, z_a, s_w, z_w] (one device tensor, so nothing here synchronises with the host)
         if _ops_state.lut_appmult is None:
             raise RuntimeError("lookup tables are not initialised: call init_lookup_tables first")
-        s_a, z_a, s_w, z_w = (quant[i:i + 1] for i in range(4))
         B, Cin, H, W = x.shape
         Cout, _, kh, kw = weight.shape
         Ho, Wo = _out_hw(H, W, kh, kw, stride, padding, dilation)
-        L, M = Ho * Wo, B * Ho * Wo
         if not (x.is_contiguous() or x.is_contiguous(memory_format=torch.channels_last)):
             x = x.contiguous()
-        codes, chansum = approx_ops.quantize_activations(x, s_a, z_a, a_qmax)
-        # weight codes as the [K, Cout] matrix of the LUT kernels + their per-tap sums; the two z_a cross terms per
-        # output position; the window sums of the channel-summed activation codes (one small kernel each)
-        wmat, wsum = approx_ops.layer_weight_prep(weight, quant, w_qmax)
-        sumw_t, taps = approx_ops.layer_cross_terms(wsum, Cin, H, W, kh, kw, stride, padding, dilation)
-        box = approx_ops.layer_window_sum(chansum, kh, kw, stride, padding, dilation)
-        # one kernel: LUT convolution with the de-quantisation applied to the sums in registers
-        out, codes_t = approx_ops.approx_conv2d_forward_layer(codes, wmat, _ops_state.lut_appmult, kh, kw, stride, padding,
-                                                              dilation, box, sumw_t, taps, s_a, s_w, z_a, z_w, bias)
+        # one call: activation codes and their channel sums; weight codes as the [K, Cout] matrix of the LUT kernels and
+        # their per-tap sums; the two z_a cross terms per output position; the window sums of the channel-summed codes; the
+        # LUT convolution with the de-quantisation applied to the sums in registers
+        out, codes, wmat, codes_t = approx_ops.conv2d_layer_pass(x, weight, bias, quant, a_qmax, w_qmax,
+                                                                 _ops_state.lut_appmult, stride, padding, dilation)
         ctx.save_for_backward(x, codes, wmat, weight, quant)
         ctx.codes_t = codes_t  # transposed unfolded codes of the forward kernel: the grad_w kernel reuses them
         ctx.cfg = (a_qmax, w_qmax, stride, padding, dilation, Ho, Wo, bias is not None)

@@ -248,6 +248,20 @@ int lutgemm_conv2d_epilogue(const uint32_t *y, const float *box, const float *su
                             float *out, long M, int L, int Cout, void *stream);
 
 /*
+ * Forward pass of an approximate convolution layer from its fp32 operands, in one call: lutgemm_quantize_activations,
+ * lutgemm_layer_weight_prep, lutgemm_layer_cross_terms, lutgemm_layer_window_sum and lutgemm_conv2d_forward_layer with the
+ * same arguments (x and weight with their strides in elements, quant = {s_a, z_a, s_w, z_w}).  Outputs: codes u8
+ * [B,C,H,W], wmat u8 [C*kh*kw, Cout], out fp32 [B*Ho*Wo, Cout].  work: lutgemm_conv2d_layer_work_floats() floats for the
+ * channel sums and cross terms (0 = bad geometry); scratch as for lutgemm_conv2d_forward_layer.
+ */
+size_t lutgemm_conv2d_layer_work_floats(int B, int C, int H, int W, int Cout, int kh, int kw, int stride, int pad, int dil);
+int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, long x_sw, const float *weight, long w_so,
+                              long w_sc, long w_sh, long w_sw, const float *bias, const float *quant, float a_qmax,
+                              float w_qmax, const uint16_t *lut, int bits, int B, int C, int H, int W, int Cout, int kh,
+                              int kw, int stride, int pad, int dil, uint8_t *codes, uint8_t *wmat, float *out, float *work,
+                              void *scratch, size_t scratch_bytes, void *stream);
+
+/*
  * Forward of a whole approximate layer in one kernel: lutgemm_conv2d_forward_ws (or lutgemm_forward_ws for a
  * linear layer, L = 1) with lutgemm_conv2d_epilogue applied to the sums while they are still in registers, so the
  * uint32 accumulators [M, Cout] are neither written nor read back:
