@@ -63,22 +63,23 @@ struct BackwardPlan {
 // ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
 // Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
 // The clocks are measured on B200, at 4096^3 unless said otherwise:
-//   slab kernels, per k and tile      packed 512 x 64: 1540 (4 and 6 bits), 1560 (7), 2180 (8); tall 1024 x 32: 1540, 1690, 1880;
+//   slab kernels, per k and tile      packed 512 x 64: grad_w 1480 (4 and 6 bits), 1500 (7), 2120 (8), grad_a and grad_x 1540,
+//                                     1580, 2180; tall 1024 x 32: 1540, 1690, 1880;
 //                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
 //                                     more launches: code transposition, zeroing, and a layer's epilogue)
 //   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
-//                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.7, 1.9, 2.8
+//                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.66, 1.72, 2.2
 // A slab kernel's time does not depend on the codes and it can cut K into many work items; a broadcast kernel has no slab
 // to build, so it stays the better one for few rows.  Against the fixed limits on M, N and tile fill that came before
 // (base_plan below) the estimates move small and ragged problems to the slab kernels: 256 x 512 x 256 at 7 bits, forward 0.291 ms,
 // grad_w 0.088 ms and grad_a 0.092 ms with the broadcast kernels, both gradients 0.034 ms with the slab kernels.
 struct FamilyClocks {
-    double packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start;
+    double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {2180, 1880, 1330, 3.1, 3.3, 4.2, 2.8, 75e3};
-    if (bits == 7) return {1560, 1690, 940, 2.33, 2.4, 2.6, 1.9, 60e3};
-    return {1540, 1540, 905, 1.48, 1.6, 1.6, 1.7, 60e3};
+    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3};
+    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3};
+    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3};
 }
 constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
@@ -91,9 +92,13 @@ double slab_grad_clocks(long rows, long cols, int K, int rt, int ct, int overhea
     const double reduce = blocks > 1 ? 8e3 + 8.0 * blocks * K * cols / kReduceBytesPerClock : 0;
     return (double)ks.waves * (ks.per + overhead) * per_step + start + reduce;
 }
-double packed_clocks(int bits, long rows, long cols, int K, int sms, int rt) {
+double packed_gw_clocks(int bits, int M, int K, int N, int sms) {
+    return slab_grad_clocks(M, N, K, 512, 64, lutgemm::kPackedGwOverhead, family_clocks(bits).packed_gw, kSlabStart, sms);
+}
+double packed_ga_clocks(int bits, int M, int K, int N, int sms) {
+    const int rt = lutgemm::packed_ga_tile_rows(bits, N);
     const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
-    return slab_grad_clocks(rows, cols, K, rt, 64, lutgemm::kPackedItemOverhead, step, kSlabStart, sms);
+    return slab_grad_clocks(N, M, K, rt, 64, lutgemm::kPackedItemOverhead, step, kSlabStart, sms);
 }
 double tall_clocks(int bits, long rows, long cols, int K, int sms) {
     const FamilyClocks f = family_clocks(bits);
@@ -152,14 +157,14 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
     BackwardPlan pl{};
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (want_gw) {
-        const double packed = packed_clocks(bits, M, N, K, sms, 512), tall = tall_clocks(bits, M, N, K, sms);
+        const double packed = packed_gw_clocks(bits, M, K, N, sms), tall = tall_clocks(bits, M, N, K, sms);
         pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
         set_gw_scratch(pl, bits, M, K, N, sms);
     }
     if (want_ga) {
-        const double packed = packed_clocks(bits, N, M, K, sms, lutgemm::packed_ga_tile_rows(bits, N)), tall = tall_clocks(bits, N, M, K, sms);
+        const double packed = packed_ga_clocks(bits, M, K, N, sms), tall = tall_clocks(bits, N, M, K, sms);
         pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
@@ -512,27 +517,40 @@ static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
 // family_clocks).  The slab kernel's time does not depend on the codes, the broadcast kernel's bank conflicts do; the
 // estimate takes the clustered codes of a trained layer.  Measured on B200, 3x3 layers at batch 256, clustered codes,
 // broadcast against slab, ms:
-//   7 bits  64 channels (576 rows) 1.79 : 2.17   128 (1152) 1.99 : 1.96   256 (2304) 2.00 : 1.81   512 (4608) 2.02 : 1.79
-//   8 bits  64 channels            2.32 : 2.81   128        2.66 : 2.57   256        2.66 : 2.39   512        2.74 : 2.36
+//   7 bits  64 channels (576 rows) 1.79 : 1.85   128 (1152) 1.99 : 1.75   256 (2304) 1.99 : 1.65   512 (4608) 2.02 : 1.64
+//   8 bits  64 channels            2.28 : 2.50   128        2.61 : 2.34   256        2.66 : 2.24   512        2.74 : 2.22
+//   256 -> 512 channels, stride 2 (classes of 2048, 1024, 1024 and 512 rows): 7 bits 1.07 : 0.96, 8 bits 1.77 : 1.35
 static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
     const int force = g_force_backward.load(std::memory_order_relaxed);
     if (force == LUTGEMM_BACKWARD_BCAST) return false;
     if (force == LUTGEMM_BACKWARD_SLAB) return true;
     const FamilyClocks f = family_clocks(bits);
     const long mt = bits == 8 ? 512 : 256;
-    double slab = 0, rows_tiles = 0;
-    long tiles = 0, most_rows = 0;
+    double slab = 0;
+    // broadcast kernel: tiles of all classes in one list, tile t on SM t mod sms (rows_of[i] rows from tile begin[i] on)
+    constexpr int kMaxListed = 16;
+    long begin[kMaxListed + 1] = {0}, rows_of[kMaxListed], most = 0;
+    int n = 0;
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(bits, rows);
-        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, 20, f.packed * (rt > 512 ? 1.12 : 1.0), kSlabStart, sms);
-        tiles += t;
-        rows_tiles += (double)t * rows;
-        if (rows > most_rows) most_rows = rows;
+        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, lutgemm::kPackedItemOverhead, f.packed * (rt > 512 ? 1.12 : 1.0), kSlabStart, sms);
+        if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
+            begin[n] += t;
+            return;
+        }
+        rows_of[n] = rows;
+        begin[n + 1] = begin[n] + t;
+        ++n;
     });
-    const double mean = (double)div_up(tiles, sms) * rows_tiles / tiles;  // (a class with pixels exists: kernel extent > stride)
-    const double per_sm = mean > most_rows ? mean : (double)most_rows;
-    return slab < per_sm * mt * f.gx_bcast + kBcastStart;
+    const long last = begin[n];
+    for (int sm = 0; sm < (n > 1 ? sms : 1); ++sm) {  // (one class: SM 0 has the most tiles)
+        long rows = 0;
+        for (int c = 0; c < n; ++c) rows += rows_of[c] * ((begin[c + 1] + sms - 1 - sm) / sms - (begin[c] + sms - 1 - sm) / sms);
+        if (rows > most) most = rows;
+        if (sm >= last) break;
+    }
+    return slab < (double)most * mt * f.gx_bcast + kBcastStart;
 }
 
 // Scratch that the choice by fixed limits (see base_plan) asked for: a buffer of at least that size is not refused, the

@@ -62,7 +62,8 @@ inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
     }
     return best;
 }
-constexpr int kPackedItemOverhead = 10, kTallItemOverhead = 4;  // in k steps: operand fetch, grad_out block, first slabs
+// in k steps: operand fetch, grad_out block (gathered in grad_a and grad_x), first slabs
+constexpr int kPackedGwOverhead = 5, kPackedItemOverhead = 10, kTallItemOverhead = 4;
 
 // rows of the reduction dimension per CTA tile of the packed-slab gradient kernels, and the block count
 constexpr int kSlabPackedRows = 512;

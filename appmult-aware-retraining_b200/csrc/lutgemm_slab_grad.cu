@@ -93,7 +93,8 @@ struct Cfg {
     static constexpr int OFF_CC = OFF_RC + 2 * RC_STAGE;
     static constexpr int OFF_PART = OFF_CC + 2 * CC_STAGE;
     static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // grad_x: image offset of each column
-    static constexpr int OFF_BAR = OFF_PIX + CT * 8;
+    static constexpr int OFF_TAP = OFF_PIX + CT * 8;                  // grad_x: output offset {rows, columns} of each tap
+    static constexpr int OFF_BAR = OFF_TAP + kMaxTaps * 8;
     static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // a full and an empty mbarrier per buffer, and the abort word
     static_assert(RW % 4 == 0 && RT % 16 == 0, "rows per warp");
     static_assert(U_BYTES % 16 == 0 && RC_STAGE % 16 == 0 && CC_STAGE % 16 == 0, "16-byte vectors");
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     uint8_t *cc_s = smem + C::OFF_CC;
     float *part_s = reinterpret_cast<float *>(smem + C::OFF_PART);
     long long *pix_s = reinterpret_cast<long long *>(smem + C::OFF_PIX);
+    int2 *tap_s = reinterpret_cast<int2 *>(smem + C::OFF_TAP);
     const uint32_t tt_addr = smem_u32(smem);
     const uint32_t u_addr = smem_u32(smem + C::OFF_U);
     const uint32_t bar_full = smem_u32(smem + C::OFF_BAR), bar_empty = bar_full + 8 * NB;
@@ -154,6 +156,12 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + table_pos<BITS>(x) * 2) = (uint16_t)p.lut[hi_idx * COL + lo_idx] ^ (uint16_t)0x8000u;
     }
     if (tid == 0) *abort_word = 0;
+    if (MODE == kGx) {
+        // pixel (hh, ww) of the class sits at h = ph + s hh; tap q connects it to output row (h - dh) / s = hh + eh
+        for (int q = tid; q < p.px.ntaps; q += THREADS)
+            tap_s[q] = make_int2((p.px.ph - p.px.dh[q]) / p.px.s, (p.px.pw - p.px.dw[q]) / p.px.s);
+        __syncthreads();
+    }
 
     // ---- operand staging: a group of 16 k is fetched into registers and written to shared memory SC k at a time:
     //      rc_s[stage][kk][r] (RT row codes per k), cc_s[stage][kk][c] (64 column codes per k) ---------------------
@@ -195,18 +203,19 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
         return make_uint4(t[0], t[1], t[2], t[3]);
     };
-    // grad_x: the code of pixel column `col` in channels kbase..kbase+15
-    auto gx_col_codes16 = [&](int col, int kbase) -> uint4 {
-        if (col >= CDIM || kbase >= K) return make_uint4(0, 0, 0, 0);
+    // grad_x: the codes of pixel column tid % 64 in channels kbase + 2 (tid / 64) and + 1 (two byte loads per thread,
+    // coalesced over the pixels)
+    static_assert(MODE != kGx || THREADS * 2 == CT * KC, "two column codes per thread");
+    auto gx_col_codes2 = [&](long long offset, bool valid, int kbase) -> uint32_t {
+        const int k = kbase + 2 * (tid / CT);
         const size_t plane = (size_t)p.px.H * p.px.W;
-        const uint8_t *src = p.a + pixel_class_offset(p.px, col) + (size_t)kbase * plane;
-        uint32_t t[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-            if (kbase + q < K) t[q >> 2] |= (uint32_t)src[q * plane] << (8 * (q & 3));
-        return make_uint4(t[0], t[1], t[2], t[3]);
+        const uint8_t *src = p.a + offset + (size_t)k * plane;
+        uint32_t t = 0;
+        if (valid && k < K) t = src[0];
+        if (valid && k + 1 < K) t |= (uint32_t)src[plane] << 8;
+        return t;
     };
-    auto fetch_group = [&](int r0, int c0, int group) {
+    auto fetch_group = [&](int r0, int c0, int group, bool first) {
         const int kbase = group * KC;
 #pragma unroll
         for (int j = 0; j < RCL; ++j) {
@@ -218,9 +227,13 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                                                      : make_uint4(0, 0, 0, 0);
             else prc[j] = MODE == kGx ? gx_row_codes16(gk, gr) : w_codes16(gk, gr);
         }
-        if (tid < CT) {
+        if (MODE == kGx) {
+            const int col = c0 + tid % CT;
+            // (the first fetch of a tile is made before its table of image offsets is written)
+            pcc.x = gx_col_codes2(first ? (long long)pixel_class_offset(p.px, min(col, CDIM - 1)) : pix_s[tid % CT], col < CDIM, kbase);
+        } else if (tid < CT) {
             if (MODE == kGw) pcc = w_codes16(kbase + tid / (CT / 16), c0 + (tid % (CT / 16)) * 16);
-            else pcc = MODE == kGx ? gx_col_codes16(c0 + tid, kbase) : a_codes16(c0 + tid, kbase);
+            else pcc = a_codes16(c0 + tid, kbase);
         }
     };
     static_assert(KC * CT / 16 == CT, "column codes: one 16-byte vector for each of the first 64 threads");
@@ -235,7 +248,14 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 *reinterpret_cast<uint4 *>(rs + (kq % SC) * RT + (idx % NSEG) * 16) =
                     make_uint4(prc[j].x & MASK4, prc[j].y & MASK4, prc[j].z & MASK4, prc[j].w & MASK4);
         }
-        if (tid < CT) {
+        if (MODE == kGx) {
+            const int k = 2 * (tid / CT);  // even, and SC is even: both codes go to the same stage
+            if (k / SC == hf || HALVES == 1) {
+                const uint32_t t = pcc.x & MASK4;
+                cs[(k % SC) * CT + tid % CT] = (uint8_t)t;
+                cs[(k % SC + 1) * CT + tid % CT] = (uint8_t)(t >> 8);
+            }
+        } else if (tid < CT) {
             const uint32_t tc[4] = {pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4};
             if (MODE == kGw) {
                 const int kq = tid / (CT / 16);
@@ -319,8 +339,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         const int r0 = tr * RT, c0 = tc * CT;
 
         // kbeg is a multiple of 16, so the first stage is half 0 of its group
-        fetch_group(r0, c0, kbeg / KC);
+        fetch_group(r0, c0, kbeg / KC, true);
 
+        // (grad_x: the offsets of the taps come from a table and row -> (tap, n) is stepped, not divided: with four divisions
+        // per load and the codes of a pixel's 16 channels read by one thread a tile of 64 channels spent a quarter of its time
+        // here; 3x3, batch 256, 7 bits: 64 channels 2.17 -> 1.85 ms, 128 1.96 -> 1.75, 256 1.81 -> 1.65, 512 1.79 -> 1.64)
         // the grad_out block of this tile: g[2 (2q + j) + i] = entries of row 4q + 2h + j of the warp for the lane's
         // column pair i (columns 4 cq + 2 i, + 1)
         // (adding -0 changes no value; it makes the pair the result of one 64-bit instruction, so that it stays in an
@@ -354,34 +377,31 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             // two rows (n, n + 1 of one output position) of four columns at a time
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const float *base[2];
-                int h[2] = {0, 0}, w[2] = {0, 0};
+                const float *base[2];          // grad_a: row of column e;  grad_x: position of tap offset 0
+                int hh[2] = {0, 0}, ww[2] = {0, 0};
                 bool valid[2];
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int col = cb + 2 * i + e;
+                    const int col = cb + 2 * i + e, cc = min(col, CDIM - 1);
                     valid[e] = col < CDIM;
                     if (MODE == kGa) {
-                        base[e] = p.gc + (size_t)min(col, CDIM - 1) * N;
+                        base[e] = p.gc + (size_t)cc * N;
                     } else {
-                        const int per = p.px.Hc * p.px.Wc, cc = min(col, CDIM - 1);
-                        const int b = cc / per, rr = cc - b * per, hh = rr / p.px.Wc;
-                        h[e] = p.px.ph + p.px.s * hh;
-                        w[e] = p.px.pw + p.px.s * (rr - hh * p.px.Wc);
-                        base[e] = p.gc + (size_t)b * p.px.Ho * p.px.Wo * N;
+                        const int per = p.px.Hc * p.px.Wc, b = cc / per, rr = cc - b * per;
+                        hh[e] = rr / p.px.Wc;
+                        ww[e] = rr - hh[e] * p.px.Wc;
+                        base[e] = p.gc + ((size_t)(b * p.px.Ho + hh[e]) * p.px.Wo + ww[e]) * N;
                     }
                 }
-                // &grad_out of (column e, row r), or nullptr where there is none
-                auto src_of = [&](int e, int r) -> const float * {
+                // &grad_out of (column e, row r = tap * N + n), or nullptr where there is none
+                auto src_of = [&](int e, int r, int tap, int n) -> const float * {
                     if (!valid[e] || r >= RDIM) return nullptr;
                     if (MODE == kGa) return base[e] + r;
-                    const int q = r / N, n = r - q * N;
-                    const int th = h[e] - p.px.dh[q], tw = w[e] - p.px.dw[q];
-                    if (th < 0 || tw < 0) return nullptr;
-                    const int oh = th / p.px.s, ow = tw / p.px.s;
-                    if (oh * p.px.s != th || ow * p.px.s != tw || oh >= p.px.Ho || ow >= p.px.Wo) return nullptr;
-                    return base[e] + ((size_t)oh * p.px.Wo + ow) * N + n;
+                    const int2 o = tap_s[tap];
+                    if ((unsigned)(hh[e] + o.x) >= (unsigned)p.px.Ho || (unsigned)(ww[e] + o.y) >= (unsigned)p.px.Wo) return nullptr;
+                    return base[e] + ((long)(o.x * p.px.Wo + o.y) * N + n);
                 };
+                int tap = MODE == kGx ? rb / N : 0, n = rb - tap * N;
 #pragma unroll
                 for (int q = 0; q < NW; ++q) {
                     const int r = rb + 4 * q;
@@ -389,17 +409,19 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         t[e] = make_float2(0.f, 0.f);
-                        const float *src = src_of(e, r);
+                        const float *src = src_of(e, r, tap, n);
                         if (p.vec_g) {  // N % 4 == 0: both rows share their tap and lie inside one 8-byte vector
                             if (src) t[e] = *reinterpret_cast<const float2 *>(src);
                         } else {
                             if (src) t[e].x = *src;
-                            src = src_of(e, r + 1);
+                            src = n + 1 < N || MODE == kGa ? src_of(e, r + 1, tap, n + 1) : src_of(e, r + 1, tap + 1, 0);
                             if (src) t[e].y = *src;
                         }
                     }
                     g[2 * (2 * q) + i] = pair(t[0].x, t[1].x);
                     g[2 * (2 * q + 1) + i] = pair(t[0].y, t[1].y);
+                    if (MODE == kGx)
+                        for (n += 4; n >= N; n -= N) ++tap;
                 }
             }
         }
@@ -503,7 +525,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
             const bool more = ks + SC < kend;
             // the registers are free for the next group once the last stage of the current one is written
-            if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC);
+            if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC, false);
             const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
             const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + AHEAD * KP * CT;  // column codes of the unit AHEAD
 #pragma unroll 1
@@ -592,7 +614,7 @@ int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStrea
     p.direct = p.tiles_r == 1;
     p.out = p.direct ? out : scratch;
     const long tiles = (long)p.tiles_r * p.tiles_c;
-    const KSplit ks = choose_ksplit(tiles, p.K, num_sms, kPackedItemOverhead);
+    const KSplit ks = choose_ksplit(tiles, p.K, num_sms, MODE == sp::kGw ? kPackedGwOverhead : kPackedItemOverhead);
     p.ksplits = ks.parts;
     p.k_per_split = ks.per;
     const long items = tiles * ks.parts;
