@@ -180,17 +180,26 @@ class _AppLinearLayer(torch.autograd.Function):
                                         codes_t=ctx.codes_t)
         ctx.codes_t = None
         gx = gwt = gb = None
+        colsum = gy.sum(dim=0) if need_w or (has_bias and ctx.needs_input_grad[2]) else None
         if need_x:
             ga.add_(z_w * gy.sum(dim=1, keepdim=True))  # cross term z_w * rowsum(q_a)
             gx = approx_ops.quantize_activations_backward(x2.view(1, M, 1, K), s_a, z_a, a_qmax, ga.view(1, M, 1, K),
                                                           None, s_w, z_w).view(M, K)
         if need_w:
             # cross term z_a * colsum(q_w), clamp mask and activation scale in one pass
-            gwt = approx_ops.layer_weight_grad(gw, gy.sum(dim=0).view(-1, 1).contiguous(), weight.view(-1, K, 1, 1), quant,
+            gwt = approx_ops.layer_weight_grad(gw, colsum.view(-1, 1), weight.view(-1, K, 1, 1), quant,
                                                w_qmax).view(weight.shape)
         if has_bias and ctx.needs_input_grad[2]:
-            gb = gy.sum(dim=0)
+            gb = colsum
         return gx, gwt, gb, None, None, None
+
+
+def _in_memory_order(x: torch.Tensor) -> torch.Tensor:
+    """The same values as a contiguous view where x is dense in channels-last order: a reduction over all of it would
+    otherwise copy it to NCHW first (0.22 ms for 64 x 256 x 56 x 56)."""
+    if x.dim() == 4 and not x.is_contiguous() and x.is_contiguous(memory_format=torch.channels_last):
+        return x.permute(0, 2, 3, 1)
+    return x
 
 
 class _MinMax(nn.Module):
@@ -242,8 +251,8 @@ class _AppQuant(nn.Module):
             return
         if fused:
             # the two range reductions, then ONE launch for both observers and the four quantisation parameters
-            a_lo, a_hi = torch.aminmax(x.detach())
-            w_lo, w_hi = torch.aminmax(w.detach())
+            a_lo, a_hi = torch.aminmax(_in_memory_order(x.detach()))
+            w_lo, w_hi = torch.aminmax(_in_memory_order(w.detach()))
             approx_ops.layer_update_ranges(a_lo, a_hi, w_lo, w_hi, self.act_range.state(), self.weight_range.state(),
                                            self.act_range.momentum, self.a_qmax, self.w_qmax, self.quant)
             return
