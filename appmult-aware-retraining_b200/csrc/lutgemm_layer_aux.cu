@@ -54,7 +54,7 @@ __global__ void update_ranges_kernel(const float *act_lo, const float *act_hi, c
 // ordered (cin, kh, kw); wsum[co, t] = sum over cin of the codes of tap t.  A thread handles one k of all CO channels, so
 // its reads are independent of each other and its codes leave in one CO-byte store; the sums are integers (exact in any
 // order; shared-memory atomics are native for integers only), added up inside the warp first where there is one tap.
-// 384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> PREP us.
+// 384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> 4.2 us.
 template <int CO>
 __global__ void __launch_bounds__(512) weight_prep_kernel(const float *__restrict__ weight, long s_co, long s_c, long s_h,
                                                           long s_w, int Cout, int Cin, int kh, int kw,

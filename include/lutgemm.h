@@ -108,6 +108,7 @@ int lutgemm_forward_ws(const uint8_t *a, const uint8_t *w, uint32_t *c, const ui
  * Scratch bytes lutgemm_backward needs for a problem (0 when none is needed).  The weight-gradient
  * kernel splits its long reduction over M into slabs whose partial sums live in this buffer, followed
  * by a transposed copy of the activation codes.
+ * A smaller buffer is accepted where kernels that need less can do the work (they are slower); LUTGEMM_E_SCRATCH otherwise.
  * No counterpart in the reference (its GB kernel never splits M, approx_gemm_backward.cu:587-608).
  */
 size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N);
@@ -333,9 +334,9 @@ int lutgemm_layer_weight_grad(const float *gwmat, const float *tapg, const float
  * allocator, code on a path where cudaMalloc's implicit synchronisation is not acceptable.
  *   - The array is LUTGEMM_NOALLOC_SCRATCH_BYTES (32 MiB) per GPU that loads the library, held until
  *     the process exits; lutgemm_noalloc_scratch_capacity() returns the figure.  A problem whose partial
- *     sums need more is refused with LUTGEMM_E_TOOLARGE (lutgemm_backward_scratch_bytes tells the need: on
- *     the slab path one K*N*4-byte block per 1024 or 512 rows of M plus a transposed copy of the codes,
- *     K*M bytes; splits*K*N*4 on the split-M path; nothing for small M).
+ *     sums need more is refused with LUTGEMM_E_TOOLARGE (the need: on the slab path
+ *     one K*N*4-byte block per 1024 or 512 rows of M plus a transposed copy of the codes, K*M bytes;
+ *     splits*K*N*4 on the split-M path; nothing for small M - the kernel family is one that fits the array).
  *   - The first call made with a given device current looks up the array's address on that device
  *     (cudaGetSymbolAddress); make that first call before any stream capture begins.
  *   - All calls share the one array per device and it keeps whatever the last call left there.  Nothing
