@@ -348,7 +348,8 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t given = scratch ? scratch_bytes : 0;
     BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0, gw != nullptr, ga != nullptr);
-    if ((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) pl = base_plan(bits, M, K, N, sms);
+    if (((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) && !g_force_backward.load(std::memory_order_relaxed))
+        pl = base_plan(bits, M, K, N, sms);
     float *sc = static_cast<float *>(scratch);
     if (gw) {
         // the weight gradient goes first: under data parallelism its all-reduce can then overlap gA
