@@ -476,7 +476,7 @@ static bool conv_windows_overlap(const lutgemm::ConvGeom &g) {
     return g.dil * (g.kh - 1) + 1 > g.stride || g.dil * (g.kw - 1) + 1 > g.stride;
 }
 
-// the stride class (ph, pw) of geometry g; false when the class has no pixels or no taps
+// the stride class (ph, pw) of geometry g; false when the class has no pixels, no taps or more than it can hold
 static bool make_pixel_class(const lutgemm::ConvGeom &g, int ph, int pw, lutgemm::PixelClass *px) {
     *px = lutgemm::PixelClass{};
     px->H = g.H; px->W = g.W; px->C = g.C; px->ph = ph; px->pw = pw; px->s = g.stride; px->Ho = g.Ho; px->Wo = g.Wo;
@@ -489,6 +489,7 @@ static bool make_pixel_class(const lutgemm::ConvGeom &g, int ph, int pw, lutgemm
             const int dh = i * g.dil - g.pad, dw = j * g.dil - g.pad;
             const int rh = (((ph - dh) % g.stride) + g.stride) % g.stride, rw = (((pw - dw) % g.stride) + g.stride) % g.stride;
             if (rh != 0 || rw != 0) continue;
+            if (n == lutgemm::kMaxTaps) return false;
             px->dh[n] = (int8_t)dh; px->dw[n] = (int8_t)dw; px->t[n] = (uint8_t)(i * g.kw + j);
             ++n;
         }
@@ -577,6 +578,7 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
     if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true).ga_scratch;
+    if (!pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
     size_t need = 0;
     if (gx_uses_slab(bits, g, Cout, sms))
         for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
