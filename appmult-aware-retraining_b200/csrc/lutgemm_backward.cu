@@ -586,8 +586,9 @@ int backward_gw(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, 
 // image the (channel, tap) of k and the (image, row, column) of the first m are decoded once per thread and m
 // advances incrementally; for a plain [M,K] matrix the byte loads of the 32 k of a block share sectors.
 __global__ void __launch_bounds__(1024) transpose_codes_kernel(const uint8_t *__restrict__ a, uint8_t *__restrict__ at,
-                                                               int M, int K, int pitch, const ConvGeom g, uint32_t mask4) {
-    const int k = blockIdx.y * 32 + threadIdx.y;
+                                                               int M, int K, int pitch, const ConvGeom g, uint32_t mask4,
+                                                               int kbeg) {
+    const int k = kbeg + blockIdx.y * 32 + threadIdx.y;
     const int m0 = (blockIdx.x * 32 + threadIdx.x) * 16;
     if (k >= K || m0 >= pitch) return;
     uint32_t v[4] = {0u, 0u, 0u, 0u};
@@ -649,11 +650,11 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
 // Plain [M,K] matrix with 16-byte aligned rows (K a multiple of 16): a CTA moves a tile of 128 rows x 64 k through
 // shared memory - 16-byte loads along k, 16-byte stores along m - instead of gathering single bytes from global memory.
 __global__ void __launch_bounds__(512) transpose_codes_tiled_kernel(const uint8_t *__restrict__ a, uint8_t *__restrict__ at,
-                                                                    int M, int K, int pitch, uint32_t mask4) {
+                                                                    int M, int K, int pitch, uint32_t mask4, int kbeg) {
     constexpr int TM = 128, TK = 64, TP = TK + 4;  // tile pitch in bytes: rows 17 words apart, the transposed byte reads
                                                    // of 32 rows fall on 32 different banks
     __shared__ __align__(16) uint8_t tile[TM * TP];
-    const int m0 = blockIdx.x * TM, k0 = blockIdx.y * TK;
+    const int m0 = blockIdx.x * TM, k0 = kbeg + blockIdx.y * TK;
     const int tid = threadIdx.x;
     {   // load: thread = (row, 16-k chunk); 4 chunks per row
         const int r = tid >> 2, q = tid & 3;
@@ -688,15 +689,17 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
         transpose_codes_plane_kernel<<<conv.B * conv.C, 256, smem, stream>>>(a, at, pitch, conv, mask4);
         return launch_status();
     }
-    if (!conv.enabled && K % 16 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (K + 63) / 64 <= 65535) {
-        const dim3 tgrid((pitch + 127) / 128, (K + 63) / 64);
-        transpose_codes_tiled_kernel<<<tgrid, 512, 0, stream>>>(a, at, M, K, pitch, mask4);
-        return launch_status();
+    // (k runs over grid.y, which ends at 65535: longer K in several launches)
+    const bool tiled = !conv.enabled && K % 16 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
+    const int rows_per_block = tiled ? 64 : 32, most = 65535 * rows_per_block;
+    for (long k = 0; k < K; k += most) {
+        const unsigned ny = (unsigned)(((K - k < most ? K - k : most) + rows_per_block - 1) / rows_per_block);
+        if (tiled) transpose_codes_tiled_kernel<<<dim3((pitch + 127) / 128, ny), 512, 0, stream>>>(a, at, M, K, pitch, mask4, (int)k);
+        else transpose_codes_kernel<<<dim3((pitch / 16 + 31) / 32, ny), dim3(32, 32), 0, stream>>>(a, at, M, K, pitch, conv, mask4, (int)k);
+        const int rc = launch_status();
+        if (rc != LUTGEMM_OK) return rc;
     }
-    const dim3 block(32, 32), grid((pitch / 16 + 31) / 32, (K + 31) / 32);
-    if (grid.y > 65535u) return LUTGEMM_E_TOOLARGE;
-    transpose_codes_kernel<<<grid, block, 0, stream>>>(a, at, M, K, pitch, conv, mask4);
-    return launch_status();
+    return LUTGEMM_OK;
 }
 
 }  // namespace lutgemm

@@ -168,3 +168,24 @@ def test_weight_codes_and_their_sums(dev, Cout, Cin, k):
         codes = torch.clamp(torch.round(w / quant[2].cpu() - quant[3].cpu()), 0, qmax)
         assert torch.equal(wmat.cpu().float(), codes.reshape(Cout, -1).t())
         assert torch.equal(wsum.cpu(), codes.reshape(Cout, Cin, k * k).sum(dim=1))
+
+
+@pytest.mark.parametrize("K", [2200001, 4200000])
+def test_forward_over_a_long_k(dev, K):
+    """The transposed code copy of the slab kernel in more than one launch (byte loads, and 16-byte loads through a tile):
+    whole numbers, so equal to the broadcast kernel's sums, which need no copy."""
+    import approx_ops
+    M, N, bits = 16, 20, 4
+    g = torch.Generator(device=dev).manual_seed(K)
+    a = torch.randint(0, 16, (M, K), generator=g, device=dev, dtype=torch.uint8)
+    w = torch.randint(0, 16, (K, N), generator=g, device=dev, dtype=torch.uint8)
+    lut = torch.from_numpy(O.pack_padded(np.random.default_rng(1).integers(0, 2 ** 16, (16, 16)), bits, np.uint16)).to(dev)
+    out = []
+    try:
+        for family in ("slab", "rowbcast"):
+            approx_ops.set_kernel_choice(forward=family)
+            out.append(torch.zeros((M, N), dtype=torch.uint32, device=dev))
+            approx_ops.approx_gemm_forward(a, w, out[-1], lut)
+    finally:
+        approx_ops.set_kernel_choice()
+    assert torch.equal(out[0].view(torch.int32), out[1].view(torch.int32))

@@ -29,3 +29,14 @@ def test_scratch_query_for_windows_of_many_taps(lib, k, stride):
     assert lib.call("lutgemm_conv2d_backward", p, p, p, None, p, p, p, *conv, p, need, None)[0] == H.OK
     rc, _ = lib.call("lutgemm_conv2d_backward", p, p, p, p, None, p, p, *conv, p, need, None)
     assert rc == (H.OK if k * k <= 128 else H.E_TOOLARGE)
+
+
+@pytest.mark.parametrize("K", [2097120, 2097121, 2200001, 4194240, 4194256, 9000001])
+def test_long_k_is_not_refused(lib, K):
+    """Few rows and a long K: the slab kernels' transposed code copy is made in as many launches as its grid needs."""
+    p, big = lib.p, H.Size(1 << 40)
+    rc, calls = lib.call("lutgemm_forward_ws", p, p, p, p, 4, 16, K, 64, p, big, None)
+    assert rc == H.OK and calls[-1][0] == "slab_fwd_kernel"
+    per_launch = 65535 * (64 if K % 16 == 0 else 32)
+    assert sum(name.startswith("transpose") for name, _ in calls) == (K + per_launch - 1) // per_launch
+    assert lib.call("lutgemm_backward", p, p, p, p, p, p, p, 4, 16, K, 64, p, big, None)[0] == H.OK
