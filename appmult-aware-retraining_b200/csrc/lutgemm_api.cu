@@ -263,6 +263,12 @@ static bool forward_uses_slab(int bits, int M, int K, int N, int sms) {
     return base_forward_uses_slab(M, N) || slab < bcast;
 }
 
+// A workspace too small for the slab kernel is refused where the slab kernel was always the choice (or is forced); elsewhere
+// the broadcast kernel, which needs none, runs.
+static bool small_workspace_refused(int M, int N) {
+    return base_forward_uses_slab(M, N) || g_force_forward.load(std::memory_order_relaxed);
+}
+
 static int codes_pitch(int M) { return (M + 15) & ~15; }
 
 // `scratch` (optional, K * codes_pitch(M) bytes, 16-byte aligned): the slab kernel then reads the activation
@@ -281,7 +287,7 @@ static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const u
     const int pitch = codes_pitch(M);
     bool slab = forward_uses_slab(bits, M, K, N, sms);
     if (slab && scratch && scratch_bytes < (size_t)pitch * K) {
-        if (base_forward_uses_slab(M, N) || g_force_forward.load(std::memory_order_relaxed)) return LUTGEMM_E_SCRATCH;
+        if (small_workspace_refused(M, N)) return LUTGEMM_E_SCRATCH;
         slab = false;
     }
     if (slab) {
@@ -710,7 +716,7 @@ static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t
     if (!layer_forward_needs_sums(bits, M, K, N, sms))
         return forward_impl(a, w, nullptr, lut, bits, M, K, N, conv, scratch, scratch_bytes, stream, &e);
     if (!scratch || scratch_bytes < layer_forward_scratch_bytes(bits, M, K, N)) {
-        if (base_forward_uses_slab(M, N) || g_force_forward.load(std::memory_order_relaxed)) return LUTGEMM_E_SCRATCH;
+        if (small_workspace_refused(M, N)) return LUTGEMM_E_SCRATCH;
         return lutgemm::forward_rowbcast(a, w, nullptr, lut, bits, M, K, N, conv, &e, sms, static_cast<cudaStream_t>(stream));
     }
     uint32_t *sums = reinterpret_cast<uint32_t *>(static_cast<char *>(scratch) + align16(codes));
@@ -871,7 +877,18 @@ int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, l
     lutgemm::ConvGeom g{};
     int rc = make_geom(B, C, H, W, kh, kw, stride, pad, dil, &g);
     if (rc != LUTGEMM_OK) return rc;
-    if (!quant || !work || Cout <= 0 || (reinterpret_cast<uintptr_t>(work) & 3)) return LUTGEMM_E_BADARG;
+    // everything the steps below would refuse, before the first of them writes anything
+    if (!lutgemm::bits_supported(bits)) return LUTGEMM_E_BITS;
+    if (!x || !weight || !quant || !lut || !codes || !wmat || !out || !work || Cout <= 0 || kh * kw > 4096 ||
+        !(a_qmax >= 1.f && a_qmax <= 255.f) || (reinterpret_cast<uintptr_t>(lut) & 1) || (reinterpret_cast<uintptr_t>(out) & 3) ||
+        (reinterpret_cast<uintptr_t>(work) & 3) || (reinterpret_cast<uintptr_t>(scratch) & 15))
+        return LUTGEMM_E_BADARG;
+    if (H > 65535 || B > 65535) return LUTGEMM_E_TOOLARGE;
+    const int sms = current_num_sms(), M = B * g.Ho * g.Wo, K = C * kh * kw;
+    if (sms <= 0) return LUTGEMM_E_CUDA;
+    if (scratch_bytes < layer_forward_scratch_bytes(bits, M, K, Cout) && small_workspace_refused(M, Cout) &&
+        (scratch || layer_forward_needs_sums(bits, M, K, Cout, sms)))
+        return LUTGEMM_E_SCRATCH;
     const size_t L = (size_t)g.Ho * g.Wo, pixels = (size_t)B * H * W;
     float *chansum = work, *wsum = chansum + pixels, *sumw_t = wsum + (size_t)Cout * kh * kw, *taps = sumw_t + L * Cout,
           *box = taps + L;

@@ -40,3 +40,32 @@ def test_long_k_is_not_refused(lib, K):
     per_launch = 65535 * (64 if K % 16 == 0 else 32)
     assert sum(name.startswith("transpose") for name, _ in calls) == (K + per_launch - 1) // per_launch
     assert lib.call("lutgemm_backward", p, p, p, p, p, p, p, 4, 16, K, 64, p, big, None)[0] == H.OK
+
+
+def layer_pass(lib, bits=7, B=4, C=64, h=8, Cout=64, k=3, a_qmax=127.0, scratch_bytes=1 << 40, **null):
+    p = lib.p
+    ptr = {name: null.get(name, p) for name in ("x", "weight", "quant", "lut", "codes", "wmat", "out", "work", "scratch")}
+    s = [H.Size(1)] * 4
+    return lib.call("lutgemm_conv2d_layer_pass", ptr["x"], *s, ptr["weight"], *s, None, ptr["quant"], a_qmax, 127.0, ptr["lut"], bits,
+                    B, C, h, h, Cout, k, k, 1, 1, 1, ptr["codes"], ptr["wmat"], ptr["out"], ptr["work"], ptr["scratch"],
+                    H.Size(scratch_bytes), None)
+
+
+@pytest.mark.parametrize("bad,status", [
+    (dict(bits=5), H.E_BITS), (dict(x=None), H.E_BADARG), (dict(weight=None), H.E_BADARG), (dict(quant=None), H.E_BADARG),
+    (dict(lut=None), H.E_BADARG), (dict(codes=None), H.E_BADARG), (dict(wmat=None), H.E_BADARG), (dict(out=None), H.E_BADARG),
+    (dict(work=None), H.E_BADARG), (dict(lut=(1 << 40) + 1), H.E_BADARG), (dict(out=(1 << 40) + 2), H.E_BADARG),
+    (dict(scratch=(1 << 40) + 8), H.E_BADARG), (dict(a_qmax=256.0), H.E_BADARG), (dict(a_qmax=0.0), H.E_BADARG),
+    (dict(k=65, h=80), H.E_BADARG), (dict(B=70000, h=3), H.E_TOOLARGE),
+    (dict(B=64, scratch_bytes=64), H.E_SCRATCH),                  # whole tiles, transposed copy only
+    (dict(B=8, C=512, scratch_bytes=64), H.E_SCRATCH), (dict(B=8, C=512, scratch=None, scratch_bytes=0), H.E_SCRATCH)])  # cut K
+def test_layer_pass_refuses_before_it_launches(lib, bad, status):
+    bad = {k: H.ctypes.c_void_p(v) if k in ("lut", "out", "scratch") and v else v for k, v in bad.items()}
+    assert layer_pass(lib, **bad) == (status, [])
+
+
+def test_layer_pass_with_a_small_workspace_where_only_the_estimate_picks_the_slab_kernel(lib):
+    assert layer_pass(lib)[1][-1][0] == "conv_epilogue_kernel"  # (K cut, sums in the workspace)
+    for kw in (dict(scratch_bytes=64), dict(scratch=None, scratch_bytes=0)):
+        rc, calls = layer_pass(lib, **kw)
+        assert rc == H.OK and "rowbcast" in calls[-1][0]
