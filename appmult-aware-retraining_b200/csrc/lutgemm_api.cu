@@ -709,7 +709,8 @@ static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t
                               const lutgemm::ConvGeom &conv, const lutgemm::LayerEpilogue &e, void *scratch,
                               size_t scratch_bytes, void *stream) {
     if (!lutgemm::bits_supported(bits)) return LUTGEMM_E_BITS;
-    if (M <= 0 || K <= 0 || N <= 0) return LUTGEMM_E_BADARG;
+    if (M <= 0 || K <= 0 || N <= 0 || (reinterpret_cast<uintptr_t>(lut) & 1) || (reinterpret_cast<uintptr_t>(scratch) & 15))
+        return LUTGEMM_E_BADARG;
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
     const size_t codes = lutgemm_forward_scratch_bytes(bits, M, K, N);

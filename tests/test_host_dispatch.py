@@ -69,3 +69,11 @@ def test_layer_pass_with_a_small_workspace_where_only_the_estimate_picks_the_sla
     for kw in (dict(scratch_bytes=64), dict(scratch=None, scratch_bytes=0)):
         rc, calls = layer_pass(lib, **kw)
         assert rc == H.OK and "rowbcast" in calls[-1][0]
+
+
+@pytest.mark.parametrize("lut,scratch", [((1 << 40) + 1, 1 << 40), (1 << 40, (1 << 40) + 4)])
+@pytest.mark.parametrize("scratch_bytes", [64, 1 << 40])
+def test_layer_forward_refuses_misaligned_buffers_whatever_the_workspace(lib, lut, scratch, scratch_bytes):
+    p = lib.p
+    assert lib.call("lutgemm_forward_layer", p, p, H.ctypes.c_void_p(lut), 7, 256, 576, 64, p, p, p, p, p, p, p, None, p,
+                    H.ctypes.c_void_p(scratch), H.Size(scratch_bytes), None) == (H.E_BADARG, [])
