@@ -119,3 +119,33 @@ def test_quantisation_division_matches_ieee_division_for_awkward_scales(dev):
                 want = torch.clamp(torch.round(x / scale - zp), 0.0, qmax)
                 want = torch.nan_to_num(want, nan=0.0).to(torch.uint8)
                 assert torch.equal(codes, want.contiguous()), (bits, hex(m), e)
+
+
+@pytest.mark.parametrize("operand", ["weight", "bias", "quant", "lut"])
+def test_layer_pass_refuses_operands_it_cannot_read(dev, operand):
+    """Operands go to the library as pointers: another type, another device, another length or stride is an error here,
+    before anything is launched."""
+    import approx_ops
+    x = torch.rand(2, 4, 6, 6, device=dev)
+    good = dict(weight=torch.randn(8, 4, 3, 3, device=dev), bias=torch.zeros(8, device=dev),
+                quant=torch.tensor([0.01, 0.0, 0.02, -60.0], device=dev), lut=torch.zeros(17408, dtype=torch.uint16, device=dev))
+    bad = [good[operand].cpu()]
+    if operand != "lut":
+        bad += [good[operand].half(), good[operand].double()]
+    if operand in ("bias", "quant"):
+        t = good[operand]
+        bad += [t[:-1], torch.zeros(2 * t.numel(), device=dev)[::2], t[:1].expand(t.numel())]
+    launches = approx_ops.library().lutgemm_kernel_launches()
+
+    def layer_pass(kw):
+        return approx_ops.conv2d_layer_pass(x, kw["weight"], kw["bias"], kw["quant"], 127.0, 127.0, kw["lut"], 1, 1, 1)
+
+    for b in bad:
+        with pytest.raises(RuntimeError):
+            layer_pass({**good, operand: b})
+        if operand in ("weight", "quant"):
+            with pytest.raises(RuntimeError):
+                approx_ops.layer_weight_prep(b if operand == "weight" else good["weight"],
+                                             b if operand == "quant" else good["quant"], 127.0)
+    assert approx_ops.library().lutgemm_kernel_launches() == launches
+    layer_pass(good)
