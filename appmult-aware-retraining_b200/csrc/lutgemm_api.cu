@@ -181,7 +181,9 @@ void record_cuda_error(cudaError_t e) { g_last_cuda_error = e; }
 
 size_t base_gw_scratch_bytes(int bits, int M, int K, int N) {
     const int sms = current_num_sms();
-    return sms > 0 ? base_plan(bits, M, K, N, sms).gw_scratch : 0;
+    if (sms <= 0) return 0;
+    if (g_force_backward.load(std::memory_order_relaxed)) return plan_backward(bits, M, K, N, sms, false, true, false).gw_scratch;
+    return base_plan(bits, M, K, N, sms).gw_scratch;
 }
 
 int launch_status() {

@@ -18,7 +18,7 @@ inline bool cuda_ok(cudaError_t e) {
 // status of the launch just made on this thread
 int launch_status();
 
-// scratch of the weight gradient under the choice by fixed limits (lutgemm_api.cu)
+// scratch of the weight gradient under the choice by fixed limits, or of the family that is forced (lutgemm_api.cu)
 size_t base_gw_scratch_bytes(int bits, int M, int K, int N);
 
 struct ConvGeom;    // lutgemm_common.cuh; geometry.enabled == 0 means `a` is a plain [M,K] matrix

@@ -77,3 +77,16 @@ def test_layer_forward_refuses_misaligned_buffers_whatever_the_workspace(lib, lu
     p = lib.p
     assert lib.call("lutgemm_forward_layer", p, p, H.ctypes.c_void_p(lut), 7, 256, 576, 64, p, p, p, p, p, p, p, None, p,
                     H.ctypes.c_void_p(scratch), H.Size(scratch_bytes), None) == (H.E_BADARG, [])
+
+
+def test_weight_gradient_without_allocation_follows_a_forced_kernel_family(lib):
+    """What fits the fixed array is the need of the kernels that run: 28 MB of codes and 4 blocks of sums for the slab
+    kernels, nothing or a few splits for the broadcast kernel."""
+    p, shape = lib.p, (4096, 7000, 320)
+    try:
+        for family, status in ((0, H.E_TOOLARGE), (1, H.OK), (2, H.E_TOOLARGE)):
+            lib.lib.lutgemm_set_kernel_choice(0, family, 0)
+            rc, calls = lib.call("lutgemm_backward_gw_noalloc", p, p, p, p, p, 8, *shape, None)
+            assert rc == status and (rc != H.OK or calls[0][0] == "gw_rowbcast_kernel")
+    finally:
+        lib.lib.lutgemm_set_kernel_choice(0, 0, 0)
