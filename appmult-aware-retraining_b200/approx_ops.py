@@ -56,6 +56,10 @@ def _load():
     lib.lutgemm_conv2d_forward_ws.argtypes = [vp, vp, vp, vp] + [ci] * 11 + [vp, sz, vp]
     lib.lutgemm_conv2d_backward_ws.restype = ci
     lib.lutgemm_conv2d_backward_ws.argtypes = [vp] * 7 + [ci] * 11 + [vp, vp, sz, vp]
+    lib.lutgemm_backward_ws_scratch_bytes.restype = sz
+    lib.lutgemm_backward_ws_scratch_bytes.argtypes = [ci] * 5
+    lib.lutgemm_conv2d_backward_ws_scratch_bytes.restype = sz
+    lib.lutgemm_conv2d_backward_ws_scratch_bytes.argtypes = [ci] * 12
     lib.lutgemm_backward_scratch_bytes.restype = sz
     lib.lutgemm_backward_scratch_bytes.argtypes = [ci, ci, ci, ci]
     lib.lutgemm_backward.restype = ci
@@ -128,6 +132,7 @@ def library():
 _FORWARD_CHOICES = {"auto": 0, "rowbcast": 1, "slab": 2}
 _BACKWARD_CHOICES = {"auto": 0, "bcast": 1, "slab": 2}
 _TILE_CHOICES = {"auto": 0, "wide": 1, "tall": 2}
+_CODES_GIVEN = 1  # LUTGEMM_SCRATCH_CODES_GIVEN
 
 
 def set_kernel_choice(forward: str = "auto", backward: str = "auto", grad_tile: str = "auto") -> None:
@@ -256,7 +261,7 @@ def approx_gemm_backward(gc: torch.Tensor, a: torch.Tensor, b: torch.Tensor, ga:
         return
     lib = _load()
     with torch.cuda.device(dev):
-        nbytes = lib.lutgemm_backward_scratch_bytes(bits, M, K, N)
+        nbytes = lib.lutgemm_backward_ws_scratch_bytes(bits, M, K, N, _CODES_GIVEN if codes_t is not None else 0)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
         if codes_t is not None:
             _check_input(codes_t, torch.uint8, "codes_t")
@@ -457,7 +462,8 @@ def approx_conv2d_backward(gy: torch.Tensor, x: torch.Tensor, wmat: torch.Tensor
             raise RuntimeError("All tensors should be on the same device")
     lib = _load()
     with torch.cuda.device(dev):
-        nbytes = lib.lutgemm_conv2d_backward_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
+        nbytes = lib.lutgemm_conv2d_backward_ws_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil,
+                                                              _CODES_GIVEN if codes_t is not None else 0)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
         if codes_t is not None:
             _check_input(codes_t, torch.uint8, "codes_t")

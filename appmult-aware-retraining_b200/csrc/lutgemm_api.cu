@@ -53,9 +53,9 @@ struct BackwardPlan {
     bool gw_tall, ga_tall;  // fp32 slab with the 1024 x 32 tile instead of the packed slab with the 512 x 64 tile
     int gw_splits;        // row-broadcast grad_w kernel: slabs of M
     size_t gw_scratch, ga_scratch;
-    // slab grad_w kernels read the activation codes from a transposed copy at[k][m] kept behind the partial
-    // sums in the scratch buffer (their row-code fetch is then coalesced; for a convolution it also
-    // replaces one implicit-im2col gather per column tile by a single one)
+    // slab grad_w kernels read the activation codes from a transposed copy at[k][m] (their row-code fetch is then
+    // coalesced; for a convolution it also replaces one implicit-im2col gather per column tile by a single one): the
+    // caller's, or one made behind the partial sums in the scratch buffer
     size_t gw_at_offset;  // bytes into the scratch buffer, a multiple of 16
     int gw_at_pitch;      // 0 = no transposed copy
 };
@@ -115,16 +115,18 @@ double ga_bcast_clocks(int bits, int M, int K, int N, int sms) {
     return (double)div_up(div_up(M, mt) * div_up(K, 32), sms) * mt * N * family_clocks(bits).ga_bcast + kBcastStart;
 }
 
-void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms) {
+void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bool have_codes) {
     pl.gw_splits = pl.gw_slab ? 1 : lutgemm::gw_num_splits(bits, M, K, N, sms);
     pl.gw_at_offset = 0;
     pl.gw_at_pitch = 0;
     if (pl.gw_slab) {
         const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::slab_packed_row_blocks(M);
         pl.gw_scratch = rb > 1 ? (size_t)rb * K * N * sizeof(float) : 0;
-        pl.gw_at_offset = (pl.gw_scratch + 15) & ~(size_t)15;
         pl.gw_at_pitch = (M + 15) & ~15;
-        pl.gw_scratch = pl.gw_at_offset + (size_t)pl.gw_at_pitch * K;
+        if (!have_codes) {
+            pl.gw_at_offset = (pl.gw_scratch + 15) & ~(size_t)15;
+            pl.gw_scratch = pl.gw_at_offset + (size_t)pl.gw_at_pitch * K;
+        }
     } else {
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
@@ -137,14 +139,14 @@ void set_ga_scratch(BackwardPlan &pl, int bits, int M, int K, int N) {
 
 // Choice by fixed limits: the plan for callers whose scratch buffer is too small for the faster one (a fixed buffer, or
 // one sized for this choice), so that what fitted such a buffer keeps running.
-BackwardPlan base_plan(int bits, int M, int K, int N, int sms) {
+BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) {
     BackwardPlan pl{};
     pl.gw_slab = bits >= 7 && M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6;
     const double ga_fill = slab_fill(N, M) > tall_fill(N, M) ? slab_fill(N, M) : tall_fill(N, M);
     pl.ga_slab = bits >= 7 && N >= 768 && M >= 32 && ga_fill >= (bits == 7 ? 0.85 : 0.7);
     pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
-    set_gw_scratch(pl, bits, M, K, N, sms);
+    set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
     set_ga_scratch(pl, bits, M, K, N);
     return pl;
 }
@@ -152,8 +154,9 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms) {
 // Choice by estimated time.  A convolution's grad_a (non-overlapping windows) gathers its column codes from the image and
 // writes in place; there the slab kernels pay from N = 768 on (1x1, 128 -> 512 channels, 7 bits: 0.75 against 0.68 ms; 1024 -> 512:
 // 1.24 against 1.22 ms).  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
-// (want_gw, want_ga: the gradients that are asked for; the plan of the other one is left empty)
-BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bool want_gw, bool want_ga) {
+// (want_gw, want_ga: the gradients that are asked for; the plan of the other one is left empty.  have_codes: the caller
+// brings the transposed activation codes)
+BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bool want_gw, bool want_ga, bool have_codes) {
     BackwardPlan pl{};
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (want_gw) {
@@ -161,7 +164,7 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
         pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_gw_scratch(pl, bits, M, K, N, sms);
+        set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
     }
     if (want_ga) {
         const double packed = packed_ga_clocks(bits, M, K, N, sms), tall = tall_clocks(bits, N, M, K, sms);
@@ -182,8 +185,8 @@ void record_cuda_error(cudaError_t e) { g_last_cuda_error = e; }
 size_t base_gw_scratch_bytes(int bits, int M, int K, int N) {
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    if (g_force_backward.load(std::memory_order_relaxed)) return plan_backward(bits, M, K, N, sms, false, true, false).gw_scratch;
-    return base_plan(bits, M, K, N, sms).gw_scratch;
+    if (g_force_backward.load(std::memory_order_relaxed)) return plan_backward(bits, M, K, N, sms, false, true, false, false).gw_scratch;
+    return base_plan(bits, M, K, N, sms, false).gw_scratch;
 }
 
 int launch_status() {
@@ -332,12 +335,16 @@ int lutgemm_selftest_bounded_wait(void *stream) {
     return lutgemm::bounded_wait_selftest(static_cast<cudaStream_t>(stream));
 }
 
-size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
+size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flags) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false, true, true);
+    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false, true, true, flags & LUTGEMM_SCRATCH_CODES_GIVEN);
     return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch;
+}
+
+size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
+    return lutgemm_backward_ws_scratch_bytes(bits, M, K, N, 0);
 }
 
 static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, float *gw,
@@ -355,9 +362,9 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t given = scratch ? scratch_bytes : 0;
-    BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0, gw != nullptr, ga != nullptr);
+    BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0, gw != nullptr, ga != nullptr, codes_t != nullptr);
     if (((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) && !g_force_backward.load(std::memory_order_relaxed))
-        pl = base_plan(bits, M, K, N, sms);
+        pl = base_plan(bits, M, K, N, sms, codes_t != nullptr);
     float *sc = static_cast<float *>(scratch);
     if (gw) {
         // the weight gradient goes first: under data parallelism its all-reduce can then overlap gA
@@ -585,7 +592,7 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     const int M = g.B * g.Ho * g.Wo, K = g.C * g.kh * g.kw;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true).ga_scratch;
+    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true, false).ga_scratch;
     if (!pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
     size_t need = 0;
     if (gx_uses_slab(bits, g, Cout, sms))
@@ -596,8 +603,8 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     return need;
 }
 
-size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
-                                             int stride, int pad, int dil) {
+size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
+                                                int stride, int pad, int dil, int flags) {
     lutgemm::ConvGeom g{};
     if (!lutgemm::bits_supported(bits) || Cout <= 0 || make_geom(B, C, H, W, kh, kw, stride, pad, dil, &g) != LUTGEMM_OK)
         return 0;
@@ -605,9 +612,14 @@ size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int 
     if (sms <= 0) return 0;
     const int M = B * g.Ho * g.Wo, K = C * kh * kw;
     // the weight-gradient and the activation-gradient kernels run one after the other on the same buffer
-    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false).gw_scratch;
+    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false, flags & LUTGEMM_SCRATCH_CODES_GIVEN).gw_scratch;
     const size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
     return gw_need > gx_need ? gw_need : gx_need;
+}
+
+size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
+                                             int stride, int pad, int dil) {
+    return lutgemm_conv2d_backward_ws_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, 0);
 }
 
 int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,

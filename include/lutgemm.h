@@ -132,7 +132,11 @@ int lutgemm_backward(const float *gc, const uint8_t *a, const uint8_t *w, float 
  * lutgemm_backward with the transposed activation codes that lutgemm_forward_ws left in its workspace for the
  * same `a` (codes_t, [K][M rounded up to 16] uint8; may be NULL): the weight-gradient kernel then skips its own
  * transposition.  Same results.  No counterpart in the reference.
+ * lutgemm_backward_ws_scratch_bytes: as lutgemm_backward_scratch_bytes; LUTGEMM_SCRATCH_CODES_GIVEN in `flags` when
+ * codes_t will be passed, so that the buffer has no room for a copy of them.
  */
+#define LUTGEMM_SCRATCH_CODES_GIVEN 1
+size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flags);
 int lutgemm_backward_ws(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, float *gw,
                         const int16_t *lut_ga, const int16_t *lut_gw, int bits, int M, int K, int N,
                         const uint8_t *codes_t, void *scratch, size_t scratch_bytes, void *stream);
@@ -197,7 +201,8 @@ int lutgemm_conv2d_backward(const float *gy, const uint8_t *x, const uint8_t *wm
  * im2col is written there once, transposed ([C*kh*kw][B*Ho*Wo rounded up to 16]), instead of being gathered
  * by every tile of the main kernel, and stays valid on return.
  * lutgemm_conv2d_backward_ws: as lutgemm_conv2d_backward; `codes_t` (may be NULL) is that buffer as the
- * forward pass of the same layer left it, which saves the weight-gradient kernel its own transposition.
+ * forward pass of the same layer left it, which saves the weight-gradient kernel its own transposition and
+ * (lutgemm_conv2d_backward_ws_scratch_bytes with LUTGEMM_SCRATCH_CODES_GIVEN) the scratch buffer that copy.
  * No counterpart in the reference (it materialises the unfolded activations in fp32, twice).
  */
 size_t lutgemm_conv2d_forward_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
@@ -205,6 +210,8 @@ size_t lutgemm_conv2d_forward_scratch_bytes(int bits, int B, int C, int H, int W
 int lutgemm_conv2d_forward_ws(const uint8_t *x, const uint8_t *wmat, uint32_t *y, const uint16_t *lut, int bits, int B,
                               int C, int H, int W, int Cout, int kh, int kw, int stride, int pad, int dil,
                               void *scratch, size_t scratch_bytes, void *stream);
+size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
+                                                int stride, int pad, int dil, int flags);
 int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
                                const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
                                int Cout, int kh, int kw, int stride, int pad, int dil, const uint8_t *codes_t,

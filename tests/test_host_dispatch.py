@@ -90,3 +90,23 @@ def test_weight_gradient_without_allocation_follows_a_forced_kernel_family(lib):
             assert rc == status and (rc != H.OK or calls[0][0] == "gw_rowbcast_kernel")
     finally:
         lib.lib.lutgemm_set_kernel_choice(0, 0, 0)
+
+
+@pytest.mark.parametrize("bits,B,Cin,Cout,h,k,stride", [(7, 64, 256, 256, 56, 3, 1), (6, 256, 64, 64, 32, 3, 1), (8, 256, 256, 512, 8, 3, 2),
+                                                        (7, 2, 24, 40, 9, 3, 1), (8, 64, 256, 64, 56, 1, 1)])
+def test_backward_scratch_has_no_room_for_codes_that_are_given(lib, bits, B, Cin, Cout, h, k, stride):
+    p, pad, ho = lib.p, k // 2, (h + 2 * (k // 2) - k) // stride + 1
+    M, K = B * ho * ho, Cin * k * k
+    conv = (bits, B, Cin, h, h, Cout, k, k, stride, pad, 1)
+    gemm = (bits, M, K, Cout)
+    for name, shape in (("lutgemm_conv2d_backward", conv), ("lutgemm_backward", gemm)):
+        full, given = (lib.query(name + "_ws_scratch_bytes", *shape, flags) for flags in (0, H.CODES_GIVEN))
+        assert full == lib.query(name + "_scratch_bytes", *shape)
+        assert full >= K * ((M + 15) // 16 * 16) > 0 and given <= full
+        rc, calls = lib.call(name + "_ws", p, p, p, p, p, p, p, *shape, p, p, H.Size(given), None)
+        assert rc == H.OK and not any("transpose" in c[0] for c in calls)
+        rc_full, calls_full = lib.call(name + "_ws", p, p, p, p, p, p, p, *shape, None, p, H.Size(full), None)
+        assert rc_full == H.OK and [c for c in calls_full if "transpose" not in c[0]] == calls
+    # one gradient alone: the copy is all that the two needs differ by
+    gw_full, gw_given = (lib.query("lutgemm_backward_ws_scratch_bytes", bits, M, K, Cout, f) for f in (0, H.CODES_GIVEN))
+    assert gw_full - gw_given <= K * ((M + 15) // 16 * 16) + 15
