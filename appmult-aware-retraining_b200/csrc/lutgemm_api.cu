@@ -86,23 +86,23 @@ constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial su
 
 long div_up(long a, long b) { return (a + b - 1) / b; }
 
-double slab_grad_clocks(long rows, long cols, int K, int rt, int ct, int overhead, double per_step, double start, int sms) {
-    const long blocks = div_up(rows, rt);
-    const lutgemm::KSplit ks = lutgemm::choose_ksplit(blocks * div_up(cols, ct), K, sms, overhead);
-    const double reduce = blocks > 1 ? 8e3 + 8.0 * blocks * K * cols / kReduceBytesPerClock : 0;
-    return (double)ks.waves * (ks.per + overhead) * per_step + start + reduce;
+double packed_clocks(const lutgemm::PackedPlan &p, long cols, int K, double per_step, bool transposed) {
+    const bool reduce = p.groups > 1 || (transposed && p.group_blocks > 1);
+    return (double)p.steps * per_step + kSlabStart + (reduce ? 8e3 + 8.0 * p.groups * K * cols / kReduceBytesPerClock : 0);
 }
 double packed_gw_clocks(int bits, int M, int K, int N, int sms) {
-    return slab_grad_clocks(M, N, K, 512, 64, lutgemm::kPackedGwOverhead, family_clocks(bits).packed_gw, kSlabStart, sms);
+    return packed_clocks(lutgemm::plan_packed_gw(M, N, K, sms), N, K, family_clocks(bits).packed_gw, false);
 }
 double packed_ga_clocks(int bits, int M, int K, int N, int sms) {
     const int rt = lutgemm::packed_ga_tile_rows(bits, N);
     const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
-    return slab_grad_clocks(N, M, K, rt, 64, lutgemm::kPackedItemOverhead, step, kSlabStart, sms);
+    return packed_clocks(lutgemm::plan_packed(N, M, K, rt, sms), M, K, step, true);
 }
 double tall_clocks(int bits, long rows, long cols, int K, int sms) {
-    const FamilyClocks f = family_clocks(bits);
-    return slab_grad_clocks(rows, cols, K, 1024, 32, lutgemm::kTallItemOverhead, f.tall, kSlabStart, sms);
+    const long blocks = div_up(rows, 1024);
+    const lutgemm::KSplit ks = lutgemm::choose_ksplit(blocks * div_up(cols, 32), K, sms, lutgemm::kTallItemOverhead);
+    const double reduce = blocks > 1 ? 8e3 + 8.0 * blocks * K * cols / kReduceBytesPerClock : 0;
+    return (double)ks.waves * (ks.per + lutgemm::kTallItemOverhead) * family_clocks(bits).tall + kSlabStart + reduce;
 }
 double gw_bcast_clocks(int bits, int M, int K, int N, int sms) {
     const long kt = N <= 128 ? 128 : 32, nt = N <= 128 ? 64 : 256, splits = lutgemm::gw_num_splits(bits, M, K, N, sms);
@@ -120,7 +120,7 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bo
     pl.gw_at_offset = 0;
     pl.gw_at_pitch = 0;
     if (pl.gw_slab) {
-        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::slab_packed_row_blocks(M);
+        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::plan_packed_gw(M, N, K, sms).groups;
         pl.gw_scratch = rb > 1 ? (size_t)rb * K * N * sizeof(float) : 0;
         pl.gw_at_pitch = (M + 15) & ~15;
         if (!have_codes) {
@@ -131,10 +131,11 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bo
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
 }
-void set_ga_scratch(BackwardPlan &pl, int bits, int M, int K, int N) {
-    const int rt = lutgemm::packed_ga_tile_rows(bits, N);
-    const int rb = !pl.ga_slab ? 1 : pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : (N + rt - 1) / rt;
-    pl.ga_scratch = rb > 1 ? (size_t)rb * K * M * sizeof(float) : 0;
+void set_ga_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms) {
+    if (!pl.ga_slab) return;
+    const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(bits, N);
+    const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::plan_packed(N, M, K, rt, sms).groups;
+    pl.ga_scratch = N > rt ? (size_t)blocks * K * M * sizeof(float) : 0;
 }
 
 // Choice by fixed limits: the plan for callers whose scratch buffer is too small for the faster one (a fixed buffer, or
@@ -147,7 +148,7 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) 
     pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
     set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
-    set_ga_scratch(pl, bits, M, K, N);
+    set_ga_scratch(pl, bits, M, K, N, sms);
     return pl;
 }
 
@@ -171,7 +172,7 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
         pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_ga_scratch(pl, bits, M, K, N);
+        set_ga_scratch(pl, bits, M, K, N, sms);
     }
     return pl;
 }
@@ -551,7 +552,7 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(bits, rows);
-        slab += slab_grad_clocks(rows, px.P, px.C, rt, 64, lutgemm::kPackedItemOverhead, f.packed * (rt > 512 ? 1.12 : 1.0), kSlabStart, sms);
+        slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, f.packed * (rt > 512 ? 1.12 : 1.0), false);
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
             return;
@@ -597,7 +598,7 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     size_t need = 0;
     if (gx_uses_slab(bits, g, Cout, sms))
         for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
-            const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B);
+            const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B, sms);
             need = n > need ? n : need;
         });
     return need;

@@ -65,9 +65,50 @@ inline KSplit choose_ksplit(long tiles, int K, int num_sms, int item_overhead) {
 // in k steps: operand fetch, grad_out block (gathered in grad_a and grad_x), first slabs
 constexpr int kPackedGwOverhead = 5, kPackedItemOverhead = 10, kTallItemOverhead = 4;
 
-// rows of the reduction dimension per CTA tile of the packed-slab gradient kernels, and the block count
+// rows of the reduction dimension per CTA tile of the packed-slab gradient kernels
 constexpr int kSlabPackedRows = 512;
-int slab_packed_row_blocks(int rdim);
+// How the packed gradient kernels deal out their work.  The row blocks of a column tile are cut into groups of
+// group_blocks; one CTA adds up a group's blocks in turn, so a group needs one block of partial sums.  A cell is (group,
+// column tile): the first main_cells of them, whole rounds of the persistent grid, are taken with their whole K, the
+// others with K cut (outputs are per k) so that the last round is full too.
+struct PackedPlan {
+    int groups, group_blocks;
+    int main_cells, tail_parts, tail_per;
+    long steps;  // k steps of the CTA that has most to do
+};
+inline PackedPlan deal_cells(long groups, long blocks, long tiles_c, int K, int num_sms, int item_overhead) {
+    const long cells = groups * tiles_c, rounds = cells / num_sms, tail = cells % num_sms;
+    const int whole = (K + 15) / 16 * 16;
+    PackedPlan p{(int)groups, (int)blocks, (int)(rounds * num_sms), 1, whole, rounds * (whole + item_overhead)};
+    if (tail) {
+        const KSplit ks = choose_ksplit(tail, K, num_sms, item_overhead);
+        p.tail_parts = ks.parts;
+        p.tail_per = ks.per;
+        p.steps += ks.waves * (ks.per + item_overhead);
+    }
+    p.steps *= blocks;
+    return p;
+}
+// Where the tiles fill the GPU anyway, the largest groups that cost no time: one block of sums per row block made the
+// buffer grow with the rows (0.9 GB for grad_w and 0.8 GB for the image gradient of a 3x3 layer of 256 channels at
+// 56 x 56, batch 64).  Fewer blocks of sums save their reading (4 bytes at 4000 per clock, a step is about 1500 clocks).
+inline PackedPlan plan_packed(long rdim, long cdim, int K, int tile_rows, int num_sms, int item_overhead = kPackedItemOverhead,
+                              long most_blocks = 1L << 30) {
+    const long tiles_r = (rdim + tile_rows - 1) / tile_rows, tiles_c = (cdim + 63) / 64;
+    const PackedPlan alone = deal_cells(tiles_r, 1, tiles_c, K, num_sms, item_overhead);
+    if (tiles_r * tiles_c < num_sms) return alone;
+    for (long blocks = tiles_r < most_blocks ? tiles_r : most_blocks; blocks > 1; --blocks) {
+        const long groups = (tiles_r + blocks - 1) / blocks;
+        if ((tiles_r + groups - 1) / groups < blocks) continue;  // as many groups of fewer blocks
+        const PackedPlan p = deal_cells(groups, blocks, tiles_c, K, num_sms, item_overhead);
+        if (p.steps <= alone.steps + alone.steps / 256 + (tiles_r - groups) * tiles_c * K / 23400) return p;
+    }
+    return alone;
+}
+// (grad_w: at most 16 blocks in a chain of additions, so that a long sum is still added up in two levels)
+inline PackedPlan plan_packed_gw(long M, long N, int K, int num_sms) {
+    return plan_packed(M, N, K, kSlabPackedRows, num_sms, kPackedGwOverhead, 16);
+}
 int packed_ga_tile_rows(int bits, int N);  // grad_a: rows of its tile (384, 512 or 576)
 // gradient slab kernels with 16-bit slab entries (converted where they are used)
 // `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
@@ -100,7 +141,7 @@ int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks,
 // activation gradient of a convolution for the input pixels of one stride class, written into gx[B,C,H,W]
 // (packed slab kernel in pixel mode: no unfolded gradient, no col2im); scratch: gx_class_scratch_bytes()
 int gx_tile_rows(int bits, long rdim);  // rows of its tile for a class of rdim = taps * Cout rows
-size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B);
+size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B, int num_sms);
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
                       int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream);
 // the same with the column-broadcast gather kernel (whole table in shared memory, no slab) for `nclasses` stride

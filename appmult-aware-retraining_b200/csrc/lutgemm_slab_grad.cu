@@ -27,8 +27,11 @@
 // Hand-over between the warps of a CTA: per slab buffer a "full" and an "empty" mbarrier with one arrival per warp
 // (see lutgemm_slab_grad_tall.cu); at 7 bits and below a buffer holds the slabs of two k, so that waits, arrivals and
 // loop overhead are paid once per two k.  Every wait is bounded (lutgemm_waits.cuh).
-// Partial sums: one per lane group, warp and k; one warp (rotating with k) adds the 32 of a column in ascending order,
-// row blocks are added by slab_reduce_blocks in ascending order: results are deterministic.
+// Partial sums: one per lane group, warp and k; one warp (rotating with k) adds the 32 of a column in ascending order.
+// A CTA takes the row blocks of a group one after the other and adds each to the group's sums in ascending order (the
+// same thread stores and adds, so the reductions need no ordering between threads); groups are added by slab_reduce_blocks
+// in ascending order: results are deterministic.  With one block of sums per row block the buffer grew with the rows: 0.82
+// GB for the image gradient of a 3x3 layer of 256 channels at 56 x 56, batch 64, 7 bits, which now needs none.
 // Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492, and for
 // grad_x the unfold backward of self_ops/ops_py/approx_ops.py:556-571.
 #include <type_traits>
@@ -110,8 +113,9 @@ struct Args {
     int M, K, N;               // kGx: M = pixels of the class (all images), K = channels, N = Cout
     int RDIM, CDIM;
     int tiles_r, tiles_c;
-    int ksplits, k_per_split;  // a tile's k range is cut into independent work items (outputs are per k)
-    int direct;
+    int groups, group_blocks;  // row blocks are dealt to groups, each summed up by one CTA per column tile and k range
+    int main_cells, tail_parts, tail_per;  // cells (group, column tile) with their whole K, and how K is cut for the others
+    int direct;                // one group, and its sums go to their final place
     int vec_a, vec_w, vec_g;
     ConvGeom conv;
     int ga_scatter;     // grad_a of a convolution whose windows do not overlap: results go straight to the image
@@ -289,14 +293,15 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             }
         }
     };
-    // add the 32 partial sums of one k in ascending order and store the tile's 64 columns (two per lane)
-    auto reduce_store = [&](int k, const float *ps, float *obase, int c0) {
+    // add the 32 partial sums of one k in ascending order and store the tile's 64 columns (two per lane), or add them to
+    // what this thread has stored for the row blocks before (reductions: nothing waits for the old value)
+    auto reduce_store = [&](int k, const float *ps, float *obase, int c0, bool add) {
         const f32x2 *p2 = reinterpret_cast<const f32x2 *>(ps) + lane;
         f32x2 v = p2[0];
 #pragma unroll 8
         for (int i = 1; i < 2 * WARPS; ++i) v = add2(v, p2[i * (CT / 2)]);
         float2 o = unpack2(v);
-        if (p.direct) {
+        if (p.direct) {  // (a power of two: the same sum whether it is scaled before or after)
             o.x *= kGradFactor;
             o.y *= kGradFactor;
         }
@@ -307,7 +312,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 if (col + e >= CDIM) break;
                 const float ov = e ? o.y : o.x;
                 if (MODE == kGx) {
-                    obase[pix_s[2 * lane + e] + (long long)k * p.px.H * p.px.W] = ov;
+                    float *dst = obase + (pix_s[2 * lane + e] + (long long)k * p.px.H * p.px.W);
+                    if (add) atomicAdd(dst, ov);
+                    else *dst = ov;
                 } else if (p.ga_scatter) {
                     const long ix = conv_scatter_index(p.conv, col + e, k);
                     if (ix >= 0) obase[ix] = ov;
@@ -319,7 +326,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
         float *dst = obase + (size_t)k * CDIM + col;
         if (col + 1 < CDIM && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-            *reinterpret_cast<float2 *>(dst) = o;
+            if (add) atomicAdd(reinterpret_cast<float2 *>(dst), o);
+            else *reinterpret_cast<float2 *>(dst) = o;
+        } else if (add) {
+            if (col < CDIM) atomicAdd(dst, o.x);
+            if (col + 1 < CDIM) atomicAdd(dst + 1, o.y);
         } else {
             if (col < CDIM) dst[0] = o.x;
             if (col + 1 < CDIM) dst[1] = o.y;
@@ -330,13 +341,20 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     const uint32_t wsel0 = (uint32_t)C::U_ROW << (16 * half), wsel1 = wsel0 << 8;  // dot-product weights of the lane's two rows
     static_assert(C::U_ROW < 256, "slab row stride must fit one byte of the dot-product operand");
 
-    const int items = p.tiles_r * p.tiles_c * p.ksplits;
+    const int items = p.main_cells + (p.groups * p.tiles_c - p.main_cells) * p.tail_parts;
     bool first_item = true;
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int tile = item / p.ksplits;
-        const int kbeg = (item % p.ksplits) * p.k_per_split, kend = min(K, kbeg + p.k_per_split);
-        const int tr = tile / p.tiles_c, tc = tile % p.tiles_c;
+    for (int item = blockIdx.x, block = 0; item < items;) {  // `block`: row block within the group
+        int cell = item, kbeg = 0, kend = K;
+        if (item >= p.main_cells) {
+            const int j = item - p.main_cells;
+            cell = p.main_cells + j / p.tail_parts;
+            kbeg = (j % p.tail_parts) * p.tail_per;
+            kend = min(K, kbeg + p.tail_per);
+        }
+        const int group = cell / p.tiles_c, tc = cell % p.tiles_c;
+        const int tr = group * p.group_blocks + block;
         const int r0 = tr * RT, c0 = tc * CT;
+        const bool add = block > 0;
 
         // kbeg is a multiple of 16, so the first stage is half 0 of its group
         fetch_group(r0, c0, kbeg / KC, true);
@@ -459,7 +477,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             mbar_arrive(bar_empty + 8 * (NB - 1));
         }
 
-        float *obase = p.out + (p.direct ? (size_t)0 : (size_t)tr * K * CDIM);
+        float *obase = p.out + (p.direct ? (size_t)0 : (size_t)group * K * CDIM);
 
         const uint32_t uc = u_addr + cq * 8;
         f32x2 acc[2][2];  // [row parity j][column pair i]
@@ -552,7 +570,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 mbar_wait(bar_empty + 8 * prev, par, 1 + NB + prev, abort_word, p.error_word);
                 if (k > kbeg && ((wp ^ (k - KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
                     const int i = wp & (KP - 1);
-                    reduce_store(k - KP + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0);
+                    reduce_store(k - KP + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0, add);
                 }
                 if (k + AHEAD * KP < kend) {
                     build_unit(prev, cb_, k + AHEAD * KP + 1 < kend);
@@ -578,7 +596,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             const int kl = kend - 1 - (kend - 1 - kbeg) % KP;  // first k of the last unit, in buffer prev
             const int i = wp & (KP - 1);
             if (kl + i < kend && ((wp ^ kl) & (WARPS - KP)) == 0)
-                reduce_store(kl + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0);
+                reduce_store(kl + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0, add);
+        }
+        if (++block == p.group_blocks || tr + 1 == p.tiles_r) {
+            block = 0;
+            item += gridDim.x;
         }
     }
 }
@@ -611,13 +633,16 @@ int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStrea
     if (!p.error_word) return LUTGEMM_E_CUDA;
     p.tiles_r = (p.RDIM + C::RT - 1) / C::RT;
     p.tiles_c = (p.CDIM + C::CT - 1) / C::CT;
-    p.direct = p.tiles_r == 1;
+    const PackedPlan pp = MODE == sp::kGw ? plan_packed_gw(p.RDIM, p.CDIM, p.K, num_sms) : plan_packed(p.RDIM, p.CDIM, p.K, C::RT, num_sms);
+    p.groups = pp.groups;
+    p.group_blocks = pp.group_blocks;
+    // (grad_a is transposed on its way to its final place, by the reduction over the groups)
+    p.direct = p.tiles_r == 1 || (MODE != sp::kGa && p.groups == 1);
     p.out = p.direct ? out : scratch;
-    const long tiles = (long)p.tiles_r * p.tiles_c;
-    const KSplit ks = choose_ksplit(tiles, p.K, num_sms, MODE == sp::kGw ? kPackedGwOverhead : kPackedItemOverhead);
-    p.ksplits = ks.parts;
-    p.k_per_split = ks.per;
-    const long items = tiles * ks.parts;
+    p.main_cells = pp.main_cells;
+    p.tail_parts = pp.tail_parts;
+    p.tail_per = pp.tail_per;
+    const long items = pp.main_cells + ((long)p.groups * p.tiles_c - pp.main_cells) * pp.tail_parts;
     const int grid = (int)(items < num_sms ? items : num_sms);
     kern<<<grid, C::THREADS, C::SMEM, stream>>>(p);
     return launch_status();
@@ -649,9 +674,9 @@ int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, floa
         rc = launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
     }
     if (rc != LUTGEMM_OK) return rc;
-    const int tiles_r = (p.RDIM + rt - 1) / rt;
-    if (tiles_r > 1)
-        return slab_reduce_blocks(scratch, out, K, p.CDIM, tiles_r, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
+    const int groups = MODE == sp::kGw ? plan_packed_gw(M, N, K, num_sms).groups : plan_packed(N, M, K, rt, num_sms).groups;
+    if (MODE == sp::kGw ? groups > 1 : p.RDIM > rt)
+        return slab_reduce_blocks(scratch, out, K, p.CDIM, groups, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
                                   kGradFactor, num_sms, stream);
     return LUTGEMM_OK;
 }
@@ -668,18 +693,16 @@ int launch_packed_gx(const float *gy, const uint8_t *x, const uint8_t *wmat, flo
     p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
     p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
     const int rw = gx_tile_rows(BITS, p.RDIM) / 16;
+    const int groups = plan_packed(p.RDIM, p.CDIM, p.K, 16 * rw, num_sms).groups;
     const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, gx, scratch, num_sms, stream)
                             : launch_packed<BITS, sp::kGx, 32>(p, gx, scratch, num_sms, stream);
     if (rc != LUTGEMM_OK) return rc;
-    const int tiles_r = (p.RDIM + 16 * rw - 1) / (16 * rw);
-    if (tiles_r > 1)
-        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, tiles_r, false, nullptr, &px, kGradFactor, num_sms, stream);
+    if (groups > 1)
+        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, groups, false, nullptr, &px, kGradFactor, num_sms, stream);
     return LUTGEMM_OK;
 }
 
 }  // namespace
-
-int slab_packed_row_blocks(int rdim) { return (rdim + kSlabPackedRows - 1) / kSlabPackedRows; }
 
 int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
                             int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
@@ -705,10 +728,10 @@ int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w,
     return LUTGEMM_E_BITS;
 }
 
-size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B) {
-    const long rdim = (long)px.ntaps * Cout, rt = gx_tile_rows(bits, rdim);
-    const long tiles_r = (rdim + rt - 1) / rt;
-    return tiles_r > 1 ? (size_t)tiles_r * px.C * ((size_t)B * px.Hc * px.Wc) * sizeof(float) : 0;
+size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B, int num_sms) {
+    const long rdim = (long)px.ntaps * Cout, cdim = (long)B * px.Hc * px.Wc;
+    const int groups = plan_packed(rdim, cdim, px.C, gx_tile_rows(bits, rdim), num_sms).groups;
+    return groups > 1 ? (size_t)groups * px.C * cdim * sizeof(float) : 0;
 }
 
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,

@@ -82,11 +82,27 @@ def test_gradients_at_the_edges_of_tiles_and_stages(dev, oracle_c, packed, bits,
     check(gw, r_gw, r_gwa)
 
 
+@pytest.mark.parametrize("bits,M,K,N", [(4, 130300, 33, 20), (6, 130300, 33, 20), (7, 130300, 33, 20), (8, 130300, 33, 20),
+                                        (7, 11015, 66, 700), (8, 11015, 66, 700)])
+def test_gradients_with_several_row_blocks_per_cta(dev, oracle_c, packed, bits, M, K, N):
+    """grad_w with two row blocks added up in each of 128 groups, the last one short; grad_a with both of its row blocks added up,
+    whole rounds of tiles and a last round with K cut.  The order of the additions is fixed: a second run is identical."""
+    la, lw = full_range_tables(bits, 11 * bits)
+    a, w, gc = problem(bits, M, K, N, bits + M)
+    ga, gw = backward(dev, gc, a, w, la, lw)
+    ga2, gw2 = backward(dev, gc, a, w, la, lw)
+    assert np.array_equal(ga, ga2) and np.array_equal(gw, gw2)
+    r_ga, r_gw, r_gaa, r_gwa = oracle_c.backward_f64(gc, a, w, la, lw, bits)
+    check(ga, r_ga, r_gaa)
+    check(gw, r_gw, r_gwa)
+
+
 @pytest.mark.parametrize("bits", [4, 6, 7, 8])
 @pytest.mark.parametrize("B,Cin,H,Cout,k,st,p", [(1, 5, 9, 64, 3, 1, 1), (2, 33, 6, 128, 3, 1, 1), (1, 18, 7, 63, 3, 1, 1),
-                                                 (1, 16, 9, 256, 3, 2, 1)])
+                                                 (1, 16, 9, 256, 3, 2, 1), (37, 20, 16, 128, 3, 1, 1), (4, 18, 40, 128, 3, 1, 1)])
 def test_image_gradient_of_convolutions(dev, oracle_c, packed, bits, B, Cin, H, Cout, k, st, p):
-    """576-row tiles (one and two of them, and a partly filled one) and the stride classes of a stride-2 convolution."""
+    """576-row tiles (one and two of them, and a partly filled one), the stride classes of a stride-2 convolution; 148 pixel
+    tiles whose two row blocks one CTA adds up, and more work items than SMs, so that a CTA takes a second one."""
     import approx_ops
     la, lw = full_range_tables(bits, 5 * bits)
     rng = np.random.default_rng(bits + Cin + Cout)

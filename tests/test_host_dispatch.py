@@ -110,3 +110,20 @@ def test_backward_scratch_has_no_room_for_codes_that_are_given(lib, bits, B, Cin
     # one gradient alone: the copy is all that the two needs differ by
     gw_full, gw_given = (lib.query("lutgemm_backward_ws_scratch_bytes", bits, M, K, Cout, f) for f in (0, H.CODES_GIVEN))
     assert gw_full - gw_given <= K * ((M + 15) // 16 * 16) + 15
+
+
+def test_plan_of_the_packed_gradient_kernels_covers_its_work(tmp_path):
+    exe = str(tmp_path / "plan")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-o", exe, os.path.join(HERE, "packed_plan_check.cpp"), "-I",
+                    os.path.join(H.ROOT, "appmult-aware-retraining_b200", "csrc"), "-I", os.path.join(H.ROOT, "include"), "-I",
+                    os.path.join(cuda, "include")], check=True)
+    res = subprocess.run([exe], capture_output=True, text=True)
+    assert res.returncode == 0, res.stdout
+
+
+@pytest.mark.parametrize("bits,B,C,h", [(7, 64, 256, 56), (7, 256, 256, 56), (7, 64, 512, 28), (6, 256, 64, 32), (4, 1024, 64, 32)])
+def test_image_gradient_needs_no_partial_sums_and_weight_gradient_one_block_per_1024_rows(lib, bits, B, C, h):
+    """3x3 layers of C channels whose pixel tiles fill the GPU."""
+    need = lib.query("lutgemm_conv2d_backward_ws_scratch_bytes", bits, B, C, h, h, C, 3, 3, 1, 1, 1, H.CODES_GIVEN)
+    assert need <= (B * h * h + 1023) // 1024 * 9 * C * C * 4
