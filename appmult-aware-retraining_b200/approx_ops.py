@@ -132,7 +132,8 @@ def library():
 _FORWARD_CHOICES = {"auto": 0, "rowbcast": 1, "slab": 2}
 _BACKWARD_CHOICES = {"auto": 0, "bcast": 1, "slab": 2}
 _TILE_CHOICES = {"auto": 0, "wide": 1, "tall": 2}
-_CODES_GIVEN = 1  # LUTGEMM_SCRATCH_CODES_GIVEN
+_CODES_GIVEN, _LEAST = 1, 2  # LUTGEMM_SCRATCH_CODES_GIVEN, LUTGEMM_SCRATCH_LEAST
+_E_SCRATCH = -4
 
 
 def set_kernel_choice(forward: str = "auto", backward: str = "auto", grad_tile: str = "auto") -> None:
@@ -189,6 +190,34 @@ def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def _backward_scratch(query, args, codes_t, dev):
+    """(buffer, bytes) of a backward call: what the fastest kernels want, or, where that cannot be had, the least that the
+    library accepts (a training step that just fits the device then runs on slower kernels)."""
+    flags = _CODES_GIVEN if codes_t is not None else 0
+    nbytes = query(*args, flags)
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes
+    except torch.OutOfMemoryError:
+        least = query(*args, flags | _LEAST)
+        if least >= nbytes:
+            raise
+        return torch.empty(least, dtype=torch.uint8, device=dev), least
+
+
+def _forward_workspace(nbytes: int, dev):
+    """(buffer or None, bytes, error) of a forward call, which can do without one unless the library says otherwise."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None, nbytes, None
+    except torch.OutOfMemoryError as e:
+        return None, 0, e.with_traceback(None)
+
+
+def _check_forward(rc: int, short, what: str) -> None:
+    if short is not None and rc == _E_SCRATCH:
+        raise short
+    _check(rc, what)
+
+
 def approx_gemm_forward(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, lut: torch.Tensor):
     """c[m,n] = sum_k lut[a[m,k]*(2^bits+2) + b[k,n]], written in place into the uint32 tensor c.
     Returns the transposed activation codes the kernel worked from (a uint8 tensor that
@@ -218,11 +247,10 @@ def approx_gemm_forward(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, lut: 
     lib = _load()
     with torch.cuda.device(dev):
         # workspace for the transposed activation codes (0 bytes when the kernel for this shape has no use for it)
-        nbytes = lib.lutgemm_forward_scratch_bytes(bits, M, K, N)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        scratch, nbytes, short = _forward_workspace(lib.lutgemm_forward_scratch_bytes(bits, M, K, N), dev)
         rc = lib.lutgemm_forward_ws(a.data_ptr(), b.data_ptr(), c.data_ptr(), lut.data_ptr(), bits, M, K, N,
                                     scratch.data_ptr() if nbytes else None, nbytes, _stream_ptr(dev))
-    _check(rc, "approx_gemm_forward")
+    _check_forward(rc, short, "approx_gemm_forward")
     return scratch
 
 
@@ -261,8 +289,7 @@ def approx_gemm_backward(gc: torch.Tensor, a: torch.Tensor, b: torch.Tensor, ga:
         return
     lib = _load()
     with torch.cuda.device(dev):
-        nbytes = lib.lutgemm_backward_ws_scratch_bytes(bits, M, K, N, _CODES_GIVEN if codes_t is not None else 0)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        scratch, nbytes = _backward_scratch(lib.lutgemm_backward_ws_scratch_bytes, (bits, M, K, N), codes_t, dev)
         if codes_t is not None:
             _check_input(codes_t, torch.uint8, "codes_t")
             if codes_t.numel() != K * ((M + 15) // 16 * 16):
@@ -270,7 +297,7 @@ def approx_gemm_backward(gc: torch.Tensor, a: torch.Tensor, b: torch.Tensor, ga:
         rc = lib.lutgemm_backward_ws(gc.data_ptr(), a.data_ptr(), b.data_ptr(), ga.data_ptr(), gb.data_ptr(),
                                      lut_grad_a.data_ptr(), lut_grad_b.data_ptr(), bits, M, K, N,
                                      codes_t.data_ptr() if codes_t is not None else None,
-                                     scratch.data_ptr() if scratch is not None else None, nbytes, _stream_ptr(dev))
+                                     scratch.data_ptr(), nbytes, _stream_ptr(dev))
     _check(rc, "approx_gemm_backward")
 
 
@@ -318,11 +345,11 @@ def approx_conv2d_forward(x: torch.Tensor, wmat: torch.Tensor, y: torch.Tensor, 
     lib = _load()
     with torch.cuda.device(x.device):
         nbytes = lib.lutgemm_conv2d_forward_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
-        codes_t = torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+        codes_t, nbytes, short = _forward_workspace(nbytes, x.device)
         rc = lib.lutgemm_conv2d_forward_ws(x.data_ptr(), wmat.data_ptr(), y.data_ptr(), lut.data_ptr(), bits, B, C, H,
                                            W, Cout, kh, kw, stride, pad, dil, codes_t.data_ptr() if nbytes else None,
                                            nbytes, _stream_ptr(x.device))
-    _check(rc, "approx_conv2d_forward")
+    _check_forward(rc, short, "approx_conv2d_forward")
     return codes_t
 
 
@@ -357,12 +384,12 @@ def approx_conv2d_forward_layer(x: torch.Tensor, wmat: torch.Tensor, lut: torch.
     with torch.cuda.device(x.device):
         ncodes = lib.lutgemm_conv2d_forward_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
         nbytes = lib.lutgemm_conv2d_forward_layer_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+        scratch, nbytes, short = _forward_workspace(nbytes, x.device)
         rc = lib.lutgemm_conv2d_forward_layer(x.data_ptr(), wmat.data_ptr(), lut.data_ptr(), bits, B, C, H, W, Cout, kh, kw,
                                               stride, pad, dil, *epi, out.data_ptr(),
                                               scratch.data_ptr() if nbytes else None, nbytes, _stream_ptr(x.device))
-    _check(rc, "approx_conv2d_forward_layer")
-    return out, (scratch[:ncodes] if ncodes else None)
+    _check_forward(rc, short, "approx_conv2d_forward_layer")
+    return out, (scratch[:ncodes] if ncodes and nbytes else None)
 
 
 def conv2d_layer_pass(x: torch.Tensor, weight: torch.Tensor, bias, quant: torch.Tensor, a_qmax: float, w_qmax: float,
@@ -396,14 +423,14 @@ def conv2d_layer_pass(x: torch.Tensor, weight: torch.Tensor, bias, quant: torch.
         wmat = torch.empty((C * kh * kw, Cout), dtype=torch.uint8, device=dev)
         out = torch.empty((B * Ho * Wo, Cout), dtype=torch.float32, device=dev)
         work = torch.empty(lib.lutgemm_conv2d_layer_work_floats(*geom), dtype=torch.float32, device=dev)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        scratch, nbytes, short = _forward_workspace(nbytes, dev)
         rc = lib.lutgemm_conv2d_layer_pass(x.data_ptr(), *x.stride(), weight.data_ptr(), *weight.stride(),
                                            bias.data_ptr() if bias is not None else None, quant.data_ptr(), float(a_qmax),
                                            float(w_qmax), lut.data_ptr(), bits, *geom, codes.data_ptr(), wmat.data_ptr(),
                                            out.data_ptr(), work.data_ptr(), scratch.data_ptr() if nbytes else None, nbytes,
                                            _stream_ptr(dev))
-    _check(rc, "conv2d_layer_pass")
-    return out, codes, wmat, (scratch[:ncodes] if ncodes else None)
+    _check_forward(rc, short, "conv2d_layer_pass")
+    return out, codes, wmat, (scratch[:ncodes] if ncodes and nbytes else None)
 
 
 def approx_gemm_forward_layer(a: torch.Tensor, b: torch.Tensor, lut: torch.Tensor, box, sumw_t, taps, s_a, s_w, z_a, z_w,
@@ -424,11 +451,11 @@ def approx_gemm_forward_layer(a: torch.Tensor, b: torch.Tensor, lut: torch.Tenso
     with torch.cuda.device(a.device):
         ncodes = lib.lutgemm_forward_scratch_bytes(bits, M, K, N)
         nbytes = lib.lutgemm_forward_layer_scratch_bytes(bits, M, K, N)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+        scratch, nbytes, short = _forward_workspace(nbytes, a.device)
         rc = lib.lutgemm_forward_layer(a.data_ptr(), b.data_ptr(), lut.data_ptr(), bits, M, K, N, *epi, out.data_ptr(),
                                        scratch.data_ptr() if nbytes else None, nbytes, _stream_ptr(a.device))
-    _check(rc, "approx_gemm_forward_layer")
-    return out, (scratch[:ncodes] if ncodes else None)
+    _check_forward(rc, short, "approx_gemm_forward_layer")
+    return out, (scratch[:ncodes] if ncodes and nbytes else None)
 
 
 def approx_conv2d_backward(gy: torch.Tensor, x: torch.Tensor, wmat: torch.Tensor, gx: torch.Tensor, gw: torch.Tensor,
@@ -462,9 +489,8 @@ def approx_conv2d_backward(gy: torch.Tensor, x: torch.Tensor, wmat: torch.Tensor
             raise RuntimeError("All tensors should be on the same device")
     lib = _load()
     with torch.cuda.device(dev):
-        nbytes = lib.lutgemm_conv2d_backward_ws_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil,
-                                                              _CODES_GIVEN if codes_t is not None else 0)
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        scratch, nbytes = _backward_scratch(lib.lutgemm_conv2d_backward_ws_scratch_bytes,
+                                            (bits, B, C, H, W, Cout, kh, kw, stride, pad, dil), codes_t, dev)
         if codes_t is not None:
             _check_input(codes_t, torch.uint8, "codes_t")
             if codes_t.numel() != K * ((B * Ho * Wo + 15) // 16 * 16):

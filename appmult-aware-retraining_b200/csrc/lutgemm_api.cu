@@ -336,12 +336,19 @@ int lutgemm_selftest_bounded_wait(void *stream) {
     return lutgemm::bounded_wait_selftest(static_cast<cudaStream_t>(stream));
 }
 
+static size_t larger_need(const BackwardPlan &pl) { return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch; }
+// of a buffer for the faster choice and one for the fixed limits, the smaller one that is accepted
+static size_t least_need(size_t need, size_t base) {
+    return base < need && !g_force_backward.load(std::memory_order_relaxed) ? base : need;
+}
+
 size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flags) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    const BackwardPlan pl = plan_backward(bits, M, K, N, sms, false, true, true, flags & LUTGEMM_SCRATCH_CODES_GIVEN);
-    return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch;
+    const bool have_codes = flags & LUTGEMM_SCRATCH_CODES_GIVEN;
+    const size_t need = larger_need(plan_backward(bits, M, K, N, sms, false, true, true, have_codes));
+    return flags & LUTGEMM_SCRATCH_LEAST ? least_need(need, larger_need(base_plan(bits, M, K, N, sms, have_codes))) : need;
 }
 
 size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
@@ -613,8 +620,14 @@ size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, i
     if (sms <= 0) return 0;
     const int M = B * g.Ho * g.Wo, K = C * kh * kw;
     // the weight-gradient and the activation-gradient kernels run one after the other on the same buffer
-    const size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false, flags & LUTGEMM_SCRATCH_CODES_GIVEN).gw_scratch;
-    const size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
+    const bool have_codes = flags & LUTGEMM_SCRATCH_CODES_GIVEN;
+    size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false, have_codes).gw_scratch;
+    size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
+    if (flags & LUTGEMM_SCRATCH_LEAST) {
+        const BackwardPlan base = base_plan(bits, M, K, Cout, sms, have_codes);
+        gw_need = least_need(gw_need, base.gw_scratch);
+        gx_need = least_need(gx_need, conv_windows_overlap(g) ? gx_base_scratch_bytes(bits, g, Cout) : base.ga_scratch);
+    }
     return gw_need > gx_need ? gw_need : gx_need;
 }
 

@@ -133,9 +133,11 @@ int lutgemm_backward(const float *gc, const uint8_t *a, const uint8_t *w, float 
  * same `a` (codes_t, [K][M rounded up to 16] uint8; may be NULL): the weight-gradient kernel then skips its own
  * transposition.  Same results.  No counterpart in the reference.
  * lutgemm_backward_ws_scratch_bytes: as lutgemm_backward_scratch_bytes; LUTGEMM_SCRATCH_CODES_GIVEN in `flags` when
- * codes_t will be passed, so that the buffer has no room for a copy of them.
+ * codes_t will be passed, so that the buffer has no room for a copy of them; LUTGEMM_SCRATCH_LEAST for the smallest
+ * buffer that is accepted instead of the one for the fastest kernels.
  */
 #define LUTGEMM_SCRATCH_CODES_GIVEN 1
+#define LUTGEMM_SCRATCH_LEAST 2
 size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flags);
 int lutgemm_backward_ws(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, float *gw,
                         const int16_t *lut_ga, const int16_t *lut_gw, int bits, int M, int K, int N,

@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 OBJ_DIR = os.path.join(ROOT, "appmult-aware-retraining_b200", "build")
 
 OK, E_BADARG, E_BITS, E_SCRATCH, E_TOOLARGE = 0, -1, -2, -4, -5
-CODES_GIVEN = 1
+CODES_GIVEN, LEAST = 1, 2
 
 
 def build(out_dir) -> str:

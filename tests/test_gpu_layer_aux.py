@@ -149,3 +149,51 @@ def test_layer_pass_refuses_operands_it_cannot_read(dev, operand):
                                              b if operand == "quant" else good["quant"], 127.0)
     assert approx_ops.library().lutgemm_kernel_launches() == launches
     layer_pass(good)
+
+
+def test_a_layer_runs_on_slower_kernels_where_the_fast_ones_do_not_fit(dev, monkeypatch):
+    """Workspaces beyond 64 kilobytes cannot be had (an allocator that says so): the operator, a convolution and a
+    linear layer give the results of the kernels that need less; what no kernel can do without is an error as before."""
+    import approx_ops
+    import self_ops
+    from lutgemm_layers import AppConv2d, AppLinear
+    from lutgemm_luts import synthetic_multiplier, window_difference_gradients
+    fp = synthetic_multiplier(7, seed=0)
+    self_ops.set_lookup_tables(dev, fp, *window_difference_gradients(fp, 8), 7)
+    torch.manual_seed(0)
+    conv = AppConv2d(64, 128, 3, 1, 1, bias=True, a_bits=7, w_bits=7, conv_impl="layer").to(dev).train()
+    lin = AppLinear(300, 700, a_bits=7, w_bits=7, impl="layer").to(dev).train()
+    x, y = torch.rand(4, 64, 10, 10, device=dev), torch.randn(350, 300, device=dev)
+    a = torch.randint(0, 128, (400, 200), device=dev).float()
+    w = torch.randint(0, 128, (200, 600), device=dev).float()
+
+    def run():
+        out = []
+        for f, args in ((conv, (x,)), (lin, (y,)), (self_ops.approx_gemm_op, (a, w))):
+            args = [t.clone().requires_grad_(True) for t in args]
+            conv.zero_grad()
+            lin.zero_grad()
+            r = f(*args)
+            r.backward(torch.ones_like(r))
+            out += [r.detach()] + [t.grad for t in args] + [p.grad.clone() for m in (conv, lin) for p in m.parameters() if p.grad is not None]
+        return out
+
+    want = run()
+    empty, refused = torch.empty, []
+
+    def short(*size, **kw):
+        n = size[0] if isinstance(size[0], int) else 0
+        if kw.get("dtype") == torch.uint8 and len(size) == 1 and n > 1 << 16:
+            refused.append(n)
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", short)
+    got = run()
+    assert len(refused) >= 6
+    for g, r in zip(got, want):
+        assert torch.linalg.vector_norm(g - r) <= 1e-5 * torch.linalg.vector_norm(r)
+    # 4096 rows: the weight gradient needs its code copy under either choice
+    a = torch.randint(0, 128, (4096, 200), device=dev).float().requires_grad_(True)
+    r = self_ops.approx_gemm_op(a, w.requires_grad_(True))
+    with pytest.raises(torch.OutOfMemoryError):
+        r.sum().backward()

@@ -127,3 +127,19 @@ def test_image_gradient_needs_no_partial_sums_and_weight_gradient_one_block_per_
     """3x3 layers of C channels whose pixel tiles fill the GPU."""
     need = lib.query("lutgemm_conv2d_backward_ws_scratch_bytes", bits, B, C, h, h, C, 3, 3, 1, 1, 1, H.CODES_GIVEN)
     assert need <= (B * h * h + 1023) // 1024 * 9 * C * C * 4
+
+
+@pytest.mark.parametrize("given", [0, H.CODES_GIVEN])
+@pytest.mark.parametrize("bits,B,Cin,Cout,h,k,stride", [(7, 64, 256, 256, 28, 3, 1), (6, 256, 64, 64, 32, 3, 1), (8, 256, 256, 512, 8, 3, 2),
+                                                        (7, 1, 64, 256, 8, 3, 1), (8, 64, 256, 64, 56, 1, 1), (7, 8, 64, 1024, 28, 1, 1)])
+def test_least_scratch_is_accepted_and_nothing_below_it(lib, given, bits, B, Cin, Cout, h, k, stride):
+    p, pad, ho = lib.p, k // 2, (h + 2 * (k // 2) - k) // stride + 1
+    codes = p if given else None
+    for name, shape in (("lutgemm_conv2d_backward", (bits, B, Cin, h, h, Cout, k, k, stride, pad, 1)),
+                        ("lutgemm_backward", (bits, B * ho * ho, Cin * k * k, Cout))):
+        need, least = (lib.query(name + "_ws_scratch_bytes", *shape, f | given) for f in (0, H.LEAST))
+        assert least <= need
+
+        def status(nbytes):
+            return lib.call(name + "_ws", p, p, p, p, p, p, p, *shape, codes, p, H.Size(nbytes), None)[0]
+        assert status(least) == H.OK and (least == 0 or status(least - 1) == H.E_SCRATCH)
