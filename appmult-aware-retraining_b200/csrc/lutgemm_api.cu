@@ -568,12 +568,12 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
         begin[n + 1] = begin[n] + t;
         ++n;
     });
-    const long last = begin[n];
-    for (int sm = 0; sm < (n > 1 ? sms : 1); ++sm) {  // (one class: SM 0 has the most tiles)
+    // what an SM gets changes only at the SMs where a class begins or ends, SM 0 (class 0) among them
+    for (int i = 0; i < n; ++i) {
+        const long sm = begin[i] % sms;
         long rows = 0;
         for (int c = 0; c < n; ++c) rows += rows_of[c] * ((begin[c + 1] + sms - 1 - sm) / sms - (begin[c] + sms - 1 - sm) / sms);
         if (rows > most) most = rows;
-        if (sm >= last) break;
     }
     return slab < (double)most * mt * f.gx_bcast + kBcastStart;
 }
@@ -596,19 +596,22 @@ static size_t gx_base_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     return need;
 }
 
+static size_t gx_slab_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+    size_t need = 0;
+    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
+        const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B, sms);
+        need = n > need ? n : need;
+    });
+    return need;
+}
+
 static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout) {
     const int M = g.B * g.Ho * g.Wo, K = g.C * g.kh * g.kw;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
     if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true, false).ga_scratch;
     if (!pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
-    size_t need = 0;
-    if (gx_uses_slab(bits, g, Cout, sms))
-        for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
-            const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B, sms);
-            need = n > need ? n : need;
-        });
-    return need;
+    return gx_uses_slab(bits, g, Cout, sms) ? gx_slab_scratch_bytes(bits, g, Cout, sms) : 0;
 }
 
 size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
@@ -670,7 +673,7 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
     if (sms <= 0) return LUTGEMM_E_CUDA;
     bool slab = gx_uses_slab(bits, g, Cout, sms);
     const size_t given = scratch ? scratch_bytes : 0;
-    if (slab && conv_gx_scratch_bytes(bits, g, Cout) > given) {
+    if (slab && gx_slab_scratch_bytes(bits, g, Cout, sms) > given) {
         if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
             return LUTGEMM_E_SCRATCH;
         slab = false;

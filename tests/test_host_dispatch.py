@@ -143,3 +143,16 @@ def test_least_scratch_is_accepted_and_nothing_below_it(lib, given, bits, B, Cin
         def status(nbytes):
             return lib.call(name + "_ws", p, p, p, p, p, p, p, *shape, codes, p, H.Size(nbytes), None)[0]
         assert status(least) == H.OK and (least == 0 or status(least - 1) == H.E_SCRATCH)
+
+
+@pytest.mark.parametrize("bits,B,Cin,Cout,h,k,stride,slab", [
+    (7, 256, 64, 64, 32, 3, 1, False), (7, 256, 128, 128, 16, 3, 1, True), (7, 256, 64, 128, 32, 3, 2, False),
+    (7, 256, 128, 256, 16, 3, 2, False), (7, 256, 256, 512, 8, 3, 2, True), (8, 256, 64, 64, 32, 3, 1, False),
+    (8, 256, 128, 256, 16, 3, 2, False), (8, 256, 256, 512, 8, 3, 2, True), (7, 16, 32, 64, 20, 5, 3, False), (7, 2, 48, 96, 30, 7, 5, False)])
+def test_kernel_family_of_image_gradients(lib, bits, B, Cin, Cout, h, k, stride, slab):
+    """The choice counts what the busiest SM gets from the tiles of all stride classes (1, 4, 9 and 25 of them here)."""
+    p = lib.p
+    rc, calls = lib.call("lutgemm_conv2d_backward", p, p, p, p, None, p, p, bits, B, Cin, h, h, Cout, k, k, stride, k // 2, 1, p,
+                         H.Size(1 << 40), None)
+    names = {c[0] for c in calls}
+    assert rc == H.OK and ("slab_grad_packed_kernel" in names, "ga_colbcast_kernel" in names) == (slab, not slab)
