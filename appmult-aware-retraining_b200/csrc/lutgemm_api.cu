@@ -94,7 +94,7 @@ double packed_gw_clocks(int bits, int M, int K, int N, int sms) {
     return packed_clocks(lutgemm::plan_packed_gw(M, N, K, sms), N, K, family_clocks(bits).packed_gw, false);
 }
 double packed_ga_clocks(int bits, int M, int K, int N, int sms) {
-    const int rt = lutgemm::packed_ga_tile_rows(bits, N);
+    const int rt = lutgemm::packed_ga_tile_rows(N);
     const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
     return packed_clocks(lutgemm::plan_packed(N, M, K, rt, sms), M, K, step, true);
 }
@@ -131,9 +131,9 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bo
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
 }
-void set_ga_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms) {
+void set_ga_scratch(BackwardPlan &pl, int M, int K, int N, int sms) {
     if (!pl.ga_slab) return;
-    const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(bits, N);
+    const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(N);
     const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::plan_packed(N, M, K, rt, sms).groups;
     pl.ga_scratch = N > rt ? (size_t)blocks * K * M * sizeof(float) : 0;
 }
@@ -148,7 +148,7 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) 
     pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
     set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
-    set_ga_scratch(pl, bits, M, K, N, sms);
+    set_ga_scratch(pl, M, K, N, sms);
     return pl;
 }
 
@@ -172,7 +172,7 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
         pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_ga_scratch(pl, bits, M, K, N, sms);
+        set_ga_scratch(pl, M, K, N, sms);
     }
     return pl;
 }
@@ -493,7 +493,7 @@ int lutgemm_conv2d_forward_ws(const uint8_t *x, const uint8_t *wmat, uint32_t *y
 // ---- activation gradient of a convolution ------------------------------------------------------------------
 // Windows that do not overlap (kernel extent <= stride, e.g. 1x1 convolutions and patch embeddings): every image
 // position receives at most one (m,k) term, so the GEMM-shaped grad_a kernels write it in place.  Overlapping
-// windows: the pixel-mode slab kernel, one launch per stride class (lutgemm_slab_grad_tall.cu).  Either way no
+// windows: the pixel-mode slab kernel, one launch per stride class (lutgemm_slab_grad.cu).  Either way no
 // unfolded gradient [M,K] exists.
 static bool conv_windows_overlap(const lutgemm::ConvGeom &g) {
     return g.dil * (g.kh - 1) + 1 > g.stride || g.dil * (g.kw - 1) + 1 > g.stride;
@@ -558,7 +558,7 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
     int n = 0;
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
-        const int rt = lutgemm::gx_tile_rows(bits, rows);
+        const int rt = lutgemm::gx_tile_rows(rows);
         slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, f.packed * (rt > 512 ? 1.12 : 1.0), false);
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
@@ -596,10 +596,10 @@ static size_t gx_base_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     return need;
 }
 
-static size_t gx_slab_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+static size_t gx_slab_scratch_bytes(const lutgemm::ConvGeom &g, int Cout, int sms) {
     size_t need = 0;
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
-        const size_t n = lutgemm::gx_class_scratch_bytes(bits, Cout, px, g.B, sms);
+        const size_t n = lutgemm::gx_class_scratch_bytes(Cout, px, g.B, sms);
         need = n > need ? n : need;
     });
     return need;
@@ -611,7 +611,7 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     if (sms <= 0) return 0;
     if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true, false).ga_scratch;
     if (!pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
-    return gx_uses_slab(bits, g, Cout, sms) ? gx_slab_scratch_bytes(bits, g, Cout, sms) : 0;
+    return gx_uses_slab(bits, g, Cout, sms) ? gx_slab_scratch_bytes(g, Cout, sms) : 0;
 }
 
 size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
@@ -673,7 +673,7 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
     if (sms <= 0) return LUTGEMM_E_CUDA;
     bool slab = gx_uses_slab(bits, g, Cout, sms);
     const size_t given = scratch ? scratch_bytes : 0;
-    if (slab && gx_slab_scratch_bytes(bits, g, Cout, sms) > given) {
+    if (slab && gx_slab_scratch_bytes(g, Cout, sms) > given) {
         if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
             return LUTGEMM_E_SCRATCH;
         slab = false;

@@ -109,7 +109,7 @@ inline PackedPlan plan_packed(long rdim, long cdim, int K, int tile_rows, int nu
 inline PackedPlan plan_packed_gw(long M, long N, int K, int num_sms) {
     return plan_packed(M, N, K, kSlabPackedRows, num_sms, kPackedGwOverhead, 16);
 }
-int packed_ga_tile_rows(int bits, int N);  // grad_a: rows of its tile (384, 512 or 576)
+int packed_ga_tile_rows(int N);  // grad_a: rows of its tile (384, 512 or 576)
 // gradient slab kernels with 16-bit slab entries (converted where they are used)
 // `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
 int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
@@ -140,8 +140,8 @@ int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks,
                        const PixelClass *px, float scale, int num_sms, cudaStream_t stream);
 // activation gradient of a convolution for the input pixels of one stride class, written into gx[B,C,H,W]
 // (packed slab kernel in pixel mode: no unfolded gradient, no col2im); scratch: gx_class_scratch_bytes()
-int gx_tile_rows(int bits, long rdim);  // rows of its tile for a class of rdim = taps * Cout rows
-size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B, int num_sms);
+int gx_tile_rows(long rdim);  // rows of its tile for a class of rdim = taps * Cout rows
+size_t gx_class_scratch_bytes(int Cout, const PixelClass &px, int B, int num_sms);
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
                       int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream);
 // the same with the column-broadcast gather kernel (whole table in shared memory, no slab) for `nclasses` stride

@@ -619,8 +619,8 @@ static int best_tile_rows(long rdim, bool with_384) {
     if (with_384 && cost(384, 0.83) < c) rt = 384;
     return rt;
 }
-int packed_ga_tile_rows(int, int N) { return best_tile_rows(N, true); }
-int gx_tile_rows(int, long rdim) { return best_tile_rows(rdim, false); }
+int packed_ga_tile_rows(int N) { return best_tile_rows(N, true); }
+int gx_tile_rows(long rdim) { return best_tile_rows(rdim, false); }
 
 namespace {
 
@@ -666,7 +666,7 @@ int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, floa
     p.vec_g = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(gc) & 15) == 0);
     int rc, rt = kSlabPackedRows;
     if constexpr (MODE == sp::kGa) {
-        rt = packed_ga_tile_rows(BITS, N);
+        rt = packed_ga_tile_rows(N);
         rc = rt == 384   ? launch_packed<BITS, MODE, 24>(p, out, scratch, num_sms, stream)
              : rt == 576 ? launch_packed<BITS, MODE, 36>(p, out, scratch, num_sms, stream)
                          : launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
@@ -692,7 +692,7 @@ int launch_packed_gx(const float *gy, const uint8_t *x, const uint8_t *wmat, flo
     p.px = px;
     p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
     p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
-    const int rw = gx_tile_rows(BITS, p.RDIM) / 16;
+    const int rw = gx_tile_rows(p.RDIM) / 16;
     const int groups = plan_packed(p.RDIM, p.CDIM, p.K, 16 * rw, num_sms).groups;
     const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, gx, scratch, num_sms, stream)
                             : launch_packed<BITS, sp::kGx, 32>(p, gx, scratch, num_sms, stream);
@@ -728,9 +728,9 @@ int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w,
     return LUTGEMM_E_BITS;
 }
 
-size_t gx_class_scratch_bytes(int bits, int Cout, const PixelClass &px, int B, int num_sms) {
+size_t gx_class_scratch_bytes(int Cout, const PixelClass &px, int B, int num_sms) {
     const long rdim = (long)px.ntaps * Cout, cdim = (long)B * px.Hc * px.Wc;
-    const int groups = plan_packed(rdim, cdim, px.C, gx_tile_rows(bits, rdim), num_sms).groups;
+    const int groups = plan_packed(rdim, cdim, px.C, gx_tile_rows(rdim), num_sms).groups;
     return groups > 1 ? (size_t)groups * px.C * cdim * sizeof(float) : 0;
 }
 

@@ -1,13 +1,12 @@
-// Gradient LUT-GEMM kernels for sm_100a, fp32 column-gathered slab with a TALL tile (16*RW rows x 32 columns).
+// Gradient LUT-GEMM kernels for sm_100a, fp32 column-gathered slab with a TALL tile (1024 rows x 32 columns).
 //
 //   grad_w:  gw[k,n] = 1/16 * sum_m T(a[m,k], w[k,n]) * gc[m,n]     rows r = m, columns c = n
 //   grad_a:  ga[m,k] = 1/16 * sum_n gc[m,n] * T(a[m,k], w[k,n])     rows r = n, columns c = m
 //
 // Per k a slab U_k[x][c] = T(x, cc[k,c]) is gathered once, then every row reads slab row rc[r,k] contiguously
-// (conflict-free: with RW = 64 half a warp per row and two fp32 columns per lane in one 64-bit load, otherwise a
-// warp per row and one column per lane) and multiplies it with its grad_out entries held in registers (RW per
-// thread).  The 2^b-row build is paid once per 16*RW rows; two slab buffers, so slab k+1 is built
-// while slab k is read.
+// (conflict-free: half a warp per row and two fp32 columns per lane in one 64-bit load) and multiplies it with its
+// grad_out entries held in registers (64 per thread).  The 2^b-row build is paid once per 1024 rows; two slab buffers, so
+// slab k+1 is built while slab k is read.
 //
 // Hand-over between the warps of a CTA: per slab buffer a "full" barrier (all 16 warps have built their part)
 // and an "empty" barrier (all 16 warps have finished reading it), both mbarriers with one arrival per warp.
@@ -27,27 +26,23 @@
 #include "lutgemm_kernels.h"
 #include "lutgemm_waits.cuh"
 
-#ifndef LUTGEMM_TALL_HALFWARP_ROWS
-#define LUTGEMM_TALL_HALFWARP_ROWS 1
-#endif
-
 namespace lutgemm {
 namespace sgt {
 
 enum { kGw = 1, kGa = 2 };
 
-template <int BITS, int RW_>
+template <int BITS>
 struct Cfg {
     static constexpr int Q = 1 << BITS;
     static constexpr bool F32_TABLE = BITS <= 7;
     static constexpr int TT_STRIDE = F32_TABLE ? Q + 1 : table_row_bytes<BITS>() / 4;  // words per table row
-    static constexpr int WARPS = 16, THREADS = 512, RW = RW_, RT = WARPS * RW, CT = 32;
+    static constexpr int WARPS = 16, THREADS = 512, RW = 64, RT = WARPS * RW, CT = 32;
     static constexpr int KC = 16;                       // k per global fetch (16 codes per row in registers)
     static constexpr int SC = BITS == 8 ? 8 : 16;       // k per shared-memory stage
     static constexpr int U_STRIDE = 34;  // words per slab row: 32 floats + 2 (8-byte aligned rows, conflict-free stores)
     static constexpr int P_STRIDE = 33;
     static constexpr int NSEG = RT / 16;                // 16-row code segments per k
-    static constexpr int RC_LOADS = (KC * NSEG + THREADS - 1) / THREADS;  // row-code vectors per thread and group
+    static constexpr int RC_LOADS = KC * NSEG / THREADS;  // row-code vectors per thread and group
     static constexpr int TT_BYTES = Q * TT_STRIDE * 4;
     static constexpr int U_BYTES = Q * U_STRIDE * 4;
     static constexpr int RC_STAGE = SC * RT, CC_STAGE = SC * CT;
@@ -58,7 +53,7 @@ struct Cfg {
     static constexpr int OFF_PART = OFF_CC + 2 * CC_STAGE;
     static constexpr int OFF_BAR = (OFF_PART + 2 * P_BYTES + 15) & ~15;
     static constexpr int SMEM = OFF_BAR + 4 * 8 + 16;   // four mbarriers and the abort word
-    static_assert(RW % 4 == 0 && RW <= 64, "rows per warp");
+    static_assert(KC * NSEG % THREADS == 0 && RT % THREADS == 0, "row-code loads shared out evenly");
 };
 
 struct Args {
@@ -85,25 +80,24 @@ struct Args {
 // USE_AT (grad_w only): the row codes come from the transposed copy p.at; the other instantiation keeps the
 // direct / implicit-im2col fetch, so neither carries the other's registers.
 // HANDOVER: per-buffer mbarriers (see the file comment) instead of one CTA barrier per k.
-template <int BITS, int MODE, int RW, bool USE_AT, bool HANDOVER>
+template <int BITS, int MODE, bool USE_AT, bool HANDOVER>
 __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
-    using C = Cfg<BITS, RW>;
-    constexpr int WARPS = C::WARPS;
+    using C = Cfg<BITS>;
+    constexpr int WARPS = C::WARPS, RW = C::RW;
     constexpr int Q = C::Q, TTS = C::TT_STRIDE, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC;
     constexpr int US = C::U_STRIDE, PS = C::P_STRIDE, THREADS = C::THREADS, NSEG = C::NSEG, RCL = C::RC_LOADS;
     constexpr int HALVES = KC / SC;  // shared-memory stages per fetched group of 16 k
     // slab reads in flight ahead of their use (per row, or per pair of columns with HW): 4 at 8 bits (2 and 3 are 1 - 2 %
     // slower, 8 is 3 % slower), 2 at 7 bits and below (4 is 1 % slower)
     constexpr int PF = BITS == 8 ? 4 : 2;
-    // HW: half a warp per slab row and two columns per lane (64-bit slab reads) instead of a warp per row and one
-    // column per lane: lanes 0-15 take the first RW/2 rows of the warp, lanes 16-31 the others
-    constexpr bool HW = LUTGEMM_TALL_HALFWARP_ROWS && RW == 64 && HANDOVER;
+    // HW: half a warp per slab row and two columns per lane (64-bit slab reads): lanes 0-15 take the first RW/2 rows of the
+    // warp, lanes 16-31 the others.  With a CTA barrier per k: a warp per row and one column per lane.
+    constexpr bool HW = HANDOVER;
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
     constexpr int COL = lut_col_num(BITS);
-    static_assert(MODE != kGw || USE_AT || RT % THREADS == 0, "grad_w without a transposed copy: whole rows per thread");
 
     const int M = p.M, K = p.K, N = p.N;
-    const int RDIM = p.RDIM, CDIM = p.CDIM;
+    const int CDIM = p.CDIM;
 
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t *rc_s = smem + C::OFF_RC;
@@ -167,7 +161,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
             for (int j = 0; j < RCL; ++j) {
                 const int idx = tid + THREADS * j;  // (k, 16-row segment)
                 const int gk = kbase + idx / NSEG, gm = r0 + (idx % NSEG) * 16;
-                prc[j] = (idx < KC * NSEG && gk < K && gm < p.at_pitch)
+                prc[j] = (gk < K && gm < p.at_pitch)
                              ? *reinterpret_cast<const uint4 *>(p.at + (size_t)gk * p.at_pitch + gm)
                              : make_uint4(0, 0, 0, 0);
             }
@@ -181,8 +175,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
             for (int j = 0; j < RCL; ++j) {
                 const int idx = tid + THREADS * j;  // (k, 16-row segment)
                 const int gk = kbase + idx / NSEG, gr = r0 + (idx % NSEG) * 16;
-                if (idx >= KC * NSEG) prc[j] = make_uint4(0, 0, 0, 0);
-                else prc[j] = w_codes16(gk, gr);
+                prc[j] = w_codes16(gk, gr);
             }
             if (tid < CT) pcc = a_codes16(c0 + tid, kbase);
         }
@@ -205,7 +198,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
 #pragma unroll
             for (int j = 0; j < RCL; ++j) {
                 const int idx = tid + THREADS * j, kq = idx / NSEG;
-                if (idx < KC * NSEG && (kq / SC == half || HALVES == 1))
+                if (kq / SC == half || HALVES == 1)
                     *reinterpret_cast<uint4 *>(rs + (kq % SC) * RT + (idx % NSEG) * 16) =
                         make_uint4(prc[j].x & MASK4, prc[j].y & MASK4, prc[j].z & MASK4, prc[j].w & MASK4);
             }
@@ -390,7 +383,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
             auto row_addr = [&](uint32_t v, int i) { return byte_scaled_add<US * 4>(v, i, ub); };
             constexpr int W0 = RB / 4, W1 = (RE + 3) / 4;  // code words (four rows each) this range touches
             uint32_t rv[W1 - W0];
-            if constexpr (RW % 16 == 0 && RB % 16 == 0 && RE % 16 == 0) {
+            if constexpr (RB % 16 == 0 && RE % 16 == 0) {
                 const uint4 *rp = reinterpret_cast<const uint4 *>(rbase);
 #pragma unroll
                 for (int q = RB / 16; q < RE / 16; ++q) {
@@ -445,9 +438,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_tall_kernel(const Args p) {
             }
         };
         using I0 = std::integral_constant<int, 0>;
-        using IH = std::integral_constant<int, (RW / 2) & ~3>;
+        using IH = std::integral_constant<int, RW / 2>;
         using IE = std::integral_constant<int, RW>;
-        using IQ = std::integral_constant<int, ((RW / 4) + 15) & ~15>;  // HW: half of a half-warp's rows
+        using IQ = std::integral_constant<int, RW / 4>;  // HW: half of a half-warp's rows
 
         for (int k = kbeg; k < kend; ++k) {
             const int chunk = k / SC, kk = k % SC, stage = chunk & 1;
@@ -516,17 +509,16 @@ namespace {
 
 bool g_tall_handover = true;  // per-buffer mbarrier hand-over (false: one CTA barrier per k)
 
-
-template <int BITS, int MODE, int RW>
+template <int BITS, int MODE>
 int launch_slab_grad_tall(sgt::Args p, float *out, float *scratch, int num_sms, cudaStream_t stream) {
-    using C = sgt::Cfg<BITS, RW>;
+    using C = sgt::Cfg<BITS>;
     static_assert(C::SMEM <= 232448, "shared memory budget");
     const bool use_at = MODE == sgt::kGw && p.at != nullptr;
     const bool ho = g_tall_handover;
-    auto kern = use_at ? (ho ? sgt::slab_grad_tall_kernel<BITS, MODE, RW, MODE == sgt::kGw, true>
-                             : sgt::slab_grad_tall_kernel<BITS, MODE, RW, MODE == sgt::kGw, false>)
-                       : (ho ? sgt::slab_grad_tall_kernel<BITS, MODE, RW, false, true>
-                             : sgt::slab_grad_tall_kernel<BITS, MODE, RW, false, false>);
+    auto kern = use_at ? (ho ? sgt::slab_grad_tall_kernel<BITS, MODE, MODE == sgt::kGw, true>
+                             : sgt::slab_grad_tall_kernel<BITS, MODE, MODE == sgt::kGw, false>)
+                       : (ho ? sgt::slab_grad_tall_kernel<BITS, MODE, false, true>
+                             : sgt::slab_grad_tall_kernel<BITS, MODE, false, false>);
     if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)))
         return LUTGEMM_E_CUDA;
     p.error_word = device_error_word();
@@ -549,8 +541,8 @@ template <int BITS, int MODE>
 int launch_gemm_grad_tall(const float *gc, const uint8_t *a, const uint8_t *w, float *out, const int16_t *lut,
                           const float *lut_f32, int M, int K, int N, const ConvGeom &conv, float *scratch,
                           const uint8_t *at, int at_pitch, int num_sms, cudaStream_t stream) {
-    static_assert(sgt::Cfg<BITS, 64>::RT == kSlabTallRows, "tile height");
-    if (lut_f32 && !sgt::Cfg<BITS, 64>::F32_TABLE) return LUTGEMM_E_BITS;
+    static_assert(sgt::Cfg<BITS>::RT == kSlabTallRows, "tile height");
+    if (lut_f32 && !sgt::Cfg<BITS>::F32_TABLE) return LUTGEMM_E_BITS;
     sgt::Args p{};
     p.a = a; p.w = w; p.lut = lut; p.gc = gc; p.M = M; p.K = K; p.N = N;
     p.lut_f32 = lut_f32;
@@ -564,7 +556,7 @@ int launch_gemm_grad_tall(const float *gc, const uint8_t *a, const uint8_t *w, f
     p.vec_a = !conv.enabled && (K % 16 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
     p.vec_w = (N % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
     p.vec_g = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(gc) & 15) == 0);
-    const int rc = launch_slab_grad_tall<BITS, MODE, 64>(p, out, scratch, num_sms, stream);
+    const int rc = launch_slab_grad_tall<BITS, MODE>(p, out, scratch, num_sms, stream);
     if (rc != LUTGEMM_OK) return rc;
     const int tiles_r = (p.RDIM + kSlabTallRows - 1) / kSlabTallRows;
     if (tiles_r > 1)
