@@ -98,7 +98,7 @@ struct Cfg {
     static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // grad_x: image offset of each column
     static constexpr int OFF_TAP = OFF_PIX + CT * 8;                  // grad_x: output offset {rows, columns} of each tap
     static constexpr int OFF_BAR = OFF_TAP + kMaxTaps * 8;
-    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // a full and an empty mbarrier per buffer, and the abort word
+    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // two mbarriers per buffer, abort word, work item
     static_assert(RW % 4 == 0 && RT % 16 == 0, "rows per warp");
     static_assert(U_BYTES % 16 == 0 && RC_STAGE % 16 == 0 && CC_STAGE % 16 == 0, "16-byte vectors");
     static_assert(SMEM <= 232448, "shared memory budget");
@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     const uint32_t u_addr = smem_u32(smem + C::OFF_U);
     const uint32_t bar_full = smem_u32(smem + C::OFF_BAR), bar_empty = bar_full + 8 * NB;
     volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 16 * NB);
+    int *work_s = reinterpret_cast<int *>(smem + C::OFF_BAR + 16 * NB + 4);  // grad_w: cell and k range of the work item
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int half = lane >> 4, cq = lane & 15;  // half-warp and column quad (columns 4 cq .. 4 cq + 3)
 
@@ -350,6 +351,15 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             cell = p.main_cells + j / p.tail_parts;
             kbeg = (j % p.tail_parts) * p.tail_per;
             kend = min(K, kbeg + p.tail_per);
+        }
+        if constexpr (MODE == kGw) {
+            // the compiler's schedule of the k loop depends on what it sees of these three: read back from shared memory
+            // grad_w takes 1.49 ms for 4096 x 4608 x 512 at 7 bits, straight from the branch 1.53 (grad_x: the other way round)
+            if (tid == 0) { work_s[0] = cell; work_s[1] = kbeg; work_s[2] = kend; }
+            __syncthreads();
+            cell = work_s[0];
+            kbeg = work_s[1];
+            kend = work_s[2];
         }
         const int group = cell / p.tiles_c, tc = cell % p.tiles_c;
         const int tr = group * p.group_blocks + block;
