@@ -168,12 +168,13 @@ def _check_input(x: torch.Tensor, dtype: torch.dtype, name: str) -> None:
         raise RuntimeError(f"{name} must be of type {dtype}")
 
 
-def _check_fp32(x: torch.Tensor, name: str, device: torch.device, numel: int = None) -> None:
-    """An fp32 operand on `device` that goes to the library as a pointer; with `numel` it has to be that many values in a row."""
-    if x.device != device:
-        raise RuntimeError(f"{name} must be on {device}, not on {x.device}")
-    if x.dtype != torch.float32:
+def _check_fp32(x: torch.Tensor, name: str, index: int, numel: int = None) -> None:
+    """An fp32 operand on CUDA device `index` that goes to the library as a pointer; with `numel` it has to be that many values
+    in a row."""
+    if x.dtype is not torch.float32:
         raise RuntimeError(f"{name} must be of type torch.float32")
+    if x.get_device() != index or index < 0:
+        raise RuntimeError(f"{name} must be on the CUDA device of the other operands, not on {x.device}")
     if numel is not None and (x.numel() != numel or not x.is_contiguous()):
         raise RuntimeError(f"{name} must be {numel} contiguous values")
 
@@ -359,7 +360,7 @@ def _epilogue_args(box, sumw_t, taps, s_a, s_w, z_a, z_w, bias, M, L, Cout):
         if tuple(t.shape) != shape:
             raise RuntimeError(f"{name} has shape {tuple(t.shape)}, expected {shape}")
     if bias is not None:
-        _check_fp32(bias, "bias_tensor", box.device, Cout)
+        _check_fp32(bias, "bias_tensor", box.get_device(), Cout)
     return [box.data_ptr(), sumw_t.data_ptr(), taps.data_ptr(), s_a.data_ptr(), s_w.data_ptr(), z_a.data_ptr(),
             z_w.data_ptr(), bias.data_ptr() if bias is not None else None]
 
@@ -408,12 +409,13 @@ def conv2d_layer_pass(x: torch.Tensor, weight: torch.Tensor, bias, quant: torch.
     bits = _bits_of(lut, "lut_appmult_tensor")
     Ho, Wo = _conv_out(H, W, kh, kw, stride, pad, dil)
     dev = x.device
-    if lut.device != dev:
+    index = x.get_device()  # (an int: comparing device objects costs more than the rest of the checks)
+    if lut.get_device() != index:
         raise RuntimeError("device id not match")
-    _check_fp32(weight, "weight_tensor", dev)
-    _check_fp32(quant, "quant_tensor", dev, 4)
+    _check_fp32(weight, "weight_tensor", index)
+    _check_fp32(quant, "quant_tensor", index, 4)
     if bias is not None:
-        _check_fp32(bias, "bias_tensor", dev, Cout)
+        _check_fp32(bias, "bias_tensor", index, Cout)
     lib = _load()
     geom = (B, C, H, W, Cout, kh, kw, stride, pad, dil)
     with torch.cuda.device(dev):
@@ -622,10 +624,9 @@ def layer_weight_prep(weight: torch.Tensor, quant: torch.Tensor, qmax: float):
     """(wmat u8 [Cin*kh*kw, Cout], wsum f32 [Cout, kh*kw]) of a 4-D fp32 weight in any dense layout: the weight
     codes transposed for the LUT kernels and their sums over the input channels per tap."""
     Cout, Cin, kh, kw = weight.shape
-    if not weight.is_cuda:
-        raise RuntimeError("weight_tensor must be a CUDA tensor")
-    _check_fp32(weight, "weight_tensor", weight.device)
-    _check_fp32(quant, "quant_tensor", weight.device, 4)
+    index = weight.get_device()
+    _check_fp32(weight, "weight_tensor", index)
+    _check_fp32(quant, "quant_tensor", index, 4)
     wmat = torch.empty((Cin * kh * kw, Cout), dtype=torch.uint8, device=weight.device)
     wsum = torch.empty((Cout, kh * kw), dtype=torch.float32, device=weight.device)
     s = weight.stride()

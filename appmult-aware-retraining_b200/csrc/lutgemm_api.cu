@@ -58,6 +58,7 @@ struct BackwardPlan {
     // caller's, or one made behind the partial sums in the scratch buffer
     size_t gw_at_offset;  // bytes into the scratch buffer, a multiple of 16
     int gw_at_pitch;      // 0 = no transposed copy
+    lutgemm::PackedPlan gw_packed, ga_packed;
 };
 
 // ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
@@ -90,13 +91,13 @@ double packed_clocks(const lutgemm::PackedPlan &p, long cols, int K, double per_
     const bool reduce = p.groups > 1 || (transposed && p.group_blocks > 1);
     return (double)p.steps * per_step + kSlabStart + (reduce ? 8e3 + 8.0 * p.groups * K * cols / kReduceBytesPerClock : 0);
 }
-double packed_gw_clocks(int bits, int M, int K, int N, int sms) {
-    return packed_clocks(lutgemm::plan_packed_gw(M, N, K, sms), N, K, family_clocks(bits).packed_gw, false);
+double packed_gw_clocks(const lutgemm::PackedPlan &plan, int bits, int K, int N) {
+    return packed_clocks(plan, N, K, family_clocks(bits).packed_gw, false);
 }
-double packed_ga_clocks(int bits, int M, int K, int N, int sms) {
+double packed_ga_clocks(const lutgemm::PackedPlan &plan, int bits, int M, int K, int N) {
     const int rt = lutgemm::packed_ga_tile_rows(N);
     const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
-    return packed_clocks(lutgemm::plan_packed(N, M, K, rt, sms), M, K, step, true);
+    return packed_clocks(plan, M, K, step, true);
 }
 double tall_clocks(int bits, long rows, long cols, int K, int sms) {
     const long blocks = div_up(rows, 1024);
@@ -120,7 +121,7 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bo
     pl.gw_at_offset = 0;
     pl.gw_at_pitch = 0;
     if (pl.gw_slab) {
-        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : lutgemm::plan_packed_gw(M, N, K, sms).groups;
+        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : pl.gw_packed.groups;
         pl.gw_scratch = rb > 1 ? (size_t)rb * K * N * sizeof(float) : 0;
         pl.gw_at_pitch = (M + 15) & ~15;
         if (!have_codes) {
@@ -131,10 +132,10 @@ void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bo
         pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
     }
 }
-void set_ga_scratch(BackwardPlan &pl, int M, int K, int N, int sms) {
+void set_ga_scratch(BackwardPlan &pl, int M, int K, int N) {
     if (!pl.ga_slab) return;
     const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(N);
-    const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : lutgemm::plan_packed(N, M, K, rt, sms).groups;
+    const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : pl.ga_packed.groups;
     pl.ga_scratch = N > rt ? (size_t)blocks * K * M * sizeof(float) : 0;
 }
 
@@ -147,8 +148,10 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) 
     pl.ga_slab = bits >= 7 && N >= 768 && M >= 32 && ga_fill >= (bits == 7 ? 0.85 : 0.7);
     pl.gw_tall = pl.gw_slab && tall_fill(M, N) >= 0.7 * slab_fill(M, N);
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
+    if (pl.gw_slab && !pl.gw_tall) pl.gw_packed = lutgemm::plan_packed_gw(M, N, K, sms);
+    if (pl.ga_slab && !pl.ga_tall) pl.ga_packed = lutgemm::plan_packed(N, M, K, lutgemm::packed_ga_tile_rows(N), sms);
     set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
-    set_ga_scratch(pl, M, K, N, sms);
+    set_ga_scratch(pl, M, K, N);
     return pl;
 }
 
@@ -161,18 +164,20 @@ BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bo
     BackwardPlan pl{};
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (want_gw) {
-        const double packed = packed_gw_clocks(bits, M, K, N, sms), tall = tall_clocks(bits, M, N, K, sms);
+        pl.gw_packed = lutgemm::plan_packed_gw(M, N, K, sms);
+        const double packed = packed_gw_clocks(pl.gw_packed, bits, K, N), tall = tall_clocks(bits, M, N, K, sms);
         pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
         set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
     }
     if (want_ga) {
-        const double packed = packed_ga_clocks(bits, M, K, N, sms), tall = tall_clocks(bits, N, M, K, sms);
+        pl.ga_packed = lutgemm::plan_packed(N, M, K, lutgemm::packed_ga_tile_rows(N), sms);
+        const double packed = packed_ga_clocks(pl.ga_packed, bits, M, K, N), tall = tall_clocks(bits, N, M, K, sms);
         pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
         pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_ga_scratch(pl, M, K, N, sms);
+        set_ga_scratch(pl, M, K, N);
     }
     return pl;
 }
@@ -386,14 +391,14 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
         }
         int rc = !pl.gw_slab ? lutgemm::backward_gw(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, pl.gw_splits, sms, s)
                  : pl.gw_tall ? lutgemm::backward_gw_slab_tall(gc, a, w, gw, lut_gw, nullptr, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s)
-                             : lutgemm::backward_gw_slab_packed(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s);
+                             : lutgemm::backward_gw_slab_packed(gc, a, w, gw, lut_gw, bits, M, K, N, conv, pl.gw_packed, sc, at, pl.gw_at_pitch, sms, s);
         if (rc != LUTGEMM_OK) return rc;
     }
     if (ga) {
         if (pl.ga_scratch > given) return LUTGEMM_E_SCRATCH;
         int rc = !pl.ga_slab ? lutgemm::backward_ga(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sms, s)
                  : pl.ga_tall ? lutgemm::backward_ga_slab_tall(gc, a, w, ga, lut_ga, nullptr, bits, M, K, N, conv, sc, sms, s)
-                             : lutgemm::backward_ga_slab_packed(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sc, sms, s);
+                             : lutgemm::backward_ga_slab_packed(gc, a, w, ga, lut_ga, bits, M, K, N, conv, pl.ga_packed, sc, sms, s);
         if (rc != LUTGEMM_OK) return rc;
     }
     return LUTGEMM_OK;
@@ -918,8 +923,9 @@ int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, l
     if (H > 65535 || B > 65535) return LUTGEMM_E_TOOLARGE;
     const int sms = current_num_sms(), M = B * g.Ho * g.Wo, K = C * kh * kw;
     if (sms <= 0) return LUTGEMM_E_CUDA;
-    if (scratch_bytes < layer_forward_scratch_bytes(bits, M, K, Cout) && small_workspace_refused(M, Cout) &&
-        (scratch || layer_forward_needs_sums(bits, M, K, Cout, sms)))
+    // (a buffer for codes and sums is enough for every choice; what the choice needs is only worked out for a smaller one)
+    if (scratch_bytes < (size_t)codes_pitch(M) * K + (size_t)M * Cout * sizeof(uint32_t) && small_workspace_refused(M, Cout) &&
+        scratch_bytes < layer_forward_scratch_bytes(bits, M, K, Cout) && (scratch || layer_forward_needs_sums(bits, M, K, Cout, sms)))
         return LUTGEMM_E_SCRATCH;
     const size_t L = (size_t)g.Ho * g.Wo, pixels = (size_t)B * H * W;
     float *chansum = work, *wsum = chansum + pixels, *sumw_t = wsum + (size_t)Cout * kh * kw, *taps = sumw_t + L * Cout,

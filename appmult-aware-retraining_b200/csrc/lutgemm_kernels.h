@@ -97,11 +97,17 @@ inline PackedPlan plan_packed(long rdim, long cdim, int K, int tile_rows, int nu
     const long tiles_r = (rdim + tile_rows - 1) / tile_rows, tiles_c = (cdim + 63) / 64;
     const PackedPlan alone = deal_cells(tiles_r, 1, tiles_c, K, num_sms, item_overhead);
     if (tiles_r * tiles_c < num_sms) return alone;
+    const unsigned sms = (unsigned)num_sms;
+    const long whole = (K + 15) / 16 * 16 + item_overhead;
     for (long blocks = tiles_r < most_blocks ? tiles_r : most_blocks; blocks > 1; --blocks) {
         const long groups = (tiles_r + blocks - 1) / blocks;
         if ((tiles_r + groups - 1) / groups < blocks) continue;  // as many groups of fewer blocks
+        const long most = alone.steps + alone.steps / 256 + (tiles_r - groups) * tiles_c * K / 23400;
+        // (most candidates cannot do it even with an even last round: the search for their K split is left out)
+        const long rounds = groups * tiles_c / sms, tail = groups * tiles_c % sms;
+        if (blocks * (rounds * whole + (tail ? tail * K / sms + item_overhead : 0)) > most) continue;
         const PackedPlan p = deal_cells(groups, blocks, tiles_c, K, num_sms, item_overhead);
-        if (p.steps <= alone.steps + alone.steps / 256 + (tiles_r - groups) * tiles_c * K / 23400) return p;
+        if (p.steps <= most) return p;
     }
     return alone;
 }
@@ -111,13 +117,14 @@ inline PackedPlan plan_packed_gw(long M, long N, int K, int num_sms) {
 }
 int packed_ga_tile_rows(int N);  // grad_a: rows of its tile (384, 512 or 576)
 // gradient slab kernels with 16-bit slab entries (converted where they are used)
-// `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
+// `at`: the row codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes); `plan`: plan_packed_gw or, for
+// grad_a, plan_packed of the problem
 int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
-                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                            int at_pitch, int num_sms, cudaStream_t stream);
+                            int bits, int M, int K, int N, const ConvGeom &conv, const PackedPlan &plan, float *scratch,
+                            const uint8_t *at, int at_pitch, int num_sms, cudaStream_t stream);
 int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
-                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
-                            cudaStream_t stream);
+                            int bits, int M, int K, int N, const ConvGeom &conv, const PackedPlan &plan, float *scratch,
+                            int num_sms, cudaStream_t stream);
 // fp32 slab entries and a tall tile (1024 rows x 32 columns)
 constexpr int kSlabTallRows = 1024;
 int slab_tall_row_blocks(int rdim);

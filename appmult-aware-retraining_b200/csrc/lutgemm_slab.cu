@@ -473,10 +473,11 @@ int slab_fwd_ksplits(int M, int K, int N, int num_sms) {
     int ksplits = 1;
     double best = -1.0;
     for (int s = 1; s <= 16 && s <= kchunks; ++s) {
-        const int per = ((kchunks + s - 1) / s) * C::KC;
-        if ((K + per - 1) / per != s) continue;  // some split would get no work
+        const int chunks = (kchunks + s - 1) / s, per = chunks * C::KC;
+        if ((kchunks + chunks - 1) / chunks != s) continue;  // some split would get no work
         const long items = tiles * s;
-        const long waves = (items + num_sms - 1) / num_sms;
+        // (32-bit division where it will do: the search is made several times per layer call)
+        const long waves = items < (1L << 31) ? (long)(((unsigned)items + num_sms - 1) / (unsigned)num_sms) : (items + num_sms - 1) / num_sms;
         const double eff = (double)items / (double)(waves * num_sms) * (double)per / (double)(per + 6);
         if (eff > best + 1e-9) { best = eff; ksplits = s; }
     }

@@ -635,7 +635,7 @@ int gx_tile_rows(long rdim) { return best_tile_rows(rdim, false); }
 namespace {
 
 template <int BITS, int MODE, int RW>
-int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStream_t stream) {
+int launch_packed(sp::Args p, const PackedPlan &pp, float *out, float *scratch, int num_sms, cudaStream_t stream) {
     using C = sp::Cfg<BITS, RW>;
     auto kern = sp::slab_grad_packed_kernel<BITS, MODE, RW>;
     if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM))) return LUTGEMM_E_CUDA;
@@ -643,7 +643,6 @@ int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStrea
     if (!p.error_word) return LUTGEMM_E_CUDA;
     p.tiles_r = (p.RDIM + C::RT - 1) / C::RT;
     p.tiles_c = (p.CDIM + C::CT - 1) / C::CT;
-    const PackedPlan pp = MODE == sp::kGw ? plan_packed_gw(p.RDIM, p.CDIM, p.K, num_sms) : plan_packed(p.RDIM, p.CDIM, p.K, C::RT, num_sms);
     p.groups = pp.groups;
     p.group_blocks = pp.group_blocks;
     // (grad_a is transposed on its way to its final place, by the reduction over the groups)
@@ -660,8 +659,8 @@ int launch_packed(sp::Args p, float *out, float *scratch, int num_sms, cudaStrea
 
 template <int BITS, int MODE>
 int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, float *out, const int16_t *lut, int M, int K,
-                       int N, const ConvGeom &conv, float *scratch, const uint8_t *at, int at_pitch, int num_sms,
-                       cudaStream_t stream) {
+                       int N, const ConvGeom &conv, const PackedPlan &plan, float *scratch, const uint8_t *at, int at_pitch,
+                       int num_sms, cudaStream_t stream) {
     static_assert(sp::Cfg<BITS, 32>::RT == kSlabPackedRows, "tile height");
     sp::Args p{};
     p.a = a; p.w = w; p.lut = lut; p.gc = gc; p.M = M; p.K = K; p.N = N;
@@ -677,16 +676,15 @@ int launch_packed_gemm(const float *gc, const uint8_t *a, const uint8_t *w, floa
     int rc, rt = kSlabPackedRows;
     if constexpr (MODE == sp::kGa) {
         rt = packed_ga_tile_rows(N);
-        rc = rt == 384   ? launch_packed<BITS, MODE, 24>(p, out, scratch, num_sms, stream)
-             : rt == 576 ? launch_packed<BITS, MODE, 36>(p, out, scratch, num_sms, stream)
-                         : launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+        rc = rt == 384   ? launch_packed<BITS, MODE, 24>(p, plan, out, scratch, num_sms, stream)
+             : rt == 576 ? launch_packed<BITS, MODE, 36>(p, plan, out, scratch, num_sms, stream)
+                         : launch_packed<BITS, MODE, 32>(p, plan, out, scratch, num_sms, stream);
     } else {
-        rc = launch_packed<BITS, MODE, 32>(p, out, scratch, num_sms, stream);
+        rc = launch_packed<BITS, MODE, 32>(p, plan, out, scratch, num_sms, stream);
     }
     if (rc != LUTGEMM_OK) return rc;
-    const int groups = MODE == sp::kGw ? plan_packed_gw(M, N, K, num_sms).groups : plan_packed(N, M, K, rt, num_sms).groups;
-    if (MODE == sp::kGw ? groups > 1 : p.RDIM > rt)
-        return slab_reduce_blocks(scratch, out, K, p.CDIM, groups, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
+    if (MODE == sp::kGw ? plan.groups > 1 : p.RDIM > rt)
+        return slab_reduce_blocks(scratch, out, K, p.CDIM, plan.groups, MODE == sp::kGa, p.ga_scatter ? &conv : nullptr, nullptr,
                                   kGradFactor, num_sms, stream);
     return LUTGEMM_OK;
 }
@@ -703,37 +701,37 @@ int launch_packed_gx(const float *gy, const uint8_t *x, const uint8_t *wmat, flo
     p.vec_w = (Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(wmat) & 15) == 0);
     p.vec_g = (Cout % 4 == 0) && ((reinterpret_cast<uintptr_t>(gy) & 15) == 0);
     const int rw = gx_tile_rows(p.RDIM) / 16;
-    const int groups = plan_packed(p.RDIM, p.CDIM, p.K, 16 * rw, num_sms).groups;
-    const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, gx, scratch, num_sms, stream)
-                            : launch_packed<BITS, sp::kGx, 32>(p, gx, scratch, num_sms, stream);
+    const PackedPlan plan = plan_packed(p.RDIM, p.CDIM, p.K, 16 * rw, num_sms);
+    const int rc = rw == 36 ? launch_packed<BITS, sp::kGx, 36>(p, plan, gx, scratch, num_sms, stream)
+                            : launch_packed<BITS, sp::kGx, 32>(p, plan, gx, scratch, num_sms, stream);
     if (rc != LUTGEMM_OK) return rc;
-    if (groups > 1)
-        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, groups, false, nullptr, &px, kGradFactor, num_sms, stream);
+    if (plan.groups > 1)
+        return slab_reduce_blocks(scratch, gx, p.K, p.CDIM, plan.groups, false, nullptr, &px, kGradFactor, num_sms, stream);
     return LUTGEMM_OK;
 }
 
 }  // namespace
 
 int backward_gw_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, const int16_t *lut_gw,
-                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, const uint8_t *at,
-                            int at_pitch, int num_sms, cudaStream_t stream) {
+                            int bits, int M, int K, int N, const ConvGeom &conv, const PackedPlan &plan, float *scratch,
+                            const uint8_t *at, int at_pitch, int num_sms, cudaStream_t stream) {
     switch (bits) {
-        case 4: return launch_packed_gemm<4, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 6: return launch_packed_gemm<6, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 7: return launch_packed_gemm<7, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
-        case 8: return launch_packed_gemm<8, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, scratch, at, at_pitch, num_sms, stream);
+        case 4: return launch_packed_gemm<4, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, plan, scratch, at, at_pitch, num_sms, stream);
+        case 6: return launch_packed_gemm<6, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, plan, scratch, at, at_pitch, num_sms, stream);
+        case 7: return launch_packed_gemm<7, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, plan, scratch, at, at_pitch, num_sms, stream);
+        case 8: return launch_packed_gemm<8, sp::kGw>(gc, a, w, gw, lut_gw, M, K, N, conv, plan, scratch, at, at_pitch, num_sms, stream);
     }
     return LUTGEMM_E_BITS;
 }
 
 int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
-                            int bits, int M, int K, int N, const ConvGeom &conv, float *scratch, int num_sms,
-                            cudaStream_t stream) {
+                            int bits, int M, int K, int N, const ConvGeom &conv, const PackedPlan &plan, float *scratch,
+                            int num_sms, cudaStream_t stream) {
     switch (bits) {
-        case 4: return launch_packed_gemm<4, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 6: return launch_packed_gemm<6, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 7: return launch_packed_gemm<7, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
-        case 8: return launch_packed_gemm<8, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, scratch, nullptr, 0, num_sms, stream);
+        case 4: return launch_packed_gemm<4, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, plan, scratch, nullptr, 0, num_sms, stream);
+        case 6: return launch_packed_gemm<6, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, plan, scratch, nullptr, 0, num_sms, stream);
+        case 7: return launch_packed_gemm<7, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, plan, scratch, nullptr, 0, num_sms, stream);
+        case 8: return launch_packed_gemm<8, sp::kGa>(gc, a, w, ga, lut_ga, M, K, N, conv, plan, scratch, nullptr, 0, num_sms, stream);
     }
     return LUTGEMM_E_BITS;
 }
