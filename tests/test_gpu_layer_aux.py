@@ -213,3 +213,46 @@ def test_narrow_layers_hold_no_code_copy_for_the_backward_pass(dev, cout, held):
             fn = fn.next_functions[0][0]
         assert (fn.codes_t is not None) == held
         out.sum().backward()
+
+
+@pytest.mark.parametrize("B,Cin,H,W,Cout,kh,kw,st,p,d", GEOMS + [(4, 40, 17, 19, 70, 3, 3, 1, 2, 2), (2, 16, 30, 30, 24, 3, 3, 2, 3, 3)])
+@pytest.mark.parametrize("channels_last", [False, True])
+def test_layer_pass_equals_its_steps(dev, B, Cin, H, W, Cout, kh, kw, st, p, d, channels_last):
+    """The one-call forward pass of a convolution layer against the five calls it stands for: identical outputs."""
+    import approx_ops
+    from lutgemm_luts import synthetic_multiplier
+    from oracle import oracle_np as O
+    torch.manual_seed(Cout)
+    fmt = torch.channels_last if channels_last else torch.contiguous_format
+    x = torch.rand(B, Cin, H, W, device=dev).contiguous(memory_format=fmt)
+    weight = torch.randn(Cout, Cin, kh, kw, device=dev).contiguous(memory_format=fmt)
+    bias = torch.randn(Cout, device=dev)
+    quant = torch.tensor([1 / 127, 0.0, 0.05, -63.0], device=dev)
+    s_a, z_a, s_w, z_w = (quant[i:i + 1] for i in range(4))
+    lut = torch.from_numpy(O.pack_padded(synthetic_multiplier(7, seed=1), 7, np.uint16)).to(dev)
+    out, codes, wmat, codes_t = approx_ops.conv2d_layer_pass(x, weight, bias, quant, 127.0, 127.0, lut, st, p, d)
+    codes_, chansum = approx_ops.quantize_activations(x, s_a, z_a, 127.0)
+    wmat_, wsum = approx_ops.layer_weight_prep(weight, quant, 127.0)
+    sumw_t, taps = approx_ops.layer_cross_terms(wsum, Cin, H, W, kh, kw, st, p, d)
+    box = approx_ops.layer_window_sum(chansum, kh, kw, st, p, d)
+    out_, codes_t_ = approx_ops.approx_conv2d_forward_layer(codes_, wmat_, lut, kh, kw, st, p, d, box, sumw_t, taps, s_a, s_w, z_a,
+                                                            z_w, bias)
+    assert torch.equal(codes, codes_) and torch.equal(wmat, wmat_) and torch.equal(out, out_)
+    assert (codes_t is None) == (codes_t_ is None) and (codes_t is None or torch.equal(codes_t, codes_t_))
+
+
+def test_ranges_of_tensors_in_any_memory_order(dev):
+    """A layer's fused range update on inputs that are contiguous, channels-last, permuted otherwise, sliced or expanded."""
+    from lutgemm_layers import AppConv2d, _in_memory_order
+    base = torch.randn(4, 6, 8, 10, device=dev)
+    wide = torch.randn(4, 6, 8, 20, device=dev)
+    for x in (base, base.contiguous(memory_format=torch.channels_last), base.permute(0, 1, 3, 2), base.permute(1, 0, 2, 3),
+              wide[..., ::2], wide[:, :, :, 3:13], base[:, :1].expand(-1, 6, -1, -1), base.reshape(4, 6, 80)):
+        y = _in_memory_order(x)
+        assert y.numel() == x.numel() and torch.equal(torch.stack(torch.aminmax(y)), torch.stack((x.min(), x.max())))
+        if x.dim() == 4:
+            ref, new = (AppConv2d(x.shape[1], 3, 3, a_bits=7, w_bits=7, conv_impl=impl).to(dev).train() for impl in ("fused", "layer"))
+            new.load_state_dict(ref.state_dict())
+            ref._refresh(x, ref.weight)
+            new._refresh(x, new.weight, fused=True)
+            assert torch.equal(ref.quant, new.quant)

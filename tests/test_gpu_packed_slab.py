@@ -1,6 +1,7 @@
 """GPU tests of the packed-slab gradient kernels (512 x 64 tiles, 576 x 64 for grad_x) at the sizes where they can go
 wrong - remainders of tiles, of the two-k slab buffers and of the 16-k operand stages - with tables over the whole int16
-range, and of what the dispatcher does when a caller's scratch buffer is too small for the faster kernel.
+range, of the forward kernel's two-k pipeline, and of what the dispatcher does when a caller's scratch buffer is too small
+for the faster kernel.
 
 Tolerance: an fp32 sum of n terms in any order is off by at most about n * 2^-24 times the sum of the absolute terms, and
 the kernels add at most 16 terms per accumulator, 32 accumulators and the row blocks in turn (fewer than 100 additions in
@@ -140,12 +141,17 @@ def test_a_small_scratch_buffer_selects_a_kernel_that_fits(dev, oracle_c, bits):
     r_ga, r_gw, r_gaa, r_gwa = oracle_c.backward_f64(gc, a, w, la, lw, bits)
     check(ga.cpu().numpy(), r_ga, r_gaa)
     check(gw.cpu().numpy(), r_gw, r_gwa)
-    # 4096 rows, the weight gradient by a slab kernel under either choice: a buffer below both needs is refused
-    M = 4096
+    # 4096 rows, the weight gradient by a slab kernel under either choice: a buffer below both needs is refused (the
+    # buffers have their full sizes, so that a call that were accepted would stay inside them)
     if bits >= 7:
+        a, w, gc = problem(bits, 4096, K, N, bits)
+        t = [torch.from_numpy(v).to(dev) for v in (gc, a, w, la, lw)]
+        ga, gw = (torch.zeros(s, dtype=torch.float32, device=dev) for s in (a.shape, w.shape))
+        scratch = torch.empty(lib.lutgemm_backward_scratch_bytes(bits, 4096, K, N), dtype=torch.uint8, device=dev)
+        launches = lib.lutgemm_kernel_launches()
         rc = lib.lutgemm_backward(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), ga.data_ptr(), gw.data_ptr(), t[3].data_ptr(),
-                                  t[4].data_ptr(), bits, M, K, N, ga.data_ptr(), 16, None)
-        assert rc == -4  # LUTGEMM_E_SCRATCH, before anything is launched
+                                  t[4].data_ptr(), bits, 4096, K, N, scratch.data_ptr(), 16, None)
+        assert rc == -4 and lib.lutgemm_kernel_launches() == launches  # LUTGEMM_E_SCRATCH, before anything is launched
 
 
 @pytest.mark.parametrize("bits", [6, 7, 8])
@@ -168,6 +174,77 @@ def test_image_gradient_without_scratch(dev, oracle_c, bits):
     col = oracle_c.im2col(x, k, k, 1, 1, 1)
     r_ga, _, r_gaa, _ = oracle_c.backward_f64(gy, col, wmat, la, lw, bits)
     check(gx.cpu().numpy(), O.col2im_f64(r_ga, x.shape, k, k, 1, 1, 1), O.col2im_f64(r_gaa, x.shape, k, k, 1, 1, 1))
+    # it is the broadcast kernel that ran, and a slab kernel that would have (their sums differ in the last bits)
+    other = {}
+    try:
+        for family in ("bcast", "auto"):
+            approx_ops.set_kernel_choice(backward=family)
+            other[family] = torch.empty_like(gx)
+            approx_ops.approx_conv2d_backward(t[0], t[1], t[2], other[family], None, t[3], t[3], k, k, 1, 1, 1)
+    finally:
+        approx_ops.set_kernel_choice()
+    assert torch.equal(gx, other["bcast"]) and not torch.equal(gx, other["auto"])
+
+
+@pytest.mark.parametrize("bits", [4, 6, 7, 8])
+@pytest.mark.parametrize("M,K,N", [(512, 80, 64), (700, 77, 90), (40, 301, 33), (512 * 296 - 100, 70, 20)])
+def test_forward_slab_kernel_without_and_with_a_workspace(dev, bits, M, K, N):
+    """Five and more 16-k operand chunks, a last one of 6, 13 or 16 k, tiles cut across CTAs and (the last) whole tiles of
+    which a CTA takes two, with the three ways to stage operands: whole numbers, so equal to the broadcast kernel's sums."""
+    import approx_ops
+    lib = approx_ops.library()
+    a, w, _ = problem(bits, M, K, N, bits + M)
+    lut = O.pack_padded(np.random.default_rng(bits).integers(0, 2 ** 16, (1 << bits, 1 << bits)), bits, np.uint16)
+    a, w, lut = (torch.from_numpy(v).to(dev) for v in (a, w, lut))
+    out = []
+
+    def run(family, ws, tma):
+        approx_ops.set_kernel_choice(forward=family)
+        lib.lutgemm_set_tma(tma)
+        nbytes = lib.lutgemm_forward_scratch_bytes(bits, M, K, N) if ws else 0
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        c = torch.full((M, N), 7, dtype=torch.int32, device=dev).view(torch.uint32)
+        assert lib.lutgemm_forward_ws(a.data_ptr(), w.data_ptr(), c.data_ptr(), lut.data_ptr(), bits, M, K, N,
+                                      scratch.data_ptr() if nbytes else None, nbytes, None) == 0
+        torch.cuda.synchronize()
+        out.append(c.view(torch.int32))
+    try:
+        run("rowbcast", False, 1)
+        run("slab", False, 1)
+        run("slab", True, 0)
+        run("slab", True, 1)
+    finally:
+        approx_ops.set_kernel_choice()
+        lib.lutgemm_set_tma(1)
+    assert approx_ops.device_error() == 0
+    assert all(torch.equal(out[0], o) for o in out[1:])
+
+
+@pytest.mark.parametrize("M,K,N", [(256, 576, 64), (300, 200, 600), (40000, 100, 24)])
+def test_forward_with_a_workspace_that_is_too_small(dev, M, K, N):
+    """Shapes where only the estimate picks the slab kernel: sums and layer outputs are those of the full workspace."""
+    import approx_ops
+    lib, bits = approx_ops.library(), 7
+    a, w, _ = problem(bits, M, K, N, M)
+    lut = O.pack_padded(np.random.default_rng(2).integers(0, 2 ** 14, (128, 128)), bits, np.uint16)
+    a, w, lut = (torch.from_numpy(v).to(dev) for v in (a, w, lut))
+    box, sumw, taps = a.sum(dim=1, dtype=torch.float32), w.sum(dim=0, dtype=torch.float32), torch.full((1,), float(K), device=dev)
+    q = torch.tensor([0.01, -3.0, 0.02, -60.0], device=dev)
+    full = lib.lutgemm_forward_scratch_bytes(bits, M, K, N)
+    full_layer = lib.lutgemm_forward_layer_scratch_bytes(bits, M, K, N)
+    assert full > 64 and full_layer > 64
+    scratch = torch.empty(max(full, full_layer), dtype=torch.uint8, device=dev)
+    c, o = [], []
+    for small in (False, True):
+        c.append(torch.zeros((M, N), dtype=torch.int32, device=dev))
+        o.append(torch.zeros((M, N), device=dev))
+        assert lib.lutgemm_forward_ws(a.data_ptr(), w.data_ptr(), c[-1].data_ptr(), lut.data_ptr(), bits, M, K, N,
+                                      scratch.data_ptr(), 64 if small else full, None) == 0
+        assert lib.lutgemm_forward_layer(a.data_ptr(), w.data_ptr(), lut.data_ptr(), bits, M, K, N, box.data_ptr(), sumw.data_ptr(),
+                                         taps.data_ptr(), q.data_ptr(), q[2:].data_ptr(), q[1:].data_ptr(), q[3:].data_ptr(), None,
+                                         o[-1].data_ptr(), scratch.data_ptr(), 64 if small else full_layer, None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(c[0], c[1]) and torch.equal(o[0], o[1])
 
 
 @pytest.mark.parametrize("Cout,Cin,k", [(8, 5, 1), (13, 700, 1), (64, 33, 3), (9, 3, 23), (1, 1, 1)])

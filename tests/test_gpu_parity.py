@@ -120,8 +120,8 @@ def test_each_forward_kernel_on_every_shape_class(dev, oracle_c, bits, kernel, k
 @pytest.mark.parametrize("kernel", ["bcast", "slab-wide", "slab-tall"])
 @pytest.mark.parametrize("bits", [4, 6, 7, 8])
 def test_each_backward_kernel_on_every_shape_class(dev, oracle_c, bits, kernel, kernel_choice):
-    """Every family of gradient kernels (selected through lutgemm_set_kernel_choice: fp32 slab with the
-    512 x 64 and the 1024 x 32 tile, broadcast) on shapes of either class."""
+    """Every family of gradient kernels (selected through lutgemm_set_kernel_choice: packed slab
+    with the 512 x 64 tile, fp32 slab with the 1024 x 32 tile, broadcast) on shapes of either class."""
     kernel_choice(backward=kernel.split("-")[0], grad_tile="tall" if kernel.endswith("-tall") else "wide")
     _, la, lw = synth_wire(bits, seed=20 + bits)
     shapes = [(1, 1, 1), (5, 33, 3), (130, 16, 64), (515, 31, 67), (1024, 48, 128), (66, 35, 520)]
