@@ -78,11 +78,11 @@ def _valid_taps(geom, device):
     return _VALID_TAPS[key]
 
 
-def _keep_codes(codes_t, M, N):
+def _keep_codes(codes_t, N):
     """The forward kernel's transposed codes ([K, M] bytes) where the backward pass should find them again.  A layer of fewer
-    than 32 outputs would hold several times its saved activations for a weight gradient that is short: there the copy is
-    made again (256 x 16 x 32 x 32, 3x3: 38 MB not held)."""
-    return codes_t if N >= 32 or M < 512 else None
+    than 32 outputs would hold several times its saved activations for a weight gradient that is short: there a copy above
+    8 MB is made again (256 x 16 x 32 x 32, 3x3: 38 MB not held); below, the launch would cost a small layer more."""
+    return codes_t if codes_t is None or N >= 32 or codes_t.numel() <= 1 << 23 else None
 
 
 class _AppConvLayer(torch.autograd.Function):
@@ -108,7 +108,7 @@ class _AppConvLayer(torch.autograd.Function):
         out, codes, wmat, codes_t = approx_ops.conv2d_layer_pass(x, weight, bias, quant, a_qmax, w_qmax,
                                                                  _ops_state.lut_appmult, stride, padding, dilation)
         ctx.save_for_backward(x, codes, wmat, weight, quant)
-        ctx.codes_t = _keep_codes(codes_t, B * Ho * Wo, Cout)  # transposed unfolded codes: the grad_w kernel reuses them
+        ctx.codes_t = _keep_codes(codes_t, Cout)  # transposed unfolded codes: the grad_w kernel reuses them
         ctx.cfg = (a_qmax, w_qmax, stride, padding, dilation, Ho, Wo, bias is not None)
         return out.view(B, Ho, Wo, Cout).permute(0, 3, 1, 2)  # NCHW view of channels-last memory
 
@@ -169,7 +169,7 @@ class _AppLinearLayer(torch.autograd.Function):
         out, codes_t = approx_ops.approx_gemm_forward_layer(codes, wmat, _ops_state.lut_appmult, box, sumw_t, taps, s_a, s_w,
                                                             z_a, z_w, bias)
         ctx.save_for_backward(x2, codes, wmat, weight, quant)
-        ctx.codes_t = _keep_codes(codes_t, M, N)  # transposed codes of the forward kernel: the grad_w kernel reuses them
+        ctx.codes_t = _keep_codes(codes_t, N)  # transposed codes of the forward kernel: the grad_w kernel reuses them
         ctx.cfg = (a_qmax, w_qmax, bias is not None)
         return out
 

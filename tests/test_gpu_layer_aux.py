@@ -199,15 +199,15 @@ def test_a_layer_runs_on_slower_kernels_where_the_fast_ones_do_not_fit(dev, monk
         r.sum().backward()
 
 
-@pytest.mark.parametrize("cout,held", [(16, False), (31, False), (32, True), (64, True)])
-def test_narrow_layers_hold_no_code_copy_for_the_backward_pass(dev, cout, held):
+@pytest.mark.parametrize("cout,batch,held", [(16, 64, False), (31, 64, False), (16, 48, True), (32, 64, True), (64, 64, True)])
+def test_narrow_layers_hold_no_large_code_copy_for_the_backward_pass(dev, cout, batch, held):
     import self_ops
     from lutgemm_layers import AppConv2d, AppLinear
     from lutgemm_luts import synthetic_multiplier, window_difference_gradients
     self_ops.set_lookup_tables(dev, synthetic_multiplier(7, seed=0), *window_difference_gradients(synthetic_multiplier(7, seed=0), 8), 7)
     conv = AppConv2d(16, cout, 3, 1, 1, bias=False, a_bits=7, w_bits=7, conv_impl="layer").to(dev).train()
     lin = AppLinear(144, cout, a_bits=7, w_bits=7, impl="layer").to(dev).train()
-    for out in (conv(torch.rand(64, 16, 32, 32, device=dev)), lin(torch.rand(65536, 144, device=dev))):
+    for out in (conv(torch.rand(batch, 16, 32, 32, device=dev)), lin(torch.rand(batch * 1024, 144, device=dev))):
         fn = out.grad_fn
         while not hasattr(fn, "codes_t"):
             fn = fn.next_functions[0][0]
