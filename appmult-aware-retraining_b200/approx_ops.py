@@ -168,10 +168,13 @@ def _check_input(x: torch.Tensor, dtype: torch.dtype, name: str) -> None:
         raise RuntimeError(f"{name} must be of type {dtype}")
 
 
+_F32 = torch.float32
+
+
 def _check_fp32(x: torch.Tensor, name: str, index: int, numel: int = None) -> None:
     """An fp32 operand on CUDA device `index` that goes to the library as a pointer; with `numel` it has to be that many values
     in a row."""
-    if x.dtype is not torch.float32:
+    if x.dtype is not _F32:
         raise RuntimeError(f"{name} must be of type torch.float32")
     if x.get_device() != index or index < 0:
         raise RuntimeError(f"{name} must be on the CUDA device of the other operands, not on {x.device}")
@@ -187,8 +190,15 @@ def _bits_of(lut: torch.Tensor, name: str) -> int:
     return bits
 
 
+# (device indices: resolving a device object takes PyTorch a microsecond each time)
+def _guard(device: torch.device):
+    if device.type != "cuda":
+        raise ValueError(f"expected a CUDA device, but got {device}")
+    return torch.cuda.device(device.index)
+
+
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch.cuda.current_stream(device.index).cuda_stream
 
 
 def _backward_scratch(query, args, codes_t, dev):
@@ -246,7 +256,7 @@ def approx_gemm_forward(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, lut: 
         c.zero_()
         return
     lib = _load()
-    with torch.cuda.device(dev):
+    with _guard(dev):
         # workspace for the transposed activation codes (0 bytes when the kernel for this shape has no use for it)
         scratch, nbytes, short = _forward_workspace(lib.lutgemm_forward_scratch_bytes(bits, M, K, N), dev)
         rc = lib.lutgemm_forward_ws(a.data_ptr(), b.data_ptr(), c.data_ptr(), lut.data_ptr(), bits, M, K, N,
@@ -289,7 +299,7 @@ def approx_gemm_backward(gc: torch.Tensor, a: torch.Tensor, b: torch.Tensor, ga:
         gb.zero_()
         return
     lib = _load()
-    with torch.cuda.device(dev):
+    with _guard(dev):
         scratch, nbytes = _backward_scratch(lib.lutgemm_backward_ws_scratch_bytes, (bits, M, K, N), codes_t, dev)
         if codes_t is not None:
             _check_input(codes_t, torch.uint8, "codes_t")
@@ -344,7 +354,7 @@ def approx_conv2d_forward(x: torch.Tensor, wmat: torch.Tensor, y: torch.Tensor, 
     if wmat.device != x.device or y.device != x.device or lut.device != x.device:
         raise RuntimeError("device id not match")
     lib = _load()
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         nbytes = lib.lutgemm_conv2d_forward_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
         codes_t, nbytes, short = _forward_workspace(nbytes, x.device)
         rc = lib.lutgemm_conv2d_forward_ws(x.data_ptr(), wmat.data_ptr(), y.data_ptr(), lut.data_ptr(), bits, B, C, H,
@@ -382,7 +392,7 @@ def approx_conv2d_forward_layer(x: torch.Tensor, wmat: torch.Tensor, lut: torch.
     epi = _epilogue_args(box, sumw_t, taps, s_a, s_w, z_a, z_w, bias, M, L, Cout)
     out = torch.empty((M, Cout), dtype=torch.float32, device=x.device)
     lib = _load()
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         ncodes = lib.lutgemm_conv2d_forward_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
         nbytes = lib.lutgemm_conv2d_forward_layer_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil)
         scratch, nbytes, short = _forward_workspace(nbytes, x.device)
@@ -418,7 +428,7 @@ def conv2d_layer_pass(x: torch.Tensor, weight: torch.Tensor, bias, quant: torch.
         _check_fp32(bias, "bias_tensor", index, Cout)
     lib = _load()
     geom = (B, C, H, W, Cout, kh, kw, stride, pad, dil)
-    with torch.cuda.device(dev):
+    with _guard(dev):
         ncodes = lib.lutgemm_conv2d_forward_scratch_bytes(bits, *geom)
         nbytes = lib.lutgemm_conv2d_forward_layer_scratch_bytes(bits, *geom)
         codes = torch.empty((B, C, H, W), dtype=torch.uint8, device=dev)
@@ -450,7 +460,7 @@ def approx_gemm_forward_layer(a: torch.Tensor, b: torch.Tensor, lut: torch.Tenso
     epi = _epilogue_args(box, sumw_t, taps, s_a, s_w, z_a, z_w, bias, M, 1, N)
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     lib = _load()
-    with torch.cuda.device(a.device):
+    with _guard(a.device):
         ncodes = lib.lutgemm_forward_scratch_bytes(bits, M, K, N)
         nbytes = lib.lutgemm_forward_layer_scratch_bytes(bits, M, K, N)
         scratch, nbytes, short = _forward_workspace(nbytes, a.device)
@@ -490,7 +500,7 @@ def approx_conv2d_backward(gy: torch.Tensor, x: torch.Tensor, wmat: torch.Tensor
         if t is not None and t.device != dev:
             raise RuntimeError("All tensors should be on the same device")
     lib = _load()
-    with torch.cuda.device(dev):
+    with _guard(dev):
         scratch, nbytes = _backward_scratch(lib.lutgemm_conv2d_backward_ws_scratch_bytes,
                                             (bits, B, C, H, W, Cout, kh, kw, stride, pad, dil), codes_t, dev)
         if codes_t is not None:
@@ -523,7 +533,7 @@ def approx_gemm_backward_f32lut(gc: torch.Tensor, a: torch.Tensor, b: torch.Tens
     if bits < 0 or bits > 7 or lut_grad_b.numel() != lut_grad_a.numel():
         raise RuntimeError("fp32 gradient tables must both have the padded length of a bit-width up to 7")
     dev = gc.device
-    with torch.cuda.device(dev):
+    with _guard(dev):
         nbytes = lib.lutgemm_backward_f32lut_scratch_bytes(bits, M, K, N)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
         rc = lib.lutgemm_backward_f32lut(gc.data_ptr(), a.data_ptr(), b.data_ptr(), ga.data_ptr(), gb.data_ptr(),
@@ -551,7 +561,7 @@ def quantize_activations(x: torch.Tensor, scale: torch.Tensor, zp_neg: torch.Ten
     codes = torch.empty((B, C, H, W), dtype=torch.uint8, device=x.device)
     chansum = torch.zeros((B, H, W), dtype=torch.float32, device=x.device) if want_chansum else None
     sb, sc, sh, sw = x.stride()
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         rc = _load().lutgemm_quantize_activations(x.data_ptr(), sb, sc, sh, sw, B, C, H, W, scale.data_ptr(),
                                                   zp_neg.data_ptr(), float(qmax), codes.data_ptr(),
                                                   chansum.data_ptr() if want_chansum else None, _stream_ptr(x.device))
@@ -574,7 +584,7 @@ def quantize_activations_backward(x: torch.Tensor, scale: torch.Tensor, zp_neg: 
         raise RuntimeError("could not allocate a gradient with the strides of input_tensor")
     if box_t is not None:
         _check_input(box_t, torch.float32, "box_t_tensor")
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         rc = _load().lutgemm_quantize_activations_backward(
             x.data_ptr(), sb, sc, sh, sw, B, C, H, W, scale.data_ptr(), zp_neg.data_ptr(), float(qmax), gcodes.data_ptr(),
             box_t.data_ptr() if box_t is not None else None, s_w.data_ptr(), z_w.data_ptr(), gx.data_ptr(),
@@ -593,7 +603,7 @@ def conv2d_epilogue(y: torch.Tensor, box: torch.Tensor, sumw_t: torch.Tensor, ta
         if tuple(t.shape) != shape:
             raise RuntimeError(f"{name} has shape {tuple(t.shape)}, expected {shape}")
     out = torch.empty((M, Cout), dtype=torch.float32, device=y.device)
-    with torch.cuda.device(y.device):
+    with _guard(y.device):
         rc = _load().lutgemm_conv2d_epilogue(y.data_ptr(), box.data_ptr(), sumw_t.data_ptr(), taps.data_ptr(),
                                              s_a.data_ptr(), s_w.data_ptr(), z_a.data_ptr(), z_w.data_ptr(),
                                              bias.data_ptr() if bias is not None else None, out.data_ptr(), M, L, Cout,
@@ -611,7 +621,7 @@ def layer_update_ranges(act_lo, act_hi, w_lo, w_hi, act_state, w_state, momentum
     {s_a, z_a, s_w, z_w}."""
     dev = quant.device
     eps = float(torch.finfo(torch.float32).eps)
-    with torch.cuda.device(dev):
+    with _guard(dev):
         rc = _load().lutgemm_layer_update_ranges(
             act_lo.data_ptr(), act_hi.data_ptr(), w_lo.data_ptr(), w_hi.data_ptr(), act_state[0].data_ptr(),
             act_state[1].data_ptr(), act_state[2].data_ptr(), w_state[0].data_ptr(), w_state[1].data_ptr(),
@@ -630,7 +640,7 @@ def layer_weight_prep(weight: torch.Tensor, quant: torch.Tensor, qmax: float):
     wmat = torch.empty((Cin * kh * kw, Cout), dtype=torch.uint8, device=weight.device)
     wsum = torch.empty((Cout, kh * kw), dtype=torch.float32, device=weight.device)
     s = weight.stride()
-    with torch.cuda.device(weight.device):
+    with _guard(weight.device):
         rc = _load().lutgemm_layer_weight_prep(weight.data_ptr(), s[0], s[1], s[2], s[3], Cout, Cin, kh, kw, quant.data_ptr(),
                                                float(qmax), wmat.data_ptr(), wsum.data_ptr(), _stream_ptr(weight.device))
     _check(rc, "layer_weight_prep")
@@ -644,7 +654,7 @@ def layer_cross_terms(wsum: torch.Tensor, Cin: int, H: int, W: int, kh: int, kw:
     Ho, Wo = _conv_out(H, W, kh, kw, stride, pad, dil)
     sumw_t = torch.empty((Ho * Wo, Cout), dtype=torch.float32, device=wsum.device)
     taps = torch.empty((Ho * Wo,), dtype=torch.float32, device=wsum.device)
-    with torch.cuda.device(wsum.device):
+    with _guard(wsum.device):
         rc = _load().lutgemm_layer_cross_terms(wsum.data_ptr(), Cout, Cin, H, W, kh, kw, stride, pad, dil, sumw_t.data_ptr(),
                                                taps.data_ptr(), _stream_ptr(wsum.device))
     _check(rc, "layer_cross_terms")
@@ -657,7 +667,7 @@ def layer_window_sum(img: torch.Tensor, kh: int, kw: int, stride: int, pad: int,
     B, H, W = img.shape
     Ho, Wo = _conv_out(H, W, kh, kw, stride, pad, dil)
     box = torch.empty((B * Ho * Wo,), dtype=torch.float32, device=img.device)
-    with torch.cuda.device(img.device):
+    with _guard(img.device):
         rc = _load().lutgemm_layer_window_sum(img.data_ptr(), B, H, W, kh, kw, stride, pad, dil, box.data_ptr(),
                                               _stream_ptr(img.device))
     _check(rc, "layer_window_sum")
@@ -669,7 +679,7 @@ def layer_window_sum_adjoint(gsum: torch.Tensor, H: int, W: int, kh: int, kw: in
     _check_input(gsum, torch.float32, "grad_sum")
     B = gsum.shape[0]
     out = torch.empty((B, H, W), dtype=torch.float32, device=gsum.device)
-    with torch.cuda.device(gsum.device):
+    with _guard(gsum.device):
         rc = _load().lutgemm_layer_window_sum_adjoint(gsum.data_ptr(), B, H, W, kh, kw, stride, pad, dil, out.data_ptr(),
                                                       _stream_ptr(gsum.device))
     _check(rc, "layer_window_sum_adjoint")
@@ -684,7 +694,7 @@ def layer_weight_grad(gwmat: torch.Tensor, tapg: torch.Tensor, weight: torch.Ten
     Cout, Cin, kh, kw = weight.shape
     gw = torch.empty((Cout, Cin, kh, kw), dtype=torch.float32, device=weight.device)
     s = weight.stride()
-    with torch.cuda.device(weight.device):
+    with _guard(weight.device):
         rc = _load().lutgemm_layer_weight_grad(gwmat.data_ptr(), tapg.data_ptr(), weight.data_ptr(), s[0], s[1], s[2], s[3],
                                                Cout, Cin, kh, kw, quant.data_ptr(), float(qmax), gw.data_ptr(),
                                                _stream_ptr(weight.device))

@@ -90,3 +90,13 @@ def test_bench_reads_dram_traffic_from_the_committed_capture_summary():
         assert "profiles/" in source
     assert bench.ncu_dram_traffic("forward", (7, 4096, 4096)) == (None, None)
     assert bench.ncu_dram_traffic("no such kernel", (8, 4096, 4096)) == (None, None)
+
+
+def test_device_guard_refuses_tensors_without_a_cuda_device():
+    import approx_ops
+    import torch
+    for f in (lambda: approx_ops.layer_cross_terms(torch.zeros(4, 9), 3, 5, 5, 3, 3, 1, 1, 1),
+              lambda: approx_ops.layer_update_ranges(*[torch.zeros(1)] * 4, [torch.zeros(1)] * 3, [torch.zeros(1)] * 3, 0.1, 127.0, 127.0,
+                                                     torch.zeros(4))):
+        with pytest.raises(ValueError):
+            f()
