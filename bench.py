@@ -715,7 +715,7 @@ def ncu_dram_traffic(kernel, config):
         for name in ("dram__bytes_read.sum", "dram__bytes_write.sum"):
             r = next(r for r in rows if r[0] == name)
             total += float(r[col].replace(",", "")) * scale[r[1]]
-        return total, f"ncu --set full capture of one launch of this kernel at this size ({NCU_TRAFFIC_PROFILE['file']})"
+        return total, f"ncu capture of one launch of this kernel at this size ({NCU_TRAFFIC_PROFILE['file']})"
     except (OSError, StopIteration, ValueError, KeyError, IndexError):
         return None, None
 
