@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     const uint32_t u_addr = smem_u32(smem + C::OFF_U);
     const uint32_t bar_full = smem_u32(smem + C::OFF_BAR), bar_empty = bar_full + 8 * NB;
     volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 16 * NB);
-    int *work_s = reinterpret_cast<int *>(smem + C::OFF_BAR + 16 * NB + 4);  // grad_w: cell and k range of the work item
+    int *work_s = reinterpret_cast<int *>(smem + C::OFF_BAR + 16 * NB + 4);  // grad_w, grad_a: cell and k range of the work item
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int half = lane >> 4, cq = lane & 15;  // half-warp and column quad (columns 4 cq .. 4 cq + 3)
 
@@ -352,9 +352,10 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             kbeg = (j % p.tail_parts) * p.tail_per;
             kend = min(K, kbeg + p.tail_per);
         }
-        if constexpr (MODE == kGw) {
+        if constexpr (MODE != kGx) {
             // the compiler's schedule of the k loop depends on what it sees of these three: read back from shared memory
-            // grad_w takes 1.49 ms for 4096 x 4608 x 512 at 7 bits, straight from the branch 1.53 (grad_x: the other way round)
+            // grad_w takes 1.49 ms for 4096 x 4608 x 512 at 7 bits and grad_a 11.11 ms for 4096^3, straight from the branch
+            // 1.53 and 11.50 (grad_x: the other way round, 6.81 against 6.93 ms at 8 bits for 16 x 256 x 56 x 56, 3x3)
             if (tid == 0) { work_s[0] = cell; work_s[1] = kbeg; work_s[2] = kend; }
             __syncthreads();
             cell = work_s[0];
