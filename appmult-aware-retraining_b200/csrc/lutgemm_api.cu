@@ -52,13 +52,16 @@ struct BackwardPlan {
     bool gw_slab, ga_slab;
     bool gw_tall, ga_tall;  // fp32 slab with the 1024 x 32 tile instead of the packed slab with the 512 x 64 tile
     int gw_splits;        // row-broadcast grad_w kernel: slabs of M
-    size_t gw_scratch, ga_scratch;
     // slab grad_w kernels read the activation codes from a transposed copy at[k][m] (their row-code fetch is then
     // coalesced; for a convolution it also replaces one implicit-im2col gather per column tile by a single one): the
     // caller's, or one made behind the partial sums in the scratch buffer
-    size_t gw_at_offset;  // bytes into the scratch buffer, a multiple of 16
-    int gw_at_pitch;      // 0 = no transposed copy
+    // (grad_a with one thread per row reads them too)
+    size_t at_offset;  // bytes into the scratch buffer, a multiple of 16
+    int at_pitch;      // 0 = no transposed copy
+    size_t scratch;    // whole buffer: sums of either gradient, which run one after the other, then the copy
     lutgemm::PackedPlan gw_packed, ga_packed;
+    bool gw_rows, ga_rows;  // one thread per output row instead of the packed or tall slab kernel
+    lutgemm::RowsPlan gw_rows_plan, ga_rows_plan;
 };
 
 // ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
@@ -75,12 +78,12 @@ struct BackwardPlan {
 // (base_plan below) the estimates move small and ragged problems to the slab kernels: 256 x 512 x 256 at 7 bits, forward 0.291 ms,
 // grad_w 0.088 ms and grad_a 0.092 ms with the broadcast kernels, both gradients 0.034 ms with the slab kernels.
 struct FamilyClocks {
-    double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start;
+    double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start, rows;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3};
-    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3};
-    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3};
+    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390};
+    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150};
+    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, bits == 6 ? 1070.0 : 1420.0};
 }
 constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
@@ -116,32 +119,36 @@ double ga_bcast_clocks(int bits, int M, int K, int N, int sms) {
     return (double)div_up(div_up(M, mt) * div_up(K, 32), sms) * mt * N * family_clocks(bits).ga_bcast + kBcastStart;
 }
 
-void set_gw_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bool have_codes) {
-    pl.gw_splits = pl.gw_slab ? 1 : lutgemm::gw_num_splits(bits, M, K, N, sms);
-    pl.gw_at_offset = 0;
-    pl.gw_at_pitch = 0;
-    if (pl.gw_slab) {
-        const int rb = pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : pl.gw_packed.groups;
-        pl.gw_scratch = rb > 1 ? (size_t)rb * K * N * sizeof(float) : 0;
-        pl.gw_at_pitch = (M + 15) & ~15;
-        if (!have_codes) {
-            pl.gw_at_offset = (pl.gw_scratch + 15) & ~(size_t)15;
-            pl.gw_scratch = pl.gw_at_offset + (size_t)pl.gw_at_pitch * K;
-        }
-    } else {
-        pl.gw_scratch = pl.gw_splits > 1 ? (size_t)pl.gw_splits * K * N * sizeof(float) : 0;
-    }
+// (`aligned`: a block's grad_out values come in 16-byte vectors; `copy`: the transposed codes have to be made for it)
+double rows_clocks(const lutgemm::RowsPlan &p, int bits, long rows, int K, bool direct, bool aligned, bool copy) {
+    const bool reduce = p.groups > 1 || !direct;
+    return p.steps * family_clocks(bits).rows + p.loads * (aligned ? 9e3 : 27e3) + (bits == 8 ? 35e3 : 25e3) + (copy ? 13e3 : 0) +
+           (reduce ? 15e3 + 8.0 * p.groups * K * rows / kReduceBytesPerClock : 0);
 }
-void set_ga_scratch(BackwardPlan &pl, int M, int K, int N) {
-    if (!pl.ga_slab) return;
-    const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(N);
-    const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : pl.ga_packed.groups;
-    pl.ga_scratch = N > rt ? (size_t)blocks * K * M * sizeof(float) : 0;
+
+void set_scratch(BackwardPlan &pl, int bits, int M, int K, int N, int sms, bool want_gw, bool want_ga, bool have_codes) {
+    size_t gw = 0, ga = 0;
+    if (want_gw) {
+        pl.gw_splits = pl.gw_slab ? 1 : lutgemm::gw_num_splits(bits, M, K, N, sms);
+        const int blocks = !pl.gw_slab ? pl.gw_splits : pl.gw_tall ? lutgemm::slab_tall_row_blocks(M) : pl.gw_packed.groups;
+        gw = pl.gw_rows ? lutgemm::rows_scratch_bytes(pl.gw_rows_plan, N, K, true, sms) : blocks > 1 ? (size_t)blocks * K * N * sizeof(float) : 0;
+    }
+    if (want_ga && pl.ga_slab) {
+        const int rt = pl.ga_tall ? lutgemm::kSlabTallRows : lutgemm::packed_ga_tile_rows(N);
+        const int blocks = pl.ga_tall ? lutgemm::slab_tall_row_blocks(N) : pl.ga_packed.groups;
+        ga = pl.ga_rows ? lutgemm::rows_scratch_bytes(pl.ga_rows_plan, M, K, false, sms) : N > rt ? (size_t)blocks * K * M * sizeof(float) : 0;
+    }
+    pl.scratch = gw > ga ? gw : ga;
+    pl.at_pitch = (want_gw && pl.gw_slab) || (want_ga && pl.ga_rows) ? (M + 15) & ~15 : 0;
+    if (pl.at_pitch && !have_codes) {
+        pl.at_offset = (pl.scratch + 15) & ~(size_t)15;
+        pl.scratch = pl.at_offset + (size_t)pl.at_pitch * K;
+    }
 }
 
 // Choice by fixed limits: the plan for callers whose scratch buffer is too small for the faster one (a fixed buffer, or
 // one sized for this choice), so that what fitted such a buffer keeps running.
-BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) {
+BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool want_gw, bool want_ga, bool have_codes) {
     BackwardPlan pl{};
     pl.gw_slab = bits >= 7 && M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6;
     const double ga_fill = slab_fill(N, M) > tall_fill(N, M) ? slab_fill(N, M) : tall_fill(N, M);
@@ -150,8 +157,7 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) 
     pl.ga_tall = pl.ga_slab && tall_fill(N, M) >= 0.7 * slab_fill(N, M);
     if (pl.gw_slab && !pl.gw_tall) pl.gw_packed = lutgemm::plan_packed_gw(M, N, K, sms);
     if (pl.ga_slab && !pl.ga_tall) pl.ga_packed = lutgemm::plan_packed(N, M, K, lutgemm::packed_ga_tile_rows(N), sms);
-    set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
-    set_ga_scratch(pl, M, K, N);
+    set_scratch(pl, bits, M, K, N, sms, want_gw, want_ga, have_codes);
     return pl;
 }
 
@@ -163,22 +169,38 @@ BackwardPlan base_plan(int bits, int M, int K, int N, int sms, bool have_codes) 
 BackwardPlan plan_backward(int bits, int M, int K, int N, int sms, bool conv, bool want_gw, bool want_ga, bool have_codes) {
     BackwardPlan pl{};
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
+    const bool rows = tile == LUTGEMM_TILE_ROWS || (!force && !tile);  // may the kernel with one thread per row be chosen?
     if (want_gw) {
         pl.gw_packed = lutgemm::plan_packed_gw(M, N, K, sms);
         const double packed = packed_gw_clocks(pl.gw_packed, bits, K, N), tall = tall_clocks(bits, M, N, K, sms);
-        pl.gw_slab = (packed < tall ? packed : tall) < gw_bcast_clocks(bits, M, K, N, sms);
+        double slab = packed < tall ? packed : tall;
+        if (rows && lutgemm::rows_supported(N, M, K)) {
+            pl.gw_rows_plan = lutgemm::plan_rows(N, M, K, sms);
+            const double t = rows_clocks(pl.gw_rows_plan, bits, N, K, true, N % 4 == 0, false);
+            pl.gw_rows = tile == LUTGEMM_TILE_ROWS || t < slab;
+            if (pl.gw_rows) slab = t;
+        }
+        pl.gw_slab = slab < gw_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.gw_slab = force == LUTGEMM_BACKWARD_SLAB;
-        pl.gw_tall = pl.gw_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_gw_scratch(pl, bits, M, K, N, sms, have_codes);
+        pl.gw_rows = pl.gw_rows && pl.gw_slab;
+        pl.gw_tall = pl.gw_slab && !pl.gw_rows && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
     }
     if (want_ga) {
         pl.ga_packed = lutgemm::plan_packed(N, M, K, lutgemm::packed_ga_tile_rows(N), sms);
         const double packed = packed_ga_clocks(pl.ga_packed, bits, M, K, N), tall = tall_clocks(bits, N, M, K, sms);
-        pl.ga_slab = (!conv || N >= 768) && (packed < tall ? packed : tall) < ga_bcast_clocks(bits, M, K, N, sms);
+        double slab = packed < tall ? packed : tall;
+        if (rows && !conv && lutgemm::rows_supported(M, N, K)) {
+            pl.ga_rows_plan = lutgemm::plan_rows(M, N, K, sms);
+            const double t = rows_clocks(pl.ga_rows_plan, bits, M, K, false, N % 4 == 0, !want_gw && !have_codes);
+            pl.ga_rows = tile == LUTGEMM_TILE_ROWS || t < slab;
+            if (pl.ga_rows) slab = t;
+        }
+        pl.ga_slab = (!conv || N >= 768) && slab < ga_bcast_clocks(bits, M, K, N, sms);
         if (force) pl.ga_slab = force == LUTGEMM_BACKWARD_SLAB;
-        pl.ga_tall = pl.ga_slab && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
-        set_ga_scratch(pl, M, K, N);
+        pl.ga_rows = pl.ga_rows && pl.ga_slab;
+        pl.ga_tall = pl.ga_slab && !pl.ga_rows && (tile ? tile == LUTGEMM_TILE_TALL : tall < packed);
     }
+    set_scratch(pl, bits, M, K, N, sms, want_gw, want_ga, have_codes);
     return pl;
 }
 
@@ -191,8 +213,8 @@ void record_cuda_error(cudaError_t e) { g_last_cuda_error = e; }
 size_t base_gw_scratch_bytes(int bits, int M, int K, int N) {
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    if (g_force_backward.load(std::memory_order_relaxed)) return plan_backward(bits, M, K, N, sms, false, true, false, false).gw_scratch;
-    return base_plan(bits, M, K, N, sms, false).gw_scratch;
+    if (g_force_backward.load(std::memory_order_relaxed)) return plan_backward(bits, M, K, N, sms, false, true, false, false).scratch;
+    return base_plan(bits, M, K, N, sms, true, false, false).scratch;
 }
 
 int launch_status() {
@@ -237,7 +259,7 @@ int lutgemm_set_handover(int on) {
 unsigned long long lutgemm_kernel_launches(void) { return g_kernel_launches.load(std::memory_order_relaxed); }
 
 int lutgemm_set_kernel_choice(int forward, int backward, int grad_tile) {
-    if (forward < 0 || forward > 2 || backward < 0 || backward > 2 || grad_tile < 0 || grad_tile > 2)
+    if (forward < 0 || forward > 2 || backward < 0 || backward > 2 || grad_tile < 0 || grad_tile > 3)
         return LUTGEMM_E_BADARG;
     g_force_forward.store(forward, std::memory_order_relaxed);
     g_force_backward.store(backward, std::memory_order_relaxed);
@@ -341,7 +363,6 @@ int lutgemm_selftest_bounded_wait(void *stream) {
     return lutgemm::bounded_wait_selftest(static_cast<cudaStream_t>(stream));
 }
 
-static size_t larger_need(const BackwardPlan &pl) { return pl.gw_scratch > pl.ga_scratch ? pl.gw_scratch : pl.ga_scratch; }
 // of a buffer for the faster choice and one for the fixed limits, the smaller one that is accepted
 static size_t least_need(size_t need, size_t base) {
     return base < need && !g_force_backward.load(std::memory_order_relaxed) ? base : need;
@@ -352,8 +373,8 @@ size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flag
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
     const bool have_codes = flags & LUTGEMM_SCRATCH_CODES_GIVEN;
-    const size_t need = larger_need(plan_backward(bits, M, K, N, sms, false, true, true, have_codes));
-    return flags & LUTGEMM_SCRATCH_LEAST ? least_need(need, larger_need(base_plan(bits, M, K, N, sms, have_codes))) : need;
+    const size_t need = plan_backward(bits, M, K, N, sms, false, true, true, have_codes).scratch;
+    return flags & LUTGEMM_SCRATCH_LEAST ? least_need(need, base_plan(bits, M, K, N, sms, true, true, have_codes).scratch) : need;
 }
 
 size_t lutgemm_backward_scratch_bytes(int bits, int M, int K, int N) {
@@ -376,27 +397,28 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t given = scratch ? scratch_bytes : 0;
     BackwardPlan pl = plan_backward(bits, M, K, N, sms, conv.enabled != 0, gw != nullptr, ga != nullptr, codes_t != nullptr);
-    if (((gw && pl.gw_scratch > given) || (ga && pl.ga_scratch > given)) && !g_force_backward.load(std::memory_order_relaxed))
-        pl = base_plan(bits, M, K, N, sms, codes_t != nullptr);
+    if (pl.scratch > given && !g_force_backward.load(std::memory_order_relaxed))
+        pl = base_plan(bits, M, K, N, sms, gw != nullptr, ga != nullptr, codes_t != nullptr);
+    if (pl.scratch > given) return LUTGEMM_E_SCRATCH;
     float *sc = static_cast<float *>(scratch);
+    const uint8_t *at = codes_t;  // left by the forward pass (same layout), or made here
+    if (pl.at_pitch && !at) {
+        uint8_t *dst = static_cast<uint8_t *>(scratch) + pl.at_offset;
+        const int trc = lutgemm::transpose_codes(a, dst, M, K, pl.at_pitch, conv, bits, s);
+        if (trc != LUTGEMM_OK) return trc;
+        at = dst;
+    }
     if (gw) {
         // the weight gradient goes first: under data parallelism its all-reduce can then overlap gA
-        if (pl.gw_scratch > given) return LUTGEMM_E_SCRATCH;
-        const uint8_t *at = codes_t;  // left by the forward pass (same layout), or made here
-        if (pl.gw_slab && pl.gw_at_pitch && !at) {
-            uint8_t *dst = static_cast<uint8_t *>(scratch) + pl.gw_at_offset;
-            const int trc = lutgemm::transpose_codes(a, dst, M, K, pl.gw_at_pitch, conv, bits, s);
-            if (trc != LUTGEMM_OK) return trc;
-            at = dst;
-        }
         int rc = !pl.gw_slab ? lutgemm::backward_gw(gc, a, w, gw, lut_gw, bits, M, K, N, conv, sc, pl.gw_splits, sms, s)
-                 : pl.gw_tall ? lutgemm::backward_gw_slab_tall(gc, a, w, gw, lut_gw, nullptr, bits, M, K, N, conv, sc, at, pl.gw_at_pitch, sms, s)
-                             : lutgemm::backward_gw_slab_packed(gc, a, w, gw, lut_gw, bits, M, K, N, conv, pl.gw_packed, sc, at, pl.gw_at_pitch, sms, s);
+                 : pl.gw_rows ? lutgemm::backward_gw_rows(gc, w, gw, lut_gw, bits, M, K, N, pl.gw_rows_plan, sc, at, pl.at_pitch, sms, s)
+                 : pl.gw_tall ? lutgemm::backward_gw_slab_tall(gc, a, w, gw, lut_gw, nullptr, bits, M, K, N, conv, sc, at, pl.at_pitch, sms, s)
+                             : lutgemm::backward_gw_slab_packed(gc, a, w, gw, lut_gw, bits, M, K, N, conv, pl.gw_packed, sc, at, pl.at_pitch, sms, s);
         if (rc != LUTGEMM_OK) return rc;
     }
     if (ga) {
-        if (pl.ga_scratch > given) return LUTGEMM_E_SCRATCH;
         int rc = !pl.ga_slab ? lutgemm::backward_ga(gc, a, w, ga, lut_ga, bits, M, K, N, conv, sms, s)
+                 : pl.ga_rows ? lutgemm::backward_ga_rows(gc, w, ga, lut_ga, bits, M, K, N, pl.ga_rows_plan, sc, at, pl.at_pitch, sms, s)
                  : pl.ga_tall ? lutgemm::backward_ga_slab_tall(gc, a, w, ga, lut_ga, nullptr, bits, M, K, N, conv, sc, sms, s)
                              : lutgemm::backward_ga_slab_packed(gc, a, w, ga, lut_ga, bits, M, K, N, conv, pl.ga_packed, sc, sms, s);
         if (rc != LUTGEMM_OK) return rc;
@@ -550,13 +572,13 @@ static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
 //   7 bits  64 channels (576 rows) 1.79 : 1.85   128 (1152) 1.99 : 1.75   256 (2304) 1.99 : 1.65   512 (4608) 2.02 : 1.64
 //   8 bits  64 channels            2.28 : 2.50   128        2.61 : 2.34   256        2.66 : 2.24   512        2.74 : 2.22
 //   256 -> 512 channels, stride 2 (classes of 2048, 1024, 1024 and 512 rows): 7 bits 1.07 : 0.96, 8 bits 1.77 : 1.35
-static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
-    const int force = g_force_backward.load(std::memory_order_relaxed);
-    if (force == LUTGEMM_BACKWARD_BCAST) return false;
-    if (force == LUTGEMM_BACKWARD_SLAB) return true;
+struct GxTimes {
+    double slab, bcast, rows;
+};
+static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
     const FamilyClocks f = family_clocks(bits);
     const long mt = bits == 8 ? 512 : 256;
-    double slab = 0;
+    double slab = 0, by_rows = 0;
     // broadcast kernel: tiles of all classes in one list, tile t on SM t mod sms (rows_of[i] rows from tile begin[i] on)
     constexpr int kMaxListed = 16;
     long begin[kMaxListed + 1] = {0}, rows_of[kMaxListed], most = 0;
@@ -565,6 +587,7 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(rows);
         slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, f.packed * (rt > 512 ? 1.12 : 1.0), false);
+        by_rows += rows_clocks(lutgemm::plan_rows(px.P, rows, px.C, sms), bits, px.P, px.C, true, Cout % 4 == 0, false);
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
             return;
@@ -580,7 +603,21 @@ static bool gx_uses_slab(int bits, const lutgemm::ConvGeom &g, int Cout, int sms
         for (int c = 0; c < n; ++c) rows += rows_of[c] * ((begin[c + 1] + sms - 1 - sm) / sms - (begin[c] + sms - 1 - sm) / sms);
         if (rows > most) most = rows;
     }
-    return slab < (double)most * mt * f.gx_bcast + kBcastStart;
+    return {slab, (double)most * mt * f.gx_bcast + kBcastStart, by_rows};
+}
+// (the kernel addresses an image by 32-bit offsets and keeps the two coordinates of a pixel in one word)
+static bool gx_rows_supported(const lutgemm::ConvGeom &g, int Cout) {
+    return g.H < 32768 && g.W < 65536 && (double)g.B * g.C * g.H * g.W < 4294967296.0 && lutgemm::rows_supported((long)g.B * g.H * g.W, (long)g.kh * g.kw * Cout, g.C);
+}
+enum GxFamily { kGxBcast, kGxSlab, kGxRows };
+static GxFamily gx_family(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows) {
+    rows = rows && gx_rows_supported(g, Cout);
+    const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
+    if (force == LUTGEMM_BACKWARD_BCAST) return kGxBcast;
+    if (force == LUTGEMM_BACKWARD_SLAB) return rows && tile == LUTGEMM_TILE_ROWS ? kGxRows : kGxSlab;
+    const GxTimes t = gx_times(bits, g, Cout, sms);
+    if (rows && t.rows < t.slab && t.rows < t.bcast) return kGxRows;
+    return t.slab < t.bcast ? kGxSlab : kGxBcast;
 }
 
 // Scratch that the choice by fixed limits (see base_plan) asked for: a buffer of at least that size is not refused, the
@@ -610,13 +647,49 @@ static size_t gx_slab_scratch_bytes(const lutgemm::ConvGeom &g, int Cout, int sm
     return need;
 }
 
+static size_t gx_rows_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+    size_t need = 0;
+    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
+        const lutgemm::RowsPlan plan = lutgemm::plan_rows(px.P, (long)px.ntaps * Cout, px.C, sms);
+        const size_t n = lutgemm::rows_scratch_bytes(plan, px.P, px.C, true, sms);
+        need = n > need ? n : need;
+    });
+    return need;
+}
+
+// 1x1 windows without padding: every pixel of class (0, 0) has the one tap
+static bool pointwise(const lutgemm::ConvGeom &g) { return g.kh == 1 && g.kw == 1 && g.pad == 0; }
+static bool pointwise_by_rows(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+    const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
+    if (!pointwise(g) || force == LUTGEMM_BACKWARD_BCAST || !gx_rows_supported(g, Cout)) return false;
+    if (force || tile) return tile == LUTGEMM_TILE_ROWS;
+    const int M = g.B * g.Ho * g.Wo;
+    const double rows = rows_clocks(lutgemm::plan_rows(M, Cout, g.C, sms), bits, M, g.C, true, Cout % 4 == 0, false);
+    double best = ga_bcast_clocks(bits, M, g.C, Cout, sms);
+    if (Cout >= 768) {
+        const lutgemm::PackedPlan pp = lutgemm::plan_packed(Cout, M, g.C, lutgemm::packed_ga_tile_rows(Cout), sms);
+        const double packed = packed_ga_clocks(pp, bits, M, g.C, Cout), tall = tall_clocks(bits, Cout, M, g.C, sms);
+        best = packed < best ? packed : best;
+        best = tall < best ? tall : best;
+    }
+    return rows < best;
+}
+
 static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout) {
     const int M = g.B * g.Ho * g.Wo, K = g.C * g.kh * g.kw;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    if (!conv_windows_overlap(g)) return plan_backward(bits, M, K, Cout, sms, true, false, true, false).ga_scratch;
-    if (!pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
-    return gx_uses_slab(bits, g, Cout, sms) ? gx_slab_scratch_bytes(g, Cout, sms) : 0;
+    if (conv_windows_overlap(g) && !pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
+    // (either entry point's choice, see lutgemm_conv2d_backward)
+    size_t need = 0, rows = 0;
+    if (!conv_windows_overlap(g)) {
+        need = plan_backward(bits, M, K, Cout, sms, true, false, true, false).scratch;
+        if (pointwise_by_rows(bits, g, Cout, sms)) rows = gx_rows_scratch_bytes(bits, g, Cout, sms);
+    } else {
+        if (gx_family(bits, g, Cout, sms, false) == kGxSlab) need = gx_slab_scratch_bytes(g, Cout, sms);
+        if (gx_family(bits, g, Cout, sms, true) == kGxRows) rows = gx_rows_scratch_bytes(bits, g, Cout, sms);
+    }
+    return need > rows ? need : rows;
 }
 
 size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
@@ -629,12 +702,12 @@ size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, i
     const int M = B * g.Ho * g.Wo, K = C * kh * kw;
     // the weight-gradient and the activation-gradient kernels run one after the other on the same buffer
     const bool have_codes = flags & LUTGEMM_SCRATCH_CODES_GIVEN;
-    size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false, have_codes).gw_scratch;
+    size_t gw_need = plan_backward(bits, M, K, Cout, sms, true, true, false, have_codes).scratch;
     size_t gx_need = conv_gx_scratch_bytes(bits, g, Cout);
     if (flags & LUTGEMM_SCRATCH_LEAST) {
-        const BackwardPlan base = base_plan(bits, M, K, Cout, sms, have_codes);
-        gw_need = least_need(gw_need, base.gw_scratch);
-        gx_need = least_need(gx_need, conv_windows_overlap(g) ? gx_base_scratch_bytes(bits, g, Cout) : base.ga_scratch);
+        gw_need = least_need(gw_need, base_plan(bits, M, K, Cout, sms, true, false, have_codes).scratch);
+        gx_need = least_need(gx_need, conv_windows_overlap(g) ? gx_base_scratch_bytes(bits, g, Cout)
+                                                              : base_plan(bits, M, K, Cout, sms, false, true, have_codes).scratch);
     }
     return gw_need > gx_need ? gw_need : gx_need;
 }
@@ -644,10 +717,11 @@ size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int 
     return lutgemm_conv2d_backward_ws_scratch_bytes(bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, 0);
 }
 
-int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
-                               const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
-                               int Cout, int kh, int kw, int stride, int pad, int dil, const uint8_t *codes_t,
-                               void *scratch, size_t scratch_bytes, void *stream) {
+// `by_rows`: the image gradient may be computed with one thread per pixel
+static int conv_backward_impl(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
+                              const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
+                              int Cout, int kh, int kw, int stride, int pad, int dil, const uint8_t *codes_t,
+                              void *scratch, size_t scratch_bytes, void *stream, bool by_rows) {
     lutgemm::ConvGeom g{};
     int rc = make_geom(B, C, H, W, kh, kw, stride, pad, dil, &g);
     if (rc != LUTGEMM_OK) return rc;
@@ -670,18 +744,24 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
     if (!every_pixel_written &&
         !lutgemm::cuda_ok(cudaMemsetAsync(gx, 0, (size_t)B * C * H * W * sizeof(float), s)))
         return LUTGEMM_E_CUDA;
-    if (!overlap)  // conv.enabled makes the grad_a kernels write (m,k) to the image position it came from
-        return backward_impl(gy, x, wmat, gx, nullptr, lut_ga, nullptr, bits, M, K, Cout, g, nullptr, scratch, scratch_bytes,
-                             stream);
-    if (!pixel_mode_supported(g)) return LUTGEMM_E_TOOLARGE;
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
-    bool slab = gx_uses_slab(bits, g, Cout, sms);
     const size_t given = scratch ? scratch_bytes : 0;
-    if (slab && gx_slab_scratch_bytes(g, Cout, sms) > given) {
-        if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
-            return LUTGEMM_E_SCRATCH;
-        slab = false;
+    GxFamily family = kGxBcast;
+    if (!overlap) {  // conv.enabled makes the grad_a kernels write (m,k) to the image position it came from
+        if (!by_rows || !pointwise_by_rows(bits, g, Cout, sms) || gx_rows_scratch_bytes(bits, g, Cout, sms) > given)
+            return backward_impl(gy, x, wmat, gx, nullptr, lut_ga, nullptr, bits, M, K, Cout, g, nullptr, scratch, scratch_bytes,
+                                 stream);
+        family = kGxRows;
+    } else {
+        if (!pixel_mode_supported(g)) return LUTGEMM_E_TOOLARGE;
+        family = gx_family(bits, g, Cout, sms, by_rows);
+        if (family == kGxRows && gx_rows_scratch_bytes(bits, g, Cout, sms) > given) family = gx_family(bits, g, Cout, sms, false);
+        if (family == kGxSlab && gx_slab_scratch_bytes(g, Cout, sms) > given) {
+            if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
+                return LUTGEMM_E_SCRATCH;
+            family = kGxBcast;
+        }
     }
     lutgemm::PixelClass px;
     lutgemm::PixelClass bcast[lutgemm::kMaxClassesPerLaunch];  // classes for the broadcast kernel, launched in groups
@@ -689,7 +769,12 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
     for (int ph = 0; ph < stride; ++ph)
         for (int pw = 0; pw < stride; ++pw) {
             if (!make_pixel_class(g, ph, pw, &px)) continue;
-            if (slab) {
+            if (family == kGxRows) {
+                rc = lutgemm::backward_gx_rows(gy, x, wmat, gx, lut_ga, bits, Cout, px, static_cast<float *>(scratch), sms, s);
+                if (rc != LUTGEMM_OK) return rc;
+                continue;
+            }
+            if (family == kGxSlab) {
                 rc = lutgemm::backward_gx_class(gy, x, wmat, gx, lut_ga, bits, Cout, px, B, static_cast<float *>(scratch), sms, s);
                 if (rc != LUTGEMM_OK) return rc;
                 continue;
@@ -705,12 +790,21 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
     return LUTGEMM_OK;
 }
 
+int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
+                               const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
+                               int Cout, int kh, int kw, int stride, int pad, int dil, const uint8_t *codes_t,
+                               void *scratch, size_t scratch_bytes, void *stream) {
+    return conv_backward_impl(gy, x, wmat, gx, gw, lut_ga, lut_gw, bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, codes_t,
+                              scratch, scratch_bytes, stream, true);
+}
+
+// (its image gradients keep the kernels, and with them the order of summation, that they have always had)
 int lutgemm_conv2d_backward(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
                             const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
                             int Cout, int kh, int kw, int stride, int pad, int dil, void *scratch,
                             size_t scratch_bytes, void *stream) {
-    return lutgemm_conv2d_backward_ws(gy, x, wmat, gx, gw, lut_ga, lut_gw, bits, B, C, H, W, Cout, kh, kw, stride, pad,
-                                      dil, nullptr, scratch, scratch_bytes, stream);
+    return conv_backward_impl(gy, x, wmat, gx, gw, lut_ga, lut_gw, bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, nullptr,
+                              scratch, scratch_bytes, stream, false);
 }
 
 // ---- forward with the layer's de-quantisation applied where the kernel stores ------------------------------------

@@ -136,6 +136,61 @@ int backward_gw_slab_tall(const float *gc, const uint8_t *a, const uint8_t *w, f
 int backward_ga_slab_tall(const float *gc, const uint8_t *a, const uint8_t *w, float *ga, const int16_t *lut_ga,
                           const float *lut_f32, int bits, int M, int K, int N, const ConvGeom &conv, float *scratch,
                           int num_sms, cudaStream_t stream);
+// ---- gradient kernel with one thread per output row (lutgemm_slab_rows.cu): tiles of 512 rows x 64 terms ------------------
+constexpr int kRowsTile = 512, kRowsTerms = 64;
+constexpr int kRowsChain = 16, kRowsRun = 8;     // term blocks added in one chain; above it, length of the runs
+constexpr int kRowsMaxPer = 128;                // k per work item where sums of runs are kept (bounds their buffer)
+constexpr int kRowsBlockOverhead = 7;         // in k steps: grad_out block, first slabs
+// How its work is dealt out.  The term blocks of a row tile are cut into groups of group_blocks; the cells (tile, group), each
+// with its K in units of four k, are laid end to end and every CTA takes an equal share of the units: pieces of at most
+// piece_k k of one cell, all term blocks of the group one after the other.
+struct RowsPlan {
+    int groups, group_blocks, piece_k;
+    double steps, loads;  // k steps of one CTA, and how often it loads a block's grad_out values and fills its slabs
+};
+constexpr int kRowsUnit = 4;
+inline long rows_units(const RowsPlan &p, long rows, int K) {
+    return (rows + kRowsTile - 1) / kRowsTile * p.groups * ((K + kRowsUnit - 1) / kRowsUnit);
+}
+// units and blocks are counted in 32 bits
+inline bool rows_supported(long rows, long terms, int K) {
+    return (double)rows / kRowsTile * 128 * (K / kRowsUnit + 1) < 1e9 && terms < (1L << 31) - kRowsTerms && rows < (1L << 31) - kRowsTile;
+}
+// The number of groups that finishes first: more groups fill the GPU where tiles and K alone do not, and spread a block's
+// grad_out loads over more k, at the price of another block of sums each.
+inline RowsPlan plan_rows(long rows, long terms, int K, int num_sms) {
+    const long tiles = (rows + kRowsTile - 1) / kRowsTile;
+    const int blocks = (int)((terms + kRowsTerms - 1) / kRowsTerms), kp = (K + kRowsUnit - 1) / kRowsUnit * kRowsUnit;
+    constexpr double kMostSums = 96e6;  // bytes of sums of several groups
+    RowsPlan best{};
+    double best_cost = 0;
+    for (int g = 1; g <= blocks && g <= 128; g += g < 4 ? 1 : g < 16 ? 2 : g < 32 ? 4 : 16) {
+        RowsPlan p{};
+        p.group_blocks = (blocks + g - 1) / g;
+        p.groups = (blocks + p.group_blocks - 1) / p.group_blocks;
+        const double sums = p.groups > 1 ? 8.0 * p.groups * K * (double)rows / 4000 / 1200 + 5 : 0;
+        if (best.groups && (sums >= best_cost || (double)p.groups * K * rows * sizeof(float) > kMostSums)) break;
+        const long share = (rows_units(p, rows, K) + num_sms - 1) / num_sms * kRowsUnit;
+        const int most = p.group_blocks > kRowsChain && kp > kRowsMaxPer ? kRowsMaxPer : kp;
+        const long pieces = (share + most - 1) / most;
+        p.piece_k = most == kp ? kp : (int)((share + pieces - 1) / pieces + kRowsUnit - 1) / kRowsUnit * kRowsUnit;
+        // (a share begins and ends inside a cell: one piece more than its length asks for, where there is more than one cell)
+        p.steps = (double)p.group_blocks * share;
+        p.loads = p.group_blocks * ((double)pieces + (tiles * p.groups > 1));
+        const double cost = p.steps + kRowsBlockOverhead * p.loads + sums;
+        if (!best.groups || cost < best_cost) { best = p; best_cost = cost; }
+    }
+    return best;
+}
+// floats of its scratch buffer: blocks of sums where they do not go to their final place, and sums of runs
+size_t rows_scratch_bytes(const RowsPlan &plan, long rows, int K, bool direct, int num_sms);
+// `at`: the activation codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
+int backward_gw_rows(const float *gc, const uint8_t *w, float *gw, const int16_t *lut_gw, int bits, int M, int K, int N,
+                     const RowsPlan &plan, float *scratch, const uint8_t *at, int at_pitch, int num_sms, cudaStream_t stream);
+int backward_ga_rows(const float *gc, const uint8_t *w, float *ga, const int16_t *lut_ga, int bits, int M, int K, int N,
+                     const RowsPlan &plan, float *scratch, const uint8_t *at, int at_pitch, int num_sms, cudaStream_t stream);
+int backward_gx_rows(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
+                     int Cout, const PixelClass &px, float *scratch, int num_sms, cudaStream_t stream);
 // reads (and clears) the device-side error word of the bounded barrier waits; synchronises the device
 int read_and_clear_device_error(int *value);
 // launches a one-warp kernel whose barrier wait can never be satisfied (it must time out with error id 99)

@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "lutgemm_common.cuh"
+#include "lutgemm_f32x2.cuh"
 #include "lutgemm_kernels.h"
 #include "lutgemm_waits.cuh"
 
@@ -44,35 +45,6 @@ namespace lutgemm {
 namespace sp {
 
 enum { kGw = 1, kGa = 2, kGx = 3 };
-
-// two fp32 values in one 64-bit register (the operand form of the packed fp32 instructions)
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 t;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(t.x), "=f"(t.y) : "l"(v));
-    return t;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// the two signed table entries of a slab word: 0x4B000000 | u is the float 2^23 + u, u = entry + 2^15
-__device__ __forceinline__ f32x2 entries2(uint32_t word, f32x2 bias) {
-    const float lo = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7610));
-    const float hi = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7632));
-    return add2(pack2(lo, hi), bias);
-}
 
 template <int BITS, int RW_>
 struct Cfg {
@@ -754,6 +726,28 @@ int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, fl
     return LUTGEMM_E_BITS;
 }
 
+// The blocks are added in 64 bits (these kernels wait for memory, the additions cost nothing) and rounded once: the rounding
+// errors of many blocks in one fp32 chain showed (64 blocks of 64 terms: 1.8e-7 relative to the sums, now 1.0e-7).
+struct Sum4 {
+    double x, y, z, w;
+    __device__ __forceinline__ float4 rounded() const { return make_float4((float)x, (float)y, (float)z, (float)w); }
+};
+__device__ __forceinline__ double sum_blocks(const float *p, size_t stride, int b0, int b1) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) s += p[b * stride];
+    return s;
+}
+__device__ __forceinline__ Sum4 sum_blocks4(const float4 *p, size_t stride, int b0, int b1) {
+    Sum4 s{0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) {
+        const float4 v = p[b * stride];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    return s;
+}
+
 // out[k][c] (TRANSPOSE=false) or out[c][k] (TRANSPOSE=true) = scale * sum_b part[b][k][c], b ascending.
 // PLACE = 1: column c is an unfolded row m of a convolution with non-overlapping windows and (m,k) goes to its
 // position in the image gradient (conv_scatter_index); PLACE = 2: column c is pixel c of a stride class and k a
@@ -776,7 +770,7 @@ __global__ void slab_reduce_blocks_kernel(const float *__restrict__ part, float 
             const int k = k0 + ty + 8 * j, c = c0 + tx;
             float s = 0.f;
             if (k < K && c < C)
-                for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * KC_ + (size_t)k * C + c];
+                s = (float)sum_blocks(part + (size_t)k * C + c, KC_, 0, nblocks);
             if (TRANSPOSE) tile[ty + 8 * j][tx] = s * scale;
             else if (k < K && c < C) {
                 if (PLACE == 1) {
@@ -818,10 +812,7 @@ __global__ void __launch_bounds__(256) slab_reduce_blocks_vec_kernel(const float
             const int k = k0 + ty + 8 * j, c = c0 + 4 * tx;
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
             if (k < K && c < C) {
-                for (int b = 0; b < nblocks; ++b) {
-                    const float4 v = *reinterpret_cast<const float4 *>(part + (size_t)b * KC_ + (size_t)k * C + c);
-                    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-                }
+                s = sum_blocks4(reinterpret_cast<const float4 *>(part + (size_t)k * C + c), KC_ / 4, 0, nblocks).rounded();
                 s.x *= scale; s.y *= scale; s.z *= scale; s.w *= scale;
                 if (!TRANSPOSE) *reinterpret_cast<float4 *>(out + (size_t)k * C + c) = s;
             }
@@ -841,35 +832,35 @@ __global__ void __launch_bounds__(256) slab_reduce_blocks_vec_kernel(const float
     }
 }
 
-// Many blocks of few sums (a convolution's grad_w: M / 512 blocks of K x Cout): the blocks of 32 vectors are shared out
-// over the 16 warps of a CTA in contiguous ranges, and the warps' sums added in ascending order.  One thread per sum
-// and all blocks in a row left most of the GPU idle: 392 blocks of 64 x 256 sums took as long as a tenth of the kernel
-// that made them.
+// Several blocks whose sums stay where they are: 32 vectors (or single sums, where blocks are not 16-byte aligned) per step
+// of a CTA, the blocks shared out over its 16 warps in contiguous ranges.  One thread per sum and all blocks in a row left
+// most of the GPU idle: 392 blocks of 64 x 256 sums took as long as a tenth of the kernel that made them, 16 blocks of
+// 777 x 333 18 us.
+template <bool VEC>
 __global__ void __launch_bounds__(512) slab_reduce_many_kernel(const float *__restrict__ part, float *__restrict__ out,
-                                                               long vecs, int nblocks, float scale) {
-    __shared__ float4 sums[16][32];
+                                                               long count, int nblocks, float scale) {
+    __shared__ Sum4 sums[16][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int b0 = (int)((long)nblocks * ty / 16), b1 = (int)((long)nblocks * (ty + 1) / 16);
-    const float4 *src = reinterpret_cast<const float4 *>(part);
-    for (long v0 = (long)blockIdx.x * 32; v0 < vecs; v0 += (long)gridDim.x * 32) {
+    for (long v0 = (long)blockIdx.x * 32; v0 < count; v0 += (long)gridDim.x * 32) {
         const long v = v0 + tx;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v < vecs) {
-#pragma unroll 4
-            for (int b = b0; b < b1; ++b) {
-                const float4 t = src[(size_t)b * vecs + v];
-                s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
-            }
+        Sum4 s{0.0, 0.0, 0.0, 0.0};
+        if (v < count) {
+            if (VEC) s = sum_blocks4(reinterpret_cast<const float4 *>(part) + v, count, b0, b1);
+            else s.x = sum_blocks(part + v, count, b0, b1);
         }
-        sums[ty][tx] = s;
+        if (VEC) sums[ty][tx] = s;
+        else sums[ty][tx].x = s.x;
         __syncthreads();
-        if (ty == 0 && v < vecs) {
+        if (ty == 0 && v < count) {
 #pragma unroll
             for (int i = 1; i < 16; ++i) {
-                const float4 t = sums[i][tx];
-                s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+                s.x += sums[i][tx].x;
+                if (VEC) { s.y += sums[i][tx].y; s.z += sums[i][tx].z; s.w += sums[i][tx].w; }
             }
-            reinterpret_cast<float4 *>(out)[v] = make_float4(s.x * scale, s.y * scale, s.z * scale, s.w * scale);
+            const float4 r = s.rounded();
+            if (VEC) reinterpret_cast<float4 *>(out)[v] = make_float4(r.x * scale, r.y * scale, r.z * scale, r.w * scale);
+            else out[v] = r.x * scale;
         }
         __syncthreads();
     }
@@ -877,10 +868,12 @@ __global__ void __launch_bounds__(512) slab_reduce_many_kernel(const float *__re
 
 int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks, bool transpose, const ConvGeom *scatter,
                        const PixelClass *px, float scale, int num_sms, cudaStream_t stream) {
-    if (!scatter && !px && !transpose && nblocks >= 16 && (long)K * C % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0 &&
-        (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-        const long vecs = (long)K * C / 4, ctas = (vecs + 31) / 32;
-        slab_reduce_many_kernel<<<(int)(ctas < 4L * num_sms ? ctas : 4L * num_sms), 512, 0, stream>>>(part, out, vecs, nblocks, scale);
+    if (!scatter && !px && !transpose && nblocks >= 4) {
+        const bool vec = (long)K * C % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+        const long count = (long)K * C / (vec ? 4 : 1), ctas = (count + 31) / 32;
+        const int grid = (int)(ctas < 4L * num_sms ? ctas : 4L * num_sms);
+        if (vec) slab_reduce_many_kernel<true><<<grid, 512, 0, stream>>>(part, out, count, nblocks, scale);
+        else slab_reduce_many_kernel<false><<<grid, 512, 0, stream>>>(part, out, count, nblocks, scale);
         return launch_status();
     }
     if (!scatter && !px && C % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0 &&
