@@ -129,7 +129,7 @@ def library():
     return _load()
 
 
-_FORWARD_CHOICES = {"auto": 0, "rowbcast": 1, "slab": 2}
+_FORWARD_CHOICES = {"auto": 0, "rowbcast": 1, "slab": 2, "rows": 3}
 _BACKWARD_CHOICES = {"auto": 0, "bcast": 1, "slab": 2}
 _TILE_CHOICES = {"auto": 0, "wide": 1, "tall": 2, "rows": 3}
 _CODES_GIVEN, _LEAST = 1, 2  # LUTGEMM_SCRATCH_CODES_GIVEN, LUTGEMM_SCRATCH_LEAST
@@ -138,7 +138,7 @@ _E_SCRATCH = -4
 
 def set_kernel_choice(forward: str = "auto", backward: str = "auto", grad_tile: str = "auto") -> None:
     """Process-wide kernel-family override (tests, A/B timing); all "auto" restores the choice by shape.
-    forward: "rowbcast" | "slab"; backward: "bcast" | "slab"; grad_tile: "wide" (512 x 64) | "tall" (1024 x 32) |
+    forward: "rowbcast" | "slab" | "rows" (two rows per thread); backward: "bcast" | "slab"; grad_tile: "wide" (512 x 64) | "tall" (1024 x 32) |
     "rows" (one thread per output row)."""
     _check(_load().lutgemm_set_kernel_choice(_FORWARD_CHOICES[forward], _BACKWARD_CHOICES[backward],
                                              _TILE_CHOICES[grad_tile]), "set_kernel_choice")

@@ -70,7 +70,9 @@ struct BackwardPlan {
 //   slab kernels, per k and tile      packed 512 x 64: grad_w 1480 (4 and 6 bits), 1500 (7), 2120 (8), grad_a and grad_x 1540,
 //                                     1580, 2180; tall 1024 x 32: 1540, 1690, 1880;
 //                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
-//                                     more launches: code transposition, zeroing, and a layer's epilogue)
+//                                     more launches: code transposition, zeroing, and a layer's epilogue);
+//   a thread per row                  gradients 512 x 64: 1420 (4 bits), 1070 (6), 1150 (7), 1390 (8) per k, 9e3 per block of
+//                                     grad_out values (27e3 where they come one by one); forward 1024 x 32: 650, 690, 845
 //   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
 //                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.66, 1.72, 2.2
 // A slab kernel's time does not depend on the codes and it can cut K into many work items; a broadcast kernel has no slab
@@ -78,12 +80,12 @@ struct BackwardPlan {
 // (base_plan below) the estimates move small and ragged problems to the slab kernels: 256 x 512 x 256 at 7 bits, forward 0.291 ms,
 // grad_w 0.088 ms and grad_a 0.092 ms with the broadcast kernels, both gradients 0.034 ms with the slab kernels.
 struct FamilyClocks {
-    double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start, rows;
+    double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start, rows, fwd_rows;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390};
-    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150};
-    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, bits == 6 ? 1070.0 : 1420.0};
+    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390, 845};
+    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150, 690};
+    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, bits == 6 ? 1070.0 : 1420.0, 650};
 }
 constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
@@ -259,7 +261,7 @@ int lutgemm_set_handover(int on) {
 unsigned long long lutgemm_kernel_launches(void) { return g_kernel_launches.load(std::memory_order_relaxed); }
 
 int lutgemm_set_kernel_choice(int forward, int backward, int grad_tile) {
-    if (forward < 0 || forward > 2 || backward < 0 || backward > 2 || grad_tile < 0 || grad_tile > 3)
+    if (forward < 0 || forward > 3 || backward < 0 || backward > 2 || grad_tile < 0 || grad_tile > 3)
         return LUTGEMM_E_BADARG;
     g_force_forward.store(forward, std::memory_order_relaxed);
     g_force_backward.store(backward, std::memory_order_relaxed);
@@ -284,16 +286,34 @@ int lutgemm_bits_from_elem_num(long elem_num) {
 // callers whose workspace is too small for it.  lutgemm_set_kernel_choice overrides the choice (tests, A/B timing).
 static bool base_forward_uses_slab(int M, int N) { return M >= 512 && N >= 32 && slab_fill(M, N) >= 0.6; }
 
+static double fwd_slab_clocks(int bits, int M, int K, int N, int sms) {
+    const FamilyClocks f = family_clocks(bits);
+    return (double)div_up(div_up(M, 512) * div_up(N, 64) * div_up(K, 16), sms) * 16 * f.fwd_slab + f.fwd_start;
+}
+static double fwd_bcast_clocks(int bits, int M, int K, int N, int sms) {
+    const long mt = N <= 128 ? 128 : 64, nt = N <= 128 ? 64 : 256;
+    return (double)div_up(div_up(M, mt) * div_up(N, nt), sms) * mt * nt * K * family_clocks(bits).fwd_bcast / 32 + kBcastStart;
+}
 static bool forward_uses_slab(int bits, int M, int K, int N, int sms) {
     const int force = g_force_forward.load(std::memory_order_relaxed);
     if (force == LUTGEMM_FORWARD_ROWBCAST) return false;
-    if (force == LUTGEMM_FORWARD_SLAB) return true;
+    if (force) return true;
+    return base_forward_uses_slab(M, N) || fwd_slab_clocks(bits, M, K, N, sms) < fwd_bcast_clocks(bits, M, K, N, sms);
+}
+
+// Two rows per thread instead of either, where the caller brings a workspace for the transposed codes: from about a thousand
+// rows on (7 bits, slab kernel against two rows per thread, ms: 512^3 0.042 : 0.044, 1000 x 777 x 333 0.067 : 0.052, 1024^3 0.140 :
+// 0.108, 200704 x 64 x 256 0.394 : 0.355).
+constexpr double kFwdTileClocks = 13e3;  // codes of the first k, sums on their way out
+static bool forward_by_rows(int bits, int M, int K, int N, int sms) {
+    const int force = g_force_forward.load(std::memory_order_relaxed);
+    if (force) return force == LUTGEMM_FORWARD_ROWS;
     const FamilyClocks f = family_clocks(bits);
-    const long tiles = div_up(M, 512) * div_up(N, 64), chunks = div_up(K, 16);
-    const double slab = (double)div_up(tiles * chunks, sms) * 16 * f.fwd_slab + f.fwd_start;
-    const long mt = N <= 128 ? 128 : 64, nt = N <= 128 ? 64 : 256;
-    const double bcast = (double)div_up(div_up(M, mt) * div_up(N, nt), sms) * mt * nt * K * f.fwd_bcast / 32 + kBcastStart;
-    return base_forward_uses_slab(M, N) || slab < bcast;
+    const long tiles = div_up(M, lutgemm::kFwdRowsTile) * div_up(N, lutgemm::kFwdRowsCols);
+    const bool cut = lutgemm::forward_rows_cut(M, K, N, sms);
+    const double k = cut ? 4.0 * div_up(tiles * div_up(K, 4), sms) : (double)div_up(tiles, sms) * K;
+    const double t = k * f.fwd_rows + (div_up(tiles, sms) + cut) * kFwdTileClocks + f.fwd_start;
+    return t < fwd_slab_clocks(bits, M, K, N, sms) && (base_forward_uses_slab(M, N) || t < fwd_bcast_clocks(bits, M, K, N, sms));
 }
 
 // A workspace too small for the slab kernel is refused where the slab kernel was always the choice (or is forced); elsewhere
@@ -304,11 +324,12 @@ static bool small_workspace_refused(int M, int N) {
 
 static int codes_pitch(int M) { return (M + 15) & ~15; }
 
-// `scratch` (optional, K * codes_pitch(M) bytes, 16-byte aligned): the slab kernel then reads the activation
-// codes from a transposed copy made there first, which stays valid on return.
+// `scratch` (optional, K * codes_pitch(M) bytes, 16-byte aligned): the slab kernels then read the activation
+// codes from a transposed copy made there first, which stays valid on return.  `may_rows`: the kernel with two rows per thread
+// may be chosen.
 static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K,
                         int N, const lutgemm::ConvGeom &conv, void *scratch, size_t scratch_bytes, void *stream,
-                        const lutgemm::LayerEpilogue *epi = nullptr) {
+                        const lutgemm::LayerEpilogue *epi = nullptr, bool may_rows = true) {
     if (!lutgemm::bits_supported(bits)) return LUTGEMM_E_BITS;
     if (!a || !w || (!c && !epi) || !lut || M <= 0 || K <= 0 || N <= 0) return LUTGEMM_E_BADARG;
     if ((reinterpret_cast<uintptr_t>(c) & 3) || (reinterpret_cast<uintptr_t>(lut) & 1) ||
@@ -318,6 +339,11 @@ static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const u
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int pitch = codes_pitch(M);
+    if (may_rows && scratch && scratch_bytes >= (size_t)pitch * K && forward_by_rows(bits, M, K, N, sms)) {
+        const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, s);
+        if (trc != LUTGEMM_OK) return trc;
+        return lutgemm::forward_rows(w, c, lut, bits, M, K, N, static_cast<const uint8_t *>(scratch), pitch, epi, sms, s);
+    }
     bool slab = forward_uses_slab(bits, M, K, N, sms);
     if (slab && scratch && scratch_bytes < (size_t)pitch * K) {
         if (small_workspace_refused(M, N)) return LUTGEMM_E_SCRATCH;
@@ -344,7 +370,7 @@ int lutgemm_forward(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint1
 size_t lutgemm_forward_scratch_bytes(int bits, int M, int K, int N) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
-    if (sms <= 0 || !forward_uses_slab(bits, M, K, N, sms)) return 0;
+    if (sms <= 0 || !(forward_uses_slab(bits, M, K, N, sms) || forward_by_rows(bits, M, K, N, sms))) return 0;
     return (size_t)codes_pitch(M) * K;
 }
 
@@ -827,12 +853,22 @@ static bool layer_forward_needs_sums(int bits, int M, int K, int N, int sms) {
     return forward_uses_slab(bits, M, K, N, sms) && lutgemm::slab_fwd_ksplits(M, K, N, sms) > 1;
 }
 
+// what the layer forward pass needs at least where it refuses a smaller buffer
+static size_t layer_forward_base_bytes(int bits, int M, int K, int N, int sms) {
+    const size_t codes = forward_uses_slab(bits, M, K, N, sms) ? align16((size_t)codes_pitch(M) * K) : 0;
+    return codes + (layer_forward_needs_sums(bits, M, K, N, sms) ? (size_t)M * N * sizeof(uint32_t) : 0);
+}
+static size_t layer_forward_rows_bytes(int M, int K, int N, int sms) {
+    return align16((size_t)codes_pitch(M) * K) + (lutgemm::forward_rows_cut(M, K, N, sms) ? (size_t)M * N * sizeof(uint32_t) : 0);
+}
+
 static size_t layer_forward_scratch_bytes(int bits, int M, int K, int N) {
     if (!lutgemm::bits_supported(bits) || M <= 0 || K <= 0 || N <= 0) return 0;
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
-    const size_t codes = align16(lutgemm_forward_scratch_bytes(bits, M, K, N));
-    return codes + (layer_forward_needs_sums(bits, M, K, N, sms) ? (size_t)M * N * sizeof(uint32_t) : 0);
+    const size_t base = layer_forward_base_bytes(bits, M, K, N, sms);
+    const size_t rows = forward_by_rows(bits, M, K, N, sms) ? layer_forward_rows_bytes(M, K, N, sms) : 0;
+    return base > rows ? base : rows;
 }
 
 static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t *lut, int bits, int M, int K, int N,
@@ -843,15 +879,16 @@ static int layer_forward_impl(const uint8_t *a, const uint8_t *w, const uint16_t
         return LUTGEMM_E_BADARG;
     const int sms = current_num_sms();
     if (sms <= 0) return LUTGEMM_E_CUDA;
-    const size_t codes = lutgemm_forward_scratch_bytes(bits, M, K, N);
-    if (!layer_forward_needs_sums(bits, M, K, N, sms))
-        return forward_impl(a, w, nullptr, lut, bits, M, K, N, conv, scratch, scratch_bytes, stream, &e);
-    if (!scratch || scratch_bytes < layer_forward_scratch_bytes(bits, M, K, N)) {
+    const size_t given = scratch ? scratch_bytes : 0, codes = (size_t)codes_pitch(M) * K;
+    const bool by_rows = forward_by_rows(bits, M, K, N, sms) && given >= layer_forward_rows_bytes(M, K, N, sms);
+    if (by_rows ? !lutgemm::forward_rows_cut(M, K, N, sms) : !layer_forward_needs_sums(bits, M, K, N, sms))
+        return forward_impl(a, w, nullptr, lut, bits, M, K, N, conv, scratch, scratch_bytes, stream, &e, by_rows);
+    if (given < (by_rows ? layer_forward_rows_bytes(M, K, N, sms) : layer_forward_base_bytes(bits, M, K, N, sms))) {
         if (small_workspace_refused(M, N)) return LUTGEMM_E_SCRATCH;
         return lutgemm::forward_rowbcast(a, w, nullptr, lut, bits, M, K, N, conv, &e, sms, static_cast<cudaStream_t>(stream));
     }
     uint32_t *sums = reinterpret_cast<uint32_t *>(static_cast<char *>(scratch) + align16(codes));
-    const int rc = forward_impl(a, w, sums, lut, bits, M, K, N, conv, scratch, codes, stream);
+    const int rc = forward_impl(a, w, sums, lut, bits, M, K, N, conv, scratch, codes, stream, nullptr, by_rows);
     if (rc != LUTGEMM_OK) return rc;
     return lutgemm::conv_epilogue(sums, e.box, e.sumw_t, e.taps, e.s_a, e.s_w, e.z_a, e.z_w, e.bias, e.out, M, e.L, N, sms,
                                   static_cast<cudaStream_t>(stream));
@@ -1019,7 +1056,7 @@ int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, l
     if (sms <= 0) return LUTGEMM_E_CUDA;
     // (a buffer for codes and sums is enough for every choice; what the choice needs is only worked out for a smaller one)
     if (scratch_bytes < (size_t)codes_pitch(M) * K + (size_t)M * Cout * sizeof(uint32_t) && small_workspace_refused(M, Cout) &&
-        scratch_bytes < layer_forward_scratch_bytes(bits, M, K, Cout) && (scratch || layer_forward_needs_sums(bits, M, K, Cout, sms)))
+        scratch_bytes < layer_forward_base_bytes(bits, M, K, Cout, sms) && (scratch || layer_forward_needs_sums(bits, M, K, Cout, sms)))
         return LUTGEMM_E_SCRATCH;
     const size_t L = (size_t)g.Ho * g.Wo, pixels = (size_t)B * H * W;
     float *chansum = work, *wsum = chansum + pixels, *sumw_t = wsum + (size_t)Cout * kh * kw, *taps = sumw_t + L * Cout,

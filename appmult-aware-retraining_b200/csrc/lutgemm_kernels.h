@@ -34,6 +34,19 @@ int forward_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t
                  const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, int num_sms,
                  cudaStream_t stream);
 
+// forward kernel with two output rows per thread (lutgemm_forward_rows.cu), tiles of 1024 rows x 32 columns; `at` as above,
+// not optional
+constexpr int kFwdRowsTile = 1024, kFwdRowsCols = 32;
+int forward_rows(const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K, int N, const uint8_t *at,
+                 int at_pitch, const LayerEpilogue *epi, int num_sms, cudaStream_t stream);
+// whether it cuts K where it is free to: whole tiles would leave the last wave of the persistent grid badly filled
+inline bool forward_rows_cut(int M, int K, int N, int num_sms) {
+    const long tiles = (long)((M + kFwdRowsTile - 1) / kFwdRowsTile) * ((N + kFwdRowsCols - 1) / kFwdRowsCols);
+    const long waves = (tiles + num_sms - 1) / num_sms;
+    // (a cut costs about as much as 24 k: two parts per CTA to zero and to combine)
+    return (double)waves * K > (double)tiles * K / num_sms + 24;
+}
+
 // operand chunks of forward_slab by bulk-tensor copies (default) or by vector loads through registers
 void slab_fwd_set_tma(bool on);
 // number of K ranges forward_slab cuts a problem into when it is free to (1 = none; a fused epilogue needs 1)

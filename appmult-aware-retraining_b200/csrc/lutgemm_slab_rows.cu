@@ -45,6 +45,7 @@
 #include "lutgemm_common.cuh"
 #include "lutgemm_f32x2.cuh"
 #include "lutgemm_kernels.h"
+#include "lutgemm_rows.cuh"
 #include "lutgemm_waits.cuh"
 
 namespace lutgemm {
@@ -60,9 +61,8 @@ struct Cfg {
     // k per unit - what the warps hand over to each other - as many as fit three times: 4096^3 at 7 bits 9.2 ms with four, 10.1
     // with two, at 8 bits there is room for one
     static constexpr int KU = BITS == 8 ? 1 : 4, NB = 3;
-    static constexpr int TT_ROW = BITS == 4 ? 36 : 2 * Q;  // bytes per table row (4 bits: padded, rows on different banks)
-    static constexpr int TT_BYTES = (Q * TT_ROW + 127) & ~127;
-    static constexpr int U_ROW = 2 * CT, U_BYTES = Q * U_ROW, UB = KU * U_BYTES;
+    using T = RowsTable<BITS>;
+    static constexpr int TT_ROW = T::ROW, TT_BYTES = T::BYTES, U_ROW = T::U_ROW, U_BYTES = T::U_BYTES, UB = KU * U_BYTES;
     static constexpr int CC_STAGE = KC * CT;
     static constexpr int OFF_U = TT_BYTES;
     // a block's grad_out values pass through the slab buffers, G_ROWS rows at a time, with grad_x's pixels behind them
@@ -72,11 +72,9 @@ struct Cfg {
     static constexpr int OFF_BAR = OFF_CC + 2 * CC_STAGE;
     static constexpr int OFF_TAP = OFF_BAR + NB * 8 + 16;  // behind an mbarrier per buffer, abort word and table range
     static constexpr int SMEM = OFF_TAP + kMaxTaps * 2;  // grad_x: output offset {rows, columns} of each tap
-    static_assert(U_ROW == 128 && OFF_U % 128 == 0, "chunks of a slab row lie on fixed bank quads");
+    static_assert(U_ROW == 2 * CT && OFF_U % 128 == 0, "chunks of a slab row lie on fixed bank quads");
     static_assert(SMEM <= 232448, "shared memory budget");
-    // the wire-format table passes through the slab buffers, ST_ROWS of its rows at a time
-    static constexpr int ST_ROWS = BITS == 8 ? 128 : Q;
-    static_assert(ST_ROWS * lut_col_num(BITS) * 2 <= NB * UB, "table staging");
+    static_assert(T::TURN_BYTES <= NB * UB, "the table passes through the slab buffers");
 };
 
 struct Args {
@@ -125,28 +123,13 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, l7 = lane & 7;
 
     // ---- stage the gradient table in offset-binary: tt[y][x], x = row code, y = term code, T = lut[a * COL + w] -----------
-    // (grad_w: rows are weight codes; grad_a / grad_x: rows are activation codes, so the table is turned: its rows pass
-    // through the slab buffers as they are - their stride is an odd number of words - and both sides stay conflict-free)
+    // (grad_w: rows are weight codes; grad_a / grad_x: rows are activation codes, so the table is turned)
     if (MODE == kGw) {
         for (int idx = tid; idx < Q * Q; idx += THREADS)
             *reinterpret_cast<uint16_t *>(smem + (idx >> BITS) * C::TT_ROW + (idx & (Q - 1)) * 2) =
                 (uint16_t)p.lut[(idx >> BITS) * COL + (idx & (Q - 1))] ^ (uint16_t)0x8000u;
     } else {
-        uint16_t *raw = reinterpret_cast<uint16_t *>(smem + C::OFF_U);
-#pragma unroll 1
-        for (int x0 = 0; x0 < Q; x0 += C::ST_ROWS) {
-            const int16_t *src = p.lut + x0 * COL;
-            if (x0) __syncthreads();
-#pragma unroll 8
-            for (int idx = tid; idx < C::ST_ROWS * COL; idx += THREADS) raw[idx] = (uint16_t)src[idx];
-            __syncthreads();
-#pragma unroll 4
-            for (int idx = tid; idx < C::ST_ROWS / 2 * Q; idx += THREADS) {
-                const int xp = idx % (C::ST_ROWS / 2), y = idx / (C::ST_ROWS / 2);
-                const uint32_t e0 = raw[2 * xp * COL + y], e1 = raw[(2 * xp + 1) * COL + y];
-                *reinterpret_cast<uint32_t *>(smem + y * C::TT_ROW + (x0 + 2 * xp) * 2) = (e0 | e1 << 16) ^ 0x80008000u;
-            }
-        }
+        stage_table_turned<BITS>(smem, smem + C::OFF_U, reinterpret_cast<const uint16_t *>(p.lut), 0x80008000u, tid);
     }
     if (tid == 0) {
         *abort_word = 0;
@@ -219,51 +202,10 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
                 make_uint4(pcc.x & MASK4, pcc.y & MASK4, pcc.z & MASK4, pcc.w & MASK4);
     };
 
-    // ---- the thread's share of a unit's slabs: four terms (quad bq) x eight codes (16 bytes of a table row; four at 6 bits, one
-    //      at 4) of slab bs ------------------------------------------------------------------------------------------------
-    const int bq = tid & 15, hx = tid >> 4;
-    const int bs = BITS < 8 ? hx >> 4 : 0;
-    const int bx = BITS == 8 ? (hx ^ (bq & 7)) * 8 : BITS == 7 ? ((hx & 15) ^ (bq & 7)) * 8
-                 : BITS == 6 ? ((hx & 15) ^ bq) * 4 : hx & 15;  // first code
-    const uint32_t tt_lane = tt_addr + bx * 2;
-    const uint32_t us = u_addr + bs * C::U_BYTES + bx * C::U_ROW + bq * 8;
-    const int cc_lane = bs * CT + bq * 4;
-    auto build_step = [&](uint32_t off, const uint8_t *codes) {  // one slab at 8 bits, two at fewer
-        const uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + cc_lane);
-        uint32_t ad[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ad[c] = tt_lane + byte_of(cw, c) * C::TT_ROW;
-        const uint32_t ub = us + off;
-        auto put = [&](int row, uint32_t lo, uint32_t hi) {
-            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(ub + row * C::U_ROW), "r"(lo), "r"(hi) : "memory");
-        };
-        if constexpr (BITS >= 6) {
-            constexpr int W = BITS == 6 ? 2 : 4;
-            uint32_t r[4][W];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                if constexpr (W == 4)
-                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(r[c][0]), "=r"(r[c][1]), "=r"(r[c][W - 2]), "=r"(r[c][W - 1]) : "r"(ad[c]));
-                else
-                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r[c][0]), "=r"(r[c][1]) : "r"(ad[c]));
-            }
-#pragma unroll
-            for (int e = 0; e < 2 * W; ++e) {
-                const uint32_t sel = e & 1 ? 0x7632u : 0x5410u;
-                put(e, __byte_perm(r[0][e / 2], r[1][e / 2], sel), __byte_perm(r[2][e / 2], r[3][e / 2], sel));
-            }
-        } else {
-            uint32_t r[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) r[c] = lds_u16(ad[c]);
-            put(0, r[0] | r[1] << 16, r[2] | r[3] << 16);
-        }
-    };
-
+    const SlabBuild<BITS> builder(tt_addr, u_addr, tid);
     auto build = [&](uint32_t off, const uint8_t *codes) {  // codes of the unit's first k
 #pragma unroll
-        for (int i = 0; i < (KU + 1) / 2; ++i) build_step(off + i * 2 * C::U_BYTES, codes + i * 2 * CT);
+        for (int i = 0; i < (KU + 1) / 2; ++i) builder.step(off + i * 2 * C::U_BYTES, codes + i * 2 * CT);
     };
 
     const float bias1 = -(8388608.0f + (float)offset);

@@ -42,13 +42,14 @@ unsigned long long lutgemm_kernel_launches(void);
  * Kernel-family override, process-wide; 0 (LUTGEMM_KERNEL_AUTO) in every position restores the automatic
  * choice by problem shape, which is the default.  Meant for tests that must reach every kernel family on one
  * shape and for A/B timing; results do not depend on it (forward bit-identical, gradients within fp32
- * summation order).  forward: row-broadcast or slab kernel; backward: broadcast or slab gradient kernels;
+ * summation order).  forward: row-broadcast or slab kernel, or two rows per thread; backward: broadcast or slab gradient kernels;
  * grad_tile: 512 x 64 or 1024 x 32 slab tile, or one thread per output row.  Call the *_scratch_bytes functions after changing it.
  * No counterpart in the reference (one kernel per operator there).
  */
 #define LUTGEMM_KERNEL_AUTO 0
 #define LUTGEMM_FORWARD_ROWBCAST 1
 #define LUTGEMM_FORWARD_SLAB 2
+#define LUTGEMM_FORWARD_ROWS 3
 #define LUTGEMM_BACKWARD_BCAST 1
 #define LUTGEMM_BACKWARD_SLAB 2
 #define LUTGEMM_TILE_WIDE 1
