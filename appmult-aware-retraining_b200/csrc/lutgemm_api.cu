@@ -67,8 +67,8 @@ struct BackwardPlan {
 // ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
 // Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
 // The clocks are measured on B200, at 4096^3 unless said otherwise:
-//   slab kernels, per k and tile      packed 512 x 64: grad_w 1480 (4 and 6 bits), 1500 (7), 2120 (8), grad_a and grad_x 1540,
-//                                     1580, 2180; tall 1024 x 32: 1540, 1690, 1880;
+//   slab kernels, per k and tile      packed 512 x 64: grad_w 1440 (4 bits), 1300 (6), 1305 (7), 1950 (8), grad_a and grad_x
+//                                     1390, 1225, 1290, 1965; tall 1024 x 32: 1540, 1690, 1880;
 //                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
 //                                     more launches: code transposition, zeroing, and a layer's epilogue);
 //   a thread per row                  gradients 512 x 64: 1420 (4 bits), 1070 (6), 1150 (7), 1390 (8) per k, 9e3 per block of
@@ -83,9 +83,10 @@ struct FamilyClocks {
     double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start, rows, fwd_rows;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {2120, 2180, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390, 845};
-    if (bits == 7) return {1500, 1580, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150, 690};
-    return {1480, 1540, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, bits == 6 ? 1070.0 : 1420.0, 650};
+    if (bits == 8) return {1950, 1965, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390, 845};
+    if (bits == 7) return {1305, 1290, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150, 690};
+    if (bits == 6) return {1300, 1225, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1070, 650};
+    return {1440, 1390, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1420, 650};
 }
 constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU
@@ -101,7 +102,7 @@ double packed_gw_clocks(const lutgemm::PackedPlan &plan, int bits, int K, int N)
 }
 double packed_ga_clocks(const lutgemm::PackedPlan &plan, int bits, int M, int K, int N) {
     const int rt = lutgemm::packed_ga_tile_rows(N);
-    const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? 1.12 : 1.0);
+    const double step = family_clocks(bits).packed * (rt == 384 ? 0.83 : rt == 576 ? lutgemm::kPacked576Step : 1.0);
     return packed_clocks(plan, M, K, step, true);
 }
 double tall_clocks(int bits, long rows, long cols, int K, int sms) {
@@ -312,7 +313,7 @@ static bool forward_by_rows(int bits, int M, int K, int N, int sms) {
     const long tiles = div_up(M, lutgemm::kFwdRowsTile) * div_up(N, lutgemm::kFwdRowsCols);
     const bool cut = lutgemm::forward_rows_cut(M, K, N, sms);
     const double k = cut ? 4.0 * div_up(tiles * div_up(K, 4), sms) : (double)div_up(tiles, sms) * K;
-    const double t = k * f.fwd_rows + (div_up(tiles, sms) + cut) * kFwdTileClocks + f.fwd_start;
+    const double t = k * f.fwd_rows + div_up(tiles, sms) * kFwdTileClocks + f.fwd_start;
     return t < fwd_slab_clocks(bits, M, K, N, sms) && (base_forward_uses_slab(M, N) || t < fwd_bcast_clocks(bits, M, K, N, sms));
 }
 
@@ -601,9 +602,12 @@ static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
 struct GxTimes {
     double slab, bcast, rows;
 };
-static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows_entry) {
     const FamilyClocks f = family_clocks(bits);
     const long mt = bits == 8 ? 512 : 256;
+    // (lutgemm_conv2d_backward keeps the lines that it was given with the slab kernel of that time: 1580 clocks per step at 7 bits)
+    const double step = rows_entry ? f.packed : bits == 8 ? 2180 : bits == 7 ? 1580 : 1540;
+    const double step576 = rows_entry ? lutgemm::kPacked576Step : 1.12;
     double slab = 0, by_rows = 0;
     // broadcast kernel: tiles of all classes in one list, tile t on SM t mod sms (rows_of[i] rows from tile begin[i] on)
     constexpr int kMaxListed = 16;
@@ -612,7 +616,7 @@ static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms)
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(rows);
-        slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, f.packed * (rt > 512 ? 1.12 : 1.0), false);
+        slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, step * (rt > 512 ? step576 : 1.0), false);
         by_rows += rows_clocks(lutgemm::plan_rows(px.P, rows, px.C, sms), bits, px.P, px.C, true, Cout % 4 == 0, false);
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
@@ -637,11 +641,12 @@ static bool gx_rows_supported(const lutgemm::ConvGeom &g, int Cout) {
 }
 enum GxFamily { kGxBcast, kGxSlab, kGxRows };
 static GxFamily gx_family(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows) {
+    const bool rows_entry = rows;
     rows = rows && gx_rows_supported(g, Cout);
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (force == LUTGEMM_BACKWARD_BCAST) return kGxBcast;
     if (force == LUTGEMM_BACKWARD_SLAB) return rows && tile == LUTGEMM_TILE_ROWS ? kGxRows : kGxSlab;
-    const GxTimes t = gx_times(bits, g, Cout, sms);
+    const GxTimes t = gx_times(bits, g, Cout, sms, rows_entry);
     if (rows && t.rows < t.slab && t.rows < t.bcast) return kGxRows;
     return t.slab < t.bcast ? kGxSlab : kGxBcast;
 }

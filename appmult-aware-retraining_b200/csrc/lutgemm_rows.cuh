@@ -24,12 +24,22 @@ __device__ __forceinline__ void stage_table_turned(uint8_t *table, uint8_t *buff
     using T = RowsTable<BITS>;
     constexpr int COL = lut_col_num(BITS), THREADS = 512;
     uint16_t *raw = reinterpret_cast<uint16_t *>(buffer);
+    const bool vec = (reinterpret_cast<uintptr_t>(lut) & 15) == 0;
+    static_assert(T::TURN_ROWS == T::Q || T::TURN_ROWS * COL % 8 == 0, "the second half is as aligned as the first");
 #pragma unroll 1
     for (int x0 = 0; x0 < T::Q; x0 += T::TURN_ROWS) {
         const uint16_t *src = lut + x0 * COL;
         if (x0) __syncthreads();
+        if (vec) {
+            constexpr int VECS = T::TURN_BYTES / 16;
+            for (int idx = tid; idx < VECS; idx += THREADS) cp_async16(raw + 8 * idx, src + 8 * idx);
+            for (int idx = 8 * VECS + tid; idx < T::TURN_ROWS * COL; idx += THREADS) raw[idx] = src[idx];
+            cp_async_commit();
+            cp_async_wait<0>();
+        } else {
 #pragma unroll 8
-        for (int idx = tid; idx < T::TURN_ROWS * COL; idx += THREADS) raw[idx] = src[idx];
+            for (int idx = tid; idx < T::TURN_ROWS * COL; idx += THREADS) raw[idx] = src[idx];
+        }
         __syncthreads();
 #pragma unroll 4
         for (int idx = tid; idx < T::TURN_ROWS / 2 * T::Q; idx += THREADS) {
@@ -38,6 +48,65 @@ __device__ __forceinline__ void stage_table_turned(uint8_t *table, uint8_t *buff
             *reinterpret_cast<uint32_t *>(table + y * T::ROW + (x0 + 2 * xp) * 2) = (e0 | e1 << 16) ^ flip;
         }
     }
+}
+
+// table[x][y] = lut[x * COL + y] ^ flip, rows as they are
+template <int BITS>
+__device__ __forceinline__ void stage_table_plain(uint8_t *table, const uint16_t *__restrict__ lut, uint32_t flip, int tid) {
+    using T = RowsTable<BITS>;
+    constexpr int COL = lut_col_num(BITS), Q = T::Q, THREADS = 512;
+    if ((reinterpret_cast<uintptr_t>(lut) & 3u) == 0) {  // (COL is even: pairs of entries are 4-byte aligned)
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(lut);
+#pragma unroll 8
+        for (int idx = tid; idx < Q * Q / 2; idx += THREADS)
+            *reinterpret_cast<uint32_t *>(table + idx / (Q / 2) * T::ROW + idx % (Q / 2) * 4) = src[idx / (Q / 2) * (COL / 2) + idx % (Q / 2)] ^ flip;
+    } else {
+        for (int idx = tid; idx < Q * Q; idx += THREADS)
+            *reinterpret_cast<uint16_t *>(table + (idx >> BITS) * T::ROW + (idx & (Q - 1)) * 2) =
+                lut[(idx >> BITS) * COL + (idx & (Q - 1))] ^ (uint16_t)flip;
+    }
+}
+
+// Gradient tables are staged in offset-binary, entry + 2^15.  Where the least entry is not far below zero (-4 min <= max: products
+// of operands and their slopes), the offset becomes the least that leaves entries unsigned, so that their bits can be used
+// as subnormal floats (`small`); the offset's share of a sum comes off at the end.  Beyond that line rounding errors of the
+// shared offset would show in the sums.  `range` (two words of shared memory) = {0xffff, 0} on entry, visible to all; the
+// table has been written and is complete after the caller's next barrier.
+template <int BITS>
+__device__ __forceinline__ int reduce_table_offset(uint8_t *table, uint32_t *range, int tid, bool *small) {
+    using T = RowsTable<BITS>;
+    constexpr int Q = T::Q, THREADS = 512;
+    auto word = [&](int idx) -> uint32_t & { return *reinterpret_cast<uint32_t *>(table + idx / (Q / 2) * T::ROW + idx % (Q / 2) * 4); };
+    uint32_t lo = 0xffffu, hi = 0u;
+#pragma unroll 4
+    for (int idx = tid; idx < Q * Q / 2; idx += THREADS) {
+        const uint32_t v = word(idx);
+        lo = min(lo, min(v & 0xffffu, v >> 16));
+        hi = max(hi, max(v & 0xffffu, v >> 16));
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((tid & 31) == 0) {
+        atomicMin(range, lo);
+        atomicMax(range + 1, hi);
+    }
+    __syncthreads();
+    const int least = min(0, (int)range[0] - 32768), most = (int)range[1] - 32768;
+    *small = -4 * least <= most;
+    if (!*small) return 32768;
+#pragma unroll 4
+    for (int idx = tid; idx < Q * Q / 2; idx += THREADS) word(idx) -= (32768u + least) * 0x10001u;
+    return -least;
+}
+
+// For values of which the largest magnitude is m: a power of two that brings them to about 2^100, or 2^127 where that is less, and
+// what takes it, and the 2^-149 of an entry used as a subnormal float, back out of a product.  `ok`: m (and with it every product)
+// stays in the range of ordinary numbers; otherwise, and with infinities or NaN (`sum` of the values), the other form is used.
+__device__ __forceinline__ void subnormal_scale(float m, float sum, float *up, float *down, bool *ok) {
+    *ok = m < 0x1p60f && (m == 0.f || m >= 0x1p-60f) && sum == sum;
+    const int e = min(127, 227 - (int)(__float_as_uint(m) >> 23));
+    *up = __uint_as_float((uint32_t)(e + 127) << 23);
+    *down = __uint_as_float((uint32_t)(149 - e + 127) << 23);
 }
 
 // A thread's share of a slab build by 512 threads: four columns (quad bq) x eight codes (16 bytes of a table row; four codes at

@@ -16,18 +16,22 @@
 // kh*kw rows of the weight matrix, and the result is written straight into the image gradient - no col2im, no atomics.  A
 // strided convolution is cut into stride^2 classes of input pixels that each see a fixed subset of the taps.
 //
-// What bounds it: the shared-memory pipe (one 128-byte wavefront per clock) and instruction issue (four per clock).
-// The slab keeps the table's own 16 bits per entry, so a look-up costs half the wavefronts of an fp32 slab; the price
-// is the conversion at each use.  It is done for two entries at a time: each 16-bit half goes, in offset-binary, behind
-// the exponent of 2^23 (one byte permutation), one packed subtraction of 2^23 + 2^15 leaves the two signed entries
-// exactly, and one packed multiply-add (fma.rn.f32x2) consumes them - 10 instructions per 128 look-ups of a warp
-// against 8 with an fp32 slab, but 512 + build instead of 1024 + build wavefronts per 32768 look-ups.  Products and
-// sums are the same fp32 operations as with an fp32 slab.
+// What bounds it: instruction issue (four per clock, packed fp32 instructions count twice) and the shared-memory pipe (one
+// 128-byte wavefront per clock).  The slab keeps the table's own 16 bits per entry, so a look-up costs half the wavefronts
+// of an fp32 slab; the price is the conversion at each use.  It is done for two entries at a time: two byte permutations
+// make them subnormal floats, and one packed multiply-add (fma.rn.f32x2) consumes them, with grad_out scaled by a
+// power of two per thread and the table's offset taken out of the thread's partial sum (lutgemm_rows.cuh).  Tables and values that this
+// does not suit, and 576-row tiles, put each entry behind the exponent of 2^23 and subtract in between: 8 against 10
+// instructions per 128 look-ups of a warp.  Products and sums are the same fp32 operations either way.
+// With one barrier per unit and the staggered slab build of lutgemm_rows.cuh, against the subtraction, two barriers per unit and padded
+// slab rows (grad_w, grad_a): 4096^3 at 7 bits 10.50, 11.12 -> 9.13, 9.07 ms, 6 bits 9.89, 10.71 -> 8.72, 8.50, 8 bits 15.19, 15.18 ->
+// 14.18, 13.70; 262144 x 576 x 64 at 7 bits, grad_w 1.51 -> 1.34 ms.
 //
-// Hand-over between the warps of a CTA: per slab buffer a "full" and an "empty" mbarrier with one arrival per warp
-// (see lutgemm_slab_grad_tall.cu); at 7 bits and below a buffer holds the slabs of two k, so that waits, arrivals and
-// loop overhead are paid once per two k.  Every wait is bounded (lutgemm_waits.cuh).
-// Partial sums: one per lane group, warp and k; one warp (rotating with k) adds the 32 of a column in ascending order.
+// Hand-over between the warps of a CTA: at 7 bits and below three buffers of two slabs each and one mbarrier per buffer
+// (lutgemm_slab_rows.cu); at 8 bits shared memory has room for two slabs, with a "full" and an "empty" mbarrier each, one arrival per
+// warp (see lutgemm_slab_grad_tall.cu).  Every wait is bounded (lutgemm_waits.cuh).
+// Partial sums: one per lane group, warp and k; one warp (rotating with k) adds the 32 of a column in four
+// chains.
 // A CTA takes the row blocks of a group one after the other and adds each to the group's sums in ascending order (the
 // same thread stores and adds, so the reductions need no ordering between threads); groups are added by slab_reduce_blocks
 // in ascending order: results are deterministic.  With one block of sums per row block the buffer grew with the rows: 0.82
@@ -39,6 +43,7 @@
 #include "lutgemm_common.cuh"
 #include "lutgemm_f32x2.cuh"
 #include "lutgemm_kernels.h"
+#include "lutgemm_rows.cuh"
 #include "lutgemm_waits.cuh"
 
 namespace lutgemm {
@@ -50,27 +55,27 @@ template <int BITS, int RW_>
 struct Cfg {
     static constexpr int Q = 1 << BITS;
     static constexpr int WARPS = 16, THREADS = 512, RW = RW_, RT = WARPS * RW, CT = 64;
-    static constexpr int E = Q >= 32 ? Q / 32 : 1;      // codes per lane in the build: x = lane + 32 j, j < E
-    static constexpr int TT_ROW = table_row_bytes<BITS>();  // table row of a column code
-    static constexpr int U_ROW = 2 * CT + 8;            // bytes per slab row: conflict-free 64-bit build stores
+    using T = RowsTable<BITS>;
+    static constexpr int U_ROW = T::U_ROW;              // bytes per slab row
+    static_assert(U_ROW == 2 * CT, "a slab row holds the tile's columns");
     static constexpr int KC = 16;                       // k per global fetch
     static constexpr int SC = BITS == 8 ? 8 : 16;       // k per shared-memory stage
     static constexpr int KP = BITS == 8 ? 1 : 2;        // slabs per buffer
     static constexpr int NB = BITS == 8 ? 2 : 3;        // buffers (shared memory has no room for a third at 8 bits)
     static constexpr int NSEG = RT / 16;                // 16-row code segments per k
     static constexpr int RC_LOADS = (KC * NSEG + THREADS - 1) / THREADS;
-    static constexpr int TT_BYTES = (Q * TT_ROW + 15) & ~15;
-    static constexpr int U_BYTES = Q * U_ROW;
+    static constexpr int TT_BYTES = T::BYTES, U_BYTES = T::U_BYTES;
     static constexpr int RC_STAGE = SC * RT, CC_STAGE = SC * CT;
     static constexpr int P_FLOATS = 2 * WARPS * CT;     // partial sums of one k: one row per half-warp
     static constexpr int OFF_U = TT_BYTES;
     static constexpr int OFF_RC = OFF_U + NB * KP * U_BYTES;
     static constexpr int OFF_CC = OFF_RC + 2 * RC_STAGE;
     static constexpr int OFF_PART = OFF_CC + 2 * CC_STAGE;
-    static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // grad_x: image offset of each column
+    static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // (a set of sums per buffer)  grad_x: image offset of each column
     static constexpr int OFF_TAP = OFF_PIX + CT * 8;                  // grad_x: output offset {rows, columns} of each tap
     static constexpr int OFF_BAR = OFF_TAP + kMaxTaps * 8;
-    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // two mbarriers per buffer, abort word, work item
+    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 24;   // two mbarriers per buffer, abort word, work item, table range
+    static_assert(T::TURN_BYTES <= OFF_PART - OFF_U, "the table passes through the slab buffers and operand stages");
     static_assert(RW % 4 == 0 && RT % 16 == 0, "rows per warp");
     static_assert(U_BYTES % 16 == 0 && RC_STAGE % 16 == 0 && CC_STAGE % 16 == 0, "16-byte vectors");
     static_assert(SMEM <= 232448, "shared memory budget");
@@ -100,12 +105,11 @@ struct Args {
 template <int BITS, int MODE, int RW>
 __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_constant__ Args p) {
     using C = Cfg<BITS, RW>;
-    constexpr int Q = C::Q, E = C::E, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC, KP = C::KP, NB = C::NB;
+    constexpr int Q = C::Q, RT = C::RT, CT = C::CT, KC = C::KC, SC = C::SC, KP = C::KP, NB = C::NB;
     constexpr int WARPS = C::WARPS, THREADS = C::THREADS, NSEG = C::NSEG, RCL = C::RC_LOADS;
     constexpr int HALVES = KC / SC;  // shared-memory stages per fetched group of 16 k
     constexpr int NW = RW / 4;       // code words per warp; half h of the warp owns rows 4q + 2h and 4q + 2h + 1
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
-    constexpr int COL = lut_col_num(BITS);
 
     const int M = p.M, K = p.K, N = p.N;
     const int RDIM = p.RDIM, CDIM = p.CDIM;
@@ -125,14 +129,21 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
     const int half = lane >> 4, cq = lane & 15;  // half-warp and column quad (columns 4 cq .. 4 cq + 3)
 
     // ---- stage the gradient table in offset-binary; x = row code, y = column code, T(x,y) = lut[a*COL + w] -------
-    // (grad_w: rows are activation codes; grad_a / grad_x: rows are weight codes)
-#pragma unroll 8
-    for (int idx = tid; idx < Q * Q; idx += THREADS) {
-        const int hi_idx = idx >> BITS, lo_idx = idx & (Q - 1);  // global read contiguous in lo_idx
-        const int x = MODE == kGw ? hi_idx : lo_idx, y = MODE == kGw ? lo_idx : hi_idx;
-        *reinterpret_cast<uint16_t *>(smem + y * C::TT_ROW + table_pos<BITS>(x) * 2) = (uint16_t)p.lut[hi_idx * COL + lo_idx] ^ (uint16_t)0x8000u;
+    // (grad_w: rows are activation codes, so the table is turned; grad_a / grad_x: rows are weight codes)
+    uint32_t *range_s = reinterpret_cast<uint32_t *>(work_s + 3);
+    const uint16_t *lut = reinterpret_cast<const uint16_t *>(p.lut);
+    if (MODE == kGw) stage_table_turned<BITS>(smem, smem + C::OFF_U, lut, 0x80008000u, tid);
+    else stage_table_plain<BITS>(smem, lut, 0x80008000u, tid);
+    if (tid == 0) {
+        *abort_word = 0;
+        range_s[0] = 0xffffu;
+        range_s[1] = 0u;
     }
-    if (tid == 0) *abort_word = 0;
+    __syncthreads();
+    bool table_unsigned;
+    const int offset = reduce_table_offset<BITS>(smem, range_s, tid, &table_unsigned);
+    // (column codes past the last k: any codes, but codes)
+    if (tid < 2 * C::CC_STAGE / 16) reinterpret_cast<uint4 *>(cc_s)[tid] = make_uint4(0, 0, 0, 0);
     if (MODE == kGx) {
         // pixel (hh, ww) of the class sits at h = ph + s hh; tap q connects it to output row (h - dh) / s = hh + eh
         for (int q = tid; q < p.px.ntaps; q += THREADS)
@@ -245,34 +256,18 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             }
         }
     };
-    // build the slab at shared address `ub` for the k at (stage, kk): warp wp fills columns 4 wp .. 4 wp + 3.  Lane l
-    // reads the entries of codes l + 32 j of each column and stores four columns of one code at a time;
-    // all table reads of the share are issued before the first store (the stores order later reads behind them).
-    const uint32_t tt_lane = tt_addr + lane * table_lane_bytes<BITS>();
-    const uint32_t us = u_addr + wp * 8 + lane * C::U_ROW;
-    auto build = [&](uint32_t off, const uint8_t *codes) {  // off: byte offset of the slab
-        const uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + wp * 4);
-        constexpr int EW = (E + 1) / 2;  // table words per lane and column
-        uint32_t r[4][EW];
-        if (Q >= 32 || lane < Q) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) load_table_entries<BITS>(tt_lane + byte_of(cw, c) * C::TT_ROW, r[c]);
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(us + off + j * 32 * C::U_ROW),
-                             "r"(__byte_perm(r[0][j / 2], r[1][j / 2], sel)), "r"(__byte_perm(r[2][j / 2], r[3][j / 2], sel))
-                             : "memory");
-            }
-        }
-    };
+    const SlabBuild<BITS> builder(tt_addr, u_addr, tid);
     // add the 32 partial sums of one k in ascending order and store the tile's 64 columns (two per lane), or add them to
     // what this thread has stored for the row blocks before (reductions: nothing waits for the old value)
     auto reduce_store = [&](int k, const float *ps, float *obase, int c0, bool add) {
+        // (four chains: their additions overlap, and their rounding errors are those of eight sums in a row)
         const f32x2 *p2 = reinterpret_cast<const f32x2 *>(ps) + lane;
-        f32x2 v = p2[0];
-#pragma unroll 8
-        for (int i = 1; i < 2 * WARPS; ++i) v = add2(v, p2[i * (CT / 2)]);
+        f32x2 c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c[i] = p2[i * (CT / 2)];
+#pragma unroll
+        for (int i = 4; i < 2 * WARPS; ++i) c[i & 3] = add2(c[i & 3], p2[i * (CT / 2)]);
+        const f32x2 v = add2(add2(c[0], c[1]), add2(c[2], c[3]));
         float2 o = unpack2(v);
         if (p.direct) {  // (a power of two: the same sum whether it is scaled before or after)
             o.x *= kGradFactor;
@@ -310,9 +305,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
     };
 
-    const f32x2 bias = pack2(-8421376.0f, -8421376.0f);  // -(2^23 + 2^15)
+    const float bias1 = -(8388608.0f + (float)offset);
+    const f32x2 bias = pack2(bias1, bias1);
     const uint32_t wsel0 = (uint32_t)C::U_ROW << (16 * half), wsel1 = wsel0 << 8;  // dot-product weights of the lane's two rows
-    static_assert(C::U_ROW < 256, "slab row stride must fit one byte of the dot-product operand");
 
     const int items = p.main_cells + (p.groups * p.tiles_c - p.main_cells) * p.tail_parts;
     bool first_item = true;
@@ -427,7 +422,33 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             }
         }
 
-        __syncthreads();  // previous item (or the table staging) is done with every buffer
+        // entries as subnormal floats (lutgemm_rows.cuh): scale of the thread's values, what takes it out of their sums, and the
+        // offset's share of the sums, which does not depend on k
+        float up = 1.f, down = 1.f;
+        bool wide = false;
+        f32x2 corr[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+        constexpr bool MAY = RW <= 32;  // (no registers left in 576-row tiles)
+        if (MAY && table_unsigned) {
+            float m = 0.f;
+#pragma unroll
+            for (int i = 0; i < RW; ++i) {
+                const float2 t = unpack2(g[i]);
+                m = fmaxf(m, fmaxf(fabsf(t.x), fabsf(t.y)));
+                corr[i & 1] = add2(corr[i & 1], g[i]);
+            }
+            const float2 t = unpack2(add2(corr[0], corr[1]));
+            bool ok;
+            subnormal_scale(m, t.x + t.y, &up, &down, &ok);
+            wide = !ok;
+            const f32x2 minus = pack2(-(float)offset, -(float)offset);
+            corr[0] = mul2(corr[0], minus);
+            corr[1] = mul2(corr[1], minus);
+        }
+        const bool fast = !__syncthreads_or(wide) && table_unsigned && MAY;  // (previous item, or the table staging, done with every buffer)
+        if (fast) {
+#pragma unroll
+            for (int i = 0; i < RW; ++i) g[i] = mul2(g[i], pack2(up, up));
+        }
         store_stage((kbeg / SC) & 1, 0);
         if (MODE == kGx && tid < CT) pix_s[tid] = (long long)pixel_class_offset(p.px, min(c0 + tid, CDIM - 1));
         if (tid == 0) {
@@ -443,21 +464,14 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         // unit u = KP consecutive k of one stage, in buffer u % NB; with NB buffers the slabs of unit u + NB - 1 are built
         // during unit u
         constexpr int UB = KP * C::U_BYTES;
-        auto build_unit = [&](uint32_t buf, const uint8_t *codes, bool second) {
-            build(buf * UB, codes);
-            if constexpr (KP == 2)
-                if (second) build(buf * UB + C::U_BYTES, codes + CT);
-        };
-#pragma unroll
-        for (int u = 0; u < NB - 1; ++u)
-            if (kbeg + u * KP < kend)
-                build_unit(u, cc_s + ((kbeg / SC) & 1) * C::CC_STAGE + u * KP * CT, kbeg + u * KP + 1 < kend);
+        // one builder step: a slab at 8 bits, the two of a unit at fewer
+        constexpr bool ONE_BARRIER = NB == 3;
+        builder.step(0, cc_s + ((kbeg / SC) & 1) * C::CC_STAGE);
         __syncwarp();
-        // the first units are complete once every warp has arrived; the last buffer starts out released
+        // the first unit is complete once every warp has arrived; with two buffers the second starts out released
         if (lane == 0) {
-#pragma unroll
-            for (int u = 0; u < NB - 1; ++u) mbar_arrive(bar_full + 8 * u);
-            mbar_arrive(bar_empty + 8 * (NB - 1));
+            mbar_arrive(bar_full);
+            if (!ONE_BARRIER) mbar_arrive(bar_empty + 8);
         }
 
         float *obase = p.out + (p.direct ? (size_t)0 : (size_t)group * K * CDIM);
@@ -465,12 +479,12 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         const uint32_t uc = u_addr + cq * 8;
         f32x2 acc[2][2];  // [row parity j][column pair i]
         // rows of code words [QB, QE) of the warp: the lane's columns of the slab at `ua`, row codes of this k at `rbase`
-        auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag) {
+        auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag, auto fast_tag) {
+            constexpr bool FAST = decltype(fast_tag)::value;
             constexpr int QB = decltype(qb_tag)::value, QE = decltype(qe_tag)::value, NR = 2 * (QE - QB);
-            // slab reads in flight ahead of their use (4096^3 at 7 bits: grad_w 10.93 / 10.87 / 10.83 / 10.55 ms with 2 / 3 / 4 / 6
-            // (6 bits 10.31 with 4, 10.69 with 6),
-            // grad_a 11.33 / 11.19 / 11.24 / 11.48; 384-row tiles, 12608 x 1536 x 384: 1.323 / 1.283 / 1.344 / 1.323)
-            constexpr int PF = MODE == kGw ? (BITS == 7 ? 6 : 4) : RW == 24 ? 3 : 4;
+            // slab reads in flight ahead of their use (4096^3 at 7 bits, grad_w / grad_a: 9.25 / 9.00 ms with 2, 9.29 / 9.14 with 4, 9.19 /
+            // 9.02 with 6, 9.12 / 8.95 with 8)
+            constexpr int PF = RW > 32 ? 4 : 8;
             uint32_t rv[QE - QB];
             if constexpr (RW % 16 == 0 && QB % 4 == 0 && QE % 4 == 0) {
 #pragma unroll
@@ -500,8 +514,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 const uint32_t a0 = w0[i % PF], a1 = w1[i % PF];
                 if (i + PF < NR) fetch(i + PF);
                 const int gi = 2 * (2 * QB + i);
-                acc[i & 1][0] = fma2(entries2(a0, bias), g[gi], acc[i & 1][0]);
-                acc[i & 1][1] = fma2(entries2(a1, bias), g[gi + 1], acc[i & 1][1]);
+                acc[i & 1][0] = fma2(FAST ? tiny2(a0) : entries2(a0, bias), g[gi], acc[i & 1][0]);
+                acc[i & 1][1] = fma2(FAST ? tiny2(a1) : entries2(a1, bias), g[gi + 1], acc[i & 1][1]);
             }
         };
         using Q0 = std::integral_constant<int, 0>;
@@ -510,76 +524,94 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         auto clear_acc = [&]() { acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = pack2(0.f, 0.f); };
         // partial sums of one k: row 2 wp + h, the lane's four columns
         float *part_lane = part_s + (2 * wp + half) * CT + 4 * cq;
-        auto store_part = [&](int slot) {
-            const float2 lo = unpack2(add2(acc[0][0], acc[1][0])), hi = unpack2(add2(acc[0][1], acc[1][1]));
+        auto store_part = [&](int slot, auto fast_tag) {
+            f32x2 a = add2(acc[0][0], acc[1][0]), b = add2(acc[0][1], acc[1][1]);
+            if (decltype(fast_tag)::value) {
+                a = fma2(a, pack2(down, down), corr[0]);
+                b = fma2(b, pack2(down, down), corr[1]);
+            }
+            const float2 lo = unpack2(a), hi = unpack2(b);
             *reinterpret_cast<float4 *>(part_lane + slot * C::P_FLOATS) = make_float4(lo.x, lo.y, hi.x, hi.y);
         };
 
-        // Unit by unit: read the slabs, release them, then - once every warp has released the unit before, whose buffer
-        // it is - add up that unit's partial sums if it is this warp's turn and build the unit NB - 1 ahead.  With three
-        // buffers each wait has a whole unit of slack, with two (8 bits) the build sits in the middle of the reads.
-        constexpr int AHEAD = NB - 1;
+        // Three buffers: unit u + 1 is built at the start of unit u into the buffer of unit u - 2, and one barrier per unit is
+        // enough (lutgemm_slab_rows.cu); a warp that has seen unit u complete also knows that every warp has stored its
+        // partial sums of unit u - 2, which are added up then.  Two buffers (8 bits): the build sits in the middle of the reads and waits
+        // until every warp has released the unit before.
         constexpr int UNITS = SC / KP;  // per stage
-        static_assert(UNITS > 2 * AHEAD, "the next stage is written while no warp can still be reading it");
-        uint32_t buf = 0, prev = NB - 1, par = 0;  // buffers of this unit and of the one before, parity of this round
-        int stage = (kbeg / SC) & 1, hf = 0;
-        for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
-            const bool more = ks + SC < kend;
-            // the registers are free for the next group once the last stage of the current one is written
-            if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC, false);
-            const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
-            const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + AHEAD * KP * CT;  // column codes of the unit AHEAD
+        static_assert(UNITS > 2, "the next stage is written while no warp can still be reading it");
+        auto k_loop = [&](auto fast_tag) {
+            uint32_t buf = 0, par = 0;  // buffer of this unit, parity of this round
+            int stage = (kbeg / SC) & 1, hf = 0;
+            for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
+                const bool more = ks + SC < kend;
+                // the registers are free for the next group once the last stage of the current one is written
+                if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC, false);
+                const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
+                const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + KP * CT;  // column codes of the unit after
 #pragma unroll 1
-            for (int it = 0; it < UNITS; ++it) {
-                const int k = ks + KP * it;
-                if (k >= kend) break;
-                const uint32_t ua = uc + buf * UB;
-                clear_acc();
-                mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);  // the slabs of this unit are complete
-                if constexpr (KP == 2) {
-                    use_rows(ua, rb_, Q0{}, QN{});
-                    store_part(buf * KP);
-                    if (k + 1 < kend) {
-                        clear_acc();
-                        use_rows(ua + C::U_BYTES, rb_ + RT, Q0{}, QN{});
-                        store_part(buf * KP + 1);
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
-                } else {
-                    use_rows(ua, rb_, Q0{}, QH{});
-                }
-                // (same parity: the last buffer, which unit 0 waits for, starts out released)
-                mbar_wait(bar_empty + 8 * prev, par, 1 + NB + prev, abort_word, p.error_word);
-                if (k > kbeg && ((wp ^ (k - KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
-                    const int i = wp & (KP - 1);
-                    reduce_store(k - KP + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0, add);
-                }
-                if (k + AHEAD * KP < kend) {
-                    build_unit(prev, cb_, k + AHEAD * KP + 1 < kend);
+                for (int it = 0; it < UNITS; ++it) {
+                    const int k = ks + KP * it;
+                    if (k >= kend) break;
+                    const uint32_t next = buf == NB - 1 ? 0 : buf + 1;
+                    const uint32_t ua = uc + buf * UB;
                     // the next stage is written before the full arrival of the unit during which its first slab is built
-                    if (it == UNITS - 2 * AHEAD && more) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_full + 8 * prev);
+                    const bool refill = it == UNITS - 3 && more;
+                    mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);  // the slabs of this unit are complete
+                    if constexpr (ONE_BARRIER) {
+                        // (buffer and set of sums `next` belong to unit u - 2 as well)
+                        if (k >= kbeg + 2 * KP && ((wp ^ (k - 2 * KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
+                            const int i = wp & (KP - 1);
+                            reduce_store(k - 2 * KP + i, part_s + (next * KP + i) * C::P_FLOATS, obase, c0, add);
+                        }
+                        builder.step(next * UB, cb_);  // (past the last k: a slab that nobody reads)
+                        if (refill) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_full + 8 * next);
+#pragma unroll
+                        for (int i = 0; i < KP; ++i) {
+                            if (i && k + i >= kend) break;
+                            clear_acc();
+                            use_rows(ua + i * C::U_BYTES, rb_ + i * RT, Q0{}, QN{}, fast_tag);
+                            store_part(buf * KP + i, fast_tag);
+                        }
+                    } else {
+                        clear_acc();
+                        use_rows(ua, rb_, Q0{}, QH{}, fast_tag);
+                        // (same parity: the second buffer, which unit 0 waits for, starts out released)
+                        mbar_wait(bar_empty + 8 * next, par, 1 + NB + next, abort_word, p.error_word);
+                        if (k > kbeg && ((wp ^ (k - 1)) & (WARPS - 1)) == 0) reduce_store(k - 1, part_s + next * C::P_FLOATS, obase, c0, add);
+                        if (k + 1 < kend) {
+                            builder.step(next * UB, cb_);
+                            if (refill) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar_full + 8 * next);
+                        }
+                        use_rows(ua, rb_, QH{}, QN{}, fast_tag);
+                        store_part(buf, fast_tag);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
+                    }
+                    rb_ += KP * RT;
+                    cb_ = it == UNITS - 2 ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
+                    if (next == 0) par ^= 1;
+                    buf = next;
                 }
-                if constexpr (KP == 1) {
-                    use_rows(ua, rb_, QH{}, QN{});
-                    store_part(buf);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
-                }
-                rb_ += KP * RT;
-                cb_ = it == UNITS - 1 - AHEAD ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
-                prev = buf;
-                if (++buf == NB) { buf = 0; par ^= 1; }
             }
-        }
-        __syncthreads();  // every warp has stored its partial sums of the last unit
+        };
+        if (MAY && fast) k_loop(std::integral_constant<bool, MAY>{});
+        else k_loop(std::false_type{});
+        __syncthreads();  // every warp has stored its partial sums of the last units
         {
-            const int kl = kend - 1 - (kend - 1 - kbeg) % KP;  // first k of the last unit, in buffer prev
+            // the last unit's, and with three buffers those of the one before it
+            const int kl = kend - 1 - (kend - 1 - kbeg) % KP;  // first k of the last unit
             const int i = wp & (KP - 1);
-            if (kl + i < kend && ((wp ^ kl) & (WARPS - KP)) == 0)
-                reduce_store(kl + i, part_s + (prev * KP + i) * C::P_FLOATS, obase, c0, add);
+#pragma unroll
+            for (int back = ONE_BARRIER ? 1 : 0; back >= 0; --back) {
+                const int ku = kl - back * KP;
+                if (ku >= kbeg && ku + i < kend && ((wp ^ ku) & (WARPS - KP)) == 0)
+                    reduce_store(ku + i, part_s + ((ku - kbeg) / KP % NB * KP + i) * C::P_FLOATS, obase, c0, add);
+            }
         }
         if (++block == p.group_blocks || tr + 1 == p.tiles_r) {
             block = 0;
@@ -598,7 +630,7 @@ static int best_tile_rows(long rdim, bool with_384) {
     auto cost = [&](long rt, double step) { return (double)((rdim + rt - 1) / rt) * step; };
     int rt = 512;
     double c = cost(512, 1.0);
-    if (cost(576, 1.12) < c) { c = cost(576, 1.12); rt = 576; }
+    if (cost(576, kPacked576Step) < c) { c = cost(576, kPacked576Step); rt = 576; }
     if (with_384 && cost(384, 0.83) < c) rt = 384;
     return rt;
 }

@@ -124,13 +124,9 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
 
     // ---- stage the gradient table in offset-binary: tt[y][x], x = row code, y = term code, T = lut[a * COL + w] -----------
     // (grad_w: rows are weight codes; grad_a / grad_x: rows are activation codes, so the table is turned)
-    if (MODE == kGw) {
-        for (int idx = tid; idx < Q * Q; idx += THREADS)
-            *reinterpret_cast<uint16_t *>(smem + (idx >> BITS) * C::TT_ROW + (idx & (Q - 1)) * 2) =
-                (uint16_t)p.lut[(idx >> BITS) * COL + (idx & (Q - 1))] ^ (uint16_t)0x8000u;
-    } else {
-        stage_table_turned<BITS>(smem, smem + C::OFF_U, reinterpret_cast<const uint16_t *>(p.lut), 0x80008000u, tid);
-    }
+    const uint16_t *lut = reinterpret_cast<const uint16_t *>(p.lut);
+    if (MODE == kGw) stage_table_plain<BITS>(smem, lut, 0x80008000u, tid);
+    else stage_table_turned<BITS>(smem, smem + C::OFF_U, lut, 0x80008000u, tid);
     if (tid == 0) {
         *abort_word = 0;
         range_s[0] = 0xffffu;
@@ -138,28 +134,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
     }
     if (tid < 2 * C::CC_STAGE / 16) reinterpret_cast<uint4 *>(cc_s)[tid] = make_uint4(0, 0, 0, 0);  // (codes past the last k)
     __syncthreads();
-    // ---- offset of the table entries: 2^15 so far, the least that makes them unsigned where that is small -----------------
-    {
-        uint32_t lo = 0xffffu, hi = 0u;
-        for (int idx = tid; idx < Q * Q / 2; idx += THREADS) {
-            const uint32_t v = *reinterpret_cast<const uint32_t *>(smem + (idx / (Q / 2)) * C::TT_ROW + (idx % (Q / 2)) * 4);
-            lo = min(lo, min(v & 0xffffu, v >> 16));
-            hi = max(hi, max(v & 0xffffu, v >> 16));
-        }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) {
-            atomicMin(range_s, lo);
-            atomicMax(range_s + 1, hi);
-        }
-        __syncthreads();
-    }
-    const int tmin = min(0, (int)range_s[0] - 32768), tmax = (int)range_s[1] - 32768;
-    const bool table_unsigned = -4 * tmin <= tmax;
-    const int offset = table_unsigned ? -tmin : 32768;
-    if (table_unsigned)
-        for (int idx = tid; idx < Q * Q / 2; idx += THREADS)
-            *reinterpret_cast<uint32_t *>(smem + (idx / (Q / 2)) * C::TT_ROW + (idx % (Q / 2)) * 4) -= (32768u - offset) * 0x10001u;
+    bool table_unsigned;
+    const int offset = reduce_table_offset<BITS>(smem, range_s, tid, &table_unsigned);
     if (MODE == kGx) {
         // pixel (hh, ww) of the class sits at h = ph + s hh; tap q connects it to output row (h - dh) / s = hh + eh
         for (int q = tid; q < p.px.ntaps; q += THREADS)
@@ -356,11 +332,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
                 }
                 const float2 t = unpack2(gs);
                 const float sum = t.x + t.y;
-                wide = !(m < 0x1p60f && (m == 0.f || m >= 0x1p-60f) && sum == sum);
+                bool ok;
+                subnormal_scale(m, sum, &scale, &fa, &ok);
+                wide = !ok;
+                fa *= factor;
                 fb = -(float)offset * sum * factor;
-                const int up = min(127, 227 - (int)(__float_as_uint(m) >> 23));  // m * 2^up is about 2^100, or less
-                fa = __uint_as_float((uint32_t)(149 - up + 127) << 23) * factor;
-                scale = __uint_as_float((uint32_t)(up + 127) << 23);
             }
 
             // where the sums of this block go
