@@ -612,39 +612,100 @@ __global__ void __launch_bounds__(1024) transpose_codes_kernel(const uint8_t *__
     *reinterpret_cast<uint4 *>(at + (size_t)k * pitch + m0) = make_uint4(v[0] & mask4, v[1] & mask4, v[2] & mask4, v[3] & mask4);
 }
 
-// The same for a convolution whose output plane is a multiple of 16 positions and whose input plane fits
-// shared memory: one CTA stages the plane x[b,c,:,:] once (coalesced) and writes the kh*kw shifted copies of
-// it, 16 output positions per thread and store.
+// The same for a convolution whose output rows are a multiple of 4 and whose output planes are a multiple of 16 positions: a CTA
+// stages `planes` input planes of one channel, with the padding's zeros around them, and writes their kh*kw shifted copies.
+// Four neighbouring outputs come from two or three aligned words and a funnel shift (stride 1 and 2), not byte by byte
+// with a test of the borders for each: 256 planes of 64 x 32 x 32, 3x3, 116 -> 51 us.  Small planes share a CTA, images after
+// one another, so that stores stay longer than a sector.
+struct PlaneStage {
+    int planes, rows, pitch;  // planes per CTA; rows and bytes per row of a staged plane
+    unsigned groups;          // CTAs per channel
+    // ceil(2^32 / d) for d = words per staged plane, words per staged row, chunks of 16 outputs per CTA and per plane, four
+    // outputs per row (0 where d is 1): n / d is the high half of n * it, for n * d < 2^32
+    unsigned by_plane, by_row, by_rows, by_chunks, by_quads;
+};
+__device__ __forceinline__ int quotient(int n, unsigned by) { return by == 0u ? n : (int)__umulhi(n, by); }
+template <int STRIDE>
 __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_t *__restrict__ x, uint8_t *__restrict__ at,
-                                                                    int pitch, const ConvGeom g, uint32_t mask4) {
+                                                                    int at_pitch, const ConvGeom g, uint32_t mask4,
+                                                                    const PlaneStage st) {
     extern __shared__ __align__(16) uint8_t plane[];
-    const int bc = blockIdx.x, b = bc / g.C, c = bc - b * g.C;
-    const int HW = g.H * g.W, L = g.Ho * g.Wo, kk = g.kh * g.kw;
-    const uint8_t *src = x + (size_t)bc * HW;
-    if ((HW & 15) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        for (int i = threadIdx.x; i < HW / 16; i += blockDim.x)
-            reinterpret_cast<uint4 *>(plane)[i] = reinterpret_cast<const uint4 *>(src)[i];
-    } else {
-        for (int i = threadIdx.x; i < HW; i += blockDim.x) plane[i] = src[i];
+    const int c = blockIdx.x / st.groups, b0 = (blockIdx.x % st.groups) * st.planes, nb = min(st.planes, g.B - b0);
+    const int HW = g.H * g.W, L = g.Ho * g.Wo, kk = g.kh * g.kw, bytes = st.rows * st.pitch, words = bytes / 4, rw = st.pitch / 4;
+    const bool aligned = (g.W & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+    const int up = (4 - g.pad) & 3;  // byte of its source word that a staged word starts at
+    // (rows and columns that no window reaches are left out)
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nb * words; i += 256) {
+        const int p = quotient(i, st.by_plane), r = i - p * words, row = quotient(r, st.by_row);
+        const int h = row - g.pad, w0 = (r - row * rw) * 4 - g.pad;
+        uint32_t v = 0u;
+        if ((unsigned)h < (unsigned)g.H) {
+            const uint8_t *src = x + ((size_t)(b0 + p) * g.C + c) * HW + h * g.W;
+            if (aligned) {
+                const int lo = w0 - up;  // (a multiple of 4)
+                const uint32_t v0 = (unsigned)lo < (unsigned)g.W ? *reinterpret_cast<const uint32_t *>(src + lo) : 0u;
+                const uint32_t v1 = up != 0 && (unsigned)(lo + 4) < (unsigned)g.W ? *reinterpret_cast<const uint32_t *>(src + lo + 4) : 0u;
+                v = __funnelshift_r(v0, v1, 8 * up);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if ((unsigned)(w0 + e) < (unsigned)g.W) v |= (uint32_t)src[w0 + e] << (8 * e);
+            }
+        }
+        reinterpret_cast<uint32_t *>(plane)[i] = v & mask4;
     }
     __syncthreads();
-    const int chunks = L / 16;
-    for (int q = threadIdx.x; q < kk * chunks; q += blockDim.x) {
-        const int tap = q / chunks, l0 = (q - tap * chunks) * 16;
-        const int i = tap / g.kw, j = tap - i * g.kw;
-        const int dh = i * g.dil - g.pad, dw = j * g.dil - g.pad;
-        int oh = l0 / g.Wo, ow = l0 - oh * g.Wo;
-        uint32_t v[4] = {0u, 0u, 0u, 0u};
+    // a thread takes 16 outputs of one kernel row and goes over its taps
+    const int chunks = L / 16, per_row = nb * chunks;
+    for (int q = threadIdx.x; q < g.kh * per_row; q += 256) {
+        const int i = nb == st.planes ? quotient(q, st.by_rows) : q / per_row;
+        const int r = q - i * per_row, p = quotient(r, st.by_chunks), l0 = (r - p * chunks) * 16;
+        int oh = quotient(l0 / 4, st.by_quads), ow = l0 - oh * g.Wo;
+        int o[4];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const int ih = oh * g.stride + dh, iw = ow * g.stride + dw;
-            if ((unsigned)ih < (unsigned)g.H && (unsigned)iw < (unsigned)g.W)
-                v[e >> 2] |= (uint32_t)plane[ih * g.W + iw] << (8 * (e & 3));
-            if (++ow == g.Wo) { ow = 0; ++oh; }
+        for (int e = 0; e < 4; ++e) {
+            o[e] = p * bytes + (i * g.dil + oh * g.stride) * st.pitch + ow * g.stride;
+            ow += 4;
+            if (ow == g.Wo) { ow = 0; ++oh; }
         }
-        *reinterpret_cast<uint4 *>(at + (size_t)(c * kk + tap) * pitch + (size_t)b * L + l0) =
-            make_uint4(v[0] & mask4, v[1] & mask4, v[2] & mask4, v[3] & mask4);
+        uint8_t *dst = at + (size_t)(c * kk + i * g.kw) * at_pitch + (size_t)(b0 + p) * L + l0;
+        for (int j = 0; j < g.kw; ++j, dst += at_pitch) {
+            uint32_t v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int ad = o[e] + j * g.dil;
+                if (STRIDE == 0) {
+                    v[e] = 0u;
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) v[e] |= (uint32_t)plane[ad + t * g.stride] << (8 * t);
+                } else {
+                    const uint32_t *w = reinterpret_cast<const uint32_t *>(plane) + (ad >> 2);
+                    const int sh = 8 * (ad & 3);
+                    const uint32_t lo = __funnelshift_r(w[0], w[1], sh);
+                    v[e] = STRIDE == 1 ? lo : __byte_perm(lo, __funnelshift_r(w[1], w[2], sh), 0x6420);
+                }
+            }
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+        }
     }
+}
+
+// 1x1 windows of stride 1 without padding: rows of L = H*W codes change places, 16 at a time.
+__global__ void __launch_bounds__(256) transpose_codes_rows_kernel(const uint8_t *__restrict__ x, uint8_t *__restrict__ at, int C, int L,
+                                                                   long M, uint32_t mask4) {
+    const long m = ((long)blockIdx.x * 256 + threadIdx.x) * 16;
+    if (m >= M) return;
+    const long b = (unsigned)m / (unsigned)L, l = m - b * L;
+    const int c0 = blockIdx.y * 4;
+    uint4 v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (c0 + e < C) v[e] = *reinterpret_cast<const uint4 *>(x + ((size_t)b * C + c0 + e) * L + l);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (c0 + e < C)
+            *reinterpret_cast<uint4 *>(at + (size_t)(c0 + e) * M + m) = make_uint4(v[e].x & mask4, v[e].y & mask4, v[e].z & mask4, v[e].w & mask4);
 }
 
 // Plain [M,K] matrix with 16-byte aligned rows (K a multiple of 16): a CTA moves a tile of 128 rows x 64 k through
@@ -678,16 +739,39 @@ __global__ void __launch_bounds__(512) transpose_codes_tiled_kernel(const uint8_
 int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, const ConvGeom &conv, int bits,
                     cudaStream_t stream) {
     const uint32_t mask4 = ((1u << bits) - 1u) * 0x01010101u;  // codes are cut to `bits` bits on their way through
-    // (small planes leave a CTA too little to do: they take the generic kernel)
-    if (conv.enabled && (conv.Ho * conv.Wo) % 16 == 0 && conv.Ho * conv.Wo >= 256 && conv.H * conv.W <= 96 * 1024 &&
-        (long)conv.B * conv.C <= 0x7fffffffL) {
+    if (conv.enabled && (conv.Ho * conv.Wo) % 16 == 0 && conv.Wo % 4 == 0) {
         // every column m < M is written (M = B * Ho * Wo is a multiple of 16, so pitch == M)
-        const int smem = (conv.H * conv.W + 15) & ~15;
-        if (smem > 48 * 1024 &&
-            !cuda_ok(cudaFuncSetAttribute(transpose_codes_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
-            return LUTGEMM_E_CUDA;
-        transpose_codes_plane_kernel<<<conv.B * conv.C, 256, smem, stream>>>(a, at, pitch, conv, mask4);
-        return launch_status();
+        const int L = conv.Ho * conv.Wo;
+        if (conv.kh * conv.kw == 1 && conv.stride == 1 && conv.pad == 0 && conv.C <= 4 * 65535 && (reinterpret_cast<uintptr_t>(a) & 15) == 0) {
+            transpose_codes_rows_kernel<<<dim3((unsigned)((M / 16 + 255) / 256), (unsigned)((conv.C + 3) / 4)), 256, 0, stream>>>(
+                a, at, conv.C, L, M, mask4);
+            return launch_status();
+        }
+        PlaneStage st{};
+        st.rows = (conv.Ho - 1) * conv.stride + (conv.kh - 1) * conv.dil + 1;
+        // (the words behind the last outputs of a row are read too)
+        st.pitch = ((conv.Wo - 1) * conv.stride + (conv.kw - 1) * conv.dil + 1 + 8 + 3) & ~3;
+        const long bytes = (long)st.rows * st.pitch;
+        // about four thousand outputs per tap and CTA
+        const int want = (4096 + L - 1) / L;
+        st.planes = want < conv.B ? want : conv.B;
+        while (st.planes > 1 && st.planes * bytes > 24 * 1024) --st.planes;
+        st.groups = (unsigned)((conv.B + st.planes - 1) / st.planes);
+        const long per_row = (long)st.planes * (L / 16);
+        if (bytes <= 96 * 1024 && (long)conv.C * st.groups < (1L << 31) && conv.kh * per_row * per_row < (1L << 32)) {
+            auto reciprocal = [](long d) { return d == 1 ? 0u : (unsigned)(((1L << 32) + d - 1) / d); };
+            st.by_plane = reciprocal(bytes / 4);
+            st.by_row = reciprocal(st.pitch / 4);
+            st.by_rows = reciprocal(per_row);
+            st.by_chunks = reciprocal(L / 16);
+            st.by_quads = reciprocal(conv.Wo / 4);
+            const int smem = (int)(st.planes * bytes) + 16;
+            auto kern = conv.stride == 1 ? transpose_codes_plane_kernel<1> : conv.stride == 2 ? transpose_codes_plane_kernel<2> : transpose_codes_plane_kernel<0>;
+            if (smem > 48 * 1024 && !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+                return LUTGEMM_E_CUDA;
+            kern<<<(unsigned)conv.C * st.groups, 256, smem, stream>>>(a, at, pitch, conv, mask4, st);
+            return launch_status();
+        }
     }
     // (k runs over grid.y, which ends at 65535: longer K in several launches)
     const bool tiled = !conv.enabled && K % 16 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
