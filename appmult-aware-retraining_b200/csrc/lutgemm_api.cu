@@ -340,10 +340,13 @@ static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const u
     if (sms <= 0) return LUTGEMM_E_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int pitch = codes_pitch(M);
+    // the copy's launch sets the sums to zero where its M * K / 16 threads have 64 words each at most
+    const bool few_sums = N <= 4 * (long)K;
     if (may_rows && scratch && scratch_bytes >= (size_t)pitch * K && forward_by_rows(bits, M, K, N, sms)) {
-        const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, s);
+        const bool zero = few_sums && !epi && lutgemm::forward_rows_cut(M, K, N, sms);
+        const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, zero ? c : nullptr, (long)M * N, s);
         if (trc != LUTGEMM_OK) return trc;
-        return lutgemm::forward_rows(w, c, lut, bits, M, K, N, static_cast<const uint8_t *>(scratch), pitch, epi, sms, s);
+        return lutgemm::forward_rows(w, c, lut, bits, M, K, N, static_cast<const uint8_t *>(scratch), pitch, epi, zero, sms, s);
     }
     bool slab = forward_uses_slab(bits, M, K, N, sms);
     if (slab && scratch && scratch_bytes < (size_t)pitch * K) {
@@ -352,12 +355,13 @@ static int forward_impl(const uint8_t *a, const uint8_t *w, uint32_t *c, const u
     }
     if (slab) {
         const uint8_t *at = nullptr;
+        const bool zero = scratch && few_sums && !epi && lutgemm::slab_fwd_ksplits(M, K, N, sms) > 1;
         if (scratch) {
-            const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, s);
+            const int trc = lutgemm::transpose_codes(a, static_cast<uint8_t *>(scratch), M, K, pitch, conv, bits, zero ? c : nullptr, (long)M * N, s);
             if (trc != LUTGEMM_OK) return trc;
             at = static_cast<const uint8_t *>(scratch);
         }
-        return lutgemm::forward_slab(a, w, c, lut, bits, M, K, N, conv, at, pitch, epi, sms, s);
+        return lutgemm::forward_slab(a, w, c, lut, bits, M, K, N, conv, at, pitch, epi, zero, sms, s);
     }
     return lutgemm::forward_rowbcast(a, w, c, lut, bits, M, K, N, conv, epi, sms, s);
 }
@@ -431,7 +435,7 @@ static int backward_impl(const float *gc, const uint8_t *a, const uint8_t *w, fl
     const uint8_t *at = codes_t;  // left by the forward pass (same layout), or made here
     if (pl.at_pitch && !at) {
         uint8_t *dst = static_cast<uint8_t *>(scratch) + pl.at_offset;
-        const int trc = lutgemm::transpose_codes(a, dst, M, K, pl.at_pitch, conv, bits, s);
+        const int trc = lutgemm::transpose_codes(a, dst, M, K, pl.at_pitch, conv, bits, nullptr, 0, s);
         if (trc != LUTGEMM_OK) return trc;
         at = dst;
     }
@@ -1066,14 +1070,10 @@ int lutgemm_conv2d_layer_pass(const float *x, long x_sb, long x_sc, long x_sh, l
     const size_t L = (size_t)g.Ho * g.Wo, pixels = (size_t)B * H * W;
     float *chansum = work, *wsum = chansum + pixels, *sumw_t = wsum + (size_t)Cout * kh * kw, *taps = sumw_t + L * Cout,
           *box = taps + L;
-    // (the quantisation kernel adds its channel tiles to the channel sums)
-    if (!lutgemm::cuda_ok(cudaMemsetAsync(chansum, 0, pixels * sizeof(float), static_cast<cudaStream_t>(stream))))
-        return LUTGEMM_E_CUDA;
-    rc = lutgemm_quantize_activations(x, x_sb, x_sc, x_sh, x_sw, B, C, H, W, quant, quant + 1, a_qmax, codes, chansum, stream);
-    if (rc == LUTGEMM_OK)
-        rc = lutgemm_layer_weight_prep(weight, w_so, w_sc, w_sh, w_sw, Cout, C, kh, kw, quant, w_qmax, wmat, wsum, stream);
-    if (rc == LUTGEMM_OK) rc = lutgemm_layer_cross_terms(wsum, Cout, C, H, W, kh, kw, stride, pad, dil, sumw_t, taps, stream);
-    if (rc == LUTGEMM_OK) rc = lutgemm_layer_window_sum(chansum, B, H, W, kh, kw, stride, pad, dil, box, stream);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    rc = lutgemm::layer_prep(x, x_sb, x_sc, x_sh, x_sw, B, C, H, W, a_qmax, weight, w_so, w_sc, w_sh, w_sw, Cout, kh, kw, w_qmax, quant,
+                             codes, chansum, wmat, wsum, sms, s);
+    if (rc == LUTGEMM_OK) rc = lutgemm::layer_sums(wsum, Cout, g, sumw_t, taps, chansum, box, sms, s);
     if (rc != LUTGEMM_OK) return rc;
     return lutgemm_conv2d_forward_layer(codes, wmat, lut, bits, B, C, H, W, Cout, kh, kw, stride, pad, dil, box, sumw_t, taps,
                                         quant, quant + 2, quant + 1, quant + 3, bias, out, scratch, scratch_bytes, stream);

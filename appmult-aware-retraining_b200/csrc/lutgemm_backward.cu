@@ -582,12 +582,30 @@ int backward_gw(const float *gc, const uint8_t *a, const uint8_t *w, float *gw, 
     return LUTGEMM_E_BITS;
 }
 
+// Words that a launch of the transposition sets to zero on the way, every thread its share: the sums that the forward kernel behind
+// it adds to.  (A launch costs the host about 5 us, as much as the kernels of a small layer take.)
+struct ZeroJob {
+    uint32_t *words;
+    long n;
+};
+__device__ __forceinline__ void zero_share(const ZeroJob &z) {
+    const long first = ((long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x * blockDim.y + threadIdx.y * blockDim.x + threadIdx.x;
+    const long threads = (long)gridDim.x * gridDim.y * blockDim.x * blockDim.y;
+    if ((reinterpret_cast<uintptr_t>(z.words) & 15) == 0) {
+        for (long i = first; i < z.n / 4; i += threads) reinterpret_cast<uint4 *>(z.words)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (first < (z.n & 3)) z.words[(z.n & ~3L) + first] = 0u;
+    } else {
+        for (long i = first; i < z.n; i += threads) z.words[i] = 0u;
+    }
+}
+
 // at[k][m..m+15] per thread: lanes run over m, so the 16-byte stores are coalesced.  For the unfolded code
 // image the (channel, tap) of k and the (image, row, column) of the first m are decoded once per thread and m
 // advances incrementally; for a plain [M,K] matrix the byte loads of the 32 k of a block share sectors.
 __global__ void __launch_bounds__(1024) transpose_codes_kernel(const uint8_t *__restrict__ a, uint8_t *__restrict__ at,
                                                                int M, int K, int pitch, const ConvGeom g, uint32_t mask4,
-                                                               int kbeg) {
+                                                               int kbeg, const ZeroJob zero) {
+    zero_share(zero);
     const int k = kbeg + blockIdx.y * 32 + threadIdx.y;
     const int m0 = (blockIdx.x * 32 + threadIdx.x) * 16;
     if (k >= K || m0 >= pitch) return;
@@ -628,8 +646,9 @@ __device__ __forceinline__ int quotient(int n, unsigned by) { return by == 0u ? 
 template <int STRIDE>
 __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_t *__restrict__ x, uint8_t *__restrict__ at,
                                                                     int at_pitch, const ConvGeom g, uint32_t mask4,
-                                                                    const PlaneStage st) {
+                                                                    const PlaneStage st, const ZeroJob zero) {
     extern __shared__ __align__(16) uint8_t plane[];
+    zero_share(zero);
     const int c = blockIdx.x / st.groups, b0 = (blockIdx.x % st.groups) * st.planes, nb = min(st.planes, g.B - b0);
     const int HW = g.H * g.W, L = g.Ho * g.Wo, kk = g.kh * g.kw, bytes = st.rows * st.pitch, words = bytes / 4, rw = st.pitch / 4;
     const bool aligned = (g.W & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
@@ -693,7 +712,8 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
 
 // 1x1 windows of stride 1 without padding: rows of L = H*W codes change places, 16 at a time.
 __global__ void __launch_bounds__(256) transpose_codes_rows_kernel(const uint8_t *__restrict__ x, uint8_t *__restrict__ at, int C, int L,
-                                                                   long M, uint32_t mask4) {
+                                                                   long M, uint32_t mask4, const ZeroJob zero) {
+    zero_share(zero);
     const long m = ((long)blockIdx.x * 256 + threadIdx.x) * 16;
     if (m >= M) return;
     const long b = (unsigned)m / (unsigned)L, l = m - b * L;
@@ -711,10 +731,12 @@ __global__ void __launch_bounds__(256) transpose_codes_rows_kernel(const uint8_t
 // Plain [M,K] matrix with 16-byte aligned rows (K a multiple of 16): a CTA moves a tile of 128 rows x 64 k through
 // shared memory - 16-byte loads along k, 16-byte stores along m - instead of gathering single bytes from global memory.
 __global__ void __launch_bounds__(512) transpose_codes_tiled_kernel(const uint8_t *__restrict__ a, uint8_t *__restrict__ at,
-                                                                    int M, int K, int pitch, uint32_t mask4, int kbeg) {
+                                                                    int M, int K, int pitch, uint32_t mask4, int kbeg,
+                                                                    const ZeroJob zero) {
     constexpr int TM = 128, TK = 64, TP = TK + 4;  // tile pitch in bytes: rows 17 words apart, the transposed byte reads
                                                    // of 32 rows fall on 32 different banks
     __shared__ __align__(16) uint8_t tile[TM * TP];
+    zero_share(zero);
     const int m0 = blockIdx.x * TM, k0 = kbeg + blockIdx.y * TK;
     const int tid = threadIdx.x;
     {   // load: thread = (row, 16-k chunk); 4 chunks per row
@@ -737,14 +759,15 @@ __global__ void __launch_bounds__(512) transpose_codes_tiled_kernel(const uint8_
 }
 
 int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, const ConvGeom &conv, int bits,
-                    cudaStream_t stream) {
+                    uint32_t *zero, long zero_words, cudaStream_t stream) {
+    ZeroJob job{zero, zero ? zero_words : 0};
     const uint32_t mask4 = ((1u << bits) - 1u) * 0x01010101u;  // codes are cut to `bits` bits on their way through
     if (conv.enabled && (conv.Ho * conv.Wo) % 16 == 0 && conv.Wo % 4 == 0) {
         // every column m < M is written (M = B * Ho * Wo is a multiple of 16, so pitch == M)
         const int L = conv.Ho * conv.Wo;
         if (conv.kh * conv.kw == 1 && conv.stride == 1 && conv.pad == 0 && conv.C <= 4 * 65535 && (reinterpret_cast<uintptr_t>(a) & 15) == 0) {
             transpose_codes_rows_kernel<<<dim3((unsigned)((M / 16 + 255) / 256), (unsigned)((conv.C + 3) / 4)), 256, 0, stream>>>(
-                a, at, conv.C, L, M, mask4);
+                a, at, conv.C, L, M, mask4, job);
             return launch_status();
         }
         PlaneStage st{};
@@ -769,7 +792,7 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
             auto kern = conv.stride == 1 ? transpose_codes_plane_kernel<1> : conv.stride == 2 ? transpose_codes_plane_kernel<2> : transpose_codes_plane_kernel<0>;
             if (smem > 48 * 1024 && !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
                 return LUTGEMM_E_CUDA;
-            kern<<<(unsigned)conv.C * st.groups, 256, smem, stream>>>(a, at, pitch, conv, mask4, st);
+            kern<<<(unsigned)conv.C * st.groups, 256, smem, stream>>>(a, at, pitch, conv, mask4, st, job);
             return launch_status();
         }
     }
@@ -778,10 +801,11 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
     const int rows_per_block = tiled ? 64 : 32, most = 65535 * rows_per_block;
     for (long k = 0; k < K; k += most) {
         const unsigned ny = (unsigned)(((K - k < most ? K - k : most) + rows_per_block - 1) / rows_per_block);
-        if (tiled) transpose_codes_tiled_kernel<<<dim3((pitch + 127) / 128, ny), 512, 0, stream>>>(a, at, M, K, pitch, mask4, (int)k);
-        else transpose_codes_kernel<<<dim3((pitch / 16 + 31) / 32, ny), dim3(32, 32), 0, stream>>>(a, at, M, K, pitch, conv, mask4, (int)k);
+        if (tiled) transpose_codes_tiled_kernel<<<dim3((pitch + 127) / 128, ny), 512, 0, stream>>>(a, at, M, K, pitch, mask4, (int)k, job);
+        else transpose_codes_kernel<<<dim3((pitch / 16 + 31) / 32, ny), dim3(32, 32), 0, stream>>>(a, at, M, K, pitch, conv, mask4, (int)k, job);
         const int rc = launch_status();
         if (rc != LUTGEMM_OK) return rc;
+        job.n = 0;
     }
     return LUTGEMM_OK;
 }

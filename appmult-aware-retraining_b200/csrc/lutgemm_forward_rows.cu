@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(512, 1) forward_rows_kernel(const Args p) {
 namespace {
 
 template <int BITS>
-int launch_forward_rows(fr::Args p, int num_sms, cudaStream_t stream) {
+int launch_forward_rows(fr::Args p, bool zeroed, int num_sms, cudaStream_t stream) {
     using C = fr::Cfg<BITS>;
     auto kern = fr::forward_rows_kernel<BITS>;
     if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM))) return LUTGEMM_E_CUDA;
@@ -283,7 +283,7 @@ int launch_forward_rows(fr::Args p, int num_sms, cudaStream_t stream) {
     if (!p.error_word) return LUTGEMM_E_CUDA;
     const long items = p.share ? p.tiles * ((p.K + 3) / 4) : p.tiles;
     const int grid = (int)(items < num_sms ? items : num_sms);
-    if (p.share && !cuda_ok(cudaMemsetAsync(p.c, 0, (size_t)p.M * p.N * sizeof(uint32_t), stream))) return LUTGEMM_E_CUDA;
+    if (p.share && !zeroed && !cuda_ok(cudaMemsetAsync(p.c, 0, (size_t)p.M * p.N * sizeof(uint32_t), stream))) return LUTGEMM_E_CUDA;
     kern<<<grid, C::THREADS, C::SMEM, stream>>>(p);
     return launch_status();
 }
@@ -291,7 +291,7 @@ int launch_forward_rows(fr::Args p, int num_sms, cudaStream_t stream) {
 }  // namespace
 
 int forward_rows(const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K, int N, const uint8_t *at,
-                 int at_pitch, const LayerEpilogue *epi, int num_sms, cudaStream_t stream) {
+                 int at_pitch, const LayerEpilogue *epi, bool zeroed, int num_sms, cudaStream_t stream) {
     fr::Args p{};
     p.at = at; p.at_pitch = at_pitch; p.w = w; p.lut = lut; p.c = c; p.M = M; p.K = K; p.N = N;
     if (epi) p.epi = *epi;
@@ -300,10 +300,10 @@ int forward_rows(const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, i
     p.share = !epi && forward_rows_cut(M, K, N, num_sms);
     p.vec_w = N % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
     switch (bits) {
-        case 4: return launch_forward_rows<4>(p, num_sms, stream);
-        case 6: return launch_forward_rows<6>(p, num_sms, stream);
-        case 7: return launch_forward_rows<7>(p, num_sms, stream);
-        case 8: return launch_forward_rows<8>(p, num_sms, stream);
+        case 4: return launch_forward_rows<4>(p, zeroed, num_sms, stream);
+        case 6: return launch_forward_rows<6>(p, zeroed, num_sms, stream);
+        case 7: return launch_forward_rows<7>(p, zeroed, num_sms, stream);
+        case 8: return launch_forward_rows<8>(p, zeroed, num_sms, stream);
     }
     return LUTGEMM_E_BITS;
 }

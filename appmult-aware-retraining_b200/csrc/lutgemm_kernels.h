@@ -29,16 +29,17 @@ struct LayerEpilogue;  // lutgemm_common.cuh; optional de-quantisation applied w
 int forward_rowbcast(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K,
                      int N, const ConvGeom &conv, const LayerEpilogue *epi, int num_sms, cudaStream_t stream);
 
-// `at` (optional): the activation codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes)
+// `at` (optional): the activation codes transposed, at[k][m] with rows at_pitch bytes apart (transpose_codes); `zeroed`: c holds
+// zeros already, which the parts of a cut K are added to
 int forward_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K, int N,
-                 const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, int num_sms,
+                 const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, bool zeroed, int num_sms,
                  cudaStream_t stream);
 
 // forward kernel with two output rows per thread (lutgemm_forward_rows.cu), tiles of 1024 rows x 32 columns; `at` as above,
 // not optional
 constexpr int kFwdRowsTile = 1024, kFwdRowsCols = 32;
 int forward_rows(const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K, int N, const uint8_t *at,
-                 int at_pitch, const LayerEpilogue *epi, int num_sms, cudaStream_t stream);
+                 int at_pitch, const LayerEpilogue *epi, bool zeroed, int num_sms, cudaStream_t stream);
 // whether it cuts K where it is free to: whole tiles would leave the last wave of the persistent grid badly filled
 inline bool forward_rows_cut(int M, int K, int N, int num_sms) {
     const long tiles = (long)((M + kFwdRowsTile - 1) / kFwdRowsTile) * ((N + kFwdRowsCols - 1) / kFwdRowsCols);
@@ -230,13 +231,17 @@ void slab_tall_set_handover(bool on);
 
 
 // at[k][m] = a[m][k] cut to `bits` bits (or the unfolded code image when conv.enabled); rows `pitch` bytes apart,
-// pitch a multiple of 16 and >= M, columns m >= M are written as 0
+// pitch a multiple of 16 and >= M, columns m >= M are written as 0.  `zero` (optional): words to set to zero in the same launch.
 int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, const ConvGeom &conv, int bits,
-                    cudaStream_t stream);
+                    uint32_t *zero, long zero_words, cudaStream_t stream);
 
 // quantisation prologue / epilogue of an approximate convolution layer (lutgemm_quant.cu); strides in elements
 int quantize_codes(const float *x, long sb, long sc, long sh, long sw, int B, int C, int H, int W, const float *scale,
                    const float *zp_neg, float qmax, uint8_t *codes, float *chansum, int num_sms, cudaStream_t stream);
+// codes and channel sums of the activations, codes and tap sums of the weights of a layer; quant = {s_a, z_a, s_w, z_w}
+int layer_prep(const float *x, long sb, long sc, long sh, long sw, int B, int C, int H, int W, float a_qmax, const float *weight,
+               long s_co, long s_c, long s_h, long s_w, int Cout, int kh, int kw, float w_qmax, const float *quant, uint8_t *codes,
+               float *chansum, uint8_t *wmat, float *wsum, int num_sms, cudaStream_t stream);
 int quantize_backward(const float *x, long sb, long sc, long sh, long sw, int B, int C, int H, int W, const float *scale,
                       const float *zp_neg, float qmax, const float *gcodes, const float *boxT, const float *s_w,
                       const float *z_w, float *gx, int num_sms, cudaStream_t stream);
@@ -253,6 +258,9 @@ int layer_weight_prep(const float *weight, long s_co, long s_c, long s_h, long s
 int layer_cross_terms(const float *wsum, int Cout, const ConvGeom &g, float *sumw_t, float *taps, int num_sms,
                       cudaStream_t stream);
 int layer_window_sum(const float *img, const ConvGeom &g, float *box, int num_sms, cudaStream_t stream);
+// the last two in one launch
+int layer_sums(const float *wsum, int Cout, const ConvGeom &g, float *sumw_t, float *taps, const float *img, float *box, int num_sms,
+               cudaStream_t stream);
 int layer_window_sum_adjoint(const float *gsum, const ConvGeom &g, float *out, int num_sms, cudaStream_t stream);
 int layer_weight_grad_finish(const float *gwmat, const float *tapg, const float *weight, long s_co, long s_c, long s_h,
                              long s_w, int Cout, int Cin, int kh, int kw, const float *quant, float qmax, float *gw,

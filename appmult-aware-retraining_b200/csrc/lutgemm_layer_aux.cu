@@ -15,16 +15,12 @@
 //                      clamp mask, activation scale (backward of :147-150 for the weight)
 // All scalars live in device memory: no call synchronises with the host.
 #include "lutgemm.h"
-#include "lutgemm_common.cuh"
+#include "lutgemm_codes.cuh"
 #include "lutgemm_kernels.h"
 
 namespace lutgemm {
 
 namespace {
-
-__device__ __forceinline__ float code_of(float x, const Divisor &scale, float zp_neg) {
-    return rintf(__fsub_rn(quotient(x, scale), zp_neg));  // two roundings, as x / scale - zp in PyTorch
-}
 
 // one thread: the layer's observers and quantisation parameters
 __global__ void update_ranges_kernel(const float *act_lo, const float *act_hi, const float *w_lo, const float *w_hi,
@@ -50,64 +46,10 @@ __global__ void update_ranges_kernel(const float *act_lo, const float *act_hi, c
     quant[3] = rintf(__fdiv_rn(wmin, s_w));
 }
 
-// One block per CO output channels: codes of weight[co, :, :, :] (any strides) written as columns of wmat[K, Cout], K
-// ordered (cin, kh, kw); wsum[co, t] = sum over cin of the codes of tap t.  A thread handles one k of all CO channels, so
-// its reads are independent of each other and its codes leave in one CO-byte store; the sums are integers (exact in any
-// order; shared-memory atomics are native for integers only), added up inside the warp first where there is one tap.
-// 384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> 4.2 us.
 template <int CO>
-__global__ void __launch_bounds__(512) weight_prep_kernel(const float *__restrict__ weight, long s_co, long s_c, long s_h,
-                                                          long s_w, int Cout, int Cin, int kh, int kw,
-                                                          const float *__restrict__ quant, float qmax,
-                                                          uint8_t *__restrict__ wmat, float *__restrict__ wsum, int vec) {
+__global__ void __launch_bounds__(512) weight_prep_kernel(const WeightPrep w) {
     extern __shared__ uint32_t tap_sum[];  // [CO][kh*kw]
-    const int T = kh * kw, K = Cin * T, co0 = blockIdx.x * CO, lane = threadIdx.x & 31;
-    const Divisor scale = make_divisor(quant[2]);
-    const float zp = quant[3];
-    for (int t = threadIdx.x; t < CO * T; t += blockDim.x) tap_sum[t] = 0u;
-    __syncthreads();
-    for (int k0 = 0; k0 < K; k0 += blockDim.x) {  // (whole warps: the sum over the warp below needs every lane)
-        const int k = k0 + threadIdx.x;
-        uint32_t q[CO];
-        int t = 0;
-        if (k < K) {
-            const int c = k / T;
-            t = k - c * T;
-            const int i = t / kw, j = t - i * kw;
-            const float *src = weight + co0 * s_co + c * s_c + i * s_h + j * s_w;
-            float x[CO];
-#pragma unroll
-            for (int e = 0; e < CO; ++e) x[e] = co0 + e < Cout ? src[e * s_co] : 0.f;
-#pragma unroll
-            for (int e = 0; e < CO; ++e)
-                q[e] = (uint32_t)(uint8_t)fminf(fmaxf(code_of(x[e], scale, zp), 0.f), qmax);
-            uint8_t *dst = wmat + (size_t)k * Cout + co0;
-            if (CO == 8 && vec) {
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(q[0] | q[1 % CO] << 8 | q[2 % CO] << 16 | q[3 % CO] << 24,
-                                                             q[4 % CO] | q[5 % CO] << 8 | q[6 % CO] << 16 | q[7 % CO] << 24);
-            } else {
-#pragma unroll
-                for (int e = 0; e < CO; ++e)
-                    if (co0 + e < Cout) dst[e] = (uint8_t)q[e];
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < CO; ++e) q[e] = 0u;
-        }
-        if (T == 1) {
-#pragma unroll
-            for (int e = 0; e < CO; ++e) {
-                const uint32_t sum = __reduce_add_sync(0xffffffffu, q[e]);
-                if (lane == 0) atomicAdd(&tap_sum[e], sum);
-            }
-        } else if (k < K) {
-#pragma unroll
-            for (int e = 0; e < CO; ++e) atomicAdd(&tap_sum[e * T + t], q[e]);
-        }
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < CO * T; t += blockDim.x)
-        if (co0 + t / T < Cout) wsum[(size_t)co0 * T + t] = (float)tap_sum[t];
+    weight_prep_columns<CO>(w, blockIdx.x, tap_sum);
 }
 
 __device__ __forceinline__ bool tap_inside(const ConvGeom &g, int oh, int ow, int i, int j) {
@@ -116,11 +58,11 @@ __device__ __forceinline__ bool tap_inside(const ConvGeom &g, int oh, int ow, in
 }
 
 // sumw_t[l, co] = sum over the taps inside the image at output position l of wsum[co, t] (ascending t);
-// taps[l] = Cin * number of those taps
-__global__ void __launch_bounds__(256) cross_terms_kernel(const float *__restrict__ wsum, int Cout, const ConvGeom g,
-                                                          float *__restrict__ sumw_t, float *__restrict__ taps) {
+// taps[l] = Cin * number of those taps.  By `threads` threads, of which this is `first`.
+__device__ __forceinline__ void cross_terms(const float *__restrict__ wsum, int Cout, const ConvGeom &g, float *__restrict__ sumw_t,
+                                            float *__restrict__ taps, long first, long threads) {
     const int L = g.Ho * g.Wo, T = g.kh * g.kw;
-    for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < (long)L * Cout; idx += (long)gridDim.x * blockDim.x) {
+    for (long idx = first; idx < (long)L * Cout; idx += threads) {
         const int l = (int)(idx / Cout), co = (int)(idx - (long)l * Cout), oh = l / g.Wo, ow = l - oh * g.Wo;
         float s = 0.f;
         int n = 0;
@@ -130,12 +72,16 @@ __global__ void __launch_bounds__(256) cross_terms_kernel(const float *__restric
         if (co == 0) taps[l] = (float)n * (float)g.C;
     }
 }
+__global__ void __launch_bounds__(256) cross_terms_kernel(const float *__restrict__ wsum, int Cout, const ConvGeom g,
+                                                          float *__restrict__ sumw_t, float *__restrict__ taps) {
+    cross_terms(wsum, Cout, g, sumw_t, taps, blockIdx.x * 256L + threadIdx.x, gridDim.x * 256L);
+}
 
 // box[(b*Ho + oh)*Wo + ow] = sum over the taps inside the image of img[b, ih, iw]   (ascending tap order)
-__global__ void __launch_bounds__(256) window_sum_kernel(const float *__restrict__ img, const ConvGeom g,
-                                                         float *__restrict__ box) {
+__device__ __forceinline__ void window_sums(const float *__restrict__ img, const ConvGeom &g, float *__restrict__ box, long first,
+                                            long threads) {
     const long M = (long)g.B * g.Ho * g.Wo;
-    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < M; m += (long)gridDim.x * blockDim.x) {
+    for (long m = first; m < M; m += threads) {
         const int ow = (int)(m % g.Wo), oh = (int)((m / g.Wo) % g.Ho);
         const long b = m / ((long)g.Wo * g.Ho);
         const float *src = img + b * g.H * g.W;
@@ -150,6 +96,20 @@ __global__ void __launch_bounds__(256) window_sum_kernel(const float *__restrict
         }
         box[m] = s;
     }
+}
+__global__ void __launch_bounds__(256) window_sum_kernel(const float *__restrict__ img, const ConvGeom g,
+                                                         float *__restrict__ box) {
+    window_sums(img, g, box, blockIdx.x * 256L + threadIdx.x, gridDim.x * 256L);
+}
+// both in one launch, the first `cross` blocks for the cross terms: neither fills the GPU in a network of small batches, and a launch
+// costs more of the host's time than either of the GPU's (4 us each for 16 images of 32 x 32)
+__global__ void __launch_bounds__(256) layer_sums_kernel(const float *__restrict__ wsum, int Cout, const ConvGeom g,
+                                                         float *__restrict__ sumw_t, float *__restrict__ taps,
+                                                         const float *__restrict__ img, float *__restrict__ box, int cross) {
+    if ((int)blockIdx.x < cross)
+        cross_terms(wsum, Cout, g, sumw_t, taps, blockIdx.x * 256L + threadIdx.x, cross * 256L);
+    else
+        window_sums(img, g, box, (blockIdx.x - cross) * 256L + threadIdx.x, (gridDim.x - cross) * 256L);
 }
 
 // out[b, h, w] = sum over the taps (i, j) that connect (h, w) to an output position of gsum[b, oh, ow]
@@ -213,14 +173,14 @@ int layer_update_ranges(const float *act_lo, const float *act_hi, const float *w
 
 int layer_weight_prep(const float *weight, long s_co, long s_c, long s_h, long s_w, int Cout, int Cin, int kh, int kw,
                       const float *quant, float qmax, uint8_t *wmat, float *wsum, cudaStream_t stream) {
-    const int T = kh * kw, K = Cin * T, threads = K >= 512 ? 512 : (K + 31) / 32 * 32;
+    const int T = kh * kw, split = weight_prep_split(s_c, s_w, T), K = split ? Cin : Cin * T;
+    const int threads = K >= 512 ? 512 : (K + 31) / 32 * 32, blocks = split ? T : 1;
+    WeightPrep w{weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw, quant, qmax, wmat, wsum, 0, split};
     if (T <= 512) {  // (the sums of eight channels have to fit shared memory)
-        const int vec = Cout % 8 == 0 && (reinterpret_cast<uintptr_t>(wmat) & 7) == 0;
-        weight_prep_kernel<8><<<(Cout + 7) / 8, threads, 8 * T * sizeof(uint32_t), stream>>>(
-            weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw, quant, qmax, wmat, wsum, vec);
+        w.vec = Cout % 8 == 0 && (reinterpret_cast<uintptr_t>(wmat) & 7) == 0;
+        weight_prep_kernel<8><<<(Cout + 7) / 8 * blocks, threads, 8 * T * sizeof(uint32_t), stream>>>(w);
     } else {
-        weight_prep_kernel<1><<<Cout, threads, T * sizeof(uint32_t), stream>>>(weight, s_co, s_c, s_h, s_w, Cout, Cin, kh, kw,
-                                                                             quant, qmax, wmat, wsum, 0);
+        weight_prep_kernel<1><<<Cout * blocks, threads, T * sizeof(uint32_t), stream>>>(w);
     }
     return launch_status();
 }
@@ -233,6 +193,13 @@ int layer_cross_terms(const float *wsum, int Cout, const ConvGeom &g, float *sum
 
 int layer_window_sum(const float *img, const ConvGeom &g, float *box, int num_sms, cudaStream_t stream) {
     window_sum_kernel<<<grid_for((long)g.B * g.Ho * g.Wo, num_sms), 256, 0, stream>>>(img, g, box);
+    return launch_status();
+}
+
+int layer_sums(const float *wsum, int Cout, const ConvGeom &g, float *sumw_t, float *taps, const float *img, float *box, int num_sms,
+               cudaStream_t stream) {
+    const int cross = grid_for((long)g.Ho * g.Wo * Cout, num_sms);
+    layer_sums_kernel<<<cross + grid_for((long)g.B * g.Ho * g.Wo, num_sms), 256, 0, stream>>>(wsum, Cout, g, sumw_t, taps, img, box, cross);
     return launch_status();
 }
 

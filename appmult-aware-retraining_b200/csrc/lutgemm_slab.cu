@@ -486,7 +486,7 @@ int slab_fwd_ksplits(int M, int K, int N, int num_sms) {
 
 template <int BITS>
 static int launch_fwd_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t *lut, int M, int K, int N,
-                           const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, int num_sms,
+                           const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, bool zeroed, int num_sms,
                            cudaStream_t stream) {
     using C = sf::Cfg<BITS>;
     // operand chunks by bulk-tensor copies where the transposed copy exists and w keeps the copy engine's alignment
@@ -518,7 +518,7 @@ static int launch_fwd_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, cons
     p.share = !epi && slab_fwd_ksplits(M, K, N, num_sms) > 1;
     const long units = p.share ? tiles * kchunks : tiles;
     const int grid = (int)(units < num_sms ? units : num_sms);
-    if (p.share && !cuda_ok(cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(uint32_t), stream)))
+    if (p.share && !zeroed && !cuda_ok(cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(uint32_t), stream)))
         return LUTGEMM_E_CUDA;
     p.vec_a = !conv.enabled && (K % 16 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
     p.vec_w = (N % 16 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
@@ -529,13 +529,13 @@ static int launch_fwd_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, cons
 }
 
 int forward_slab(const uint8_t *a, const uint8_t *w, uint32_t *c, const uint16_t *lut, int bits, int M, int K, int N,
-                 const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, int num_sms,
+                 const ConvGeom &conv, const uint8_t *at, int at_pitch, const LayerEpilogue *epi, bool zeroed, int num_sms,
                  cudaStream_t stream) {
     switch (bits) {
-        case 4: return launch_fwd_slab<4>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, num_sms, stream);
-        case 6: return launch_fwd_slab<6>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, num_sms, stream);
-        case 7: return launch_fwd_slab<7>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, num_sms, stream);
-        case 8: return launch_fwd_slab<8>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, num_sms, stream);
+        case 4: return launch_fwd_slab<4>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, zeroed, num_sms, stream);
+        case 6: return launch_fwd_slab<6>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, zeroed, num_sms, stream);
+        case 7: return launch_fwd_slab<7>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, zeroed, num_sms, stream);
+        case 8: return launch_fwd_slab<8>(a, w, c, lut, M, K, N, conv, at, at_pitch, epi, zeroed, num_sms, stream);
     }
     return LUTGEMM_E_BITS;
 }

@@ -81,3 +81,31 @@ def test_dequantisation(dev, M, L, Cout, with_bias):
     acc = y.float() + (z_w * box)[:, None] + z_a * sumw[l] + ((z_a * z_w) * taps[l])[:, None]
     want = (s_a * s_w) * acc
     assert torch.equal(out, want + bias if with_bias else want)
+
+
+@pytest.mark.parametrize("B,C,H,W,Cout,k,s,p", [(2, 64, 8, 8, 64, 3, 1, 1), (1, 4, 1, 1, 8, 1, 1, 0), (3, 132, 7, 7, 20, 3, 2, 1), (1, 516, 3, 5, 9, 1, 1, 0), (40, 516, 14, 14, 16, 3, 1, 1),
+                                                (2, 68, 9, 9, 40, 5, 1, 2), (2, 3, 9, 9, 24, 3, 1, 1), (1, 4, 30, 30, 8, 23, 1, 0)])
+@pytest.mark.parametrize("channels_last", [False, True])
+def test_prologue_of_a_layer_in_one_launch(dev, B, C, H, W, Cout, k, s, p, channels_last):
+    """One call against the entry points that it joins: all of them whole numbers until the last, so the results are equal."""
+    import approx_ops
+    import self_ops
+    from lutgemm_luts import synthetic_multiplier, window_difference_gradients
+    from self_ops.ops_py import approx_ops as state
+    fp = synthetic_multiplier(7, seed=0)
+    self_ops.set_lookup_tables(dev, fp, *window_difference_gradients(fp, 8), 7)
+    gen = torch.Generator(device=dev).manual_seed(C + Cout)
+    fmt = torch.channels_last if channels_last else torch.contiguous_format
+    x = torch.randn(B, C, H, W, generator=gen, device=dev).contiguous(memory_format=fmt)
+    weight = torch.randn(Cout, C, k, k, generator=gen, device=dev).contiguous(memory_format=fmt)
+    quant = torch.tensor([0.04, -50.0, 0.03, -61.0], device=dev)
+    s_a, z_a, s_w, z_w = (quant[i:i + 1] for i in range(4))
+    codes, chansum = approx_ops.quantize_activations(x, s_a, z_a, 127.0)
+    wq = torch.clamp(torch.round(weight / s_w - z_w), 0, 127.0)
+    wmat, wsum = approx_ops.layer_weight_prep(weight, quant, 127.0)
+    assert torch.equal(wmat.float(), wq.reshape(Cout, -1).t()) and torch.equal(wsum.view(Cout, -1), wq.sum(dim=1).reshape(Cout, -1))
+    sumw_t, taps = approx_ops.layer_cross_terms(wsum, C, H, W, k, k, s, p, 1)
+    box = approx_ops.layer_window_sum(chansum, k, k, s, p, 1)
+    out, _ = approx_ops.approx_conv2d_forward_layer(codes, wmat, state.lut_appmult, k, k, s, p, 1, box, sumw_t, taps, s_a, s_w, z_a, z_w, None)
+    got = approx_ops.conv2d_layer_pass(x, weight, None, quant, 127.0, 127.0, state.lut_appmult, s, p, 1)
+    assert torch.equal(got[0].reshape(out.shape), out) and torch.equal(got[1], codes) and torch.equal(got[2], wmat)
