@@ -91,6 +91,8 @@ def _load():
     lib.lutgemm_layer_window_sum.argtypes = [vp] + [ci] * 8 + [vp, vp]
     lib.lutgemm_layer_window_sum_adjoint.restype = ci
     lib.lutgemm_layer_window_sum_adjoint.argtypes = [vp] + [ci] * 8 + [vp, vp]
+    lib.lutgemm_layer_row_sums.restype = ci
+    lib.lutgemm_layer_row_sums.argtypes = [vp, cl, ci, vp, vp]
     lib.lutgemm_layer_weight_grad.restype = ci
     lib.lutgemm_layer_weight_grad.argtypes = [vp, vp, vp, cl, cl, cl, cl, ci, ci, ci, ci, vp, cf, vp, vp]
     lib.lutgemm_conv2d_forward_layer_scratch_bytes.restype = sz
@@ -685,6 +687,19 @@ def layer_window_sum_adjoint(gsum: torch.Tensor, H: int, W: int, kh: int, kw: in
                                                       _stream_ptr(gsum.device))
     _check(rc, "layer_window_sum_adjoint")
     return out
+
+
+def layer_row_sums(g: torch.Tensor) -> torch.Tensor:
+    """[M, N] f32 -> [M] f32: sums of the rows."""
+    _check_input(g, torch.float32, "grad_output_tensor")
+    M, N = g.shape
+    if M == 0 or N == 0:
+        return torch.zeros(M, dtype=torch.float32, device=g.device)
+    sums = torch.empty(M, dtype=torch.float32, device=g.device)
+    with _guard(g.device):
+        rc = _load().lutgemm_layer_row_sums(g.data_ptr(), M, N, sums.data_ptr(), _stream_ptr(g.device))
+    _check(rc, "layer_row_sums")
+    return sums
 
 
 def layer_weight_grad(gwmat: torch.Tensor, tapg: torch.Tensor, weight: torch.Tensor, quant: torch.Tensor, qmax: float):

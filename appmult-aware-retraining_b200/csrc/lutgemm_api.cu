@@ -1028,6 +1028,13 @@ int lutgemm_layer_window_sum_adjoint(const float *gsum, int B, int H, int W, int
     return lutgemm::layer_window_sum_adjoint(gsum, g, out, sms, static_cast<cudaStream_t>(stream));
 }
 
+int lutgemm_layer_row_sums(const float *g, long M, int N, float *sums, void *stream) {
+    if (!g || !sums || M <= 0 || N <= 0) return LUTGEMM_E_BADARG;
+    const int sms = current_num_sms();
+    if (sms <= 0) return LUTGEMM_E_CUDA;
+    return lutgemm::layer_row_sums(g, M, N, sums, sms, static_cast<cudaStream_t>(stream));
+}
+
 int lutgemm_layer_weight_grad(const float *gwmat, const float *tapg, const float *weight, long s_co, long s_c, long s_h,
                               long s_w, int Cout, int Cin, int kh, int kw, const float *quant, float qmax, float *gw,
                               void *stream) {

@@ -262,6 +262,7 @@ int layer_window_sum(const float *img, const ConvGeom &g, float *box, int num_sm
 int layer_sums(const float *wsum, int Cout, const ConvGeom &g, float *sumw_t, float *taps, const float *img, float *box, int num_sms,
                cudaStream_t stream);
 int layer_window_sum_adjoint(const float *gsum, const ConvGeom &g, float *out, int num_sms, cudaStream_t stream);
+int layer_row_sums(const float *g, long M, int N, float *sums, int num_sms, cudaStream_t stream);
 int layer_weight_grad_finish(const float *gwmat, const float *tapg, const float *weight, long s_co, long s_c, long s_h,
                              long s_w, int Cout, int Cin, int kh, int kw, const float *quant, float qmax, float *gw,
                              int num_sms, cudaStream_t stream);

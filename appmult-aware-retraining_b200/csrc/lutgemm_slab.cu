@@ -1,4 +1,5 @@
-// Forward LUT-GEMM for sm_100a, "column-gathered slab" kernel (large M):
+// Forward LUT-GEMM for sm_100a, "column-gathered slab" kernel with tiles of 512 x 64 (where tiles of 1024 x 32, lutgemm_forward_rows.cu,
+// leave the GPU emptier: few rows or a short K; without a workspace; small problems):
 //     c[m,n] = sum_k LUT[a[m,k]][w[k,n]]        exact uint32 accumulate
 //
 // A warp-wide table gather whose 32 column indices are random costs ~2.8 shared-memory wavefronts at

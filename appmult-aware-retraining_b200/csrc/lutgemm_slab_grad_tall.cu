@@ -17,8 +17,9 @@
 // Partial sums: one per lane, warp and k; the 16 warps are added in ascending order by one warp (rotating
 // with k), row blocks by slab_reduce_blocks in ascending order: results are deterministic.
 // grad_w takes its row codes from a transposed copy at[k][m] of the activation codes when the caller has one.
-// Used at 8 bits, where the slab build weighs most and its 1024 rows halve it (4096^3: 13.33 and 13.47 ms for grad_w and
-// grad_a, against 15.0 and 15.5 ms with the packed slab of lutgemm_slab_grad.cu), for short K, and for fp32 tables.
+// Used where its 1024-row tiles are filled and the 512-row tiles of lutgemm_slab_rows.cu are not worth their block overhead (64 x 256 x
+// 56 x 56 with 64 outputs, 1x1, 8 bits: grad_w 0.72 ms; 4096^3 at 8 bits takes 13.33 and 13.47 ms here, 10.95 and 11.02 ms there), for
+// short K, and for fp32 tables.
 // Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492.
 #include <type_traits>
 

@@ -318,6 +318,7 @@ int lutgemm_forward_layer(const uint8_t *a, const uint8_t *w, const uint16_t *lu
  * lutgemm_layer_window_sum: box[b, oh, ow] = sum of img[b, ., .] over the kernel window (zero padding), img the
  *   channel sums of the activation codes (the convolution with a constant weight of :178).
  * lutgemm_layer_window_sum_adjoint: out[b, h, w] = sum of gsum[b, oh, ow] over the windows that contain (h, w).
+ * lutgemm_layer_row_sums: sums[m] = sum over n of g[m, n], a contiguous fp32 matrix: the gradient of the z_w-terms.
  * lutgemm_layer_weight_grad: gw[co,c,i,j] = [0 <= round(weight/s_w - z_w) <= qmax] * s_a *
  *   (gwmat[(c*kh+i)*kw+j, co] + z_a * tapg[co, i*kw+j]), gw contiguous.
  */
@@ -333,6 +334,7 @@ int lutgemm_layer_window_sum(const float *img, int B, int H, int W, int kh, int 
                              float *box, void *stream);
 int lutgemm_layer_window_sum_adjoint(const float *gsum, int B, int H, int W, int kh, int kw, int stride, int pad, int dil,
                                      float *out, void *stream);
+int lutgemm_layer_row_sums(const float *g, long M, int N, float *sums, void *stream);
 int lutgemm_layer_weight_grad(const float *gwmat, const float *tapg, const float *weight, long s_co, long s_c, long s_h,
                               long s_w, int Cout, int Cin, int kh, int kw, const float *quant, float qmax, float *gw,
                               void *stream);

@@ -109,3 +109,14 @@ def test_prologue_of_a_layer_in_one_launch(dev, B, C, H, W, Cout, k, s, p, chann
     out, _ = approx_ops.approx_conv2d_forward_layer(codes, wmat, state.lut_appmult, k, k, s, p, 1, box, sumw_t, taps, s_a, s_w, z_a, z_w, None)
     got = approx_ops.conv2d_layer_pass(x, weight, None, quant, 127.0, 127.0, state.lut_appmult, s, p, 1)
     assert torch.equal(got[0].reshape(out.shape), out) and torch.equal(got[1], codes) and torch.equal(got[2], wmat)
+
+
+@pytest.mark.parametrize("M,N", [(1, 1), (3, 2), (7, 33), (1001, 5), (517, 4), (130, 8), (65, 60), (4099, 64), (33, 132), (5, 1536), (9, 777), (200000, 12)])
+def test_row_sums(dev, M, N):
+    """|error| <= (4 + ceil(N / 128) + 5) * 2^-24 * sum |g|: four values of a vector, a lane's vectors one after the other (single
+    values where N is odd: ceil(N / 32) of them), five halvings of a warp."""
+    import approx_ops
+    g = torch.randn(M, N, generator=torch.Generator(device=dev).manual_seed(N), device=dev)
+    want = g.double().sum(dim=1)
+    bound = (9 + -(-N // 32)) * 2.0 ** -24 * g.double().abs().sum(dim=1)
+    assert bool(((approx_ops.layer_row_sums(g).double() - want).abs() <= bound).all())
