@@ -67,11 +67,11 @@ struct BackwardPlan {
 // ---- estimated times of the kernel families, in SM clocks --------------------------------------------------------
 // Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
 // The clocks are measured on B200, at 4096^3 unless said otherwise:
-//   slab kernels, per k and tile      packed 512 x 64: grad_w 1440 (4 bits), 1300 (6), 1305 (7), 1950 (8), grad_a and grad_x
-//                                     1390, 1225, 1290, 1965; tall 1024 x 32: 1540, 1690, 1880;
+//   slab kernels, per k and tile      packed 512 x 64: grad_w 1275 (4 bits), 1315 (6), 1365 (7), 1945 (8), grad_a and grad_x
+//                                     1290, 1320, 1390, 2055; tall 1024 x 32: 1540, 1690, 1880;
 //                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
 //                                     more launches: code transposition, zeroing, and a layer's epilogue);
-//   a thread per row                  gradients 512 x 64: 1420 (4 bits), 1070 (6), 1150 (7), 1390 (8) per k, 9e3 per block of
+//   a thread per row                  gradients 512 x 64: 1185 (4 bits), 1210 (6 and 7), 1490 (8) per k, 9e3 per block of
 //                                     grad_out values (27e3 where they come one by one); forward 1024 x 32: 650, 690, 845
 //   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
 //                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.66, 1.72, 2.2
@@ -83,10 +83,10 @@ struct FamilyClocks {
     double packed_gw, packed, tall, fwd_slab, fwd_bcast, gw_bcast, ga_bcast, gx_bcast, fwd_start, rows, fwd_rows;
 };
 FamilyClocks family_clocks(int bits) {
-    if (bits == 8) return {1950, 1965, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1390, 845};
-    if (bits == 7) return {1305, 1290, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1150, 690};
-    if (bits == 6) return {1300, 1225, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1070, 650};
-    return {1440, 1390, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1420, 650};
+    if (bits == 8) return {1945, 2055, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1490, 845};
+    if (bits == 7) return {1365, 1390, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1210, 690};
+    if (bits == 6) return {1315, 1320, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1210, 650};
+    return {1275, 1290, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1185, 650};
 }
 constexpr double kBcastStart = 12e3, kSlabStart = 10e3;
 constexpr double kReduceBytesPerClock = 4000;  // reading and writing partial sums, whole GPU

@@ -33,10 +33,6 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-// the two unsigned entries of a slab word times 2^-149: as the bits of a float an integer below 2^23 is a subnormal number
-__device__ __forceinline__ f32x2 tiny2(uint32_t word) {
-    return pack2(__uint_as_float(__byte_perm(word, 0u, 0x4410)), __uint_as_float(__byte_perm(word, 0u, 0x4432)));
-}
 // the two signed table entries of a slab word: 0x4B000000 | u is the float 2^23 + u, u = entry + 2^15
 __device__ __forceinline__ f32x2 entries2(uint32_t word, f32x2 bias) {
     const float lo = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7610));

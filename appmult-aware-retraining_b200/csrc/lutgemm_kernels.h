@@ -81,7 +81,7 @@ constexpr int kPackedGwOverhead = 5, kPackedItemOverhead = 10, kTallItemOverhead
 
 // rows of the reduction dimension per CTA tile of the packed-slab gradient kernels
 constexpr int kSlabPackedRows = 512;
-constexpr double kPacked576Step = 1.37;  // time of a k step with 576 rows (72 registers of values leave none for the faster form)
+constexpr double kPacked576Step = 1.13;  // time of a k step with 576 rows
 // How the packed gradient kernels deal out their work.  The row blocks of a column tile are cut into groups of
 // group_blocks; one CTA adds up a group's blocks in turn, so a group needs one block of partial sums.  A cell is (group,
 // column tile): the first main_cells of them, whole rounds of the persistent grid, are taken with their whole K, the

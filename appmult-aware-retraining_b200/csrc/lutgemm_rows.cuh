@@ -67,48 +67,6 @@ __device__ __forceinline__ void stage_table_plain(uint8_t *table, const uint16_t
     }
 }
 
-// Gradient tables are staged in offset-binary, entry + 2^15.  Where the least entry is not far below zero (-4 min <= max: products
-// of operands and their slopes), the offset becomes the least that leaves entries unsigned, so that their bits can be used
-// as subnormal floats (`small`); the offset's share of a sum comes off at the end.  Beyond that line rounding errors of the
-// shared offset would show in the sums.  `range` (two words of shared memory) = {0xffff, 0} on entry, visible to all; the
-// table has been written and is complete after the caller's next barrier.
-template <int BITS>
-__device__ __forceinline__ int reduce_table_offset(uint8_t *table, uint32_t *range, int tid, bool *small) {
-    using T = RowsTable<BITS>;
-    constexpr int Q = T::Q, THREADS = 512;
-    auto word = [&](int idx) -> uint32_t & { return *reinterpret_cast<uint32_t *>(table + idx / (Q / 2) * T::ROW + idx % (Q / 2) * 4); };
-    uint32_t lo = 0xffffu, hi = 0u;
-#pragma unroll 4
-    for (int idx = tid; idx < Q * Q / 2; idx += THREADS) {
-        const uint32_t v = word(idx);
-        lo = min(lo, min(v & 0xffffu, v >> 16));
-        hi = max(hi, max(v & 0xffffu, v >> 16));
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((tid & 31) == 0) {
-        atomicMin(range, lo);
-        atomicMax(range + 1, hi);
-    }
-    __syncthreads();
-    const int least = min(0, (int)range[0] - 32768), most = (int)range[1] - 32768;
-    *small = -4 * least <= most;
-    if (!*small) return 32768;
-#pragma unroll 4
-    for (int idx = tid; idx < Q * Q / 2; idx += THREADS) word(idx) -= (32768u + least) * 0x10001u;
-    return -least;
-}
-
-// For values of which the largest magnitude is m: a power of two that brings them to about 2^100, or 2^127 where that is less, and
-// what takes it, and the 2^-149 of an entry used as a subnormal float, back out of a product.  `ok`: m (and with it every product)
-// stays in the range of ordinary numbers; otherwise, and with infinities or NaN (`sum` of the values), the other form is used.
-__device__ __forceinline__ void subnormal_scale(float m, float sum, float *up, float *down, bool *ok) {
-    *ok = m < 0x1p60f && (m == 0.f || m >= 0x1p-60f) && sum == sum;
-    const int e = min(127, 227 - (int)(__float_as_uint(m) >> 23));
-    *up = __uint_as_float((uint32_t)(e + 127) << 23);
-    *down = __uint_as_float((uint32_t)(149 - e + 127) << 23);
-}
-
 // A thread's share of a slab build by 512 threads: four columns (quad bq) x eight codes (16 bytes of a table row; four codes at
 // 6 bits, one at 4).  One step builds a slab at 8 bits, two at fewer.  The lanes are staggered over the table rows' chunks, so
 // that reads are free of bank conflicts whatever the column codes are, and a half-warp stores sixteen different quads.

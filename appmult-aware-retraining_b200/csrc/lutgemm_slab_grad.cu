@@ -17,15 +17,16 @@
 // strided convolution is cut into stride^2 classes of input pixels that each see a fixed subset of the taps.
 //
 // What bounds it: instruction issue (four per clock, packed fp32 instructions count twice) and the shared-memory pipe (one
-// 128-byte wavefront per clock).  The slab keeps the table's own 16 bits per entry, so a look-up costs half the wavefronts
-// of an fp32 slab; the price is the conversion at each use.  It is done for two entries at a time: two byte permutations
-// make them subnormal floats, and one packed multiply-add (fma.rn.f32x2) consumes them, with grad_out scaled by a
-// power of two per thread and the table's offset taken out of the thread's partial sum (lutgemm_rows.cuh).  Tables and values that this
-// does not suit, and 576-row tiles, put each entry behind the exponent of 2^23 and subtract in between: 8 against 10
-// instructions per 128 look-ups of a warp.  Products and sums are the same fp32 operations either way.
-// With one barrier per unit and the staggered slab build of lutgemm_rows.cuh, against the subtraction, two barriers per unit and padded
-// slab rows (grad_w, grad_a): 4096^3 at 7 bits 10.50, 11.12 -> 9.13, 9.07 ms, 6 bits 9.89, 10.71 -> 8.72, 8.50, 8 bits 15.19, 15.18 ->
-// 14.18, 13.70; 262144 x 576 x 64 at 7 bits, grad_w 1.51 -> 1.34 ms.
+// 128-byte wavefront per clock): 7 bits, grad_w of 4096 x 512 x 4096, per k and tile 3690 instructions, 1060 of them packed, and 980
+// wavefronts in 1360 clocks; 8 bits 4860, 1335 and 1935.  The slab keeps the table's own 16 bits per entry, so a look-up costs half the
+// wavefronts of an fp32 slab; the price is the conversion at each use.  It is done for two entries at a time: each 16-bit half goes, in
+// offset-binary, behind the exponent of 2^23 (one byte permutation), one packed subtraction of 2^23 + 2^15 leaves the two signed entries
+// exactly, and one packed multiply-add (fma.rn.f32x2) consumes them - 10 instructions per 128 look-ups of a warp
+// against 8 with an fp32 slab, but 512 + build instead of 1024 + build wavefronts per 32768 look-ups.  Products and
+// sums are the same fp32 operations as with an fp32 slab.
+// With one barrier per unit and the staggered slab build of lutgemm_rows.cuh, against two barriers per unit and padded slab rows
+// (grad_w, grad_a): 4096^3 at 7 bits 10.50, 11.12 -> 9.99, 10.09 ms, 6 bits 9.89, 10.71 -> 9.62, 9.63, 8 bits 15.19, 15.18 -> 14.15, 14.95;
+// 262144 x 576 x 64 at 7 bits, grad_w 1.51 -> 1.46 ms.
 //
 // Hand-over between the warps of a CTA: at 7 bits and below three buffers of two slabs each and one mbarrier per buffer
 // (lutgemm_slab_rows.cu); at 8 bits shared memory has room for two slabs, with a "full" and an "empty" mbarrier each, one arrival per
@@ -74,7 +75,7 @@ struct Cfg {
     static constexpr int OFF_PIX = OFF_PART + NB * KP * P_FLOATS * 4;  // (a set of sums per buffer)  grad_x: image offset of each column
     static constexpr int OFF_TAP = OFF_PIX + CT * 8;                  // grad_x: output offset {rows, columns} of each tap
     static constexpr int OFF_BAR = OFF_TAP + kMaxTaps * 8;
-    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 24;   // two mbarriers per buffer, abort word, work item, table range
+    static constexpr int SMEM = OFF_BAR + 2 * NB * 8 + 16;   // two mbarriers per buffer, abort word, work item
     static_assert(T::TURN_BYTES <= OFF_PART - OFF_U, "the table passes through the slab buffers and operand stages");
     static_assert(RW % 4 == 0 && RT % 16 == 0, "rows per warp");
     static_assert(U_BYTES % 16 == 0 && RC_STAGE % 16 == 0 && CC_STAGE % 16 == 0, "16-byte vectors");
@@ -130,18 +131,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
 
     // ---- stage the gradient table in offset-binary; x = row code, y = column code, T(x,y) = lut[a*COL + w] -------
     // (grad_w: rows are activation codes, so the table is turned; grad_a / grad_x: rows are weight codes)
-    uint32_t *range_s = reinterpret_cast<uint32_t *>(work_s + 3);
     const uint16_t *lut = reinterpret_cast<const uint16_t *>(p.lut);
     if (MODE == kGw) stage_table_turned<BITS>(smem, smem + C::OFF_U, lut, 0x80008000u, tid);
     else stage_table_plain<BITS>(smem, lut, 0x80008000u, tid);
-    if (tid == 0) {
-        *abort_word = 0;
-        range_s[0] = 0xffffu;
-        range_s[1] = 0u;
-    }
+    if (tid == 0) *abort_word = 0;
     __syncthreads();
-    bool table_unsigned;
-    const int offset = reduce_table_offset<BITS>(smem, range_s, tid, &table_unsigned);
     // (column codes past the last k: any codes, but codes)
     if (tid < 2 * C::CC_STAGE / 16) reinterpret_cast<uint4 *>(cc_s)[tid] = make_uint4(0, 0, 0, 0);
     if (MODE == kGx) {
@@ -305,8 +299,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
     };
 
-    const float bias1 = -(8388608.0f + (float)offset);
-    const f32x2 bias = pack2(bias1, bias1);
+    const f32x2 bias = pack2(-8421376.0f, -8421376.0f);  // -(2^23 + 2^15)
     const uint32_t wsel0 = (uint32_t)C::U_ROW << (16 * half), wsel1 = wsel0 << 8;  // dot-product weights of the lane's two rows
 
     const int items = p.main_cells + (p.groups * p.tiles_c - p.main_cells) * p.tail_parts;
@@ -321,8 +314,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         }
         if constexpr (MODE != kGx) {
             // the compiler's schedule of the k loop depends on what it sees of these three: read back from shared memory
-            // grad_w takes 1.49 ms for 4096 x 4608 x 512 at 7 bits and grad_a 11.11 ms for 4096^3, straight from the branch
-            // 1.53 and 11.50 (grad_x: the other way round, 6.81 against 6.93 ms at 8 bits for 16 x 256 x 56 x 56, 3x3)
+            // grad_w / grad_a take 10.00 / 10.09 ms for 4096^3 at 7 bits, straight from the branch 10.10 / 10.23 (grad_x: the other way
+            // round, 6.81 against 6.93 ms at 8 bits for 16 x 256 x 56 x 56, 3x3)
             if (tid == 0) { work_s[0] = cell; work_s[1] = kbeg; work_s[2] = kend; }
             __syncthreads();
             cell = work_s[0];
@@ -422,33 +415,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
             }
         }
 
-        // entries as subnormal floats (lutgemm_rows.cuh): scale of the thread's values, what takes it out of their sums, and the
-        // offset's share of the sums, which does not depend on k
-        float up = 1.f, down = 1.f;
-        bool wide = false;
-        f32x2 corr[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
-        constexpr bool MAY = RW <= 32;  // (no registers left in 576-row tiles)
-        if (MAY && table_unsigned) {
-            float m = 0.f;
-#pragma unroll
-            for (int i = 0; i < RW; ++i) {
-                const float2 t = unpack2(g[i]);
-                m = fmaxf(m, fmaxf(fabsf(t.x), fabsf(t.y)));
-                corr[i & 1] = add2(corr[i & 1], g[i]);
-            }
-            const float2 t = unpack2(add2(corr[0], corr[1]));
-            bool ok;
-            subnormal_scale(m, t.x + t.y, &up, &down, &ok);
-            wide = !ok;
-            const f32x2 minus = pack2(-(float)offset, -(float)offset);
-            corr[0] = mul2(corr[0], minus);
-            corr[1] = mul2(corr[1], minus);
-        }
-        const bool fast = !__syncthreads_or(wide) && table_unsigned && MAY;  // (previous item, or the table staging, done with every buffer)
-        if (fast) {
-#pragma unroll
-            for (int i = 0; i < RW; ++i) g[i] = mul2(g[i], pack2(up, up));
-        }
+        __syncthreads();  // previous item (or the table staging) is done with every buffer
         store_stage((kbeg / SC) & 1, 0);
         if (MODE == kGx && tid < CT) pix_s[tid] = (long long)pixel_class_offset(p.px, min(c0 + tid, CDIM - 1));
         if (tid == 0) {
@@ -479,12 +446,11 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         const uint32_t uc = u_addr + cq * 8;
         f32x2 acc[2][2];  // [row parity j][column pair i]
         // rows of code words [QB, QE) of the warp: the lane's columns of the slab at `ua`, row codes of this k at `rbase`
-        auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag, auto fast_tag) {
-            constexpr bool FAST = decltype(fast_tag)::value;
+        auto use_rows = [&](uint32_t ua, const uint8_t *rbase, auto qb_tag, auto qe_tag) {
             constexpr int QB = decltype(qb_tag)::value, QE = decltype(qe_tag)::value, NR = 2 * (QE - QB);
-            // slab reads in flight ahead of their use (4096^3 at 7 bits, grad_w / grad_a: 9.25 / 9.00 ms with 2, 9.29 / 9.14 with 4, 9.19 /
-            // 9.02 with 6, 9.12 / 8.95 with 8)
-            constexpr int PF = RW > 32 ? 4 : 8;
+            // slab reads in flight ahead of their use (4096^3, grad_w / grad_a: 7 bits 10.03 / 10.08 ms with 2, 10.00 / 10.09 with 4, 10.08 /
+            // 10.16 with 6, 10.14 / 10.31 with 8; 8 bits 14.62 / 14.96, 14.16 / 14.96, 14.95 / 14.96, 14.95 / 14.96)
+            constexpr int PF = 4;
             uint32_t rv[QE - QB];
             if constexpr (RW % 16 == 0 && QB % 4 == 0 && QE % 4 == 0) {
 #pragma unroll
@@ -503,7 +469,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 for (int q = 0; q < QE - QB; ++q) rv[q] = reinterpret_cast<const uint32_t *>(rbase + QB * 4)[q];
             }
             uint32_t w0[PF], w1[PF];
-            auto fetch = [&](int i) {  // slab row address = base + 136 * code in one integer dot-product instruction
+            auto fetch = [&](int i) {  // slab row address = base + 128 * code in one integer dot-product instruction
                 asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w0[i % PF]), "=r"(w1[i % PF])
                              : "r"(__dp4a(rv[i >> 1], i & 1 ? wsel1 : wsel0, ua)));
             };
@@ -514,8 +480,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
                 const uint32_t a0 = w0[i % PF], a1 = w1[i % PF];
                 if (i + PF < NR) fetch(i + PF);
                 const int gi = 2 * (2 * QB + i);
-                acc[i & 1][0] = fma2(FAST ? tiny2(a0) : entries2(a0, bias), g[gi], acc[i & 1][0]);
-                acc[i & 1][1] = fma2(FAST ? tiny2(a1) : entries2(a1, bias), g[gi + 1], acc[i & 1][1]);
+                acc[i & 1][0] = fma2(entries2(a0, bias), g[gi], acc[i & 1][0]);
+                acc[i & 1][1] = fma2(entries2(a1, bias), g[gi + 1], acc[i & 1][1]);
             }
         };
         using Q0 = std::integral_constant<int, 0>;
@@ -524,13 +490,8 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         auto clear_acc = [&]() { acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = pack2(0.f, 0.f); };
         // partial sums of one k: row 2 wp + h, the lane's four columns
         float *part_lane = part_s + (2 * wp + half) * CT + 4 * cq;
-        auto store_part = [&](int slot, auto fast_tag) {
-            f32x2 a = add2(acc[0][0], acc[1][0]), b = add2(acc[0][1], acc[1][1]);
-            if (decltype(fast_tag)::value) {
-                a = fma2(a, pack2(down, down), corr[0]);
-                b = fma2(b, pack2(down, down), corr[1]);
-            }
-            const float2 lo = unpack2(a), hi = unpack2(b);
+        auto store_part = [&](int slot) {
+            const float2 lo = unpack2(add2(acc[0][0], acc[1][0])), hi = unpack2(add2(acc[0][1], acc[1][1]));
             *reinterpret_cast<float4 *>(part_lane + slot * C::P_FLOATS) = make_float4(lo.x, lo.y, hi.x, hi.y);
         };
 
@@ -540,67 +501,63 @@ __global__ void __launch_bounds__(512, 1) slab_grad_packed_kernel(const __grid_c
         // until every warp has released the unit before.
         constexpr int UNITS = SC / KP;  // per stage
         static_assert(UNITS > 2, "the next stage is written while no warp can still be reading it");
-        auto k_loop = [&](auto fast_tag) {
-            uint32_t buf = 0, par = 0;  // buffer of this unit, parity of this round
-            int stage = (kbeg / SC) & 1, hf = 0;
-            for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
-                const bool more = ks + SC < kend;
-                // the registers are free for the next group once the last stage of the current one is written
-                if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC, false);
-                const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
-                const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + KP * CT;  // column codes of the unit after
+        uint32_t buf = 0, par = 0;  // buffer of this unit, parity of this round
+        int stage = (kbeg / SC) & 1, hf = 0;
+        for (int ks = kbeg; ks < kend; ks += SC, stage ^= 1, hf = HALVES == 1 ? 0 : hf ^ 1) {
+            const bool more = ks + SC < kend;
+            // the registers are free for the next group once the last stage of the current one is written
+            if (more && (HALVES == 1 || hf == 1)) fetch_group(r0, c0, (ks + SC) / KC, false);
+            const uint8_t *rb_ = rc_s + stage * C::RC_STAGE + wp * RW;
+            const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + KP * CT;  // column codes of the unit after
 #pragma unroll 1
-                for (int it = 0; it < UNITS; ++it) {
-                    const int k = ks + KP * it;
-                    if (k >= kend) break;
-                    const uint32_t next = buf == NB - 1 ? 0 : buf + 1;
-                    const uint32_t ua = uc + buf * UB;
-                    // the next stage is written before the full arrival of the unit during which its first slab is built
-                    const bool refill = it == UNITS - 3 && more;
-                    mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);  // the slabs of this unit are complete
-                    if constexpr (ONE_BARRIER) {
-                        // (buffer and set of sums `next` belong to unit u - 2 as well)
-                        if (k >= kbeg + 2 * KP && ((wp ^ (k - 2 * KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
-                            const int i = wp & (KP - 1);
-                            reduce_store(k - 2 * KP + i, part_s + (next * KP + i) * C::P_FLOATS, obase, c0, add);
-                        }
-                        builder.step(next * UB, cb_);  // (past the last k: a slab that nobody reads)
+            for (int it = 0; it < UNITS; ++it) {
+                const int k = ks + KP * it;
+                if (k >= kend) break;
+                const uint32_t next = buf == NB - 1 ? 0 : buf + 1;
+                const uint32_t ua = uc + buf * UB;
+                // the next stage is written before the full arrival of the unit during which its first slab is built
+                const bool refill = it == UNITS - 3 && more;
+                mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);  // the slabs of this unit are complete
+                if constexpr (ONE_BARRIER) {
+                    // (buffer and set of sums `next` belong to unit u - 2 as well)
+                    if (k >= kbeg + 2 * KP && ((wp ^ (k - 2 * KP)) & (WARPS - KP)) == 0) {  // KP warps in turn
+                        const int i = wp & (KP - 1);
+                        reduce_store(k - 2 * KP + i, part_s + (next * KP + i) * C::P_FLOATS, obase, c0, add);
+                    }
+                    builder.step(next * UB, cb_);  // (past the last k: a slab that nobody reads)
+                    if (refill) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + 8 * next);
+#pragma unroll
+                    for (int i = 0; i < KP; ++i) {
+                        if (i && k + i >= kend) break;
+                        clear_acc();
+                        use_rows(ua + i * C::U_BYTES, rb_ + i * RT, Q0{}, QN{});
+                        store_part(buf * KP + i);
+                    }
+                } else {
+                    clear_acc();
+                    use_rows(ua, rb_, Q0{}, QH{});
+                    // (same parity: the second buffer, which unit 0 waits for, starts out released)
+                    mbar_wait(bar_empty + 8 * next, par, 1 + NB + next, abort_word, p.error_word);
+                    if (k > kbeg && ((wp ^ (k - 1)) & (WARPS - 1)) == 0) reduce_store(k - 1, part_s + next * C::P_FLOATS, obase, c0, add);
+                    if (k + 1 < kend) {
+                        builder.step(next * UB, cb_);
                         if (refill) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_full + 8 * next);
-#pragma unroll
-                        for (int i = 0; i < KP; ++i) {
-                            if (i && k + i >= kend) break;
-                            clear_acc();
-                            use_rows(ua + i * C::U_BYTES, rb_ + i * RT, Q0{}, QN{}, fast_tag);
-                            store_part(buf * KP + i, fast_tag);
-                        }
-                    } else {
-                        clear_acc();
-                        use_rows(ua, rb_, Q0{}, QH{}, fast_tag);
-                        // (same parity: the second buffer, which unit 0 waits for, starts out released)
-                        mbar_wait(bar_empty + 8 * next, par, 1 + NB + next, abort_word, p.error_word);
-                        if (k > kbeg && ((wp ^ (k - 1)) & (WARPS - 1)) == 0) reduce_store(k - 1, part_s + next * C::P_FLOATS, obase, c0, add);
-                        if (k + 1 < kend) {
-                            builder.step(next * UB, cb_);
-                            if (refill) store_stage(stage ^ 1, HALVES == 1 ? 0 : hf ^ 1);
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(bar_full + 8 * next);
-                        }
-                        use_rows(ua, rb_, QH{}, QN{}, fast_tag);
-                        store_part(buf, fast_tag);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
                     }
-                    rb_ += KP * RT;
-                    cb_ = it == UNITS - 2 ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
-                    if (next == 0) par ^= 1;
-                    buf = next;
+                    use_rows(ua, rb_, QH{}, QN{});
+                    store_part(buf);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
                 }
+                rb_ += KP * RT;
+                cb_ = it == UNITS - 2 ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KP * CT;
+                if (next == 0) par ^= 1;
+                buf = next;
             }
-        };
-        if (MAY && fast) k_loop(std::integral_constant<bool, MAY>{});
-        else k_loop(std::false_type{});
+        }
         __syncthreads();  // every warp has stored its partial sums of the last units
         {
             // the last unit's, and with three buffers those of the one before it

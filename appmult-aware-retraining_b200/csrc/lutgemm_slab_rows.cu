@@ -17,21 +17,19 @@
 // stores four terms of one code at a time, each half-warp on sixteen different bank pairs: reads and stores are
 // conflict-free too.
 //
-// From 16-bit entries to products: the table is staged with an offset that makes its entries unsigned.  Where the least entry
-// is not far below zero (-4 min <= max: products of operands and their slopes), the entry's bits taken as those of a float
-// are the subnormal number entry * 2^-149; the thread's grad_out values are scaled by a power of two, so that products
-// are ordinary numbers and exact up to the accumulation as before, and the offset comes off at the end as offset * sum of
-// grad_out, which does not depend on k.  Two byte permutations and one packed multiply-add per two look-ups.  Tables that reach
-// further below zero, and blocks with values beyond 2^60 or tiny throughout, infinities or NaN, put each entry behind the
-// exponent of 2^23 and subtract (another packed addition per two look-ups).  Errors against 64-bit sums, 2-norm: 0.9e-7 to
-// 1.3e-7 over 4 to 8 bits, 320 to 60000 terms (with terms across lanes 1.1e-7 to 1.6e-7).
+// From 16-bit entries to products, two at a time: the table is staged in offset-binary, each half of a slab word goes behind
+// the exponent of 2^23 (a byte permutation), one packed subtraction of 2^23 + 2^15 leaves the two signed entries exactly, and one
+// packed multiply-add (fma.rn.f32x2) consumes them.  Entries that are zero add nothing, whatever else the table holds.  With
+// an offset left in the entries and taken off the sum (their bits as subnormal floats: 9.06 ms instead of 9.74 at 4096^3 and 7 bits)
+// sums of small entries keep the rounding errors of the offset: sparse codes, of which 99 % are zero, were off by up to 3.5e-6.
+// Errors against 64-bit sums, 2-norm, 4 to 8 bits, 320 to 60000 terms: 0.9e-7 to 1.1e-7 for uniform codes, less where half of them and
+// more are zero (with terms across lanes, lutgemm_slab_grad.cu, 0.8e-7 to 1.0e-7).
 //
-// What bounds it: instruction issue - a packed fp32 instruction takes two slots - and the shared-memory pipe together.
-// 4096^3 at 7 bits, per k and tile (32768 look-ups): 2950 warp instructions, 590 of them packed, 920 shared-memory
-// wavefronts, 1150 clocks; with terms across lanes (lutgemm_slab_grad.cu) 3960, 1000 and 1490.  grad_w / grad_a, 4096^3:
-// 8 bits 13.36 / 13.48 -> 10.95 / 11.02 ms, 7 bits 10.51 / 11.11 -> 9.07 / 9.12, 6 bits 9.89 / 11.30 -> 8.42 / 8.66;
-// 3x3, 64 channels at 32 x 32, batch 256, 7 bits, grad_x 1.93 -> 1.33 ms; 1x1, 256 -> 64 channels at 56 x 56, batch
-// 64, 8 bits, 1.46 -> 0.53 ms.  Two rows per thread of 32 terms each (half the slab build): 11.4 ms at 7 bits, 12.7 at 8.
+// What bounds it: instruction issue, as a packed fp32 instruction takes two slots.  7 bits, 4096 x 512 x 4096, per k and tile (32768
+// look-ups): 3390 warp instructions, 1060 of them packed, 1250 clocks: 90 % of the issue slots; 810 shared-memory wavefronts,
+// 62 % of that pipe.  8 bits: 4100 instructions, 1100 wavefronts, 1535 clocks.  grad_w / grad_a of 4096^3 against the kernel with terms
+// across lanes: 8 bits 14.15 / 14.95 -> 11.76 / 11.77 ms, 7 bits 9.99 / 10.09 -> 9.76 / 9.77, 6 bits 9.62 / 9.63 -> 9.64 / 9.67; grad_x: 3x3,
+// 64 channels at 32 x 32, batch 256, 7 bits 1.80 -> 1.47 ms; 1x1, 256 -> 64 channels at 56 x 56, batch 64, 8 bits, 1.44 (broadcast) -> 0.56.
 //
 // A CTA takes the term blocks of a group one after the other and adds each to the group's sums.  More than kRowsChain
 // blocks are added in two levels (blocks of a run of kRowsRun into a buffer of the CTA, runs into the group's sums), so that
@@ -40,8 +38,6 @@
 // Every wait on a barrier is bounded (lutgemm_waits.cuh).
 // Replaces ApproxGemmBackwardKernelForGA / ForGB, self_ops/src/approx_gemm_backward.cu:13-258, 261-492, and for
 // grad_x the unfold backward of self_ops/ops_py/approx_ops.py:556-571.
-#include <type_traits>
-
 #include "lutgemm_common.cuh"
 #include "lutgemm_f32x2.cuh"
 #include "lutgemm_kernels.h"
@@ -58,8 +54,8 @@ struct Cfg {
     static constexpr int Q = 1 << BITS;
     static constexpr int WARPS = 16, THREADS = 512, RT = kRowsTile, CT = kRowsTerms;
     static constexpr int KC = 16;                        // k per operand stage
-    // k per unit - what the warps hand over to each other - as many as fit three times: 4096^3 at 7 bits 9.2 ms with four, 10.1
-    // with two, at 8 bits there is room for one
+    // k per unit - what the warps hand over to each other - as many as fit three times: grad_w / grad_a of 4096^3 at 7 bits 9.75 /
+    // 9.75 ms with four, 9.96 / 10.24 with two; at 8 bits there is room for one
     static constexpr int KU = BITS == 8 ? 1 : 4, NB = 3;
     using T = RowsTable<BITS>;
     static constexpr int TT_ROW = T::ROW, TT_BYTES = T::BYTES, U_ROW = T::U_ROW, U_BYTES = T::U_BYTES, UB = KU * U_BYTES;
@@ -70,7 +66,7 @@ struct Cfg {
     static constexpr int G_BYTES = G_ROWS * CT * 4;
     static constexpr int OFF_CC = OFF_U + (NB * UB > G_BYTES + RT * 8 ? NB * UB : G_BYTES + RT * 8);
     static constexpr int OFF_BAR = OFF_CC + 2 * CC_STAGE;
-    static constexpr int OFF_TAP = OFF_BAR + NB * 8 + 16;  // behind an mbarrier per buffer, abort word and table range
+    static constexpr int OFF_TAP = OFF_BAR + NB * 8 + 8;  // behind an mbarrier per buffer and the abort word
     static constexpr int SMEM = OFF_TAP + kMaxTaps * 2;  // grad_x: output offset {rows, columns} of each tap
     static_assert(U_ROW == 2 * CT && OFF_U % 128 == 0, "chunks of a slab row lie on fixed bank quads");
     static_assert(SMEM <= 232448, "shared memory budget");
@@ -110,7 +106,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
     using C = Cfg<BITS>;
     constexpr int Q = C::Q, RT = C::RT, CT = C::CT, KC = C::KC, KU = C::KU, NB = C::NB, UB = C::UB, THREADS = C::THREADS;
     constexpr uint32_t MASK4 = (Q - 1) * 0x01010101u;
-    constexpr int COL = lut_col_num(BITS);
     const int K = p.K, N = p.N;
 
     extern __shared__ __align__(128) uint8_t smem[];
@@ -119,7 +114,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
     const uint32_t tt_addr = smem_u32(smem), u_addr = smem_u32(smem + C::OFF_U);
     const uint32_t bar_full = smem_u32(smem + C::OFF_BAR);
     volatile int *abort_word = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + 8 * NB);
-    uint32_t *range_s = reinterpret_cast<uint32_t *>(smem + C::OFF_BAR + 8 * NB + 4);  // least and largest table entry
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, l7 = lane & 7;
 
     // ---- stage the gradient table in offset-binary: tt[y][x], x = row code, y = term code, T = lut[a * COL + w] -----------
@@ -127,20 +121,12 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
     const uint16_t *lut = reinterpret_cast<const uint16_t *>(p.lut);
     if (MODE == kGw) stage_table_plain<BITS>(smem, lut, 0x80008000u, tid);
     else stage_table_turned<BITS>(smem, smem + C::OFF_U, lut, 0x80008000u, tid);
-    if (tid == 0) {
-        *abort_word = 0;
-        range_s[0] = 0xffffu;
-        range_s[1] = 0u;
-    }
+    if (tid == 0) *abort_word = 0;
     if (tid < 2 * C::CC_STAGE / 16) reinterpret_cast<uint4 *>(cc_s)[tid] = make_uint4(0, 0, 0, 0);  // (codes past the last k)
-    __syncthreads();
-    bool table_unsigned;
-    const int offset = reduce_table_offset<BITS>(smem, range_s, tid, &table_unsigned);
     if (MODE == kGx) {
         // pixel (hh, ww) of the class sits at h = ph + s hh; tap q connects it to output row (h - dh) / s = hh + eh
         for (int q = tid; q < p.px.ntaps; q += THREADS)
             tap_s[q] = make_char2((p.px.ph - p.px.dh[q]) / p.px.s, (p.px.pw - p.px.dw[q]) / p.px.s);
-        __syncthreads();
     }
 
     // ---- term codes: 16 k x 64 terms per stage, one 16-byte vector for each of the first 64 threads ---------------------
@@ -184,8 +170,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
         for (int i = 0; i < (KU + 1) / 2; ++i) builder.step(off + i * 2 * C::U_BYTES, codes + i * 2 * CT);
     };
 
-    const float bias1 = -(8388608.0f + (float)offset);
-    const f32x2 bias = pack2(bias1, bias1);
+    const f32x2 bias = pack2(-8421376.0f, -8421376.0f);  // -(2^23 + 2^15)
     const f32x2 minus_zero = pack2(-0.0f, -0.0f);
     const uint32_t ul = u_addr + (l7 << 4);
     const float factor = p.direct ? kGradFactor : 1.0f;
@@ -318,27 +303,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
                 }
             }
 
-            // scale for the form without a subtraction (see the file comment)
-            float fa = factor, fb = 0.f, scale = 1.f;
-            bool wide = false;  // some value is outside its range
-            if (table_unsigned) {
-                float m = 0.f;
-                f32x2 gs = g[0];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float2 t = unpack2(g[i]);
-                    m = fmaxf(m, fmaxf(fabsf(t.x), fabsf(t.y)));
-                    if (i) gs = add2(gs, g[i]);
-                }
-                const float2 t = unpack2(gs);
-                const float sum = t.x + t.y;
-                bool ok;
-                subnormal_scale(m, sum, &scale, &fa, &ok);
-                wide = !ok;
-                fa *= factor;
-                fb = -(float)offset * sum * factor;
-            }
-
             // where the sums of this block go
             float *dst = out0;
             const uint32_t doff = two_level ? tid : ooff;
@@ -350,7 +314,7 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
                 add = block % kRowsRun != 0;
             }
 
-            const bool fast = !__syncthreads_or(wide) && table_unsigned;  // (and every value has been read)
+            __syncthreads();  // every value has been read
             store_cols(0);
             if (tid == 0) {
                 // fresh barriers for this block: phases restart at 0 (nobody is waiting or arriving here)
@@ -361,13 +325,6 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
                 }
             }
             first_block = false;
-            if (fast) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) g[i] = mul2(g[i], pack2(scale, scale));
-            } else {
-                fa = factor;
-                fb = 0.f;
-            }
             __syncthreads();
             // Unit u's slabs are built at the start of unit u - 1, after the wait for that one's own slabs, into the buffer of
             // unit u - 3.  A warp that has seen unit u - 1 complete knows that every warp has built it, and so has left unit
@@ -378,80 +335,75 @@ __global__ void __launch_bounds__(512, 1) slab_grad_rows_kernel(const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_full);
 
-            auto k_loop = [&](auto fast_tag) {
-                constexpr bool FAST = decltype(fast_tag)::value;
-                uint32_t buf = 0, next = 1, par = 0;  // buffers of this unit and of the one after, parity of this round
-                int stage = 0;
-                for (int ks = kbeg; ks < kend; ks += KC, stage ^= 1) {
-                    const bool more = ks + KC < kend;
-                    if (more) fetch_cols(t0, ks + KC);
-                    const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + KU * CT;  // term codes of the unit after
+            uint32_t buf = 0, next = 1, par = 0;  // buffers of this unit and of the one after, parity of this round
+            int stage = 0;
+            for (int ks = kbeg; ks < kend; ks += KC, stage ^= 1) {
+                const bool more = ks + KC < kend;
+                if (more) fetch_cols(t0, ks + KC);
+                const uint8_t *cb_ = cc_s + stage * C::CC_STAGE + KU * CT;  // term codes of the unit after
 #pragma unroll 1
-                    for (int k4 = 0; k4 < KC / 4; ++k4) {
-                        const int kg = ks + 4 * k4;
-                        if (kg >= kend) break;
-                        const uint32_t rw = __byte_perm(__byte_perm(raw[0], raw[1], 0x0040), __byte_perm(raw[2], raw[3], 0x0040), 0x5410) & MASK4;
-                        fetch_rows(kg + 4);
-                        auto begin_unit = [&](int it) {
-                            mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);
-                            build(next * UB, cb_);  // (past the last k: a slab that nobody reads)
-                            if (it == UNITS - 3 && more) store_cols(stage ^ 1);
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(bar_full + 8 * next);
-                            cb_ = it == UNITS - 2 ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KU * CT;
+                for (int k4 = 0; k4 < KC / 4; ++k4) {
+                    const int kg = ks + 4 * k4;
+                    if (kg >= kend) break;
+                    const uint32_t rw = __byte_perm(__byte_perm(raw[0], raw[1], 0x0040), __byte_perm(raw[2], raw[3], 0x0040), 0x5410) & MASK4;
+                    fetch_rows(kg + 4);
+                    auto begin_unit = [&](int it) {
+                        mbar_wait(bar_full + 8 * buf, par, 1 + buf, abort_word, p.error_word);
+                        build(next * UB, cb_);  // (past the last k: a slab that nobody reads)
+                        if (it == UNITS - 3 && more) store_cols(stage ^ 1);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_full + 8 * next);
+                        cb_ = it == UNITS - 2 ? cc_s + (stage ^ 1) * C::CC_STAGE : cb_ + KU * CT;
+                    };
+                    auto end_unit = [&]() {
+                        if (next == 0) par ^= 1;
+                        buf = next;
+                        if (++next == NB) next = 0;
+                    };
+                    // dot product of the slab row at `base` (bits 4 - 6 of it select the lane's first chunk)
+                    auto dot = [&](uint32_t base) -> float {
+                        constexpr int PF = 2;  // slab reads in flight ahead of their use
+                        uint32_t q[PF][4];
+                        auto fetch = [&](int j) {
+                            uint32_t *d = q[j % PF];
+                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(base ^ (j << 4)));
                         };
-                        auto end_unit = [&]() {
-                            if (next == 0) par ^= 1;
-                            buf = next;
-                            if (++next == NB) next = 0;
-                        };
-                        // dot product of the slab row at `base` (bits 4 - 6 of it select the lane's first chunk)
-                        auto dot = [&](uint32_t base) -> float {
-                            constexpr int PF = 2;  // slab reads in flight ahead of their use
-                            uint32_t q[PF][4];
-                            auto fetch = [&](int j) {
-                                uint32_t *d = q[j % PF];
-                                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                             : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(base ^ (j << 4)));
-                            };
 #pragma unroll
-                            for (int j = 0; j < PF; ++j) fetch(j);
-                            f32x2 acc[2];
+                        for (int j = 0; j < PF; ++j) fetch(j);
+                        f32x2 acc[2];
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const uint32_t w[4] = {q[j % PF][0], q[j % PF][1], q[j % PF][2], q[j % PF][3]};
-                                if (j + PF < 8) fetch(j + PF);
+                        for (int j = 0; j < 8; ++j) {
+                            const uint32_t w[4] = {q[j % PF][0], q[j % PF][1], q[j % PF][2], q[j % PF][3]};
+                            if (j + PF < 8) fetch(j + PF);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const f32x2 e = FAST ? tiny2(w[i]) : entries2(w[i], bias);
-                                    acc[i % 2] = j == 0 && i < 2 ? mul2(e, g[i]) : fma2(e, g[4 * j + i], acc[i % 2]);
-                                }
+                            for (int i = 0; i < 4; ++i) {
+                                const f32x2 e = entries2(w[i], bias);
+                                acc[i % 2] = j == 0 && i < 2 ? mul2(e, g[i]) : fma2(e, g[4 * j + i], acc[i % 2]);
                             }
-                            const float2 t = unpack2(add2(acc[0], acc[1]));
-                            return t.x + t.y;
-                        };
-                        float v[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if (i % KU == 0) begin_unit(KU == 4 ? k4 : 4 * k4 + i);
-                            v[i] = dot(__dp4a(rw, (uint32_t)C::U_ROW << (8 * i), ul + buf * UB + i % KU * C::U_BYTES));
-                            if (i % KU == KU - 1) end_unit();
                         }
-                        // (all four sums at the end: between the reads their branches cost 4 % and more)
-                        float *d = dst + doff;
-                        if (add) {
+                        const float2 t = unpack2(add2(acc[0], acc[1]));
+                        return t.x + t.y;
+                    };
+                    float v[4];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) put<true>(d + i * dstride, fmaf(v[i], fa, fb), in && kg + i < kend);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) put<false>(d + i * dstride, fmaf(v[i], fa, fb), in && kg + i < kend);
-                        }
-                        dst += 4 * dstride;
+                    for (int i = 0; i < 4; ++i) {
+                        if (i % KU == 0) begin_unit(KU == 4 ? k4 : 4 * k4 + i);
+                        v[i] = dot(__dp4a(rw, (uint32_t)C::U_ROW << (8 * i), ul + buf * UB + i % KU * C::U_BYTES));
+                        if (i % KU == KU - 1) end_unit();
                     }
+                    // (all four sums at the end: between the reads their branches cost 4 % and more)
+                    float *d = dst + doff;
+                    if (add) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) put<true>(d + i * dstride, v[i] * factor, in && kg + i < kend);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) put<false>(d + i * dstride, v[i] * factor, in && kg + i < kend);
+                    }
+                    dst += 4 * dstride;
                 }
-            };
-            if (fast) k_loop(std::true_type{});
-            else k_loop(std::false_type{});
+            }
             if (two_level && in && (block % kRowsRun == kRowsRun - 1 || block == nblocks - 1)) {
                 // the run is complete (its sums are this thread's own)
                 float *o = out0 + ooff;
