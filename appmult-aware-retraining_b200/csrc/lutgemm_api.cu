@@ -68,13 +68,13 @@ struct BackwardPlan {
 // Each estimate is (waves of the kernel's own tiling) x (clocks of one work item) + a fixed start (launch, table staging).
 // The clocks are measured on B200, at 4096^3 unless said otherwise:
 //   slab kernels, per k and tile      packed 512 x 64: grad_w 1275 (4 bits), 1315 (6), 1365 (7), 1945 (8), grad_a and grad_x
-//                                     1290, 1320, 1390, 2055; tall 1024 x 32: 1540, 1690, 1880;
+//                                     1290, 1320, 1390, 2055 (grad_x: 9.5e3 more per work item, 2e3 at 8 bits); tall 1024 x 32: 1540, 1690, 1880;
 //                                     forward 512 x 64: 905, 940, 1330 and 60e3 / 75e3 at the start (up to three
 //                                     more launches: code transposition, zeroing, and a layer's epilogue);
 //   a thread per row                  gradients 512 x 64: 1185 (4 bits), 1210 (6 and 7), 1490 (8) per k, 9e3 per block of
 //                                     grad_out values (27e3 where they come one by one); forward 1024 x 32: 650, 690, 845
 //   broadcast kernels, per 32 look-ups (1 = no bank conflict): forward 1.48, 2.33, 3.1; grad_w 1.6, 2.4, 3.3;
-//                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.66, 1.72, 2.2
+//                                     grad_a 1.6, 2.6, 4.2; grad_x of clustered codes 1.66, 1.7, 2.2
 // A slab kernel's time does not depend on the codes and it can cut K into many work items; a broadcast kernel has no slab
 // to build, so it stays the better one for few rows.  Against the fixed limits on M, N and tile fill that came before
 // (base_plan below) the estimates move small and ragged problems to the slab kernels: 256 x 512 x 256 at 7 bits, forward 0.291 ms,
@@ -84,7 +84,7 @@ struct FamilyClocks {
 };
 FamilyClocks family_clocks(int bits) {
     if (bits == 8) return {1945, 2055, 1880, 1330, 3.1, 3.3, 4.2, 2.2, 75e3, 1490, 845};
-    if (bits == 7) return {1365, 1390, 1690, 940, 2.33, 2.4, 2.6, 1.72, 60e3, 1210, 690};
+    if (bits == 7) return {1365, 1390, 1690, 940, 2.33, 2.4, 2.6, 1.7, 60e3, 1210, 690};
     if (bits == 6) return {1315, 1320, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1210, 650};
     return {1275, 1290, 1540, 905, 1.48, 1.6, 1.6, 1.66, 60e3, 1185, 650};
 }
@@ -600,18 +600,17 @@ static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
 // family_clocks).  The slab kernel's time does not depend on the codes, the broadcast kernel's bank conflicts do; the
 // estimate takes the clustered codes of a trained layer.  Measured on B200, 3x3 layers at batch 256, clustered codes,
 // broadcast against slab, ms:
-//   7 bits  64 channels (576 rows) 1.79 : 1.85   128 (1152) 1.99 : 1.75   256 (2304) 1.99 : 1.65   512 (4608) 2.02 : 1.64
-//   8 bits  64 channels            2.28 : 2.50   128        2.61 : 2.34   256        2.66 : 2.24   512        2.74 : 2.22
-//   256 -> 512 channels, stride 2 (classes of 2048, 1024, 1024 and 512 rows): 7 bits 1.07 : 0.96, 8 bits 1.77 : 1.35
+//   7 bits  64 channels (576 rows) 1.79 : 1.79   128 (1152) 1.99 : 1.60   256 (2304) 2.00 : 1.55   512 (4608) 2.00 : 1.49
+//   8 bits  64 channels            2.27 : 2.49   128        2.55 : 2.32   256        2.55 : 2.23   512        2.57 : 2.26
+//   stride 2, 128 -> 256 channels: 7 bits 1.03 : 0.99, 8 bits 1.31 : 1.42; 256 -> 512 (classes of 2048, 1024, 1024 and 512 rows):
+//   7 bits 1.08 : 0.88, 8 bits 1.73 : 1.30
+// or, for callers that allow it (`rows`), the kernel with one thread per pixel (lutgemm_slab_rows.cu).
 struct GxTimes {
     double slab, bcast, rows;
 };
-static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows_entry) {
+static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
     const FamilyClocks f = family_clocks(bits);
     const long mt = bits == 8 ? 512 : 256;
-    // (lutgemm_conv2d_backward keeps the lines that it was given with the slab kernel of that time: 1580 clocks per step at 7 bits)
-    const double step = rows_entry ? f.packed : bits == 8 ? 2180 : bits == 7 ? 1580 : 1540;
-    const double step576 = rows_entry ? lutgemm::kPacked576Step : 1.12;
     double slab = 0, by_rows = 0;
     // broadcast kernel: tiles of all classes in one list, tile t on SM t mod sms (rows_of[i] rows from tile begin[i] on)
     constexpr int kMaxListed = 16;
@@ -620,7 +619,8 @@ static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms,
     for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(rows);
-        slab += packed_clocks(lutgemm::plan_packed(rows, px.P, px.C, rt, sms), px.P, px.C, step * (rt > 512 ? step576 : 1.0), false);
+        const lutgemm::PackedPlan plan = lutgemm::plan_packed(rows, px.P, px.C, rt, sms);
+        slab += packed_clocks(plan, px.P, px.C, f.packed * (rt > 512 ? lutgemm::kPacked576Step : 1.0), false) + plan.items * (bits == 8 ? 2e3 : 9.5e3);
         by_rows += rows_clocks(lutgemm::plan_rows(px.P, rows, px.C, sms), bits, px.P, px.C, true, Cout % 4 == 0, false);
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
@@ -645,12 +645,11 @@ static bool gx_rows_supported(const lutgemm::ConvGeom &g, int Cout) {
 }
 enum GxFamily { kGxBcast, kGxSlab, kGxRows };
 static GxFamily gx_family(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows) {
-    const bool rows_entry = rows;
     rows = rows && gx_rows_supported(g, Cout);
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (force == LUTGEMM_BACKWARD_BCAST) return kGxBcast;
     if (force == LUTGEMM_BACKWARD_SLAB) return rows && tile == LUTGEMM_TILE_ROWS ? kGxRows : kGxSlab;
-    const GxTimes t = gx_times(bits, g, Cout, sms, rows_entry);
+    const GxTimes t = gx_times(bits, g, Cout, sms);
     if (rows && t.rows < t.slab && t.rows < t.bcast) return kGxRows;
     return t.slab < t.bcast ? kGxSlab : kGxBcast;
 }
@@ -833,7 +832,8 @@ int lutgemm_conv2d_backward_ws(const float *gy, const uint8_t *x, const uint8_t 
                               scratch, scratch_bytes, stream, true);
 }
 
-// (its image gradients keep the kernels, and with them the order of summation, that they have always had)
+// (the tests hold its image gradients to the packed and the broadcast kernel; by the same estimates, so that the one query serves
+// both entry points)
 int lutgemm_conv2d_backward(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, float *gw,
                             const int16_t *lut_ga, const int16_t *lut_gw, int bits, int B, int C, int H, int W,
                             int Cout, int kh, int kw, int stride, int pad, int dil, void *scratch,

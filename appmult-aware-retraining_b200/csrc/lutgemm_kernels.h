@@ -89,19 +89,21 @@ constexpr double kPacked576Step = 1.13;  // time of a k step with 576 rows
 struct PackedPlan {
     int groups, group_blocks;
     int main_cells, tail_parts, tail_per;
-    long steps;  // k steps of the CTA that has most to do
+    long steps, items;  // k steps of the CTA that has most to do, its item overheads among them, and its work items (row blocks each)
 };
 inline PackedPlan deal_cells(long groups, long blocks, long tiles_c, int K, int num_sms, int item_overhead) {
     const long cells = groups * tiles_c, rounds = cells / num_sms, tail = cells % num_sms;
     const int whole = (K + 15) / 16 * 16;
-    PackedPlan p{(int)groups, (int)blocks, (int)(rounds * num_sms), 1, whole, rounds * (whole + item_overhead)};
+    PackedPlan p{(int)groups, (int)blocks, (int)(rounds * num_sms), 1, whole, rounds * (whole + item_overhead), rounds};
     if (tail) {
         const KSplit ks = choose_ksplit(tail, K, num_sms, item_overhead);
         p.tail_parts = ks.parts;
         p.tail_per = ks.per;
         p.steps += ks.waves * (ks.per + item_overhead);
+        p.items += ks.waves;
     }
     p.steps *= blocks;
+    p.items *= blocks;
     return p;
 }
 // Where the tiles fill the GPU anyway, the largest groups that cost no time: one block of sums per row block made the

@@ -190,6 +190,8 @@ size_t lutgemm_conv2d_backward_scratch_bytes(int bits, int B, int C, int H, int 
  * taps joins the sum over n); the unfolded activation gradient [B*Ho*Wo, C*kh*kw] the reference forms and folds
  * back (autograd of F.unfold) never exists.  Overlapping windows with more than 128 taps are refused
  * (LUTGEMM_E_TOOLARGE).  Sums are deterministic.
+ * gx comes from the kernels with terms across lanes; lutgemm_conv2d_backward_ws may choose the one with a thread per
+ * pixel as well, which is the faster one for most large layers.
  * Replaces the autograd chain of approx_conv2d_op (unfold backward + approx_gemm_backward),
  * self_ops/ops_py/approx_ops.py:181-205,556-571.
  */
