@@ -404,7 +404,12 @@ size_t lutgemm_backward_ws_scratch_bytes(int bits, int M, int K, int N, int flag
     const int sms = current_num_sms();
     if (sms <= 0) return 0;
     const bool have_codes = flags & LUTGEMM_SCRATCH_CODES_GIVEN;
-    const size_t need = plan_backward(bits, M, K, N, sms, false, true, true, have_codes).scratch;
+    const BackwardPlan both = plan_backward(bits, M, K, N, sms, false, true, true, have_codes);
+    size_t need = both.scratch;
+    if (both.ga_rows && !have_codes) {  // (alone, grad_a has the code copy made for itself and may choose another kernel)
+        const size_t alone = plan_backward(bits, M, K, N, sms, false, false, true, false).scratch;
+        need = alone > need ? alone : need;
+    }
     return flags & LUTGEMM_SCRATCH_LEAST ? least_need(need, base_plan(bits, M, K, N, sms, true, true, have_codes).scratch) : need;
 }
 

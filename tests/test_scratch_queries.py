@@ -45,3 +45,26 @@ def test_convolution_backward(lib, gx, gw):
             assert exact[0] == H.OK and exact == lib.call("lutgemm_conv2d_backward_ws", *args, codes, p, big, None), shape
             least = lib.query("lutgemm_conv2d_backward_ws_scratch_bytes", *shape, flag | H.LEAST)
             assert lib.call("lutgemm_conv2d_backward_ws", *args, codes, p, H.Size(least), None)[0] == H.OK, shape
+
+
+def products():
+    rng = random.Random(2)
+    # (the first six: the activation gradient alone ran on a slower kernel with the size that the query named)
+    return [(6, 5104, 1095, 2537), (6, 3631, 3095, 670), (4, 3195, 2987, 1832), (8, 1673, 2932, 667), (6, 4776, 3739, 1468),
+            (4, 1396, 2477, 3692)] + [
+        (rng.choice([4, 6, 7, 8]), log_uniform(rng, 1, 16384), log_uniform(rng, 1, 8192), log_uniform(rng, 1, 8192)) for _ in range(4000)]
+
+
+@pytest.mark.parametrize("ga,gw", [(True, True), (True, False), (False, True)])
+def test_operator_backward(lib, ga, gw):
+    p, big = lib.p, H.Size(1 << 40)
+    for shape in products():
+        args = (p, p, p, p if ga else None, p if gw else None, p, p, *shape)
+        need = lib.query("lutgemm_backward_scratch_bytes", *shape)
+        exact = lib.call("lutgemm_backward", *args, p, H.Size(need), None)
+        assert exact[0] == H.OK and exact == lib.call("lutgemm_backward", *args, p, big, None), shape
+        for codes, flag in ((None, 0), (p, H.CODES_GIVEN)):
+            need, least = (lib.query("lutgemm_backward_ws_scratch_bytes", *shape, flag | f) for f in (0, H.LEAST))
+            exact = lib.call("lutgemm_backward_ws", *args, codes, p, H.Size(need), None)
+            assert exact[0] == H.OK and exact == lib.call("lutgemm_backward_ws", *args, codes, p, big, None), shape
+            assert lib.call("lutgemm_backward_ws", *args, codes, p, H.Size(least), None)[0] == H.OK, shape
