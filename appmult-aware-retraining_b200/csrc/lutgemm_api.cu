@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "lutgemm.h"
@@ -610,13 +611,19 @@ static void for_each_pixel_class(const lutgemm::ConvGeom &g, F f) {
 //   stride 2, 128 -> 256 channels: 7 bits 1.03 : 0.99, 8 bits 1.31 : 1.42; 256 -> 512 (classes of 2048, 1024, 1024 and 512 rows):
 //   7 bits 1.08 : 0.88, 8 bits 1.73 : 1.30
 // or, for callers that allow it (`rows`), the kernel with one thread per pixel (lutgemm_slab_rows.cu).
+// (the kernel with a thread per pixel addresses an image by 32-bit offsets and keeps the two coordinates of a pixel in one word)
+static bool gx_rows_supported(const lutgemm::ConvGeom &g, int Cout) {
+    return g.H < 32768 && g.W < 65536 && (double)g.B * g.C * g.H * g.W < 4294967296.0 && lutgemm::rows_supported((long)g.B * g.H * g.W, (long)g.kh * g.kw * Cout, g.C);
+}
 struct GxTimes {
-    double slab, bcast, rows;
+    double slab, bcast, rows;  // rows: 0 where that kernel is no choice
+    size_t slab_bytes, rows_bytes;
 };
-static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows_allowed) {
     const FamilyClocks f = family_clocks(bits);
     const long mt = bits == 8 ? 512 : 256;
-    double slab = 0, by_rows = 0;
+    const bool may_rows = rows_allowed && gx_rows_supported(g, Cout);
+    GxTimes times{};
     // broadcast kernel: tiles of all classes in one list, tile t on SM t mod sms (rows_of[i] rows from tile begin[i] on)
     constexpr int kMaxListed = 16;
     long begin[kMaxListed + 1] = {0}, rows_of[kMaxListed], most = 0;
@@ -625,8 +632,13 @@ static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms)
         const long rows = (long)px.ntaps * Cout, t = div_up(px.P, mt) * div_up(px.C, 32);
         const int rt = lutgemm::gx_tile_rows(rows);
         const lutgemm::PackedPlan plan = lutgemm::plan_packed(rows, px.P, px.C, rt, sms);
-        slab += packed_clocks(plan, px.P, px.C, f.packed * (rt > 512 ? lutgemm::kPacked576Step : 1.0), false) + plan.items * (bits == 8 ? 2e3 : 9.5e3);
-        by_rows += rows_clocks(lutgemm::plan_rows(px.P, rows, px.C, sms), bits, px.P, px.C, true, Cout % 4 == 0, false);
+        times.slab += packed_clocks(plan, px.P, px.C, f.packed * (rt > 512 ? lutgemm::kPacked576Step : 1.0), false) + plan.items * (bits == 8 ? 2e3 : 9.5e3);
+        times.slab_bytes = std::max(times.slab_bytes, lutgemm::gx_class_scratch_bytes(plan, px));
+        if (may_rows) {
+            const lutgemm::RowsPlan by_rows = lutgemm::plan_rows(px.P, rows, px.C, sms);
+            times.rows += rows_clocks(by_rows, bits, px.P, px.C, true, Cout % 4 == 0, false);
+            times.rows_bytes = std::max(times.rows_bytes, lutgemm::rows_scratch_bytes(by_rows, px.P, px.C, true, sms));
+        }
         if (n == kMaxListed) {  // (more stride classes than this: the rest counts as tiles of the last one)
             begin[n] += t;
             return;
@@ -642,19 +654,15 @@ static GxTimes gx_times(int bits, const lutgemm::ConvGeom &g, int Cout, int sms)
         for (int c = 0; c < n; ++c) rows += rows_of[c] * ((begin[c + 1] + sms - 1 - sm) / sms - (begin[c] + sms - 1 - sm) / sms);
         if (rows > most) most = rows;
     }
-    return {slab, (double)most * mt * f.gx_bcast + kBcastStart, by_rows};
-}
-// (the kernel addresses an image by 32-bit offsets and keeps the two coordinates of a pixel in one word)
-static bool gx_rows_supported(const lutgemm::ConvGeom &g, int Cout) {
-    return g.H < 32768 && g.W < 65536 && (double)g.B * g.C * g.H * g.W < 4294967296.0 && lutgemm::rows_supported((long)g.B * g.H * g.W, (long)g.kh * g.kw * Cout, g.C);
+    times.bcast = (double)most * mt * f.gx_bcast + kBcastStart;
+    return times;
 }
 enum GxFamily { kGxBcast, kGxSlab, kGxRows };
-static GxFamily gx_family(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, bool rows) {
-    rows = rows && gx_rows_supported(g, Cout);
+static GxFamily gx_family(const GxTimes &t, bool rows) {
+    rows = rows && t.rows > 0;
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (force == LUTGEMM_BACKWARD_BCAST) return kGxBcast;
     if (force == LUTGEMM_BACKWARD_SLAB) return rows && tile == LUTGEMM_TILE_ROWS ? kGxRows : kGxSlab;
-    const GxTimes t = gx_times(bits, g, Cout, sms);
     if (rows && t.rows < t.slab && t.rows < t.bcast) return kGxRows;
     return t.slab < t.bcast ? kGxSlab : kGxBcast;
 }
@@ -677,33 +685,16 @@ static size_t gx_base_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     return need;
 }
 
-static size_t gx_slab_scratch_bytes(const lutgemm::ConvGeom &g, int Cout, int sms) {
-    size_t need = 0;
-    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
-        const size_t n = lutgemm::gx_class_scratch_bytes(Cout, px, g.B, sms);
-        need = n > need ? n : need;
-    });
-    return need;
-}
-
-static size_t gx_rows_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
-    size_t need = 0;
-    for_each_pixel_class(g, [&](const lutgemm::PixelClass &px) {
-        const lutgemm::RowsPlan plan = lutgemm::plan_rows(px.P, (long)px.ntaps * Cout, px.C, sms);
-        const size_t n = lutgemm::rows_scratch_bytes(plan, px.P, px.C, true, sms);
-        need = n > need ? n : need;
-    });
-    return need;
-}
-
-// 1x1 windows without padding: every pixel of class (0, 0) has the one tap
+// 1x1 windows without padding: every pixel of class (0, 0), of which there are as many as output positions, has the one tap
 static bool pointwise(const lutgemm::ConvGeom &g) { return g.kh == 1 && g.kw == 1 && g.pad == 0; }
-static bool pointwise_by_rows(int bits, const lutgemm::ConvGeom &g, int Cout, int sms) {
+static bool pointwise_by_rows(int bits, const lutgemm::ConvGeom &g, int Cout, int sms, size_t *bytes) {
     const int force = g_force_backward.load(std::memory_order_relaxed), tile = g_force_tile.load(std::memory_order_relaxed);
     if (!pointwise(g) || force == LUTGEMM_BACKWARD_BCAST || !gx_rows_supported(g, Cout)) return false;
-    if (force || tile) return tile == LUTGEMM_TILE_ROWS;
     const int M = g.B * g.Ho * g.Wo;
-    const double rows = rows_clocks(lutgemm::plan_rows(M, Cout, g.C, sms), bits, M, g.C, true, Cout % 4 == 0, false);
+    const lutgemm::RowsPlan plan = lutgemm::plan_rows(M, Cout, g.C, sms);
+    *bytes = lutgemm::rows_scratch_bytes(plan, M, g.C, true, sms);
+    if (force || tile) return tile == LUTGEMM_TILE_ROWS;
+    const double rows = rows_clocks(plan, bits, M, g.C, true, Cout % 4 == 0, false);
     double best = ga_bcast_clocks(bits, M, g.C, Cout, sms);
     if (Cout >= 768) {
         const lutgemm::PackedPlan pp = lutgemm::plan_packed(Cout, M, g.C, lutgemm::packed_ga_tile_rows(Cout), sms);
@@ -720,15 +711,13 @@ static size_t conv_gx_scratch_bytes(int bits, const lutgemm::ConvGeom &g, int Co
     if (sms <= 0) return 0;
     if (conv_windows_overlap(g) && !pixel_mode_supported(g)) return 0;  // the gradient is refused, whatever the buffer
     // (either entry point's choice, see lutgemm_conv2d_backward)
-    size_t need = 0, rows = 0;
     if (!conv_windows_overlap(g)) {
-        need = plan_backward(bits, M, K, Cout, sms, true, false, true, false).scratch;
-        if (pointwise_by_rows(bits, g, Cout, sms)) rows = gx_rows_scratch_bytes(bits, g, Cout, sms);
-    } else {
-        if (gx_family(bits, g, Cout, sms, false) == kGxSlab) need = gx_slab_scratch_bytes(g, Cout, sms);
-        if (gx_family(bits, g, Cout, sms, true) == kGxRows) rows = gx_rows_scratch_bytes(bits, g, Cout, sms);
+        const size_t need = plan_backward(bits, M, K, Cout, sms, true, false, true, false).scratch;
+        size_t rows = 0;
+        return pointwise_by_rows(bits, g, Cout, sms, &rows) ? std::max(need, rows) : need;
     }
-    return need > rows ? need : rows;
+    const GxTimes t = gx_times(bits, g, Cout, sms, true);
+    return std::max(gx_family(t, false) == kGxSlab ? t.slab_bytes : 0, gx_family(t, true) == kGxRows ? t.rows_bytes : 0);
 }
 
 size_t lutgemm_conv2d_backward_ws_scratch_bytes(int bits, int B, int C, int H, int W, int Cout, int kh, int kw,
@@ -788,15 +777,17 @@ static int conv_backward_impl(const float *gy, const uint8_t *x, const uint8_t *
     const size_t given = scratch ? scratch_bytes : 0;
     GxFamily family = kGxBcast;
     if (!overlap) {  // conv.enabled makes the grad_a kernels write (m,k) to the image position it came from
-        if (!by_rows || !pointwise_by_rows(bits, g, Cout, sms) || gx_rows_scratch_bytes(bits, g, Cout, sms) > given)
+        size_t need = 0;
+        if (!by_rows || !pointwise_by_rows(bits, g, Cout, sms, &need) || need > given)
             return backward_impl(gy, x, wmat, gx, nullptr, lut_ga, nullptr, bits, M, K, Cout, g, nullptr, scratch, scratch_bytes,
                                  stream);
         family = kGxRows;
     } else {
         if (!pixel_mode_supported(g)) return LUTGEMM_E_TOOLARGE;
-        family = gx_family(bits, g, Cout, sms, by_rows);
-        if (family == kGxRows && gx_rows_scratch_bytes(bits, g, Cout, sms) > given) family = gx_family(bits, g, Cout, sms, false);
-        if (family == kGxSlab && gx_slab_scratch_bytes(g, Cout, sms) > given) {
+        const GxTimes t = gx_times(bits, g, Cout, sms, by_rows);
+        family = gx_family(t, by_rows);
+        if (family == kGxRows && t.rows_bytes > given) family = gx_family(t, false);
+        if (family == kGxSlab && t.slab_bytes > given) {
             if (g_force_backward.load(std::memory_order_relaxed) || gx_base_scratch_bytes(bits, g, Cout) > given)
                 return LUTGEMM_E_SCRATCH;
             family = kGxBcast;

@@ -220,7 +220,7 @@ int slab_reduce_blocks(const float *part, float *out, int K, int C, int nblocks,
 // activation gradient of a convolution for the input pixels of one stride class, written into gx[B,C,H,W]
 // (packed slab kernel in pixel mode: no unfolded gradient, no col2im); scratch: gx_class_scratch_bytes()
 int gx_tile_rows(long rdim);  // rows of its tile for a class of rdim = taps * Cout rows
-size_t gx_class_scratch_bytes(int Cout, const PixelClass &px, int B, int num_sms);
+size_t gx_class_scratch_bytes(const PackedPlan &plan, const PixelClass &px);  // plan_packed of the class
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
                       int Cout, const PixelClass &px, int B, float *scratch, int num_sms, cudaStream_t stream);
 // the same with the column-broadcast gather kernel (whole table in shared memory, no slab) for `nclasses` stride

@@ -698,10 +698,8 @@ int backward_ga_slab_packed(const float *gc, const uint8_t *a, const uint8_t *w,
     return LUTGEMM_E_BITS;
 }
 
-size_t gx_class_scratch_bytes(int Cout, const PixelClass &px, int B, int num_sms) {
-    const long rdim = (long)px.ntaps * Cout, cdim = (long)B * px.Hc * px.Wc;
-    const int groups = plan_packed(rdim, cdim, px.C, gx_tile_rows(rdim), num_sms).groups;
-    return groups > 1 ? (size_t)groups * px.C * cdim * sizeof(float) : 0;
+size_t gx_class_scratch_bytes(const PackedPlan &plan, const PixelClass &px) {
+    return plan.groups > 1 ? (size_t)plan.groups * px.C * px.P * sizeof(float) : 0;
 }
 
 int backward_gx_class(const float *gy, const uint8_t *x, const uint8_t *wmat, float *gx, const int16_t *lut_ga, int bits,
