@@ -630,11 +630,13 @@ __global__ void __launch_bounds__(1024) transpose_codes_kernel(const uint8_t *__
     *reinterpret_cast<uint4 *>(at + (size_t)k * pitch + m0) = make_uint4(v[0] & mask4, v[1] & mask4, v[2] & mask4, v[3] & mask4);
 }
 
-// The same for a convolution whose output rows are a multiple of 4 and whose output planes are a multiple of 16 positions: a CTA
-// stages `planes` input planes of one channel, with the padding's zeros around them, and writes their kh*kw shifted copies.
+// The same for a convolution whose output planes are a multiple of 16 positions: a CTA stages `planes` input planes of one channel, with
+// the padding's zeros around them, and writes their kh*kw shifted copies.
 // Four neighbouring outputs come from two or three aligned words and a funnel shift (stride 1 and 2), not byte by byte
 // with a test of the borders for each: 256 planes of 64 x 32 x 32, 3x3, 116 -> 51 us.  Small planes share a CTA, images after
-// one another, so that stores stay longer than a sector.
+// one another, so that stores stay longer than a sector.  STRIDE 0: any stride, by bytes; -1: also output rows that are no multiple of
+// 4, whose outputs pass from row to row one by one (256 x 64 x 16 x 18, 3x3: 38 us, 75 with a thread per 16 outputs from global memory;
+// 64 x 64 x 32 x 34, 5x5: 55, 196).
 struct PlaneStage {
     int planes, rows, pitch;  // planes per CTA; rows and bytes per row of a staged plane
     unsigned groups;          // CTAs per channel
@@ -680,12 +682,13 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
     for (int q = threadIdx.x; q < g.kh * per_row; q += 256) {
         const int i = nb == st.planes ? quotient(q, st.by_rows) : q / per_row;
         const int r = q - i * per_row, p = quotient(r, st.by_chunks), l0 = (r - p * chunks) * 16;
-        int oh = quotient(l0 / 4, st.by_quads), ow = l0 - oh * g.Wo;
-        int o[4];
+        constexpr int STEP = STRIDE < 0 ? 1 : 4;  // outputs that certainly share their row
+        int oh = STRIDE < 0 ? l0 / g.Wo : quotient(l0 / 4, st.by_quads), ow = l0 - oh * g.Wo;
+        int o[16 / STEP];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 16 / STEP; ++e) {
             o[e] = p * bytes + (i * g.dil + oh * g.stride) * st.pitch + ow * g.stride;
-            ow += 4;
+            ow += STEP;
             if (ow == g.Wo) { ow = 0; ++oh; }
         }
         uint8_t *dst = at + (size_t)(c * kk + i * g.kw) * at_pitch + (size_t)(b0 + p) * L + l0;
@@ -693,11 +696,12 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
             uint32_t v[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int ad = o[e] + j * g.dil;
-                if (STRIDE == 0) {
+                const int ad = o[e * 4 / STEP] + j * g.dil;
+                if (STRIDE <= 0) {
                     v[e] = 0u;
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) v[e] |= (uint32_t)plane[ad + t * g.stride] << (8 * t);
+                    for (int t = 0; t < 4; ++t)
+                        v[e] |= (uint32_t)plane[STRIDE < 0 ? o[(4 * e + t) / STEP] + j * g.dil : ad + t * g.stride] << (8 * t);
                 } else {
                     const uint32_t *w = reinterpret_cast<const uint32_t *>(plane) + (ad >> 2);
                     const int sh = 8 * (ad & 3);
@@ -762,7 +766,7 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
                     uint32_t *zero, long zero_words, cudaStream_t stream) {
     ZeroJob job{zero, zero ? zero_words : 0};
     const uint32_t mask4 = ((1u << bits) - 1u) * 0x01010101u;  // codes are cut to `bits` bits on their way through
-    if (conv.enabled && (conv.Ho * conv.Wo) % 16 == 0 && conv.Wo % 4 == 0) {
+    if (conv.enabled && (conv.Ho * conv.Wo) % 16 == 0) {
         // every column m < M is written (M = B * Ho * Wo is a multiple of 16, so pitch == M)
         const int L = conv.Ho * conv.Wo;
         if (conv.kh * conv.kw == 1 && conv.stride == 1 && conv.pad == 0 && conv.C <= 4 * 65535 && (reinterpret_cast<uintptr_t>(a) & 15) == 0) {
@@ -787,9 +791,11 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
             st.by_row = reciprocal(st.pitch / 4);
             st.by_rows = reciprocal(per_row);
             st.by_chunks = reciprocal(L / 16);
-            st.by_quads = reciprocal(conv.Wo / 4);
+            st.by_quads = conv.Wo % 4 == 0 ? reciprocal(conv.Wo / 4) : 0u;
             const int smem = (int)(st.planes * bytes) + 16;
-            auto kern = conv.stride == 1 ? transpose_codes_plane_kernel<1> : conv.stride == 2 ? transpose_codes_plane_kernel<2> : transpose_codes_plane_kernel<0>;
+            auto kern = conv.Wo % 4 != 0   ? transpose_codes_plane_kernel<-1>
+                        : conv.stride == 1 ? transpose_codes_plane_kernel<1>
+                        : conv.stride == 2 ? transpose_codes_plane_kernel<2> : transpose_codes_plane_kernel<0>;
             if (smem > 48 * 1024 && !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
                 return LUTGEMM_E_CUDA;
             kern<<<(unsigned)conv.C * st.groups, 256, smem, stream>>>(a, at, pitch, conv, mask4, st, job);

@@ -120,3 +120,10 @@ def test_row_sums(dev, M, N):
     want = g.double().sum(dim=1)
     bound = (9 + -(-N // 32)) * 2.0 ** -24 * g.double().abs().sum(dim=1)
     assert bool(((approx_ops.layer_row_sums(g).double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("B,C,H,W,k,s,p,d", [(2, 3, 24, 18, 3, 1, 1, 1), (70, 2, 8, 6, 3, 1, 1, 1), (3, 2, 48, 36, 3, 2, 1, 1), (2, 3, 16, 17, 3, 1, 1, 1),
+                                             (2, 2, 16, 22, 5, 1, 2, 1), (5, 3, 8, 2, 1, 1, 0, 1), (3, 2, 16, 1, 3, 1, 1, 1), (2, 2, 48, 50, 3, 3, 0, 1),
+                                             (2, 3, 18, 24, 3, 1, 2, 2), (1, 2, 64, 66, 7, 1, 3, 1)])
+def test_transposed_codes_of_output_rows_that_are_no_multiple_of_four(dev, B, C, H, W, k, s, p, d):
+    test_transposed_codes_of_a_convolution(dev, B, C, H, W, k, s, p, d)
