@@ -25,18 +25,16 @@ __host__ __device__ inline bool weight_prep_split(long s_c, long s_w, int taps) 
 // By block number `block`, CO output channels, one tap of them or all: codes of weight[co, :, :, :] (any strides) written as columns of
 // wmat[K, Cout], K ordered (cin, kh, kw); wsum[co, t] = sum over cin of the codes of tap t.  A thread handles one k of all CO
 // channels, so its reads are independent of each other and its codes leave in one CO-byte store; those of its next k are
-// on their way meanwhile.  Threads follow the weights' own order (channels-last weights have the input channel innermost).
-// The sums are integers (exact in any order; shared-memory atomics are native for integers only), added up inside the warp
-// first where it has one tap.  384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> 4.2 us.
+// on their way meanwhile.  Threads follow the weights' own order (channels-last weights, one tap of them at a time, have the input
+// channel innermost).  The sums are integers (exact in any order; shared-memory atomics are native for integers only), added up
+// inside the warp first where there is one tap.  384 x 1536 linear layer: 44.7 us with one channel per block, byte stores and fp32 atomics -> 4.2 us.
 // Channels-last 3x3 weights of ResNet-18, all layers and with their activations: 280 us with a block per eight channels, 185 us by taps.
 template <int CO>
 __device__ __forceinline__ void weight_prep_columns(const WeightPrep &w, int block, uint32_t *tap_sum) {
     const int groups = (w.Cout + CO - 1) / CO, co0 = block % groups * CO, T = w.kh * w.kw;
     const int t0 = w.split ? block / groups : 0, nt = w.split ? 1 : T;
     const int K = w.Cin * nt, lane = threadIdx.x & 31, threads = blockDim.x;
-    const bool channel_inner = w.s_c < w.s_w;
-    const int inner = channel_inner ? w.Cin : T;
-    const bool one_tap = nt == 1 || (channel_inner && w.Cin % 32 == 0);  // per warp
+    const bool one_tap = nt == 1;
     const Divisor scale = make_divisor(w.quant[2]);
     const float zp = w.quant[3];
     for (int u = threadIdx.x; u < CO * nt; u += threads) tap_sum[u] = 0u;
@@ -44,9 +42,8 @@ __device__ __forceinline__ void weight_prep_columns(const WeightPrep &w, int blo
     int c = 0, t = t0;
     float x[CO];
     auto load = [&](int i) {
-        const int hi = i / inner, lo = i - hi * inner;
-        c = channel_inner ? lo : hi;
-        t = t0 + (channel_inner ? hi : lo);
+        c = one_tap ? i : i / T;
+        t = one_tap ? t0 : i - c * T;
         const int row = t / w.kw, col = t - row * w.kw;
         const float *src = w.weight + co0 * w.s_co + c * w.s_c + row * w.s_h + col * w.s_w;
 #pragma unroll
@@ -74,7 +71,7 @@ __device__ __forceinline__ void weight_prep_columns(const WeightPrep &w, int blo
 #pragma unroll
             for (int e = 0; e < CO; ++e) {
                 const uint32_t sum = __reduce_add_sync(0xffffffffu, q[e]);
-                if (lane == 0) atomicAdd(&tap_sum[e * nt + tap], sum);  // (a warp behind the last k adds 0 to a tap it had before)
+                if (lane == 0) atomicAdd(&tap_sum[e], sum);  // (a warp behind the last k adds 0)
             }
         } else if (i < K) {
 #pragma unroll
