@@ -32,7 +32,7 @@ def rows():
 
 
 def slope_tables(bits, seed, least):
-    """Entries from `least` up to 2040: with a least one of -100 their offset is small enough for the subnormal form."""
+    """Entries from `least` up to 2040, as slopes of products have them."""
     rng = np.random.default_rng(seed)
     q = 1 << bits
     out = []
@@ -73,7 +73,7 @@ def test_long_sums(dev, oracle_c, rows, bits, M, K, N):
 @pytest.mark.parametrize("least", [0, -100, -510, -511])
 @pytest.mark.parametrize("scale", [1.0, 1e-17, 1e17, 1e-19, 1e19, 1e-37, 1e33])
 def test_grad_out_of_any_size(dev, oracle_c, rows, least, scale):
-    """Both sides of the lines between the two forms: -4 min <= max of the table, 2^-60 and 2^60 of grad_out."""
+    """Values near both ends of the fp32 range, and tables that reach below zero by a quarter of their largest entry."""
     bits, M, K, N = 7, 530, 20, 200
     la, lw = slope_tables(bits, 5, least)
     a, w, gc = problem(bits, M, K, N, 3)

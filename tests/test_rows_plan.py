@@ -22,21 +22,23 @@ def test_plan_covers_its_work(tmp_path):
     assert res.returncode == 0, res.stdout
 
 
-@pytest.mark.parametrize("bits,B,Cin,Cout,h,k,stride,rows", [
-    (7, 256, 64, 64, 32, 3, 1, True), (8, 64, 256, 64, 56, 1, 1, True), (8, 256, 256, 512, 8, 3, 2, True), (7, 1, 64, 64, 8, 3, 1, False)])
-def test_image_gradients(lib, bits, B, Cin, Cout, h, k, stride, rows):
-    """One thread per pixel where the caller brings its workspace; a buffer that is too small selects the kernels of before."""
+ROWS, PACKED, BCAST = "slab_grad_rows_kernel", "slab_grad_packed_kernel", "ga_colbcast_kernel"
+
+
+@pytest.mark.parametrize("bits,B,Cin,Cout,h,k,stride,kernel,without", [
+    (7, 256, 64, 64, 32, 3, 1, ROWS, ROWS), (8, 64, 256, 64, 56, 1, 1, ROWS, ROWS), (8, 256, 256, 512, 8, 3, 2, ROWS, None),
+    (7, 1, 64, 64, 8, 3, 1, PACKED, PACKED), (7, 64, 256, 256, 56, 3, 1, ROWS, PACKED), (8, 16, 128, 256, 10, 3, 1, ROWS, BCAST),
+    (7, 2, 256, 1024, 6, 3, 1, PACKED, None)])
+def test_image_gradients(lib, bits, B, Cin, Cout, h, k, stride, kernel, without):
+    """One thread per pixel where the caller brings its workspace; without one the kernels that need none, or a refusal where a
+    buffer has always been asked for (`without` None)."""
     p = lib.p
     conv = (bits, B, Cin, h, h, Cout, k, k, stride, k // 2, 1)
-    names = {}
-    for nbytes in (1 << 40, 0):
-        rc, calls = lib.call("lutgemm_conv2d_backward_ws", p, p, p, p, None, p, p, *conv, None, p if nbytes else None, H.Size(nbytes), None)
-        names[nbytes] = {c[0] for c in calls}
-        assert rc in (H.OK, H.E_SCRATCH)
-    assert ("slab_grad_rows_kernel" in names[1 << 40]) == rows
     need = lib.query("lutgemm_conv2d_backward_ws_scratch_bytes", *conv, H.CODES_GIVEN)
-    rc, calls = lib.call("lutgemm_conv2d_backward_ws", p, p, p, p, None, p, p, *conv, None, p, H.Size(need), None)
-    assert rc == H.OK and {c[0] for c in calls} == names[1 << 40]
+    for nbytes, expected in ((1 << 40, kernel), (need, kernel), (0, without if need else kernel)):
+        rc, calls = lib.call("lutgemm_conv2d_backward_ws", p, p, p, p, None, p, p, *conv, None, p if nbytes else None, H.Size(nbytes), None)
+        assert rc == (H.OK if expected else H.E_SCRATCH)
+        assert {c[0] for c in calls} & {ROWS, PACKED, BCAST} == ({expected} if expected else set())
 
 
 def test_operator_gradients_fall_back_where_the_buffer_is_small(lib):
