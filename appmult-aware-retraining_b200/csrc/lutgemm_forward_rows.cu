@@ -14,6 +14,7 @@
 // 4 bits 6.48 -> 4.48 (620); 262144 x 576 x 64 at 7 bits 1.09 -> 0.85 ms.
 // Slab buffers change hands through one mbarrier per unit: see lutgemm_slab_rows.cu.  The activation codes come from
 // the transposed copy at[k][m], 16 bits (both rows) per k.
+// 512 threads leave a thread 128 registers: 4 and 6 bits spill 48 and 52 bytes, 7 and 8 bits none.
 // Tiles and cut K as in lutgemm_slab.cu: whole tiles where they fill the persistent grid's waves, otherwise every CTA takes an
 // equal contiguous share of all (tile, four k) units, and the parts of a tile that is cut are combined with integer atomics,
 // which are exact in any order.  The sums leave through shared memory, so that rows are stored as whole 128-byte lines, with the layer's

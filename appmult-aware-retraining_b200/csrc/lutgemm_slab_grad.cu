@@ -24,6 +24,7 @@
 // exactly, and one packed multiply-add (fma.rn.f32x2) consumes them - 10 instructions per 128 look-ups of a warp
 // against 8 with an fp32 slab, but 512 + build instead of 1024 + build wavefronts per 32768 look-ups.  Products and
 // sums are the same fp32 operations as with an fp32 slab.
+// 576-row tiles keep 72 registers of grad_out values and spill 4 to 16 bytes.
 // With one barrier per unit and the staggered slab build of lutgemm_rows.cuh, against two barriers per unit and padded slab rows
 // (grad_w, grad_a): 4096^3 at 7 bits 10.50, 11.12 -> 9.99, 10.09 ms, 6 bits 9.89, 10.71 -> 9.62, 9.63, 8 bits 15.19, 15.18 -> 14.15, 14.95;
 // 262144 x 576 x 64 at 7 bits, grad_w 1.51 -> 1.46 ms.

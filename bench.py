@@ -697,7 +697,7 @@ def run_layers(args, local_rank):
 
 # DRAM traffic of the three main kernels: read at run time from the committed summary of the ncu capture of this
 # workload (a profiler cannot run inside a timed run, so the figure is a property of the kernel at that size)
-NCU_TRAFFIC_PROFILE = {"config": (8, 4096, 4096), "file": os.path.join("profiles", "slab_kernels_b8_4096.md")}
+NCU_TRAFFIC_PROFILE = {"config": (8, 4096, 4096), "file": os.path.join("profiles", "row_kernels_b8_4096.md")}
 
 
 def ncu_dram_traffic(kernel, config):
