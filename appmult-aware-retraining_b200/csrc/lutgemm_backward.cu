@@ -636,9 +636,10 @@ __global__ void __launch_bounds__(1024) transpose_codes_kernel(const uint8_t *__
 // with a test of the borders for each: 256 planes of 64 x 32 x 32, 3x3, 116 -> 51 us.  Small planes share a CTA, images after
 // one another, so that stores stay longer than a sector.  STRIDE 0: any stride, by bytes; -1: also output rows that are no multiple of
 // 4, whose outputs pass from row to row one by one (256 x 64 x 16 x 18, 3x3: 38 us, 75 with a thread per 16 outputs from global memory;
-// 64 x 64 x 32 x 34, 5x5: 55, 196).
+// 64 x 64 x 32 x 34, 5x5: 55, 196).  Windows one row high leave out the rows between (64 x 256 x 56 x 56, 1x1, stride 2: 82 -> 57 us).
 struct PlaneStage {
     int planes, rows, pitch;  // planes per CTA; rows and bytes per row of a staged plane
+    int row_step;             // image rows per staged row: the stride where windows are one row high, otherwise 1
     unsigned groups;          // CTAs per channel
     // ceil(2^32 / d) for d = words per staged plane, words per staged row, chunks of 16 outputs per CTA and per plane, four
     // outputs per row (0 where d is 1): n / d is the high half of n * it, for n * d < 2^32
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
 #pragma unroll 4
     for (int i = threadIdx.x; i < nb * words; i += 256) {
         const int p = quotient(i, st.by_plane), r = i - p * words, row = quotient(r, st.by_row);
-        const int h = row - g.pad, w0 = (r - row * rw) * 4 - g.pad;
+        const int h = row * st.row_step - g.pad, w0 = (r - row * rw) * 4 - g.pad;
         uint32_t v = 0u;
         if ((unsigned)h < (unsigned)g.H) {
             const uint8_t *src = x + ((size_t)(b0 + p) * g.C + c) * HW + h * g.W;
@@ -677,6 +678,7 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
         reinterpret_cast<uint32_t *>(plane)[i] = v & mask4;
     }
     __syncthreads();
+    const int out_step = g.kh == 1 ? 1 : g.stride;  // staged rows between two output rows
     // a thread takes 16 outputs of one kernel row and goes over its taps
     const int chunks = L / 16, per_row = nb * chunks;
     for (int q = threadIdx.x; q < g.kh * per_row; q += 256) {
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(256) transpose_codes_plane_kernel(const uint8_
         int o[16 / STEP];
 #pragma unroll
         for (int e = 0; e < 16 / STEP; ++e) {
-            o[e] = p * bytes + (i * g.dil + oh * g.stride) * st.pitch + ow * g.stride;
+            o[e] = p * bytes + (i * g.dil + oh * out_step) * st.pitch + ow * g.stride;
             ow += STEP;
             if (ow == g.Wo) { ow = 0; ++oh; }
         }
@@ -775,7 +777,8 @@ int transpose_codes(const uint8_t *a, uint8_t *at, int M, int K, int pitch, cons
             return launch_status();
         }
         PlaneStage st{};
-        st.rows = (conv.Ho - 1) * conv.stride + (conv.kh - 1) * conv.dil + 1;
+        st.row_step = conv.kh == 1 ? conv.stride : 1;
+        st.rows = conv.kh == 1 ? conv.Ho : (conv.Ho - 1) * conv.stride + (conv.kh - 1) * conv.dil + 1;
         // (the words behind the last outputs of a row are read too)
         st.pitch = ((conv.Wo - 1) * conv.stride + (conv.kw - 1) * conv.dil + 1 + 8 + 3) & ~3;
         const long bytes = (long)st.rows * st.pitch;

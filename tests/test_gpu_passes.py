@@ -127,3 +127,9 @@ def test_row_sums(dev, M, N):
                                              (2, 3, 18, 24, 3, 1, 2, 2), (1, 2, 64, 66, 7, 1, 3, 1)])
 def test_transposed_codes_of_output_rows_that_are_no_multiple_of_four(dev, B, C, H, W, k, s, p, d):
     test_transposed_codes_of_a_convolution(dev, B, C, H, W, k, s, p, d)
+
+
+@pytest.mark.parametrize("B,C,H,W,k,s,p,d", [(2, 2, 48, 48, 1, 3, 0, 1), (2, 3, 47, 35, 1, 2, 0, 1), (3, 2, 14, 14, 1, 2, 1, 1), (9, 3, 8, 8, 1, 2, 0, 1),
+                                             (1, 2, 64, 64, 1, 4, 0, 1)])
+def test_transposed_codes_of_windows_one_row_high(dev, B, C, H, W, k, s, p, d):
+    test_transposed_codes_of_a_convolution(dev, B, C, H, W, k, s, p, d)
